@@ -4,6 +4,8 @@
 // (embed rows, rmsnorm(+residual)(+rope), split+rope+paged-append, greedy argmax).
 #include "kernels.h"
 
+#include <atomic>
+
 namespace ak {
 
 // ============================================================================ embedding
@@ -191,6 +193,148 @@ __global__ void rmsnorm_rows_kernel(float* __restrict__ x, const float* __restri
     }
 }
 
+// Large launches (a prefill's rows): a few CTAs per SM stay for the whole launch and every warp walks over rows, the next
+// row's loads in flight while the current one is finished. HBM bound (32768 x 768 f32 -> bf16: 151 MB). What a warp needs
+// for every row stays in registers: its norm weights and, with RoPE, the frequency of the one or two angles it evaluates
+// (the one-row-per-warp kernel spends a powf per angle and CTA of four rows, and starts each row with an empty pipeline:
+// with RoPE 33.0 us at that size, this one 24.6 us). NV = float4 per lane and row (size <= 128 NV); rows of more than 1024
+// elements are not prefetched (64 registers a row), there the warps of an SM cover the latency for each other.
+// Same arithmetic, in the same order, as rmsnorm_rows_kernel.
+template <typename OT, bool HAS_RES, bool ROPE, int NV>
+__global__ void __launch_bounds__(128)
+rmsnorm_stream_kernel(float* __restrict__ x, const float* __restrict__ residual, const float* __restrict__ w, OT* __restrict__ y,
+                      const int32_t* __restrict__ positions, uint32_t rows, uint32_t size, float eps, uint32_t head_dim, uint32_t rows_per_warp) {
+    constexpr bool AHEAD = NV <= 8;
+    const uint32_t lane = threadIdx.x & 31, nv = size >> 2;
+    // rows_per_warp == 0: a grid of resident CTAs strides over the rows; else CTA b takes 4 * rows_per_warp consecutive rows
+    const uint32_t step = rows_per_warp ? 4 : gridDim.x * 4;
+    uint32_t row = blockIdx.x * 4 * (rows_per_warp ? rows_per_warp : 1) + (threadIdx.x >> 5);
+    const uint32_t row_end = rows_per_warp ? min(rows, (blockIdx.x + 1) * 4 * rows_per_warp) : rows;
+    float4 g[AHEAD ? NV : 1];
+    if (AHEAD) {
+#pragma unroll
+        for (int c = 0; c < NV; c++) {
+            const uint32_t i = lane + 32u * c;
+            g[AHEAD ? c : 0] = i < nv ? reinterpret_cast<const float4*>(w)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    // head_dim divides 128 (launcher), so all of a lane's float4 sit at the same offset d0 of their heads. head_dim <= 64:
+    // lane j evaluates angle j mod (head_dim / 2) and lanes trade; head_dim = 128: every lane evaluates its own two.
+    const uint32_t half = head_dim >> 1, d0 = ROPE ? (lane * 4) % head_dim : 0;
+    float f0 = 0.0f, f1 = 0.0f;
+    if (ROPE) {
+        f0 = 1.0f / powf(10000.0f, (float)(head_dim <= 64 ? 2 * (lane & (half - 1)) : d0) / (float)head_dim);
+        if (head_dim > 64) f1 = 1.0f / powf(10000.0f, (float)(d0 + 2) / (float)head_dim);
+    }
+    pdl_wait();
+    pdl_trigger();
+    float4 v[NV], nx[AHEAD ? NV : 1], nr[AHEAD && HAS_RES ? NV : 1];
+    int32_t pos = 0, npos = 0;
+    auto request = [&](uint32_t r) {   // the row's loads into the "next" registers
+        const float4* xr = reinterpret_cast<const float4*>(x + (size_t)r * size);
+        const float4* rr = HAS_RES ? reinterpret_cast<const float4*>(residual + (size_t)r * size) : nullptr;
+#pragma unroll
+        for (int c = 0; c < NV; c++) {
+            const uint32_t i = lane + 32u * c;
+            if (i < nv) {
+                nx[AHEAD ? c : 0] = xr[i];
+                if (HAS_RES) nr[AHEAD && HAS_RES ? c : 0] = rr[i];
+            }
+        }
+        if (ROPE) npos = positions[r];
+    };
+    if (AHEAD && row < row_end) request(row);
+    for (; row < row_end; row += step) {
+        float4* xr = reinterpret_cast<float4*>(x + (size_t)row * size);
+        float ss = 0.0f;
+        if (!AHEAD) {
+#pragma unroll
+            for (int c = 0; c < NV; c++) {
+                const uint32_t i = lane + 32u * c;
+                if (i < nv) v[c] = xr[i];
+            }
+            if (ROPE) npos = positions[row];
+        }
+#pragma unroll
+        for (int c = 0; c < NV; c++) {
+            const uint32_t i = lane + 32u * c;
+            if (i < nv) {
+                if (AHEAD) v[c] = nx[AHEAD ? c : 0];
+                if (HAS_RES) {
+                    const float4 r = AHEAD ? nr[AHEAD && HAS_RES ? c : 0] : reinterpret_cast<const float4*>(residual + (size_t)row * size)[i];
+                    v[c].x += r.x; v[c].y += r.y; v[c].z += r.z; v[c].w += r.w;
+                    xr[i] = v[c];
+                }
+                ss += v[c].x * v[c].x + v[c].y * v[c].y + v[c].z * v[c].z + v[c].w * v[c].w;
+            }
+        }
+        pos = npos;
+        if (AHEAD && row + step < row_end) request(row + step);
+        ss = warp_sum(ss);
+        const float rs = 1.0f / sqrtf((ss / (float)size) + eps);
+        float s0 = 0.f, c0 = 1.f, s1 = 0.f, c1 = 1.f;
+        if (ROPE) {
+            sincosf((float)pos * f0, &s0, &c0);
+            if (head_dim <= 64) {
+                const float sn = s0, cs = c0;
+                const uint32_t i0 = d0 >> 1;
+                s0 = __shfl_sync(0xffffffffu, sn, i0); c0 = __shfl_sync(0xffffffffu, cs, i0);
+                s1 = __shfl_sync(0xffffffffu, sn, i0 + 1); c1 = __shfl_sync(0xffffffffu, cs, i0 + 1);
+            } else {
+                sincosf((float)pos * f1, &s1, &c1);
+            }
+        }
+        OT* yr = y + (size_t)row * size;
+#pragma unroll
+        for (int c = 0; c < NV; c++) {
+            const uint32_t i = lane + 32u * c;
+            if (i >= nv) continue;
+            const float4 gg = AHEAD ? g[AHEAD ? c : 0] : reinterpret_cast<const float4*>(w)[i];
+            float o0 = v[c].x * rs * gg.x, o1 = v[c].y * rs * gg.y, o2 = v[c].z * rs * gg.z, o3 = v[c].w * rs * gg.w;
+            if (ROPE) {
+                const float a = o0 * c0 - o1 * s0, b = o0 * s0 + o1 * c0, e = o2 * c1 - o3 * s1, d = o2 * s1 + o3 * c1;
+                o0 = a; o1 = b; o2 = e; o3 = d;
+            }
+            if constexpr (sizeof(OT) == 4) {
+                reinterpret_cast<float4*>(yr)[i] = make_float4(o0, o1, o2, o3);
+            } else {
+                bf162 p0 = __floats2bfloat162_rn(o0, o1), p1 = __floats2bfloat162_rn(o2, o3);
+                reinterpret_cast<uint2*>(yr)[i] = make_uint2(*reinterpret_cast<uint32_t*>(&p0), *reinterpret_cast<uint32_t*>(&p1));
+            }
+        }
+    }
+}
+
+template <typename OT, bool HAS_RES, bool ROPE, int NV>
+static int rmsnorm_stream_launch(cudaStream_t st, float* x, const float* residual, const float* w, OT* y, const int32_t* positions, uint32_t rows,
+                                 uint32_t size, float eps, uint32_t head_dim) {
+    // With a residual two rows per warp and as many CTAs as that takes: the 14 bytes per element (8 read, 4 written back, 2
+    // out) want rows in flight near each other in memory (32768 x 768 with RoPE: 53.5 us, against 58.2 us for the resident
+    // grid, whose warps drift apart). Without one the resident grid is the faster (24.6 us against 27.2 us).
+    uint32_t rpw = HAS_RES ? 2 : 0, ctas = cdiv(rows, 8);
+    if (!HAS_RES) {
+        static std::atomic<int> per_sm{0};   // resident CTAs of this instantiation
+        int occ = per_sm.load(std::memory_order_relaxed);
+        if (!occ) {
+            AK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rmsnorm_stream_kernel<OT, HAS_RES, ROPE, NV>, 128, 0));
+            per_sm.store(occ, std::memory_order_relaxed);
+        }
+        ctas = cdiv(rows, 4);
+        if (ctas > B200_SMS * (uint32_t)occ) ctas = B200_SMS * (uint32_t)occ;
+    }
+    return launch_k(rmsnorm_stream_kernel<OT, HAS_RES, ROPE, NV>, dim3(ctas), dim3(128), 0, st, NO_CLUSTER, x, residual, w, y, positions, rows, size,
+                    eps, head_dim, rpw);
+}
+
+template <typename OT, bool HAS_RES, bool ROPE>
+static int rmsnorm_stream_nv(cudaStream_t st, float* x, const float* residual, const float* w, OT* y, const int32_t* positions, uint32_t rows,
+                             uint32_t size, float eps, uint32_t head_dim) {
+    if (size <= 384) return rmsnorm_stream_launch<OT, HAS_RES, ROPE, 3>(st, x, residual, w, y, positions, rows, size, eps, head_dim);
+    if (size <= 768) return rmsnorm_stream_launch<OT, HAS_RES, ROPE, 6>(st, x, residual, w, y, positions, rows, size, eps, head_dim);
+    if (size <= 1024) return rmsnorm_stream_launch<OT, HAS_RES, ROPE, 8>(st, x, residual, w, y, positions, rows, size, eps, head_dim);
+    return rmsnorm_stream_launch<OT, HAS_RES, ROPE, 16>(st, x, residual, w, y, positions, rows, size, eps, head_dim);
+}
+
 template <typename OT>
 static int rmsnorm_dispatch(cudaStream_t st, float* x, const float* residual, const float* w, OT* y,
                             const int32_t* row_map, const int32_t* positions, uint32_t rows, uint32_t size,
@@ -198,6 +342,15 @@ static int rmsnorm_dispatch(cudaStream_t st, float* x, const float* residual, co
     const int WARPS = 4;   // 8-warp CTAs (the RoPE frequency table shared by twice the rows) measured slower: 0.64 against 0.69 of peak
     dim3 grid(cdiv(rows, WARPS)), block(WARPS * 32);
     const bool rope = head_dim != 0, early = rows <= 1024;
+    // Streaming form: rows enough for every warp of the machine (below, one row per warp is as good) and either RoPE or
+    // short rows, where the per-CTA setup of the other kernel shows; with long rows, a residual and no RoPE the two tie,
+    // and a plain long-row norm is at 0.97 of the HBM peak without it.
+    if (rows > 2048 && !row_map && (size & 3u) == 0 && size <= 2048 && (rope ? 128u % head_dim == 0 : size <= 384)) {
+        if (residual && rope) return rmsnorm_stream_nv<OT, true, true>(st, x, residual, w, y, positions, rows, size, eps, head_dim);
+        if (rope) return rmsnorm_stream_nv<OT, false, true>(st, x, residual, w, y, positions, rows, size, eps, head_dim);
+        if (residual) return rmsnorm_stream_launch<OT, true, false, 3>(st, x, residual, w, y, positions, rows, size, eps, head_dim);
+        return rmsnorm_stream_launch<OT, false, false, 3>(st, x, residual, w, y, positions, rows, size, eps, head_dim);
+    }
 #define AK_NORM_LAUNCH(RES, ROPE_, EARLY)                                                                                          \
     AK_TRY(launch_k(rmsnorm_rows_kernel<OT, RES, ROPE_, EARLY>, dim3(grid), dim3(block), 0, st, NO_CLUSTER, x, residual, w, y, row_map, \
                     positions, rows, size, eps, head_dim))

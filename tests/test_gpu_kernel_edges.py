@@ -1,0 +1,62 @@
+"""GPU: the kernels at the edges of their dispatch rules and tiles (remainders, the smallest and largest sizes of a variant),
+against plain float64 / float32 references of the same operation."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def host(t):
+    return t.float().cpu().numpy()
+
+
+# the streaming RMSNorm (more than 2048 rows): every register width, a row count that leaves a short last CTA
+@pytest.mark.parametrize("rows,size,hd,with_res", [(2049, 320, 64, True), (2053, 320, 0, False), (2500, 384, 0, True), (2051, 768, 64, False),
+                                                   (4097, 1024, 128, True), (2050, 2048, 128, False), (2049, 2048, 32, True), (9001, 196, 4, False)])
+@pytest.mark.parametrize("out_dtype", [0, 1])
+def test_rmsnorm_stream(ak, torch_cuda, rows, size, hd, with_res, out_dtype):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(rows + size)
+    x = torch.randn(rows, size, device="cuda", generator=g)
+    r = torch.randn(rows, size, device="cuda", generator=g) if with_res else None
+    w = 1.0 + 0.1 * torch.randn(size, device="cuda", generator=g)
+    pos = torch.randint(0, 4096, (rows,), device="cuda", generator=g, dtype=torch.int32)
+    h = x + r if with_res else x.clone()
+    want = (h.double() * torch.rsqrt(h.double().square().mean(-1, keepdim=True) + 1e-5) * w.double())
+    if hd:
+        # the angle is formed in f32 (position times a f32 frequency), as the reference forms it
+        freq = 1.0 / torch.pow(torch.tensor(10000.0), torch.arange(0, hd, 2, dtype=torch.float32) / hd).cuda()
+        ang = (pos.float()[:, None] * freq[None, :]).double().repeat(1, size // hd)
+        a, b = want[:, 0::2].clone(), want[:, 1::2].clone()
+        want[:, 0::2], want[:, 1::2] = a * ang.cos() - b * ang.sin(), a * ang.sin() + b * ang.cos()
+    y = torch.full((rows, size), float("nan"), device="cuda", dtype=torch.float32 if out_dtype == 0 else torch.bfloat16)
+    ak.ops.rmsnorm_rope_residual(x, r, w, y, pos if hd else None, rows, size, 1e-5, hd, out_dtype)
+    torch.cuda.synchronize()
+    # f32: a frequency one ulp off turns position 4095 by 4095 * 2^-24 ~ 2.5e-4 rad on values up to ~5; bf16: half an ulp of 2^-8
+    tol = 2e-3 if out_dtype == 0 else 2e-3 + 5.0 * 2.0 ** -8
+    assert float((y.double() - want).abs().max()) < tol
+    if with_res:
+        assert torch.equal(x, h)
+
+
+# the CTA-pair GEMM's two output paths: TMA pieces (tails in m and n, a padded pitch) and direct stores (pitch no multiple of 16 bytes)
+@pytest.mark.parametrize("epi", [0, 1, 2, 3])
+@pytest.mark.parametrize("m,n,k,ldc", [(1024, 256, 64, 256), (1025, 300, 136, 304), (1311, 391, 72, 392), (1311, 391, 72, 391), (2049, 257, 320, 259),
+                                       (1281, 1000, 8, 1000)])
+def test_gemm_pair_outputs(ak, torch_cuda, epi, m, n, k, ldc):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    wt = (0.25 * torch.randn(n, k, device="cuda", generator=g)).bfloat16()
+    cdt = torch.float32 if epi <= 1 else torch.bfloat16
+    c = torch.full((m, ldc), 3.0, device="cuda", dtype=cdt)
+    ak.ops.gemm_bf16(a, wt, c, m, n, k, epi, ldc=ldc)
+    torch.cuda.synchronize()
+    acc = a.double() @ wt.double().T
+    want = {0: acc, 1: acc + 3.0, 2: acc, 3: acc / (1.0 + (-acc).exp())}[epi]
+    scale = float(acc.abs().max())
+    # f32: k sums in f32; bf16: half an ulp of the largest value
+    tol = 2.0 ** -22 * k * max(1.0, scale) + 1e-6 if epi <= 1 else 2.0 ** -8 * max(1.0, scale)
+    assert float((c[:, :n].double() - want).abs().max()) < tol
+    assert bool((c[:, n:] == 3.0).all())
+    ak.check(ak.lib().ak_check_device_status(None))
