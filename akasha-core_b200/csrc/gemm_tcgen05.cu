@@ -62,6 +62,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
         : "r"(taddr)
         : "memory");
 }
+// 32 lanes x 32 consecutive 32-bit columns.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
+          "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]),
+          "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor, K-major operand, 128-byte swizzle, rows of 128 bytes:
@@ -125,6 +137,11 @@ struct GemmEpi {
 
 enum { EPI_ARGMAX = 4, EPI_STORE_F32_ARGMAX = 5 };
 
+// x * sigmoid(x): ex2 + rcp on the special-function unit (both within 2 ulp of f32, far below the bf16 rounding that
+// follows). The IEEE division costs ~20 instructions per element and was what a large SiLU launch spent its time on:
+// 32768 x 3072 x 768 took 423 us with it, against 144 us without the activation.
+__device__ __forceinline__ float epi_silu(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
+
 // Store W consecutive accumulator columns of one row with the epilogue op. gcol % 4 == 0.
 template <int EPI, int W>
 __device__ __forceinline__ void epi_store(const GemmEpi& ep, uint32_t row, uint32_t gcol, const float* v, uint32_t n) {
@@ -154,7 +171,7 @@ __device__ __forceinline__ void epi_store(const GemmEpi& ep, uint32_t row, uint3
         bf16* dst = reinterpret_cast<bf16*>(ep.c) + (size_t)row * ep.ldc + gcol;
         float t[W];
 #pragma unroll
-        for (int j = 0; j < W; j++) t[j] = (EPI == AK_EPI_SILU_BF16) ? v[j] / (1.0f + __expf(-v[j])) : v[j];
+        for (int j = 0; j < W; j++) t[j] = (EPI == AK_EPI_SILU_BF16) ? epi_silu(v[j]) : v[j];
         const bool vec = (gcol + W <= n) && ((ep.ldc & 3u) == 0);
         if (W % 8 == 0 && vec && (ep.ldc & 7u) == 0 && (gcol & 7u) == 0) {
             // 16-byte stores: half as many L2 write requests per 32-byte sector as 8-byte ones
@@ -232,8 +249,8 @@ __device__ __forceinline__ void epi_store16(const GemmEpi& ep, uint32_t row, boo
         uint32_t pk[8];
 #pragma unroll
         for (int e = 0; e < 8; e++) {
-            const float t0 = (EPI == AK_EPI_SILU_BF16) ? v[2 * e] / (1.0f + __expf(-v[2 * e])) : v[2 * e];
-            const float t1 = (EPI == AK_EPI_SILU_BF16) ? v[2 * e + 1] / (1.0f + __expf(-v[2 * e + 1])) : v[2 * e + 1];
+            const float t0 = (EPI == AK_EPI_SILU_BF16) ? epi_silu(v[2 * e]) : v[2 * e];
+            const float t1 = (EPI == AK_EPI_SILU_BF16) ? epi_silu(v[2 * e + 1]) : v[2 * e + 1];
             bf162 a = __floats2bfloat162_rn(t0, t1);
             pk[e] = *reinterpret_cast<uint32_t*>(&a);
         }
@@ -525,7 +542,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 //   empty[s]     one per CTA; after the MMAs of a K block the leader commits to its own and to the peer's
 //                (two plain tcgen05.commit, the peer's addressed through the cluster window);
 //   acc_full[b]  one per CTA, committed by the leader after a tile's last MMA;
-//   acc_empty[b] leader's barrier, 8 arrivals: one per epilogue warp of both CTAs (the peer's arrive remotely).
+//   acc_empty[b] leader's barrier, 16 arrivals: one per epilogue warp of both CTAs (the peer's arrive remotely).
 // TMEM is allocated and freed with the .cta_group::2 forms by warp 1 of both CTAs, with cluster barriers after the
 // allocation and before the release.
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -574,12 +591,16 @@ template <int BN> struct PairCfg {
     static constexpr int B_BYTES = (BN / 2) * GB_K * 2;      // this CTA's half of the weight tile
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int TMEM_COLS = 512;                    // two accumulator buffers of kseg * BN columns
+    static constexpr int OUT_WARP_BYTES = 32 * 128;          // an epilogue warp's output staging: one piece of 32 rows x 128 B
 };
+constexpr int PAIR_EPI_WARPS = 8;
+constexpr int PAIR_THREADS = 64 + PAIR_EPI_WARPS * 32;
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(G_THREADS, 1)
-gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmEpi ep,
-                      uint32_t m, uint32_t n, uint32_t k, uint32_t stages, uint32_t kseg, uint32_t tiles_n, uint32_t tiles_total) {
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+                      const GemmEpi ep, uint32_t m, uint32_t n, uint32_t k, uint32_t stages, uint32_t kseg, uint32_t tiles_n,
+                      uint32_t tiles_total, uint32_t tma_out) {
     using C = PairCfg<BN>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full_bar[G_MAX_STAGES], empty_bar[G_MAX_STAGES], acc_full[2], acc_empty[2];
@@ -598,7 +619,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < stages; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        for (uint32_t b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+        for (uint32_t b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * PAIR_EPI_WARPS); }
         fail_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&tmA);
@@ -682,56 +703,88 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             }
         }
     } else {
-        // ---------------- epilogue warps 2..5 of both CTAs: thread <-> accumulator row of THIS CTA's TMEM
-        const uint32_t quad = warp & 3u;
+        // ---------------- epilogue warps of both CTAs: thread <-> accumulator row of THIS CTA's TMEM, 8 warps: the two
+        // warps of a TMEM lane quadrant take one half of the columns each. `tma_out`: 128-byte wide pieces (64 bf16 or
+        // 32 f32 columns of 32 rows) go through a swizzled staging buffer and leave as TMA stores (or TMA adds into f32):
+        // whole lines, no address arithmetic, tails clipped by the tensor map. Otherwise (row pitch of C not a multiple of
+        // 16 bytes) registers are stored directly.
+        const uint32_t quad = warp & 3u, half = (warp - 2) >> 2;
+        constexpr bool OUT_BF16 = (EPI == AK_EPI_STORE_BF16 || EPI == AK_EPI_SILU_BF16);
+        constexpr uint32_t CW = OUT_BF16 ? 64 : 32;   // columns of a staged piece
+        uint8_t* const stage_sm = smem + (size_t)stages * C::STAGE_BYTES + (size_t)(warp - 2) * C::OUT_WARP_BYTES;
         pdl_wait();
         uint32_t tc = 0;
         for (uint32_t t = pair; t < tiles_total; t += n_pairs, tc++) {
             const uint32_t buf = n_bufs == 2 ? (tc & 1u) : 0u, acc_ph = (n_bufs == 2 ? (tc >> 1) : tc) & 1u;
-            const uint32_t row = ((t / tiles_n) * 2 + rank) * GB_M + quad * 32 + lane;
-            const uint32_t n0 = (t % tiles_n) * BN;
-            bool got = num_kb == 0 || mbar_wait(&acc_full[buf], acc_ph);
+            const uint32_t row0 = ((t / tiles_n) * 2 + rank) * GB_M + quad * 32, row = row0 + lane;
+            const uint32_t n0 = (t % tiles_n) * BN + half * (BN / 2);
+            bool got = mbar_wait(&acc_full[buf], acc_ph);
             if (!got && lane == 0) atomicExch(&fail_flag, 3u);
             got = __all_sync(0xffffffffu, got);
             if (!got) break;
             tc_fence_after();
-            float best = -INFINITY;
-            uint32_t best_i = 0xffffffffu;
+            const uint32_t acc0 = tmem_base + ((quad * 32u) << 16) + buf * buf_cols + half * (BN / 2);
 #pragma unroll 1
-            for (uint32_t c0 = 0; c0 < (uint32_t)BN; c0 += 16) {
-                uint32_t r[16];
-                float v[16];
-                if (num_kb > 0) {
-                    tmem_ld16(tmem_base + ((quad * 32u) << 16) + buf * buf_cols + c0, r);
+            for (uint32_t c0 = 0; c0 < (uint32_t)BN / 2; c0 += 32) {
+                uint32_t r[32];
+                tmem_ld32(acc0 + c0, r);
+                tmem_ld_wait();
+                for (uint32_t seg = 1; seg < kseg; seg++) {
+                    uint32_t r2[32];
+                    tmem_ld32(acc0 + seg * BN + c0, r2);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
-                    for (uint32_t seg = 1; seg < kseg; seg++) {
-                        tmem_ld16(tmem_base + ((quad * 32u) << 16) + buf * buf_cols + seg * BN + c0, r);
-                        tmem_ld_wait();
+                    for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+                }
+                if (c0 + 32 == (uint32_t)BN / 2) {   // this warp has read its part of the buffer: the leader's MMA thread may reuse it
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
+                }
+                const uint32_t col = n0 + (OUT_BF16 ? (c0 & ~32u) : c0);   // first column of the staged piece
+                // a store is clipped at n in whole 16-byte units only: a ragged last piece is stored from registers
+                if (!tma_out || (col + CW > n && (n * (OUT_BF16 ? 2u : 4u)) % 16u != 0)) {
 #pragma unroll
-                        for (int j = 0; j < 16; j++) v[j] += __uint_as_float(r[j]);
+                    for (int j = 0; j < 32; j += 16) epi_store16<EPI>(ep, row, row < m, n0 + c0 + j, reinterpret_cast<const float*>(r) + j, n, lane);
+                    continue;
+                }
+                const bool first_part = !OUT_BF16 || (c0 & 32u) == 0;
+                if (first_part) {   // the previous piece has been read out of the buffer
+                    if (lane == 0) tma_store_wait_read<0>();
+                    __syncwarp();
+                }
+                uint8_t* const srow = stage_sm + lane * 128;
+                if (OUT_BF16) {
+#pragma unroll
+                    for (int q4 = 0; q4 < 4; q4++) {
+                        uint32_t pk[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const float t0 = __uint_as_float(r[8 * q4 + 2 * e]), t1 = __uint_as_float(r[8 * q4 + 2 * e + 1]);
+                            const bf162 v = (EPI == AK_EPI_SILU_BF16) ? __floats2bfloat162_rn(epi_silu(t0), epi_silu(t1)) : __floats2bfloat162_rn(t0, t1);
+                            pk[e] = *reinterpret_cast<const uint32_t*>(&v);
+                        }
+                        const uint32_t ch = (c0 & 32u) / 8 + q4;
+                        *reinterpret_cast<uint4*>(srow + ((ch ^ (lane & 7u)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                     }
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 16; j++) v[j] = 0.0f;
+                    for (uint32_t ch = 0; ch < 8; ch++)
+                        *reinterpret_cast<uint4*>(srow + ((ch ^ (lane & 7u)) << 4)) = make_uint4(r[4 * ch], r[4 * ch + 1], r[4 * ch + 2], r[4 * ch + 3]);
                 }
-                if (EPI != EPI_ARGMAX) epi_store16<EPI>(ep, row, row < m, n0 + c0, v, n, lane);
-                if (row < m && (EPI == EPI_ARGMAX || EPI == EPI_STORE_F32_ARGMAX)) {
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (n0 + c0 + j < n && v[j] > best) { best = v[j]; best_i = n0 + c0 + j; }
+                if (OUT_BF16 && first_part) continue;
+                tma_store_fence();
+                __syncwarp();
+                if (lane == 0) {
+                    if (row0 < m && col < n) {
+                        if (EPI == AK_EPI_ADD_F32) tma_reduce_add_2d(&tmC, stage_sm, (int32_t)col, (int32_t)row0);
+                        else tma_store_2d(&tmC, stage_sm, (int32_t)col, (int32_t)row0);
+                    }
+                    tma_store_commit();
                 }
             }
-            if ((EPI == EPI_ARGMAX || EPI == EPI_STORE_F32_ARGMAX) && row < m) {
-                ep.amax_val[(size_t)row * ep.amax_ld + (t % tiles_n)] = best;
-                ep.amax_idx[(size_t)row * ep.amax_ld + (t % tiles_n)] = best_i;
-            }
-            // this warp has read its part of the buffer: let the leader's MMA thread reuse it
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
         }
+        if (tma_out && lane == 0) tma_store_wait<0>();
     }
     // ---------------- common exit: nobody frees TMEM or leaves while the pair may still use this CTA's memory
     tc_fence_before();
@@ -753,6 +806,7 @@ struct GemmPlan {
 
 static constexpr uint32_t SMEM_TWO_PER_SM = 112 * 1024;   // two CTAs fit one SM below this
 static constexpr uint32_t SMEM_ONE_PER_SM = 220 * 1024;
+static constexpr uint32_t SMEM_PAIR = 226 * 1024;         // the pair kernel: all a CTA may have but its few hundred static bytes
 static constexpr uint32_t SMEM_THREE_PER_SM = 74 * 1024;  // three CTAs fit one SM below this (228 KB, 1 KB reserved and ~0.25 KB static per CTA)
 
 // Rows of the activation TMA box: a decode batch fills only part of the 128-row MMA tile, and rows the
@@ -955,26 +1009,32 @@ static int launch_planned(cudaStream_t st, const void* a, const void* wt, const 
 template <int BN, int EPI>
 static int launch_pair_cfg(cudaStream_t st, const void* a, const void* wt, const GemmEpi& ep, uint32_t m, uint32_t n, uint32_t k, uint32_t kseg) {
     using C = PairCfg<BN>;
-    uint32_t stages = (SMEM_ONE_PER_SM - 1024) / C::STAGE_BYTES;
+    constexpr uint32_t OUT_BYTES = PAIR_EPI_WARPS * C::OUT_WARP_BYTES;
+    uint32_t stages = (SMEM_PAIR - 1024 - OUT_BYTES) / C::STAGE_BYTES;
     if (stages > G_MAX_STAGES) stages = G_MAX_STAGES;
-    const size_t smem = (size_t)stages * C::STAGE_BYTES + 1024;
+    const size_t smem = (size_t)stages * C::STAGE_BYTES + OUT_BYTES + 1024;
     {
         static bool attr_set[64] = {};
         int dev = 0;
         AK_CUDA(cudaGetDevice(&dev));
         std::lock_guard<std::mutex> lock(device_cache_mutex());
         if (!attr_set[dev & 63]) {
-            AK_CUDA(cudaFuncSetAttribute(gemm_bf16_pair_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_ONE_PER_SM));
+            AK_CUDA(cudaFuncSetAttribute(gemm_bf16_pair_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_PAIR));
             attr_set[dev & 63] = true;
         }
     }
     CUtensorMap tmA, tmB;
     AK_TRY(make_tmap_2d(&tmA, a, 2, k, m, (uint64_t)k * 2, GB_K, GB_M, TMA_SWIZZLE_128B));
     AK_TRY(make_tmap_2d(&tmB, wt, 2, k, n, (uint64_t)k * 2, GB_K, BN / 2, TMA_SWIZZLE_128B));
+    // C as 32-row x 128-byte boxes for the TMA epilogue; a row pitch that is no multiple of 16 bytes cannot have a tensor map
+    constexpr uint32_t esz = (EPI == AK_EPI_STORE_BF16 || EPI == AK_EPI_SILU_BF16) ? 2 : 4;
+    const uint32_t tma_out = ((uint64_t)ep.ldc * esz) % 16 == 0 && (uintptr_t)ep.c % 16 == 0;
+    CUtensorMap tmC = tmA;
+    if (tma_out) AK_TRY(make_tmap_2d(&tmC, ep.c, esz, n, m, (uint64_t)ep.ldc * esz, 128 / esz, 32, TMA_SWIZZLE_128B));
     const uint32_t tiles_n = cdiv(n, BN), tiles_total = tiles_n * cdiv(m, 2 * GB_M);
     const uint32_t n_pairs = tiles_total < 74 ? tiles_total : 74;   // one pair per TPC of the 148 SMs
-    return launch_k(gemm_bf16_pair_kernel<BN, EPI>, dim3(2 * n_pairs, 1, 1), dim3(G_THREADS), smem, st, dim3(2, 1, 1), tmA, tmB, ep, m, n, k,
-                    stages, kseg, tiles_n, tiles_total);
+    return launch_k(gemm_bf16_pair_kernel<BN, EPI>, dim3(2 * n_pairs, 1, 1), dim3(PAIR_THREADS), smem, st, dim3(2, 1, 1), tmA, tmB, tmC, ep, m, n,
+                    k, stages, kseg, tiles_n, tiles_total, tma_out);
 }
 template <int BN>
 static int launch_pair(cudaStream_t st, const void* a, const void* wt, const GemmEpi& ep, uint32_t m, uint32_t n, uint32_t k, uint32_t epi,
