@@ -689,8 +689,9 @@ int launch_bf16_to_f32(cudaStream_t st, const void* src, float* dst, uint64_t n)
     AK_CHECK_LAUNCH();
     return AK_OK;
 }
-// w_kn [k,n] f32  ->  wt_nk [n,k] bf16 through a 32x32 shared tile (both sides coalesced).
-__global__ void transpose_to_bf16_kernel(const float* __restrict__ w, bf16* __restrict__ wt, uint32_t k, uint32_t n) {
+// w_kn [k,n] f32  <->  wt_nk [n,k] through a 32x32 shared tile (both sides coalesced).
+template <typename T>
+__global__ void transpose_to_kernel(const float* __restrict__ w, T* __restrict__ wt, uint32_t k, uint32_t n) {
     __shared__ float tile[32][33];
     uint32_t n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
     for (uint32_t r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -700,15 +701,16 @@ __global__ void transpose_to_bf16_kernel(const float* __restrict__ w, bf16* __re
     __syncthreads();
     for (uint32_t r = threadIdx.y; r < 32; r += blockDim.y) {
         uint32_t nn = n0 + r, kk = k0 + threadIdx.x;
-        if (nn < n && kk < k) wt[(size_t)nn * k + kk] = __float2bfloat16_rn(tile[threadIdx.x][r]);
+        if (nn < n && kk < k) wt[(size_t)nn * k + kk] = Cvt<T>::from_f(tile[threadIdx.x][r]);
     }
 }
-__global__ void transpose_from_bf16_kernel(const bf16* __restrict__ wt, float* __restrict__ w, uint32_t k, uint32_t n) {
+template <typename T>
+__global__ void transpose_from_kernel(const T* __restrict__ wt, float* __restrict__ w, uint32_t k, uint32_t n) {
     __shared__ float tile[32][33];
     uint32_t n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
     for (uint32_t r = threadIdx.y; r < 32; r += blockDim.y) {
         uint32_t nn = n0 + r, kk = k0 + threadIdx.x;
-        tile[r][threadIdx.x] = (nn < n && kk < k) ? __bfloat162float(wt[(size_t)nn * k + kk]) : 0.0f;
+        tile[r][threadIdx.x] = (nn < n && kk < k) ? Cvt<T>::to_f(wt[(size_t)nn * k + kk]) : 0.0f;
     }
     __syncthreads();
     for (uint32_t r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -716,16 +718,18 @@ __global__ void transpose_from_bf16_kernel(const bf16* __restrict__ wt, float* _
         if (kk < k && nn < n) w[(size_t)kk * n + nn] = tile[threadIdx.x][r];
     }
 }
-int launch_transpose_to_bf16(cudaStream_t st, const float* w_kn, void* wt_nk, uint32_t k, uint32_t n) {
+int launch_transpose_to(cudaStream_t st, const float* w_kn, void* wt_nk, uint32_t dtype, uint32_t k, uint32_t n) {
     dim3 grid(cdiv(n, 32), cdiv(k, 32)), block(32, 8);
-    transpose_to_bf16_kernel<<<grid, block, 0, st>>>(w_kn, (bf16*)wt_nk, k, n);
+    if (dtype == AK_F32) transpose_to_kernel<float><<<grid, block, 0, st>>>(w_kn, (float*)wt_nk, k, n);
+    else transpose_to_kernel<bf16><<<grid, block, 0, st>>>(w_kn, (bf16*)wt_nk, k, n);
     AK_COUNT_LAUNCH();
     AK_CHECK_LAUNCH();
     return AK_OK;
 }
-int launch_transpose_from_bf16(cudaStream_t st, const void* wt_nk, float* w_kn, uint32_t k, uint32_t n) {
+int launch_transpose_from(cudaStream_t st, const void* wt_nk, uint32_t dtype, float* w_kn, uint32_t k, uint32_t n) {
     dim3 grid(cdiv(n, 32), cdiv(k, 32)), block(32, 8);
-    transpose_from_bf16_kernel<<<grid, block, 0, st>>>((const bf16*)wt_nk, w_kn, k, n);
+    if (dtype == AK_F32) transpose_from_kernel<float><<<grid, block, 0, st>>>((const float*)wt_nk, w_kn, k, n);
+    else transpose_from_kernel<bf16><<<grid, block, 0, st>>>((const bf16*)wt_nk, w_kn, k, n);
     AK_COUNT_LAUNCH();
     AK_CHECK_LAUNCH();
     return AK_OK;
@@ -937,7 +941,7 @@ int ak_rmsnorm_rope_residual(void* stream, float* x, const float* residual, cons
 
 int ak_transpose_to_bf16(void* stream, const float* w_kn, void* wt_nk, uint32_t k, uint32_t n) {
     AK_REQUIRE(w_kn && wt_nk, AK_ERR_INVALID_ARG, "ak_transpose_to_bf16: null pointer");
-    return launch_transpose_to_bf16(as_stream(stream), w_kn, wt_nk, k, n);
+    return launch_transpose_to(as_stream(stream), w_kn, wt_nk, AK_BF16, k, n);
 }
 int ak_f32_to_bf16(void* stream, const float* src, void* dst, uint64_t n) {
     return launch_f32_to_bf16(as_stream(stream), src, dst, n);

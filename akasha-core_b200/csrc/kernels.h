@@ -35,8 +35,9 @@ int launch_sample_rows(cudaStream_t st, const float* logits, uint32_t rows, uint
                        uint64_t step, const int32_t* row_active, uint32_t* out_idx);
 int launch_f32_to_bf16(cudaStream_t st, const float* src, void* dst, uint64_t n);
 int launch_bf16_to_f32(cudaStream_t st, const void* src, float* dst, uint64_t n);
-int launch_transpose_to_bf16(cudaStream_t st, const float* w_kn, void* wt_nk, uint32_t k, uint32_t n);
-int launch_transpose_from_bf16(cudaStream_t st, const void* wt_nk, float* w_kn, uint32_t k, uint32_t n);
+// f32 [k,n] <-> [n,k] of dtype
+int launch_transpose_to(cudaStream_t st, const float* w_kn, void* wt_nk, uint32_t dtype, uint32_t k, uint32_t n);
+int launch_transpose_from(cudaStream_t st, const void* wt_nk, uint32_t dtype, float* w_kn, uint32_t k, uint32_t n);
 int launch_fill_normal(cudaStream_t st, void* dst, uint32_t dtype, uint64_t n, uint64_t seed, uint64_t stream_id,
                        float mean, float std);
 // Matrix fill for (possibly sliced) weights: local element (i, c) of a [lin, lout] slice takes the
@@ -55,6 +56,8 @@ enum { GEMM_ADD = 1, GEMM_SILU = 2 };
 // C[m,n] (+)= A[m,k] @ B[k,n], row-major f32. m == 1 uses the cluster split-K GEMV.
 int launch_gemm_f32(cudaStream_t st, const float* a, const float* b, float* c, uint32_t m, uint32_t n,
                     uint32_t k, uint32_t flags);
+// C[m,n] (+)= A[m,k] @ Wt[n,k]^T, row-major f32 (gemm_f32_nt.cu): the runner's f32 projections, stored [out,in].
+int launch_gemm_f32_nt(cudaStream_t st, const float* a, const float* wt, float* c, uint32_t m, uint32_t n, uint32_t k, uint32_t flags);
 
 // ---- gemm_tcgen05.cu (bf16 tensor cores) --------------------------------------------------------
 // invariant: keep the K summation structure a function of (n, k) only, so a row's result is the

@@ -160,14 +160,14 @@ int ak_weights_set_param(ak_weights* w, uint32_t index, const float* host, uint6
                 memcpy(&slice[(size_t)i * pr.lout + (size_t)b * bl], host + (size_t)i * pr.out + (size_t)b * bg + (size_t)w->tp_rank * bl, (size_t)bl * 4);
         src = slice.data();
     }
-    if (w->dtype == AK_F32 || pr.kind == 0) {
+    if (pr.kind == 0 || (w->dtype == AK_F32 && pr.kind == 1)) {
         AK_CUDA(cudaMemcpyAsync(*pr.ptr, src, pr.llen * 4, cudaMemcpyHostToDevice, st));
     } else {
         int rc = ensure_staging(w, pr.llen);
         if (rc) return rc;
         AK_CUDA(cudaMemcpyAsync(w->staging, src, pr.llen * 4, cudaMemcpyHostToDevice, st));
         rc = (pr.kind == 1) ? launch_f32_to_bf16(st, w->staging, *pr.ptr, pr.llen)
-                            : launch_transpose_to_bf16(st, w->staging, *pr.ptr, pr.lin, pr.lout);
+                            : launch_transpose_to(st, w->staging, *pr.ptr, w->dtype, pr.lin, pr.lout);
         if (rc) return rc;
     }
     AK_CUDA(cudaStreamSynchronize(st));
@@ -182,13 +182,13 @@ int ak_weights_get_param(ak_weights* w, uint32_t index, float* host, uint64_t n_
     AK_REQUIRE(pr.split == 0, AK_ERR_UNSUPPORTED, "ak_weights_get_param: tensor %u is sliced across tensor-parallel ranks", index);
     AK_CUDA(cudaSetDevice(w->ctx->device));
     cudaStream_t st = w->ctx->stream;
-    if (w->dtype == AK_F32 || pr.kind == 0) {
+    if (pr.kind == 0 || (w->dtype == AK_F32 && pr.kind == 1)) {
         AK_CUDA(cudaMemcpyAsync(host, *pr.ptr, pr.len * 4, cudaMemcpyDeviceToHost, st));
     } else {
         int rc = ensure_staging(w, pr.len);
         if (rc) return rc;
         rc = (pr.kind == 1) ? launch_bf16_to_f32(st, *pr.ptr, w->staging, pr.len)
-                            : launch_transpose_from_bf16(st, *pr.ptr, w->staging, pr.in, pr.out);
+                            : launch_transpose_from(st, *pr.ptr, w->dtype, w->staging, pr.in, pr.out);
         if (rc) return rc;
         AK_CUDA(cudaMemcpyAsync(host, w->staging, pr.len * 4, cudaMemcpyDeviceToHost, st));
     }
@@ -205,7 +205,7 @@ int ak_weights_init_synthetic(ak_weights* w, uint64_t seed, float std) {
         if (pr.kind == 2) {
             const uint32_t nblk = pr.split == 3 ? 3 : 1;
             const uint32_t bl = pr.lout / nblk, bg = pr.out / nblk;
-            rc = launch_fill_normal_2d(w->ctx->stream, *pr.ptr, w->dtype, w->dtype == AK_BF16, pr.lin, pr.lout, pr.out,
+            rc = launch_fill_normal_2d(w->ctx->stream, *pr.ptr, w->dtype, true, pr.lin, pr.lout, pr.out,
                                        pr.split == 1 ? w->tp_rank * pr.lin : 0, pr.split == 3 ? 3 : 0,
                                        (pr.split == 2 || pr.split == 3) ? w->tp_rank * bl : 0, bl, bg, seed, i, 0.0f, std);
         } else {
@@ -374,7 +374,7 @@ int Runner::gemm(const void* a, const void* wt, void* c, uint32_t m, uint32_t n,
     cudaStream_t st = ctx_->stream;
     if (w_->dtype == AK_F32) {
         uint32_t flags = mode == 1 ? GEMM_ADD : (mode == 2 ? GEMM_SILU : 0);
-        return launch_gemm_f32(st, (const float*)a, (const float*)wt, (float*)c, m, n, k, flags);
+        return launch_gemm_f32_nt(st, (const float*)a, (const float*)wt, (float*)c, m, n, k, flags);
     }
     uint32_t epi = mode == 1 ? AK_EPI_ADD_F32 : (mode == 2 ? AK_EPI_SILU_BF16 : AK_EPI_STORE_F32);
     return launch_gemm_bf16(st, a, wt, c, m, n, k, epi, n, true);
@@ -411,7 +411,7 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
         auto gemm_s = [&](cudaStream_t s, const void* a, const void* wt, void* cc, uint32_t m, uint32_t n, uint32_t k, int mode) -> int {
             if (dt == AK_F32) {
                 const uint32_t flags = mode == 1 ? GEMM_ADD : (mode == 2 ? GEMM_SILU : 0);
-                return launch_gemm_f32(s, (const float*)a, (const float*)wt, (float*)cc, m, n, k, flags);
+                return launch_gemm_f32_nt(s, (const float*)a, (const float*)wt, (float*)cc, m, n, k, flags);
             }
             const uint32_t epi = mode == 1 ? AK_EPI_ADD_F32 : (mode == 2 ? AK_EPI_SILU_BF16 : AK_EPI_STORE_F32);
             return launch_gemm_bf16(s, a, wt, cc, m, n, k, epi, n, true);

@@ -19,9 +19,9 @@ struct ak_weights {
     ak_ctx* ctx = nullptr;
     ak_model_config cfg{};
     uint32_t dtype = AK_F32;
-    // Device tensors. f32 mode: matrices f32 [in,out] (the reference layout, src/nn/weights.rs:32-47).
-    // bf16 mode: embedding bf16 [vocab,dim]; projection matrices bf16 [out,in] (transposed once at
-    // upload so both tcgen05 operands are K-major); norm gains stay f32.
+    // Device tensors of the reference's layout (src/nn/weights.rs:32-47): embedding [vocab,dim]; projection matrices
+    // transposed once at upload to [out,in] (both GEMM operands K-major, and a batch-1 step streams whole rows);
+    // in `dtype`. Norm gains stay f32.
     void* embedding = nullptr;
     struct Block {
         float* norm_1 = nullptr;
