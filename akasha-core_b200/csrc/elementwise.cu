@@ -964,6 +964,7 @@ namespace ak {
 
 constexpr int SMP_THREADS = 1024;
 constexpr int SMP_MAX_K = 1024;
+constexpr int SMP_MAX_SMEM = 214 * 1024;   // 227 KB less the kernel's static variables
 
 __device__ __forceinline__ uint64_t smp_mix(uint64_t z) {
     z += 0x9E3779B97F4A7C15ull;
@@ -1088,118 +1089,214 @@ __device__ uint32_t smp_sample_untruncated(const float* srow, uint32_t n, float 
     return scan[SMP_THREADS];
 }
 
+// Largest t such that at least k of the CTA's threads hold a key >= t, bit by bit.
+__device__ uint32_t smp_kth_key(uint32_t key, uint32_t k) {
+    uint32_t t = 0;
+    for (int b = 31; b >= 0; b--) {
+        const uint32_t t2 = t | (1u << b);
+        if ((uint32_t)__syncthreads_count(key >= t2) >= k) t = t2;
+    }
+    return t;
+}
+
+// One CTA per row, the row in shared memory. Top-k: the k-th largest of the 1024 threads' own maxima is a bound that at least k
+// elements reach and few others do, so the elements at or above it (a list of some tens for k = 40) are all that has to be
+// ordered: each finds its rank by counting the better ones. (Taking the maximum k times over the whole row cost ~4 us per
+// candidate.) A row with more elements at the bound than the list holds (ties, k near 1024) still goes through the repeated maximum. The f64
+// exponentials and quotients are formed by one thread per candidate; only the sums, whose order the reference fixes, are
+// serial. 50257 logits, k = 40: 200 us with both done serially.
+constexpr uint32_t SMP_LIST = 2048;
+
 __global__ void __launch_bounds__(SMP_THREADS)
-sample_rows_kernel(const float* __restrict__ logits, uint32_t n, uint32_t ld, const uint32_t* __restrict__ seen,
-                   const uint32_t* __restrict__ seen_off, float penalty, float temperature, uint32_t top_k, float top_p,
-                   uint64_t seed, uint64_t step, const int32_t* __restrict__ row_active, uint32_t* __restrict__ out_idx) {
-    extern __shared__ float srow[];                       // n logits, then the seen-id bitmap
+sample_rows_kernel(const float* __restrict__ logits, uint32_t n, uint32_t ld, const uint32_t* __restrict__ seen, const uint32_t* __restrict__ seen_off,
+                   uint32_t seen_len, float penalty, float temperature, uint32_t top_k, float top_p, uint64_t seed, uint64_t step,
+                   const int32_t* __restrict__ row_active, uint32_t* __restrict__ out_idx, uint32_t list_cap, const SampleSink sink) {
+    extern __shared__ __align__(16) float srow[];         // n logits, then list_cap words: the seen-id bitmap, later the candidate list
     uint32_t* bits = reinterpret_cast<uint32_t*>(srow + n);
     __shared__ float wv[32];
     __shared__ uint32_t wi[32];
     __shared__ __align__(8) float cand_v[SMP_MAX_K];
     __shared__ uint32_t cand_i[SMP_MAX_K + 1];
+    __shared__ uint32_t n_list;
     const uint32_t row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (row_active && row_active[row] < 0) return;
     const float* l = logits + (size_t)row * ld;
     const uint32_t nwords = (n + 31) / 32;
+    auto finish = [&](uint32_t pick) {   // one thread
+        out_idx[row] = pick;
+        if (sink.hist) *sink.hist = pick;
+        if (sink.done_host) {
+            __threadfence_system();
+            *(volatile uint64_t*)sink.done_host = (uint64_t)pick | ((uint64_t)sink.tag << 32);
+        }
+    };
     for (uint32_t i = tid; i < nwords; i += SMP_THREADS) bits[i] = 0u;
+#pragma unroll 8
     for (uint32_t i = tid; i < n; i += SMP_THREADS) srow[i] = l[i];
     __syncthreads();
     if (penalty != 1.0f && seen) {
-        for (uint32_t i = seen_off[row] + tid; i < seen_off[row + 1]; i += SMP_THREADS) {
-            uint32_t id = seen[i];
-            if (id < n) atomicOr(&bits[id >> 5], 1u << (id & 31));
+        const uint32_t s0 = seen_off ? seen_off[row] : 0u, s1 = seen_off ? seen_off[row + 1] : seen_len;
+        // every distinct id once: the thread that sets an id's bit applies the penalty to it
+        for (uint32_t i = s0 + tid; i < s1; i += SMP_THREADS) {
+            const uint32_t id = seen[i];
+            if (id < n && !(atomicOr(&bits[id >> 5], 1u << (id & 31)) & (1u << (id & 31))))
+                srow[id] = srow[id] > 0.0f ? srow[id] / penalty : srow[id] * penalty;
         }
-        __syncthreads();
-        for (uint32_t i = tid; i < n; i += SMP_THREADS)
-            if (bits[i >> 5] & (1u << (i & 31))) srow[i] = srow[i] > 0.0f ? srow[i] / penalty : srow[i] * penalty;
         __syncthreads();
     }
     if (temperature > 0.0f && (top_k == 0 || top_k >= n)) {
-        // no truncation: bisection over the whole row (the selection loop below only serves small k)
+        // no truncation: bisection over the whole row
         double* red = reinterpret_cast<double*>(cand_v);          // 64 doubles
         const uint64_t bitsr = smp_mix(seed ^ smp_mix(step * 0x632BE59BD9B4E019ull + row + 1));
         const double r = (double)(bitsr >> 11) * (1.0 / 9007199254740992.0);
         const uint32_t pick = smp_sample_untruncated(srow, n, temperature, top_p, r, red, cand_i);
-        if (tid == 0) out_idx[row] = pick;
+        if (tid == 0) finish(pick);
         return;
     }
     const uint32_t k = (temperature <= 0.0f) ? 1u : top_k;
-    for (uint32_t c = 0; c < k; c++) {
-        float best = -INFINITY;
-        uint32_t bi = 0xffffffffu;
+    // ---- the bound, and the elements that reach it (NaN never does; -inf is no candidate, as below)
+    uint32_t key = 0;
+#pragma unroll 4
+    for (uint32_t i = tid; i < n; i += SMP_THREADS) {
+        const float v = srow[i];
+        if (v > -INFINITY) key = max(key, smp_key(v + 0.0f));   // (-0 and 0 are equal)
+    }
+    uint32_t bound = smp_kth_key(key, k);
+    if (bound == 0) bound = 1;   // fewer than k threads hold a candidate: all of them
+    uint32_t* const list = bits;
+    if (tid == 0) n_list = 0;
+    __syncthreads();
+    if (key >= bound)
         for (uint32_t i = tid; i < n; i += SMP_THREADS) {
-            float v = srow[i];
-            if (v > best || (v == best && i < bi)) { best = v; bi = i; }
+            const float v = srow[i];
+            if (v > -INFINITY && smp_key(v + 0.0f) >= bound) {
+                const uint32_t at = atomicAdd(&n_list, 1u);
+                if (at < list_cap) list[at] = i;
+            }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            float ov = __shfl_xor_sync(0xffffffffu, best, o);
-            uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            argmax_combine(best, bi, ov, oi);
+    for (uint32_t j = tid; j < k; j += SMP_THREADS) cand_i[j] = 0xffffffffu;
+    __syncthreads();
+    const uint32_t m_list = n_list;
+    if (m_list <= list_cap) {
+        for (uint32_t c = tid; c < m_list; c += SMP_THREADS) {   // rank: value descending, index ascending
+            const uint32_t i = list[c];
+            const float v = srow[i];
+            uint32_t rank = 0;
+            for (uint32_t o = 0; o < m_list; o++) {
+                const uint32_t oi = list[o];
+                const float ov = srow[oi];
+                rank += (ov > v || (ov == v && oi < i)) ? 1u : 0u;
+            }
+            if (rank < k) { cand_v[rank] = v; cand_i[rank] = i; }
         }
-        if (lane == 0) { wv[warp] = best; wi[warp] = bi; }
         __syncthreads();
-        if (warp == 0) {
-            best = wv[lane];
-            bi = wi[lane];
+    } else {
+        for (uint32_t c = 0; c < k; c++) {
+            float best = -INFINITY;
+            uint32_t bi = 0xffffffffu;
+            for (uint32_t i = tid; i < n; i += SMP_THREADS) {
+                float v = srow[i];
+                if (v > best || (v == best && i < bi)) { best = v; bi = i; }
+            }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 float ov = __shfl_xor_sync(0xffffffffu, best, o);
                 uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
                 argmax_combine(best, bi, ov, oi);
             }
-            if (lane == 0) {
-                cand_v[c] = best;
-                cand_i[c] = bi;
-                if (bi != 0xffffffffu) srow[bi] = -INFINITY;  // taken
+            if (lane == 0) { wv[warp] = best; wi[warp] = bi; }
+            __syncthreads();
+            if (warp == 0) {
+                best = wv[lane];
+                bi = wi[lane];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    float ov = __shfl_xor_sync(0xffffffffu, best, o);
+                    uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                    argmax_combine(best, bi, ov, oi);
+                }
+                if (lane == 0) {
+                    cand_v[c] = best;
+                    cand_i[c] = bi;
+                    if (bi != 0xffffffffu) srow[bi] = -INFINITY;  // taken
+                }
             }
+            __syncthreads();
         }
-        __syncthreads();
     }
-    if (tid != 0) return;
-    if (temperature <= 0.0f) { out_idx[row] = cand_i[0] == 0xffffffffu ? 0u : cand_i[0]; return; }
-    // candidates that ran out (-inf everywhere) end the list
-    uint32_t m = 0;
-    while (m < k && cand_i[m] != 0xffffffffu) m++;
-    if (m == 0) { out_idx[row] = 0; return; }
-    // f64 softmax over the candidates, reusing srow as f64 scratch is not possible (taken marks):
-    // k <= 1024 doubles are recomputed on the fly instead of stored.
+    if (temperature <= 0.0f) {
+        if (tid == 0) finish(cand_i[0] == 0xffffffffu ? 0u : cand_i[0]);
+        return;
+    }
+    // ---- f64 softmax over the candidates (candidates that ran out end the list)
+    double* const e = reinterpret_cast<double*>(srow);   // the row is not needed any more: k <= n, and (n + bitmap) floats hold k doubles for n >= 2 k; else in place below
+    __shared__ double shared_sum;
+    const bool room = 2 * k <= n;
     const double mx = (double)cand_v[0], T = (double)temperature;
-    double sum = 0.0;
-    for (uint32_t j = 0; j < m; j++) sum += exp(((double)cand_v[j] - mx) / T);
+    __syncthreads();
+    if (room)
+        for (uint32_t j = tid; j < k; j += SMP_THREADS) e[j] = cand_i[j] != 0xffffffffu ? exp(((double)cand_v[j] - mx) / T) : 0.0;
+    __syncthreads();
+    auto e_of = [&](uint32_t j) { return room ? e[j] : exp(((double)cand_v[j] - mx) / T); };
+    uint32_t m = 0;
+    if (tid == 0) {
+        double sum = 0.0;
+        while (m < k && cand_i[m] != 0xffffffffu) { sum += e_of(m); m++; }
+        shared_sum = sum;
+    }
+    __syncthreads();
+    const double sum = shared_sum;
+    if (room)
+        for (uint32_t j = tid; j < k; j += SMP_THREADS) e[j] = e[j] / sum;
+    __syncthreads();
+    auto p_of = [&](uint32_t j) { return room ? e[j] : exp(((double)cand_v[j] - mx) / T) / sum; };
+    if (tid != 0) return;
+    if (m == 0) { finish(0u); return; }
     uint32_t keep = m;
+    double s2 = 0.0;
     if (top_p < 1.0f) {
         double cum = 0.0;
         for (uint32_t j = 0; j < m; j++) {
-            cum += exp(((double)cand_v[j] - mx) / T) / sum;
+            cum += p_of(j);
             if (cum >= (double)top_p) { keep = j + 1; break; }
         }
+        s2 = cum;   // the kept probabilities in list order: the same sum
+    } else {
+        for (uint32_t j = 0; j < keep; j++) s2 += p_of(j);
     }
-    double s2 = 0.0;
-    for (uint32_t j = 0; j < keep; j++) s2 += exp(((double)cand_v[j] - mx) / T) / sum;
     const uint64_t bitsr = smp_mix(seed ^ smp_mix(step * 0x632BE59BD9B4E019ull + row + 1));
     double r = (double)(bitsr >> 11) * (1.0 / 9007199254740992.0);  // [0, 1)
     uint32_t pick = cand_i[keep - 1];
     for (uint32_t j = 0; j < keep; j++) {
-        double p = (exp(((double)cand_v[j] - mx) / T) / sum) / s2;
+        const double p = p_of(j) / s2;
         if (r < p) { pick = cand_i[j]; break; }
         r -= p;
     }
-    out_idx[row] = pick;
+    finish(pick);
 }
 
-int launch_sample_rows(cudaStream_t st, const float* logits, uint32_t rows, uint32_t n, uint32_t ld, const uint32_t* seen,
-                       const uint32_t* seen_off, float penalty, float temperature, uint32_t top_k, float top_p, uint64_t seed,
-                       uint64_t step, const int32_t* row_active, uint32_t* out_idx) {
+int launch_sample_rows(cudaStream_t st, const float* logits, uint32_t rows, uint32_t n, uint32_t ld, const uint32_t* seen, const uint32_t* seen_off,
+                       uint32_t seen_len, float penalty, float temperature, uint32_t top_k, float top_p, uint64_t seed, uint64_t step,
+                       const int32_t* row_active, uint32_t* out_idx, const SampleSink& sink) {
     if (rows == 0 || n == 0) return AK_OK;
     AK_REQUIRE(temperature <= 0.0f || top_k <= SMP_MAX_K || top_k >= n, AK_ERR_UNSUPPORTED,
                "sampler: top_k must be 0 (no truncation) or 1..%d on the device (got %u)", SMP_MAX_K, top_k);
-    const size_t smem = (size_t)n * 4 + (size_t)((n + 31) / 32) * 4;
-    AK_REQUIRE(smem <= 214 * 1024, AK_ERR_UNSUPPORTED, "sampler: vocabulary of %u does not fit shared memory", n);
-    AK_CUDA(cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    sample_rows_kernel<<<rows, SMP_THREADS, smem, st>>>(logits, n, ld, seen, seen_off, penalty, temperature, top_k, top_p, seed, step,
-                                                        row_active, out_idx);
+    size_t words = (n + 31) / 32;
+    if (words < SMP_LIST && ((size_t)n + SMP_LIST) * 4 <= SMP_MAX_SMEM) words = SMP_LIST;
+    const size_t smem = ((size_t)n + words) * 4;
+    AK_REQUIRE(smem <= SMP_MAX_SMEM, AK_ERR_UNSUPPORTED, "sampler: vocabulary of %u does not fit shared memory", n);
+    {
+        static bool attr_set[64] = {};
+        int dev = 0;
+        AK_CUDA(cudaGetDevice(&dev));
+        std::lock_guard<std::mutex> lock(device_cache_mutex());
+        if (!attr_set[dev & 63]) {
+            AK_CUDA(cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMP_MAX_SMEM));
+            attr_set[dev & 63] = true;
+        }
+    }
+    sample_rows_kernel<<<rows, SMP_THREADS, smem, st>>>(logits, n, ld, seen, seen_off, seen_len, penalty, temperature, top_k, top_p, seed, step,
+                                                        row_active, out_idx, (uint32_t)words, sink);
     AK_COUNT_LAUNCH();
     AK_CHECK_LAUNCH();
     return AK_OK;
@@ -1212,6 +1309,6 @@ extern "C" int ak_sample_token(void* stream, const float* logits, uint32_t rows,
                                uint64_t seed, uint64_t step, uint32_t* out_idx) {
     AK_REQUIRE(logits && out_idx, AK_ERR_INVALID_ARG, "ak_sample_token: null pointer");
     AK_REQUIRE(repetition_penalty == 1.0f || (seen && seen_off), AK_ERR_INVALID_ARG, "ak_sample_token: a repetition penalty needs the seen ids");
-    return ak::launch_sample_rows(ak::as_stream(stream), logits, rows, n, n, seen, seen_off, repetition_penalty, temperature, top_k,
-                                  top_p, seed, step, nullptr, out_idx);
+    return ak::launch_sample_rows(ak::as_stream(stream), logits, rows, n, n, seen, seen_off, 0, repetition_penalty, temperature, top_k,
+                                  top_p, seed, step, nullptr, out_idx, ak::SampleSink{});
 }

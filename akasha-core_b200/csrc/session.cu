@@ -207,10 +207,8 @@ int ak_session_generate(ak_session* s, const uint32_t* prompt, uint32_t n, uint3
     uint32_t hist_len = n;
     for (uint32_t i = 0; i < max_new; i++) {
         // sample from the logits of the step just run; the id replaces the greedy one the step left for the next decode row
-        const uint32_t off[2] = {0u, hist_len};
-        AK_CUDA(cudaMemcpyAsync(s->d_hist_off, off, 8, cudaMemcpyHostToDevice, st));
-        rc = launch_sample_rows(st, r.logits_dev(), 1, V, r.logits_ld(), s->d_hist, s->d_hist_off, repetition_penalty, temperature, top_k,
-                                top_p, seed, i, nullptr, r.sampled_dev());
+        rc = launch_sample_rows(st, r.logits_dev(), 1, V, r.logits_ld(), s->d_hist, nullptr, hist_len, repetition_penalty, temperature, top_k,
+                                top_p, seed, i, nullptr, r.sampled_dev(), SampleSink{});
         if (rc) return rc;
         AK_CUDA(cudaMemcpyAsync(s->d_hist + hist_len, r.sampled_dev(), 4, cudaMemcpyDeviceToDevice, st));
         AK_CUDA(cudaMemcpyAsync(&next, r.sampled_dev(), 4, cudaMemcpyDeviceToHost, st));

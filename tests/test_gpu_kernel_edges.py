@@ -60,3 +60,24 @@ def test_gemm_pair_outputs(ak, torch_cuda, epi, m, n, k, ldc):
     assert float((c[:, :n].double() - want).abs().max()) < tol
     assert bool((c[:, n:] == 3.0).all())
     ak.check(ak.lib().ak_check_device_status(None))
+
+
+# the candidate list of the sampler: a small vocabulary, ties that overflow the list, k close to the thread count
+@pytest.mark.parametrize("n,k,kind", [(40, 40 - 1, "random"), (300, 7, "random"), (50257, 40, "ties"), (50257, 1000, "random"), (5000, 1024, "few"), (50257, 40, "zeros")])
+def test_sampler_candidates(ak, orc, torch_cuda, n, k, kind):
+    torch = torch_cuda
+    rng = np.random.default_rng(n + k)
+    logits = (rng.standard_normal((3, n)) * 2.0).astype(np.float32)
+    if kind == "ties":
+        logits = np.round(logits)                 # thousands of equal logits: index order decides
+    if kind == "zeros":
+        logits[:] = np.where(rng.random((3, n)) < 0.5, -0.0, 0.0)
+    if kind == "few":
+        logits[:, 50:] = -1e30
+    d = torch.from_numpy(logits).cuda()
+    for step in range(6):
+        out = torch.full((3,), -1, dtype=torch.int32, device="cuda")
+        ak.ops.sample_token(d, 3, n, out, 1.3, k, 0.97, 99, step)
+        got = out.cpu().numpy()
+        for r in range(3):
+            assert int(got[r]) == orc.sample_token(logits[r], 1.3, k, 0.97, np.zeros(0, np.uint32), 1.0, r=ak.ops.sampler_uniform(99, step, r))
