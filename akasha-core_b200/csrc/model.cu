@@ -7,6 +7,7 @@
 
 #include <stdlib.h>
 
+#include <atomic>
 #include <chrono>
 
 using namespace ak;
@@ -251,6 +252,9 @@ Runner::~Runner() {
     cudaFree(amax_val_); cudaFree(amax_idx_); cudaFree(tp_tmp_);
     cudaFree(xf_); cudaFree(logits_); cudaFree(attn_scratch_); cudaFree(rope_table_);
     cudaFree(d_desc_); cudaFree(d_sampled_);
+    cudaFree(d_solo_layers_); cudaFree(d_solo_xch_);
+    if (h_solo_done_) cudaFreeHost(h_solo_done_);
+    if (h_logits_) cudaFreeHost(h_logits_);
     for (Bank& b : banks_) {
         if (b.h_desc) cudaFreeHost(b.h_desc);
         if (b.h_sampled) cudaFreeHost(b.h_sampled);
@@ -365,7 +369,70 @@ int Runner::init(ak_ctx* ctx, ak_weights* w, uint32_t max_seqs, uint32_t max_seq
     AK_CUDA(cudaStreamCreateWithFlags(&st_time_, cudaStreamNonBlocking));
     AK_CUDA(cudaEventCreateWithFlags(&ev_tfork_, cudaEventDisableTiming));
     AK_CUDA(cudaEventCreateWithFlags(&ev_tjoin_, cudaEventDisableTiming));
+    solo_ = max_seqs == 1 && tp_ == 1 && solo_supported(w->dtype, D, F, H, c.num_layers);
+    if (solo_) {
+        std::vector<SoloLayer> sl(c.num_layers);
+        for (uint32_t l = 0; l < c.num_layers; l++) {
+            const auto& b = w->blocks[l];
+            sl[l] = {b.norm_1, b.qkv, b.out, b.norm_2, b.up, b.down, k_pool_[l], v_pool_[l]};
+        }
+        const size_t words = solo_xch_words(D, F, H, c.num_layers);
+        AK_CUDA(cudaMalloc((void**)&d_solo_layers_, sl.size() * sizeof(SoloLayer)));
+        AK_CUDA(cudaMemcpyAsync(d_solo_layers_, sl.data(), sl.size() * sizeof(SoloLayer), cudaMemcpyHostToDevice, ctx->stream));
+        AK_CUDA(cudaMalloc((void**)&d_solo_xch_, words * 8));
+        AK_CUDA(cudaMemsetAsync(d_solo_xch_, 0, words * 8, ctx->stream));
+        AK_CUDA(cudaMallocHost((void**)&h_solo_done_, SOLO_AHEAD * 8));
+        memset(h_solo_done_, 0, SOLO_AHEAD * 8);
+        AK_CUDA(cudaMallocHost((void**)&h_logits_, (size_t)V * 4));
+    }
     AK_CUDA(cudaStreamSynchronize(ctx->stream));
+    return AK_OK;
+}
+
+SoloArgs Runner::solo_args(int32_t tok_src, uint32_t pos) {
+    const ak_model_config& c = w_->cfg;
+    SoloArgs a{};
+    a.layers = d_solo_layers_;
+    a.embedding = w_->embedding;
+    a.final_norm = w_->final_norm;
+    a.lm_head = w_->lm_head;
+    a.rope = rope_table_;
+    a.xch = d_solo_xch_;
+    a.sampled = d_sampled_;
+    a.n_layers = c.num_layers; a.dim = c.dim; a.ffn = c.ffn_hidden; a.heads = c.num_heads; a.vocab = c.vocab_size;
+    a.pos = pos;
+    a.tok_src = tok_src;
+    if (++solo_step_ == 0) solo_step_ = 1;   // 0 is what a fresh exchange buffer holds
+    a.step = solo_step_;
+    a.eps = c.norm_eps;
+    a.scale = 1.0f / sqrtf((float)(c.dim / c.num_heads));
+    return a;
+}
+
+int Runner::solo_launch(int32_t tok_src, uint32_t pos, bool want_logits, bool host_logits, uint32_t& ticket) {
+    AK_CUDA(cudaSetDevice(ctx_->device));
+    SoloArgs a = solo_args(tok_src, pos);
+    a.logits = want_logits ? logits_ : nullptr;
+    a.logits_host = host_logits ? h_logits_ : nullptr;
+    a.done_host = h_solo_done_ + a.step % SOLO_AHEAD;
+    ticket = a.step;
+    return launch_solo(ctx_->stream, w_->dtype, a);
+}
+
+int Runner::wait_word(const uint64_t* w, uint32_t tag, uint32_t& value) {
+    const volatile uint64_t* word = w;
+    for (uint64_t n = 1;; n++) {
+        const uint64_t v = *word;
+        if ((uint32_t)(v >> 32) == tag) { value = (uint32_t)v; break; }
+        if ((n & 0xfff) == 0) {   // now and then: has the stream stopped without reporting?
+            const cudaError_t e = cudaStreamQuery(ctx_->stream);
+            if (e == cudaErrorNotReady) continue;
+            if (e != cudaSuccess) return cuda_fail(e, "batch-1 step", __FILE__, __LINE__);
+            const uint64_t last = *word;
+            AK_REQUIRE((uint32_t)(last >> 32) == tag, AK_ERR_CUDA, "batch-1 step ended without a result");
+        }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);   // what was written before the word
     return AK_OK;
 }
 

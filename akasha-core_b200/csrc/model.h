@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "solo.h"
 
 struct ak_ctx {
     int device = 0;
@@ -94,6 +95,18 @@ class Runner {
     // Any step (decode rows + optional prefill rows) through a per-bucket captured graph.
     int run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_pf_len);
     int sync();
+    // A decode step of the only slot as one persistent kernel (batch 1, solo.cu), where the model allows it. The token fed in
+    // is `tok_src` (< 0: the token last sampled on the device) at position `pos`; block i of the cache is block i of the
+    // sequence. solo_launch() may be called again before the step before has finished (steps run in order); solo_wait(t)
+    // blocks until step t (the value solo_launch gave) is done and returns its greedy token. At most SOLO_AHEAD steps may
+    // be unwaited for. logits_host (with `want_logits`): the step's logits in pinned host memory, valid after solo_wait.
+    static constexpr uint32_t SOLO_AHEAD = 4;
+    bool solo() const { return solo_; }
+    int solo_launch(int32_t tok_src, uint32_t pos, bool want_logits, bool host_logits, uint32_t& ticket);
+    int solo_wait(uint32_t ticket, uint32_t& token) { return wait_word(h_solo_done_ + ticket % SOLO_AHEAD, ticket, token); }
+    // spin until a device-written pinned word {value, tag} carries `tag`
+    int wait_word(const uint64_t* word, uint32_t tag, uint32_t& value);
+    const float* solo_logits_host() const { return h_logits_; }
     // Two banks of host-side step state (pinned descriptor, pinned result buffer, timing events, captured
     // graphs), so that the host can describe and launch step N+1 while step N is still running. The
     // accessors above and run()/run_graph() use the current bank; the device buffers are shared and
@@ -181,6 +194,13 @@ class Runner {
         bool ev_valid = false, ev_g_valid = false;
     } banks_[2];
     uint32_t bank_ = 0;
+    bool solo_ = false;
+    SoloLayer* d_solo_layers_ = nullptr;
+    uint64_t* d_solo_xch_ = nullptr;
+    uint64_t* h_solo_done_ = nullptr;   // pinned: one word per step in flight
+    float* h_logits_ = nullptr;         // pinned, [vocab]
+    uint32_t solo_step_ = 0;
+    SoloArgs solo_args(int32_t tok_src, uint32_t pos);
     // Admission steps: the admitted prompts' rows run on a second stream, concurrently with the decode
     // rows (different sequences: they share nothing until the final norm).
     cudaStream_t st2_ = nullptr;

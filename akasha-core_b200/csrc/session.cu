@@ -3,6 +3,7 @@
 // The KV cache is the runner's paged pool with the identity block table (block i = positions
 // 16i .. 16i+15), so a gathered read reproduces the reference's contiguous [max_ctx, dim] rows.
 #include <limits.h>
+#include <string.h>
 
 #include "model.h"
 
@@ -17,11 +18,14 @@ struct ak_session {
     Runner runner;
     // sampled generation: the history (prompt + generated ids) on the device for the repetition penalty
     uint32_t* d_hist = nullptr;
-    uint32_t* d_hist_off = nullptr;   // {0, history length}
     uint32_t hist_cap = 0;
+    // tokens sampled ahead: pinned words the sampler reports them in, and the tag each waits for
+    static constexpr uint32_t PICKS = 4;
+    uint64_t* h_pick = nullptr;
+    uint32_t pick_of[PICKS] = {}, pick_tag = 0;
     ~ak_session() {
         if (d_hist) cudaFree(d_hist);
-        if (d_hist_off) cudaFree(d_hist_off);
+        if (h_pick) cudaFreeHost(h_pick);
     }
 };
 
@@ -104,7 +108,7 @@ int ak_session_prefill(ak_session* s, const uint32_t* tokens, uint32_t n, float*
     return AK_OK;
 }
 
-static int decode_one(ak_session* s, int32_t tok_src) {
+static int decode_one(ak_session* s, int32_t tok_src) {   // models the persistent kernel does not take
     Runner& r = s->runner;
     const uint32_t pos = s->cur_len;
     r.h_rows()[0] = {tok_src, (int32_t)pos, (int32_t)pos, 0};
@@ -116,17 +120,41 @@ static int decode_one(ak_session* s, int32_t tok_src) {
     return AK_OK;
 }
 
+// Launch the decode step that feeds tok_src (< 0: the device's last pick) at position pos; logits stay on the device.
+static int decode_launch(ak_session* s, int32_t tok_src, uint32_t pos) {
+    Runner& r = s->runner;
+    uint32_t ticket = 0;
+    if (r.solo()) return r.solo_launch(tok_src, pos, true, false, ticket);
+    s->cur_len = pos;
+    AK_TRY(decode_one(s, tok_src));
+    return r.sync();   // (one descriptor buffer: the step before has to be done with it)
+}
+// One decode step, waited for: cur_len grows, the greedy token in *tok, and (host) logits in r.solo_logits_host() or on the device.
+static int decode_any(ak_session* s, int32_t tok_src, bool want_logits, uint32_t* tok, float* logits_out = nullptr) {
+    Runner& r = s->runner;
+    if (r.solo()) {
+        uint32_t ticket = 0;
+        AK_TRY(r.solo_launch(tok_src, s->cur_len, want_logits, logits_out != nullptr, ticket));
+        AK_TRY(r.solo_wait(ticket, *tok));
+        s->cur_len++;
+        if (logits_out) memcpy(logits_out, r.solo_logits_host(), (size_t)s->w->cfg.vocab_size * 4);
+        return AK_OK;
+    }
+    AK_TRY(decode_one(s, tok_src));
+    AK_TRY(r.sync());
+    *tok = r.h_sampled()[0];
+    if (logits_out) return r.read_logits(0, logits_out);
+    return AK_OK;
+}
+
 // src/nn/inference.rs:178-262
 int ak_session_decode_step(ak_session* s, uint32_t token, float* logits_out, uint32_t* argmax_out) {
     AK_REQUIRE(s, AK_ERR_INVALID_ARG, "ak_session_decode_step: null session");
     AK_REQUIRE(s->has_cache, AK_NO_CACHE, "no cache attached (call ak_session_attach_cache or generate first)");
     AK_REQUIRE(s->cur_len < s->max_ctx, AK_CONTEXT_FULL, "context window is full (%u tokens)", s->max_ctx);
-    int rc = decode_one(s, token > 0x7fffffffu ? INT_MAX : (int32_t)token);
-    if (rc) return rc;
-    rc = s->runner.sync();
-    if (rc) return rc;
-    if (argmax_out) *argmax_out = s->runner.h_sampled()[0];
-    if (logits_out) return s->runner.read_logits(0, logits_out);
+    uint32_t tok = 0;
+    AK_TRY(decode_any(s, token > 0x7fffffffu ? INT_MAX : (int32_t)token, logits_out != nullptr, &tok, logits_out));
+    if (argmax_out) *argmax_out = tok;
     return AK_OK;
 }
 
@@ -153,6 +181,31 @@ int ak_session_generate_greedy(ak_session* s, const uint32_t* prompt, uint32_t n
         }
     }
     const uint32_t eos = s->w->cfg.eos_token;
+    if (s->runner.solo()) {
+        // Steps are launched ahead of the tokens they produce (each feeds on the device's last pick), so the GPU goes from
+        // one to the next. A step launched past an end-of-sequence token only writes cache rows beyond cur_len.
+        Runner& r = s->runner;
+        uint32_t tickets[Runner::SOLO_AHEAD] = {}, launched = 0, done = 0;   // of the decode steps after `next`
+        const uint32_t room = s->max_ctx - s->cur_len, base = s->cur_len;
+        const uint32_t most = max_new < room ? max_new : room;               // decode steps that may run
+        for (uint32_t i = 0; i < max_new; i++) {
+            out_tokens[(*n_out)++] = next;
+            if ((stop_on_eos && next == eos) || i >= most) break;            // also: out of context mid-generation
+            while (launched < most && launched - done < Runner::SOLO_AHEAD - 1) {
+                AK_TRY(r.solo_launch(-1, base + launched, false, false, tickets[launched % Runner::SOLO_AHEAD]));
+                launched++;
+            }
+            AK_TRY(r.solo_wait(tickets[done % Runner::SOLO_AHEAD], next));
+            done++;
+            s->cur_len = base + done;
+        }
+        while (done < launched) {   // steps past the end: let them finish before anyone else uses the cache
+            uint32_t unused;
+            AK_TRY(r.solo_wait(tickets[done % Runner::SOLO_AHEAD], unused));
+            done++;
+        }
+        return AK_OK;
+    }
     for (uint32_t i = 0; i < max_new; i++) {
         out_tokens[(*n_out)++] = next;
         if (stop_on_eos && next == eos) break;
@@ -189,7 +242,10 @@ int ak_session_generate(ak_session* s, const uint32_t* prompt, uint32_t n, uint3
         AK_CUDA(cudaMalloc((void**)&s->d_hist, (size_t)need * 4));
         s->hist_cap = need;
     }
-    if (!s->d_hist_off) AK_CUDA(cudaMalloc((void**)&s->d_hist_off, 8));
+    if (!s->h_pick) {
+        AK_CUDA(cudaMallocHost((void**)&s->h_pick, ak_session::PICKS * 8));
+        memset(s->h_pick, 0, ak_session::PICKS * 8);
+    }
     AK_CUDA(cudaMemcpyAsync(s->d_hist, prompt, (size_t)n * 4, cudaMemcpyHostToDevice, st));
     uint32_t next = 0;
     int rc;
@@ -198,31 +254,49 @@ int ak_session_generate(ak_session* s, const uint32_t* prompt, uint32_t n, uint3
         if (rc) return rc;
     } else {
         for (uint32_t i = 0; i < n; i++) {
-            rc = ak_session_decode_step(s, prompt[i], nullptr, &next);
+            AK_REQUIRE(s->cur_len < s->max_ctx, AK_CONTEXT_FULL, "context window is full (%u tokens)", s->max_ctx);
+            rc = decode_any(s, prompt[i] > 0x7fffffffu ? INT_MAX : (int32_t)prompt[i], true, &next);
             if (rc) return rc;
         }
     }
     Runner& r = s->runner;
     const uint32_t V = s->w->cfg.vocab_size, eos = s->w->cfg.eos_token;
-    uint32_t hist_len = n;
+    const uint32_t base = s->cur_len, room = s->max_ctx - base, most = max_new < room ? max_new : room;   // decode steps that may run
+    // Token i is sampled from the logits of the step before it, replaces the greedy pick that step left for the next one and
+    // joins the history, all on the device; the host learns it from a word the sampler writes last. Samplers and decode steps
+    // are launched ahead of the tokens: a step past an end-of-sequence token only writes cache rows beyond cur_len.
+    uint32_t launched = 0;
+    const uint32_t ahead = r.solo() ? ak_session::PICKS - 1 : 1;
+    auto launch = [&](uint32_t i) -> int {   // decode step i - 1 (i > 0), then the sampler of token i
+        if (i > 0) AK_TRY(decode_launch(s, -1, base + i - 1));
+        if (++s->pick_tag == 0) s->pick_tag = 1;
+        SampleSink sink;
+        sink.hist = s->d_hist + n + i;
+        sink.done_host = s->h_pick + i % ak_session::PICKS;
+        sink.tag = s->pick_tag;
+        s->pick_of[i % ak_session::PICKS] = s->pick_tag;
+        return launch_sample_rows(st, r.logits_dev(), 1, V, r.logits_ld(), s->d_hist, nullptr, n + i, repetition_penalty, temperature, top_k, top_p, seed,
+                                  i, nullptr, r.sampled_dev(), sink);
+    };
     for (uint32_t i = 0; i < max_new; i++) {
-        // sample from the logits of the step just run; the id replaces the greedy one the step left for the next decode row
-        rc = launch_sample_rows(st, r.logits_dev(), 1, V, r.logits_ld(), s->d_hist, nullptr, hist_len, repetition_penalty, temperature, top_k,
-                                top_p, seed, i, nullptr, r.sampled_dev(), SampleSink{});
+        while (launched < max_new && launched <= most && launched < i + ahead) {
+            rc = launch(launched);
+            if (rc) return rc;
+            launched++;
+        }
+        rc = r.wait_word(s->h_pick + i % ak_session::PICKS, s->pick_of[i % ak_session::PICKS], next);
         if (rc) return rc;
-        AK_CUDA(cudaMemcpyAsync(s->d_hist + hist_len, r.sampled_dev(), 4, cudaMemcpyDeviceToDevice, st));
-        AK_CUDA(cudaMemcpyAsync(&next, r.sampled_dev(), 4, cudaMemcpyDeviceToHost, st));
-        AK_CUDA(cudaStreamSynchronize(st));
-        hist_len++;
         out_tokens[(*n_out)++] = next;
+        s->cur_len = base + i;
         if (stop_on_eos && next == eos) break;
-        if (s->cur_len >= s->max_ctx) break;  // out of context mid-generation: return what we have
-        rc = decode_one(s, -1);               // the sampled id is read on the device
-        if (rc) return rc;
-        rc = r.sync();
-        if (rc) return rc;
+        if (i >= most) break;                                // out of context mid-generation: return what we have
+        if (i + 1 == max_new) {                              // the last token is fed too, as in the reference's loop
+            rc = decode_launch(s, -1, base + i);
+            if (rc) return rc;
+            s->cur_len = base + i + 1;
+        }
     }
-    return AK_OK;
+    return r.sync();   // steps launched past the end have finished before anyone else uses the cache
 }
 
 int ak_session_read_cache(ak_session* s, uint32_t layer, float* k_out, float* v_out) {

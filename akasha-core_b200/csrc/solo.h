@@ -1,0 +1,45 @@
+// Batch-1 decode step as one persistent kernel (solo.cu): launch interface.
+#pragma once
+#include "kernels.h"
+
+namespace ak {
+
+constexpr uint32_t SOLO_MAX_SPLITS = 4;   // CTAs a head's positions are divided over
+
+struct SoloLayer {   // device array, one per layer; matrices [out, in]
+    const float* norm_1;
+    const void* qkv;
+    const void* out;
+    const float* norm_2;
+    const void* up;
+    const void* down;
+    void* k_pool;
+    void* v_pool;
+};
+
+struct SoloArgs {
+    const SoloLayer* layers;
+    const void* embedding;
+    const float* final_norm;
+    const void* lm_head;
+    const float2* rope;          // [rope_len][head_dim / 2] (cos, sin)
+    const int32_t* table;        // block table of the sequence on the device; nullptr = identity
+    uint64_t* xch;               // solo_xch_words() 64-bit words, zero before the first launch
+    uint32_t* sampled;           // device word: the token fed back when tok_src < 0, overwritten by the greedy pick
+    float* logits;               // [vocab] device, or nullptr
+    float* logits_host;          // [vocab] mapped host memory, or nullptr
+    uint32_t* sampled_host;      // mapped host word, or nullptr
+    uint64_t* done_host;         // mapped host word {token, step}: written after everything else, or nullptr
+    uint32_t n_layers, dim, ffn, heads, vocab;
+    uint32_t pos;                // position of the token fed in; positions 0 .. pos are attended to
+    int32_t tok_src;             // >= 0 literal id; < 0: *sampled
+    uint32_t step;               // non-zero, different for every launch on the same xch
+    float eps, scale;
+};
+
+bool solo_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers);
+size_t solo_xch_words(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers);
+int launch_solo(cudaStream_t st, uint32_t dtype, const SoloArgs& a);
+int solo_status(unsigned int* out);
+
+}  // namespace ak

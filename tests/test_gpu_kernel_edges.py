@@ -62,6 +62,38 @@ def test_gemm_pair_outputs(ak, torch_cuda, epi, m, n, k, ldc):
     ak.check(ak.lib().ak_check_device_status(None))
 
 
+# The batch-1 step kernel: a decode step's logits equal the last row of a prefill of the same tokens (another set of kernels).
+# Shapes: one slice of K per warp or none; fewer rows than SMs; rows in pieces (ffn wider than a ring slot) and several row
+# blocks per SM; head_dim 128; positions that need 1, 2, 3, 4 splits and several rounds of cache tiles, at block boundaries.
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("vocab,dim,heads,layers,ffn,lens", [
+    (37, 64, 1, 2, 256, (1, 15, 16, 17)),
+    (1000, 320, 5, 2, 1280, (1, 33, 191, 192, 300)),
+    (50257, 768, 12, 1, 3072, (95, 96, 97, 383, 385, 700)),
+    (777, 1024, 8, 2, 6200, (8, 127, 129, 640)),
+    (601, 2048, 16, 1, 8192, (40, 257)),
+])
+def test_solo_step_equals_prefill(ak, ctx, dtype, vocab, dim, heads, layers, ffn, lens):
+    cfg = ak.ModelConfig(vocab, dim, heads, layers, 1024, ffn)
+    w = ak.ModelWeights(ctx, cfg, dtype)
+    w.init_synthetic(5, 0.05)
+    s, ref = ak.InferenceSession(ctx, w, 768), ak.InferenceSession(ctx, w, 768)
+    for n in lens:
+        toks = ak.uniform_tokens(n + 3, vocab, seed=n)
+        s.replace_cache()
+        s.prefill(toks[:n])
+        for j in range(3):
+            got, am = s.decode_step(int(toks[n + j]))
+            ref.replace_cache()
+            want, _ = ref.prefill(toks[:n + j + 1])
+            assert np.isfinite(got).all() and am == int(np.argmax(got))
+            rel = np.linalg.norm(got.astype(np.float64) - want) / np.linalg.norm(want.astype(np.float64))
+            # f32: sums of up to 8192 terms in another order; bf16: the prefill rounds its activations to bf16 (2^-9 each, a dozen per layer)
+            assert rel < (2e-5 if dtype == 0 else 2e-2), (n, j, rel)
+    ctx.check_device_status()
+    s.close(); ref.close(); w.close()
+
+
 # the candidate list of the sampler: a small vocabulary, ties that overflow the list, k close to the thread count
 @pytest.mark.parametrize("n,k,kind", [(40, 40 - 1, "random"), (300, 7, "random"), (50257, 40, "ties"), (50257, 1000, "random"), (5000, 1024, "few"), (50257, 40, "zeros")])
 def test_sampler_candidates(ak, orc, torch_cuda, n, k, kind):
