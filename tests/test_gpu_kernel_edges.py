@@ -113,3 +113,49 @@ def test_sampler_candidates(ak, orc, torch_cuda, n, k, kind):
         got = out.cpu().numpy()
         for r in range(3):
             assert int(got[r]) == orc.sample_token(logits[r], 1.3, k, 0.97, np.zeros(0, np.uint32), 1.0, r=ak.ops.sampler_uniform(99, step, r))
+
+
+# Prefill attention with more items than SMs (two query tiles per block, the persistent path): tile and block edges, an empty
+# sequence, scores that grow by more than the rescaling threshold. A sequence alone (one query tile per block, its own launch)
+# gives the same bits.
+@pytest.mark.parametrize("heads,hd", [(12, 64), (16, 128)])
+@pytest.mark.parametrize("q_scale", [1.0, 12.0])
+def test_attn_prefill_many_items(ak, torch_cuda, heads, hd, q_scale):
+    torch = torch_cuda
+    lens = [257, 1, 128, 0, 129, 255, 256, 127, 384, 385, 511, 513, 640, 17, 700]
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    n, mx = len(lens), max(lens)
+    mb = (mx + 15) // 16
+    nb = n * mb
+    kp, vp = (torch.randn(nb, heads, 16, hd, device="cuda", generator=g).bfloat16() for _ in range(2))
+    tables = torch.randperm(nb, device="cuda", generator=g).to(torch.int32).reshape(n, mb)
+    for i, L in enumerate(lens):                      # what was never written may hold anything
+        for b in range(mb):
+            used = min(max(L - b * 16, 0), 16)
+            if used < 16:
+                vp[tables[i, b].long(), :, used:] = float("nan") if used else vp[tables[i, b].long(), :, used:]
+    cu = np.zeros(n + 1, np.int32)
+    cu[1:] = np.cumsum(lens)
+    rows = int(cu[-1])
+    q = (torch.randn(rows, heads * hd, device="cuda", generator=g) * q_scale).bfloat16()
+    slot = torch.arange(n, dtype=torch.int32, device="cuda")
+    run = lambda qq, tt, c, out, k, m: ak.ops.attn_prefill_paged(qq, kp, vp, tt, mb, torch.from_numpy(c).cuda(), slot, out, k, m, qq.shape[0], heads, hd,
+                                                                 hd ** -0.5, ak.AK_BF16, nb)
+    out = torch.full_like(q, float("nan"))
+    run(q, tables, cu, out, n, mx)
+    ak.check(ak.lib().ak_check_device_status(None))
+    for i, L in enumerate(lens):
+        if not L:
+            continue
+        rows_i = slice(int(cu[i]), int(cu[i + 1]))
+        k, v = (p[tables[i].long()].transpose(1, 2).reshape(mb * 16, heads, hd)[:L].double().transpose(0, 1) for p in (kp, vp))
+        s = torch.einsum("lhd,hkd->hlk", q[rows_i].double().reshape(L, heads, hd), k) * hd ** -0.5
+        s.masked_fill_(torch.ones(L, L, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+        want = torch.einsum("hlk,hkd->lhd", s.softmax(-1), v).reshape(L, -1)
+        # P is rounded to bf16 on both sides of the quotient (2 * 2^-9 of the largest value), the output once more
+        tol = (2 ** -8 + 2 ** -9) * float(v.abs().max())
+        assert float((out[rows_i].double() - want).abs().max()) < tol, (i, L)
+        alone = torch.empty_like(q[rows_i])
+        run(q[rows_i].contiguous(), tables[i:i + 1].contiguous(), np.array([0, L], np.int32), alone, 1, L)
+        assert torch.equal(alone, out[rows_i]), (i, L)
+    ak.check(ak.lib().ak_check_device_status(None))
