@@ -536,6 +536,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // 128 x BN slice of output: half the weight traffic from L2 per flop of the one-CTA kernel, which is what bounds that
 // kernel. The 512 TMEM columns hold TWO accumulator buffers: the epilogue warps drain tile i while the MMAs of tile
 // i+1 run, so no second CTA per SM is needed to hide the epilogue and the ring can use the whole shared memory.
+// Where K is partitioned in segments the buffers alternate by segment and the epilogue adds a tile's segments in registers
+// (128 a thread): the MMAs never wait for it. (Accumulators for every segment of a tile side by side filled TMEM and ran
+// 22144 x 3072 x 768 in 215 us, 486 TFLOP/s, in the one-CTA kernel.)
 // Synchronisation (every wait bounded):
 //   full[s]      leader's barrier; both CTAs' TMA loads (.cta_group::2, no multicast: each CTA fetches its own tiles)
 //                complete on it, the leader arms it with the bytes of both;
@@ -590,13 +593,19 @@ template <int BN> struct PairCfg {
     static constexpr int A_BYTES = GB_M * GB_K * 2;          // this CTA's 128 rows of A: 16 KB
     static constexpr int B_BYTES = (BN / 2) * GB_K * 2;      // this CTA's half of the weight tile
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int TMEM_COLS = 512;                    // two accumulator buffers of kseg * BN columns
+    static constexpr int TMEM_COLS = 2 * BN;                 // two accumulator buffers
     static constexpr int OUT_WARP_BYTES = 32 * 128;          // an epilogue warp's output staging: one piece of 32 rows x 128 B
 };
 constexpr int PAIR_EPI_WARPS = 8;
-constexpr int PAIR_THREADS = 64 + PAIR_EPI_WARPS * 32;
+// The first warpgroup holds the TMA and the MMA warp. The epilogue's two warpgroups keep 128 sums a thread when K is segmented:
+// they take the registers that the first one gives back (of the 168 that 384 threads can be launched with).
+constexpr int PAIR_THREADS = 128 + PAIR_EPI_WARPS * 32;
+constexpr int PAIR_REGS_FIRST = 56, PAIR_REGS_EPI = 224;
+static_assert(PAIR_REGS_FIRST * 128 + PAIR_REGS_EPI * 256 <= 168 * PAIR_THREADS, "the split draws on the registers of the launch");
 
-template <int BN, int EPI>
+// SEG: K in kseg segments, each a sum of its own, added in segment order (the partition of a skinny launch of the same n and k,
+// so that a row's bits do not depend on how many rows share the launch).
+template <int BN, int EPI, bool SEG>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                       const GemmEpi ep, uint32_t m, uint32_t n, uint32_t k, uint32_t stages, uint32_t kseg, uint32_t tiles_n,
@@ -612,11 +621,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const uint32_t rank = cluster_ctarank();          // 0 = leader (issues the MMAs), 1 = peer
     const uint32_t pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const uint32_t num_kb = (k + GB_K - 1) / GB_K;
-    const uint32_t buf_cols = kseg * BN;
-    // two accumulator buffers when they fit the 512 columns (the epilogue of a tile then runs under the next tile's
-    // MMAs), else one (K split in two segments of 256 columns each: the epilogue is exposed)
-    const uint32_t n_bufs = (2 * buf_cols <= (uint32_t)C::TMEM_COLS) ? 2u : 1u;
-
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < stages; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
         for (uint32_t b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * PAIR_EPI_WARPS); }
@@ -637,6 +641,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const uint32_t tmem_base = tmem_base_sm;
     pdl_trigger();   // only after the TMEM allocation (see the one-CTA kernel)
 
+    if (SEG && warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PAIR_REGS_FIRST));
     if (warp == 0) {
         // ---------------- TMA producer (one per CTA; bytes are counted on the leader's full barriers)
         if (lane == 0) {
@@ -674,16 +679,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         // ---------------- MMA issuer: one thread of the leader CTA drives both SMs' tensor cores
         if (lane == 0 && rank == 0) {
             constexpr uint32_t idesc = make_idesc(2 * GB_M, BN);
-            const uint32_t per_seg = (num_kb + kseg - 1) / kseg;
-            uint32_t tc = 0, s = 0, ph = 0;   // ring position and phase are carried: no division in the K loop
+            const uint32_t per_seg = SEG ? (num_kb + kseg - 1) / kseg : num_kb;
+            uint32_t tc = 0, s = 0, ph = 0;   // accumulations (a tile's, or a segment's) so far; ring position and phase are carried: no division in the K loop
             bool ok = true;
-            for (uint32_t t = pair; t < tiles_total && ok; t += n_pairs, tc++) {
-                const uint32_t buf = n_bufs == 2 ? (tc & 1u) : 0u, acc_ph = (n_bufs == 2 ? (tc >> 1) : tc) & 1u;
-                // the epilogue warps of both CTAs have drained this buffer (it was last used by tile tc - n_bufs)
-                if (tc >= n_bufs && !mbar_wait(&acc_empty[buf], acc_ph ^ 1u)) { atomicExch(&fail_flag, 4u); break; }
-                tc_fence_after();
-                uint32_t in_seg = 0, acc_col = tmem_base + buf * buf_cols;
+            for (uint32_t t = pair; t < tiles_total && ok; t += n_pairs) {
+                uint32_t in_seg = 0, acc_col = 0, buf = 0;
                 for (uint32_t kb = 0; kb < num_kb; kb++) {
+                    if (in_seg == 0) {
+                        buf = tc & 1u;
+                        acc_col = tmem_base + buf * BN;
+                        // the epilogue warps of both CTAs have drained this buffer (it was last used two accumulations ago)
+                        if (tc >= 2 && !mbar_wait(&acc_empty[buf], ((tc >> 1) & 1u) ^ 1u)) { atomicExch(&fail_flag, 4u); ok = false; break; }
+                        tc_fence_after();
+                    }
                     if (!mbar_wait(&full_bar[s], ph)) { atomicExch(&fail_flag, 2u); ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + (size_t)s * C::STAGE_BYTES);
@@ -695,58 +703,76 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                     tc_commit2(map_to_cta(smem_u32(&empty_bar[s]), 0));
                     tc_commit2(map_to_cta(smem_u32(&empty_bar[s]), 1));
                     if (++s == stages) { s = 0; ph ^= 1u; }
-                    if (++in_seg == per_seg) { in_seg = 0; acc_col += BN; }
+                    if (++in_seg == per_seg || kb + 1 == num_kb) {
+                        tc_commit2(map_to_cta(smem_u32(&acc_full[buf]), 0));
+                        tc_commit2(map_to_cta(smem_u32(&acc_full[buf]), 1));
+                        in_seg = 0;
+                        tc++;
+                    }
                 }
-                if (!ok) break;
-                tc_commit2(map_to_cta(smem_u32(&acc_full[buf]), 0));
-                tc_commit2(map_to_cta(smem_u32(&acc_full[buf]), 1));
             }
         }
-    } else {
+    } else if (warp >= 4) {
         // ---------------- epilogue warps of both CTAs: thread <-> accumulator row of THIS CTA's TMEM, 8 warps: the two
         // warps of a TMEM lane quadrant take one half of the columns each. `tma_out`: 128-byte wide pieces (64 bf16 or
         // 32 f32 columns of 32 rows) go through a swizzled staging buffer and leave as TMA stores (or TMA adds into f32):
         // whole lines, no address arithmetic, tails clipped by the tensor map. Otherwise (row pitch of C not a multiple of
         // 16 bytes) registers are stored directly.
-        const uint32_t quad = warp & 3u, half = (warp - 2) >> 2;
+        if (SEG) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PAIR_REGS_EPI));
+        const uint32_t quad = warp & 3u, half = (warp - 4) >> 2;
         constexpr bool OUT_BF16 = (EPI == AK_EPI_STORE_BF16 || EPI == AK_EPI_SILU_BF16);
         constexpr uint32_t CW = OUT_BF16 ? 64 : 32;   // columns of a staged piece
-        uint8_t* const stage_sm = smem + (size_t)stages * C::STAGE_BYTES + (size_t)(warp - 2) * C::OUT_WARP_BYTES;
+        uint8_t* const stage_sm = smem + (size_t)stages * C::STAGE_BYTES + (size_t)(warp - 4) * C::OUT_WARP_BYTES;
         pdl_wait();
         uint32_t tc = 0;
-        for (uint32_t t = pair; t < tiles_total; t += n_pairs, tc++) {
-            const uint32_t buf = n_bufs == 2 ? (tc & 1u) : 0u, acc_ph = (n_bufs == 2 ? (tc >> 1) : tc) & 1u;
-            const uint32_t row0 = ((t / tiles_n) * 2 + rank) * GB_M + quad * 32, row = row0 + lane;
-            const uint32_t n0 = (t % tiles_n) * BN + half * (BN / 2);
-            bool got = mbar_wait(&acc_full[buf], acc_ph);
+        // accumulation tc is complete
+        auto wait_acc = [&]() -> bool {
+            bool got = mbar_wait(&acc_full[tc & 1u], (tc >> 1) & 1u);
             if (!got && lane == 0) atomicExch(&fail_flag, 3u);
             got = __all_sync(0xffffffffu, got);
-            if (!got) break;
             tc_fence_after();
-            const uint32_t acc0 = tmem_base + ((quad * 32u) << 16) + buf * buf_cols + half * (BN / 2);
-#pragma unroll 1
-            for (uint32_t c0 = 0; c0 < (uint32_t)BN / 2; c0 += 32) {
-                uint32_t r[32];
-                tmem_ld32(acc0 + c0, r);
-                tmem_ld_wait();
-                for (uint32_t seg = 1; seg < kseg; seg++) {
-                    uint32_t r2[32];
-                    tmem_ld32(acc0 + seg * BN + c0, r2);
-                    tmem_ld_wait();
+            return got;
+        };
+        auto free_acc = [&]() {   // this warp has read its part of the buffer: the leader's MMA thread may reuse it
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[tc & 1u]), 0));
+            tc++;
+        };
+        for (uint32_t t = pair; t < tiles_total; t += n_pairs) {
+            const uint32_t row0 = ((t / tiles_n) * 2 + rank) * GB_M + quad * 32, row = row0 + lane;
+            const uint32_t n0 = (t % tiles_n) * BN + half * (BN / 2);
+            const uint32_t acc0 = tmem_base + ((quad * 32u) << 16) + half * (BN / 2);
+            float sum[SEG ? BN / 2 : 1];   // the segments added so far (registers): the buffers alternate by segment, none waits for the epilogue
+            if (SEG) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+                for (uint32_t j = 0; j < (SEG ? BN / 2 : 1); j++) sum[j] = 0.0f;
+                bool got = true;
+#pragma unroll 1
+                for (uint32_t seg = 0; seg < kseg; seg++) {
+                    got = wait_acc();
+                    if (!got) break;
+#pragma unroll
+                    for (uint32_t c0 = 0; c0 < (uint32_t)BN / 2; c0 += 32) {
+                        uint32_t r[32];
+                        tmem_ld32(acc0 + (tc & 1u) * BN + c0, r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; j++) sum[(c0 + j) % (SEG ? BN / 2 : 1)] += __uint_as_float(r[j]);
+                    }
+                    free_acc();
                 }
-                if (c0 + 32 == (uint32_t)BN / 2) {   // this warp has read its part of the buffer: the leader's MMA thread may reuse it
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
-                }
+                if (!got) break;
+            } else if (!wait_acc()) {
+                break;
+            }
+            auto piece = [&](uint32_t c0, const uint32_t (&r)[32]) {
                 const uint32_t col = n0 + (OUT_BF16 ? (c0 & ~32u) : c0);   // first column of the staged piece
                 // a store is clipped at n in whole 16-byte units only: a ragged last piece is stored from registers
                 if (!tma_out || (col + CW > n && (n * (OUT_BF16 ? 2u : 4u)) % 16u != 0)) {
 #pragma unroll
                     for (int j = 0; j < 32; j += 16) epi_store16<EPI>(ep, row, row < m, n0 + c0 + j, reinterpret_cast<const float*>(r) + j, n, lane);
-                    continue;
+                    return;
                 }
                 const bool first_part = !OUT_BF16 || (c0 & 32u) == 0;
                 if (first_part) {   // the previous piece has been read out of the buffer
@@ -772,7 +798,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                     for (uint32_t ch = 0; ch < 8; ch++)
                         *reinterpret_cast<uint4*>(srow + ((ch ^ (lane & 7u)) << 4)) = make_uint4(r[4 * ch], r[4 * ch + 1], r[4 * ch + 2], r[4 * ch + 3]);
                 }
-                if (OUT_BF16 && first_part) continue;
+                if (OUT_BF16 && first_part) return;
                 tma_store_fence();
                 __syncwarp();
                 if (lane == 0) {
@@ -781,6 +807,24 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                         else tma_store_2d(&tmC, stage_sm, (int32_t)col, (int32_t)row0);
                     }
                     tma_store_commit();
+                }
+            };
+            if (SEG) {
+#pragma unroll
+                for (uint32_t c0 = 0; c0 < (uint32_t)BN / 2; c0 += 32) {
+                    uint32_t r[32];
+#pragma unroll
+                    for (int j = 0; j < 32; j++) r[j] = __float_as_uint(sum[(c0 + j) % (SEG ? BN / 2 : 1)]);
+                    piece(c0, r);
+                }
+            } else {
+#pragma unroll 1
+                for (uint32_t c0 = 0; c0 < (uint32_t)BN / 2; c0 += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(acc0 + (tc & 1u) * BN + c0, r);
+                    tmem_ld_wait();
+                    if (c0 + 32 == (uint32_t)BN / 2) free_acc();
+                    piece(c0, r);
                 }
             }
         }
@@ -1006,7 +1050,7 @@ static int launch_planned(cudaStream_t st, const void* a, const void* wt, const 
 }
 
 // ---- the CTA-pair kernel's launch
-template <int BN, int EPI>
+template <int BN, int EPI, bool SEG>
 static int launch_pair_cfg(cudaStream_t st, const void* a, const void* wt, const GemmEpi& ep, uint32_t m, uint32_t n, uint32_t k, uint32_t kseg) {
     using C = PairCfg<BN>;
     constexpr uint32_t OUT_BYTES = PAIR_EPI_WARPS * C::OUT_WARP_BYTES;
@@ -1019,7 +1063,7 @@ static int launch_pair_cfg(cudaStream_t st, const void* a, const void* wt, const
         AK_CUDA(cudaGetDevice(&dev));
         std::lock_guard<std::mutex> lock(device_cache_mutex());
         if (!attr_set[dev & 63]) {
-            AK_CUDA(cudaFuncSetAttribute(gemm_bf16_pair_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_PAIR));
+            AK_CUDA(cudaFuncSetAttribute(gemm_bf16_pair_kernel<BN, EPI, SEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_PAIR));
             attr_set[dev & 63] = true;
         }
     }
@@ -1033,34 +1077,29 @@ static int launch_pair_cfg(cudaStream_t st, const void* a, const void* wt, const
     if (tma_out) AK_TRY(make_tmap_2d(&tmC, ep.c, esz, n, m, (uint64_t)ep.ldc * esz, 128 / esz, 32, TMA_SWIZZLE_128B));
     const uint32_t tiles_n = cdiv(n, BN), tiles_total = tiles_n * cdiv(m, 2 * GB_M);
     const uint32_t n_pairs = tiles_total < 74 ? tiles_total : 74;   // one pair per TPC of the 148 SMs
-    return launch_k(gemm_bf16_pair_kernel<BN, EPI>, dim3(2 * n_pairs, 1, 1), dim3(PAIR_THREADS), smem, st, dim3(2, 1, 1), tmA, tmB, tmC, ep, m, n,
+    return launch_k(gemm_bf16_pair_kernel<BN, EPI, SEG>, dim3(2 * n_pairs, 1, 1), dim3(PAIR_THREADS), smem, st, dim3(2, 1, 1), tmA, tmB, tmC, ep, m, n,
                     k, stages, kseg, tiles_n, tiles_total, tma_out);
+}
+template <int BN, int EPI>
+static int launch_pair_seg(cudaStream_t st, const void* a, const void* wt, const GemmEpi& ep, uint32_t m, uint32_t n, uint32_t k, uint32_t kseg) {
+    return kseg > 1 ? launch_pair_cfg<BN, EPI, true>(st, a, wt, ep, m, n, k, kseg) : launch_pair_cfg<BN, EPI, false>(st, a, wt, ep, m, n, k, kseg);
 }
 template <int BN>
 static int launch_pair(cudaStream_t st, const void* a, const void* wt, const GemmEpi& ep, uint32_t m, uint32_t n, uint32_t k, uint32_t epi,
                        uint32_t kseg) {
     switch (epi) {
-        case AK_EPI_STORE_F32: return launch_pair_cfg<BN, AK_EPI_STORE_F32>(st, a, wt, ep, m, n, k, kseg);
-        case AK_EPI_ADD_F32: return launch_pair_cfg<BN, AK_EPI_ADD_F32>(st, a, wt, ep, m, n, k, kseg);
-        case AK_EPI_STORE_BF16: return launch_pair_cfg<BN, AK_EPI_STORE_BF16>(st, a, wt, ep, m, n, k, kseg);
-        case AK_EPI_SILU_BF16: return launch_pair_cfg<BN, AK_EPI_SILU_BF16>(st, a, wt, ep, m, n, k, kseg);
+        case AK_EPI_STORE_F32: return launch_pair_seg<BN, AK_EPI_STORE_F32>(st, a, wt, ep, m, n, k, kseg);
+        case AK_EPI_ADD_F32: return launch_pair_seg<BN, AK_EPI_ADD_F32>(st, a, wt, ep, m, n, k, kseg);
+        case AK_EPI_STORE_BF16: return launch_pair_seg<BN, AK_EPI_STORE_BF16>(st, a, wt, ep, m, n, k, kseg);
+        case AK_EPI_SILU_BF16: return launch_pair_seg<BN, AK_EPI_SILU_BF16>(st, a, wt, ep, m, n, k, kseg);
     }
     set_error("gemm_bf16: unknown epilogue %u", epi);
     return AK_ERR_INVALID_ARG;
 }
-// Large m goes to the CTA-pair kernel when its K partition is a single accumulator of 256 columns (two TMEM
-// buffers, the epilogue of a tile overlapped with the next tile's MMAs).
-static bool pair_plan(uint32_t m, uint32_t n, uint32_t k, bool allow_split, bool invariant, uint32_t& bn, uint32_t& kseg) {
+// Large m goes to the CTA-pair kernel, with the K partition of the skinny launch where the bits have to be the same.
+static bool pair_plan(uint32_t m, uint32_t n, uint32_t k, bool allow_split, bool invariant, uint32_t& kseg) {
     if (m < 1024 || n < 256) return false;
-    kseg = 1;
-    if (invariant && allow_split) {
-        // With K split in two segments of 256 columns the accumulators fill TMEM, the epilogue is exposed and the
-        // kernel is no faster than the one-CTA kernel (measured on the 1.4B prefill: 12.0 s against 11.9 s): only
-        // unsplit K partitions go to the pair kernel. (The kernel itself handles kseg = 2 with a single buffer.)
-        const GemmPlan sk = plan_gemm(GB_M, n, k, true, false);
-        if (sk.ks > 1) return false;
-    }
-    bn = 256;
+    kseg = invariant && allow_split ? plan_gemm(GB_M, n, k, true, false).ks : 1;
     return true;
 }
 
@@ -1082,8 +1121,8 @@ int launch_gemm_bf16(cudaStream_t st, const void* a, const void* wt, void* c, ui
     ep.ldc = ldc ? ldc : n;
     // the split-K exchange stores 4-column groups: it needs 4-aligned rows
     const bool allow_split = (ep.ldc % 4) == 0;
-    uint32_t pbn = 0, pkseg = 1;
-    if (pair_plan(m, n, k, allow_split, invariant, pbn, pkseg)) return launch_pair<256>(st, a, wt, ep, m, n, k, epilogue, pkseg);
+    uint32_t pkseg = 1;
+    if (pair_plan(m, n, k, allow_split, invariant, pkseg)) return launch_pair<256>(st, a, wt, ep, m, n, k, epilogue, pkseg);
     return launch_planned(st, a, wt, ep, m, n, k, epilogue, plan_gemm(m, n, k, allow_split, invariant));
 }
 

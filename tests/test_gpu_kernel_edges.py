@@ -159,3 +159,25 @@ def test_attn_prefill_many_items(ak, torch_cuda, heads, hd, q_scale):
         run(q[rows_i].contiguous(), tables[i:i + 1].contiguous(), np.array([0, L], np.int32), alone, 1, L)
         assert torch.equal(alone, out[rows_i]), (i, L)
     ak.check(ak.lib().ak_check_device_status(None))
+
+
+# Prompts of 1024 rows and more (the CTA-pair kernel, its K segmented as the skinny launches split it) give the tokens that they
+# give when they are prefilled in chunks beside a decoding sequence (skinny launches): the row's sums have the same bits.
+@pytest.mark.parametrize("dim,heads,ffn", [(320, 5, 1280), (768, 12, 3072), (2048, 16, 8192)])
+def test_gemm_pair_segments(ak, ctx, dim, heads, ffn):
+    cfg = ak.ModelConfig(1000, dim, heads, 2, 2048, ffn)
+    w = ak.ModelWeights(ctx, cfg, ak.AK_BF16)
+    w.init_synthetic(7, 0.05)
+    prompts = [ak.uniform_tokens(n, 1000, seed=n) for n in (3, 1024, 1290)]
+    out = []
+    for chunk in (0, 100):
+        e = ak.Engine(ctx, w, max_seqs=3, max_seq_len=1400, prefill_chunk_rows=chunk)
+        ids = [e.submit(prompts[0], 1400)]
+        e.step()
+        ids += [e.submit(p, p.size + 40) for p in prompts[1:]]
+        e.run_to_completion()
+        out.append([e.poll(i)[0].tolist()[:200] for i in ids])
+        e.close()
+    assert out[0] == out[1]
+    ctx.check_device_status()
+    w.close()
