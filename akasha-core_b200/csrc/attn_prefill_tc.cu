@@ -81,12 +81,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
         : "r"(taddr)
         : "memory");
 }
-// one lane of a converged warp
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ float ex2(float x) {   // 2^x, hardware approximation (2 ulp), ex2(-inf) = 0
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

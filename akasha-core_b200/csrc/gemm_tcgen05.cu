@@ -304,7 +304,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint8_t* const b_base = smem + (size_t)stages * a_bytes;
     const uint32_t overrun = (GB_M - a_rows) * (GB_K * 2), b_total = stages * C::B_BYTES;
     float* red = reinterpret_cast<float*>(b_base + b_total + (overrun > b_total ? overrun - b_total : 0u));  // used when ks > 1
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t m0 = blockIdx.y * GB_M, n0 = blockIdx.x * BN;
     const uint32_t num_kb_total = (k + GB_K - 1) / GB_K;
     const uint32_t per = (num_kb_total + ks - 1) / ks;
@@ -373,29 +373,31 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer (one thread)
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(GB_M, BN);
-            const uint32_t per_seg = (num_kb + kseg - 1) / kseg;
-            uint32_t s = 0, ph = 0, in_seg = 0, acc_col = tmem_base;   // carried (no division in the loop, see the producer)
-            for (uint32_t i = 0; i < num_kb; i++) {
-                if (!mbar_wait(&full_bar[s], ph)) { atomicExch(&fail_flag, 2u); break; }
-                tc_fence_after();
-                const uint32_t a_addr = smem_u32(smem + (size_t)s * a_bytes);
-                const uint32_t b_addr = smem_u32(b_base + (size_t)s * C::B_BYTES);
-                const uint64_t da = make_smem_desc(a_addr), db = make_smem_desc(b_addr);
+        // ---------------- MMA issuer. The warp stays converged and its operands are warp-uniform: descriptors and loop state live
+        // in uniform registers. With one lane alone in the branch an MMA took ~100 cycles to issue, 0.2 us per K block.
+        constexpr uint32_t idesc = make_idesc(GB_M, BN);
+        const uint32_t per_seg = (num_kb + kseg - 1) / kseg;
+        uint32_t s = 0, ph = 0, in_seg = 0, acc_col = tmem_base;   // carried (no division in the loop, see the producer)
+        const uint64_t da0 = make_smem_desc(smem_u32(smem)), db0 = make_smem_desc(smem_u32(b_base));
+        const uint32_t da_step = a_bytes >> 4;
+        for (uint32_t i = 0; i < num_kb; i++) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], ph))) { if (lane == 0) atomicExch(&fail_flag, 2u); break; }
+            tc_fence_after();
+            const uint64_t da = da0 + s * da_step, db = db0 + s * (uint32_t)(C::B_BYTES >> 4);
+            if (elect_one()) {
 #pragma unroll
                 for (uint32_t kk = 0; kk < GB_K / 16; kk++) {
                     // advance 16 bf16 = 32 bytes along K inside the swizzle row: +2 in the address field
                     tc_mma_f16(acc_col, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (in_seg == 0 && kk == 0) ? 0u : 1u);
                 }
                 if (num_kb > stages) tc_commit(&empty_bar[s]);  // stage reusable once these MMAs have read it (nobody waits when the ring holds the whole K range)
-                if (++s == stages) { s = 0; ph ^= 1u; }
-                if (++in_seg == per_seg) { in_seg = 0; acc_col += BN; }
+                if (i + 1 == num_kb) tc_commit(&acc_bar);       // accumulator complete
             }
-            if (num_kb > 0) tc_commit(&acc_bar);  // accumulator complete
-            else mbar_arrive(&acc_bar);           // nothing to accumulate: this CTA contributes zeros
+            __syncwarp();
+            if (++s == stages) { s = 0; ph ^= 1u; }
+            if (++in_seg == per_seg) { in_seg = 0; acc_col += BN; }
         }
+        if (num_kb == 0 && lane == 0) mbar_arrive(&acc_bar);    // nothing to accumulate: this CTA contributes zeros
     }
 
     // ---------------- epilogue warps 2..5: thread <-> accumulator row (TMEM lane)
@@ -617,7 +619,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     __shared__ uint32_t fail_flag;
 
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();          // 0 = leader (issues the MMAs), 1 = peer
     const uint32_t pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const uint32_t num_kb = (k + GB_K - 1) / GB_K;
@@ -676,12 +678,16 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer: one thread of the leader CTA drives both SMs' tensor cores
-        if (lane == 0 && rank == 0) {
+        // ---------------- MMA issuer: one thread of the leader CTA drives both SMs' tensor cores (from a converged warp, see the
+        // one-CTA kernel)
+        if (rank == 0) {
             constexpr uint32_t idesc = make_idesc(2 * GB_M, BN);
             const uint32_t per_seg = SEG ? (num_kb + kseg - 1) / kseg : num_kb;
             uint32_t tc = 0, s = 0, ph = 0;   // accumulations (a tile's, or a segment's) so far; ring position and phase are carried: no division in the K loop
             bool ok = true;
+            const uint64_t d0 = make_smem_desc(smem_u32(smem));
+            const uint32_t empty0 = map_to_cta(smem_u32(&empty_bar[0]), 0), empty1 = map_to_cta(smem_u32(&empty_bar[0]), 1);
+            const uint32_t acc_full0 = map_to_cta(smem_u32(&acc_full[0]), 0), acc_full1 = map_to_cta(smem_u32(&acc_full[0]), 1);
             for (uint32_t t = pair; t < tiles_total && ok; t += n_pairs) {
                 uint32_t in_seg = 0, acc_col = 0, buf = 0;
                 for (uint32_t kb = 0; kb < num_kb; kb++) {
@@ -689,26 +695,33 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                         buf = tc & 1u;
                         acc_col = tmem_base + buf * BN;
                         // the epilogue warps of both CTAs have drained this buffer (it was last used two accumulations ago)
-                        if (tc >= 2 && !mbar_wait(&acc_empty[buf], ((tc >> 1) & 1u) ^ 1u)) { atomicExch(&fail_flag, 4u); ok = false; break; }
+                        if (tc >= 2 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((tc >> 1) & 1u) ^ 1u))) {
+                            if (lane == 0) atomicExch(&fail_flag, 4u);
+                            ok = false;
+                            break;
+                        }
                         tc_fence_after();
                     }
-                    if (!mbar_wait(&full_bar[s], ph)) { atomicExch(&fail_flag, 2u); ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], ph))) { if (lane == 0) atomicExch(&fail_flag, 2u); ok = false; break; }
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + (size_t)s * C::STAGE_BYTES);
-                    const uint64_t da = make_smem_desc(a_addr), db = make_smem_desc(a_addr + C::A_BYTES);
+                    const uint64_t da = d0 + s * (uint32_t)(C::STAGE_BYTES >> 4), db = da + (uint32_t)(C::A_BYTES >> 4);
+                    const bool last = in_seg + 1 == per_seg || kb + 1 == num_kb;
+                    if (elect_one()) {
 #pragma unroll
-                    for (uint32_t kk = 0; kk < GB_K / 16; kk++)
-                        tc_mma2_f16(acc_col, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (in_seg == 0 && kk == 0) ? 0u : 1u);
-                    // the stage is reusable in BOTH CTAs once these MMAs have read it
-                    tc_commit2(map_to_cta(smem_u32(&empty_bar[s]), 0));
-                    tc_commit2(map_to_cta(smem_u32(&empty_bar[s]), 1));
-                    if (++s == stages) { s = 0; ph ^= 1u; }
-                    if (++in_seg == per_seg || kb + 1 == num_kb) {
-                        tc_commit2(map_to_cta(smem_u32(&acc_full[buf]), 0));
-                        tc_commit2(map_to_cta(smem_u32(&acc_full[buf]), 1));
-                        in_seg = 0;
-                        tc++;
+                        for (uint32_t kk = 0; kk < GB_K / 16; kk++)
+                            tc_mma2_f16(acc_col, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (in_seg == 0 && kk == 0) ? 0u : 1u);
+                        // the stage is reusable in BOTH CTAs once these MMAs have read it
+                        tc_commit2(empty0 + s * 8);
+                        tc_commit2(empty1 + s * 8);
+                        if (last) {
+                            tc_commit2(acc_full0 + buf * 8);
+                            tc_commit2(acc_full1 + buf * 8);
+                        }
                     }
+                    __syncwarp();
+                    if (++s == stages) { s = 0; ph ^= 1u; }
+                    in_seg++;
+                    if (last) { in_seg = 0; tc++; }
                 }
             }
         }
