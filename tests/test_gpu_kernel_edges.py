@@ -181,3 +181,19 @@ def test_gemm_pair_segments(ak, ctx, dim, heads, ffn):
     assert out[0] == out[1]
     ctx.check_device_status()
     w.close()
+
+
+# a few long rows: a block per row (up to 148 rows), the warp-per-row kernel above; the same bits on both sides
+@pytest.mark.parametrize("size", [1028, 1536, 2048, 4096])
+def test_rmsnorm_wide(ak, torch_cuda, size):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(size)
+    x = torch.randn(149, size, device="cuda", generator=g)
+    w = 1.0 + 0.1 * torch.randn(size, device="cuda", generator=g)
+    y = [torch.empty(149, size, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    ak.ops.rmsnorm_rope_residual(x, None, w, y[0], None, 149, size, 1e-5, 0, ak.AK_BF16)
+    for r0, n in ((0, 1), (1, 148)):
+        ak.ops.rmsnorm_rope_residual(x[r0:], None, w, y[1][r0:], None, n, size, 1e-5, 0, ak.AK_BF16)
+    assert torch.equal(y[0], y[1])
+    want = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    assert float(((y[1].double() - want).abs() / (want.abs() + 1e-6)).max()) < 2 ** -8   # one rounding to bf16
