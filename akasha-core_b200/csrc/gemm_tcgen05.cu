@@ -973,15 +973,13 @@ static GemmPlan plan_gemm(uint32_t m, uint32_t n, uint32_t k, bool allow_split, 
     for (int bi = 0; bi < 3; bi++)
         for (int ki = 0; ki < 4; ki++) {
             const uint32_t bn = bns[bi], ks = kss[ki];
-            // One MMA (M = 128 or 64, K = 16) occupies the tensor core 50 cycles for any N <= 64 (64 cycles at
-            // N = 128, 128 at N = 256), and the issuing thread needs ~0.2 us per K block (wait, four MMAs, commit),
-            // so a CTA's main loop costs the same however narrow its tile; a cluster exchange costs ~1.2 us, the
-            // boundary to the next launch ~2 us. Split long K chains (K > 1024), and
-            // short ones four ways only when the unsplit grid would cover less than half of the SMs.
-            // Other short chains are halved at most (two accumulators still leave 256-column tiles to
-            // the large-m plan) and only with tiles of 32 columns or more per exchange.
+            // A launch in a chain costs ~3 us whatever it computes, a K block ~0.15 us (one MMA of M = 128 or 64 and K = 16
+            // occupies the tensor core 50 cycles for any N <= 64), a cluster exchange ~1.2 us. Split long K chains (K > 1024),
+            // and short ones only when the unsplit grid would cover less than half of the SMs. Measured in a chain of
+            // launches: 64 x 2304 x 768 4.4 us unsplit (144 CTAs of 16 columns), 5.6 us in two halves; 8 x 1280 x 320 3.1
+            // against 4.3 us; 8 x 768 x 768 3.4 us split four ways, 5.2 us unsplit.
             const bool short_k_ok = cdiv(n, 16) * 2 <= B200_SMS;
-            if (ks > 1 && num_kb <= 16 && !short_k_ok && (ks > 2 || bn < 32)) continue;
+            if (ks > 1 && num_kb <= 16 && !short_k_ok) continue;
             if (ks > 1 && (!allow_split || ks * 2 > num_kb || (bn / ks) % 4 != 0)) continue;
             const uint32_t per = cdiv(num_kb, ks);
             if (ks > 1 && (ks - 1) * per >= num_kb) continue;  // every CTA of the cluster gets work
