@@ -46,6 +46,12 @@ thread_local bool g_attn_early = false;
 constexpr int DEC_WARPS = 4;
 constexpr int DEC_BS = 16;          // positions per KV block
 constexpr int DEC_MIN_BLOCKS = 4;   // a split never gets fewer KV blocks than this (one per warp)
+// Sequences of up to this many blocks stay in one CTA: four blocks per warp cost less than publishing, counting and merging
+// partials. Decode step of the 162M model, 8 sequences: 399 us unsplit against 415 us at 200 positions, 437 against 423 at 440.
+constexpr uint32_t DEC_UNSPLIT_BLOCKS = 16;
+// ... and a launch that would have to clear the arrival counters first (another ~2.5 us on the stream) splits later still: one
+// sequence x 12 heads, clearing included, 8.2 us unsplit against 10.1 us at 512 positions, 11.7 against 10.3 at 800.
+constexpr uint32_t DEC_UNSPLIT_BLOCKS_CLEAR = 40;
 constexpr int DEC_MAX_SPLITS = 32;
 
 template <typename T, int HD, int ST> struct DecCfg {
@@ -122,6 +128,7 @@ struct DecFused {
 __device__ __forceinline__ void split_plan(uint32_t nblk, uint32_t n_splits, uint32_t& n_act, uint32_t& bps) {
     n_act = (nblk + DEC_MIN_BLOCKS - 1) / DEC_MIN_BLOCKS;
     if (n_act > n_splits) n_act = n_splits;
+    if (nblk <= DEC_UNSPLIT_BLOCKS) n_act = 1;
     if (n_act < 1) n_act = 1;
     bps = (nblk + n_act - 1) / n_act;
     if (bps) n_act = (nblk + bps - 1) / bps;
@@ -219,11 +226,11 @@ attn_decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int32_t* table = block_tables + (size_t)row * max_blocks;
     // Lane j holds the block-table entry of this warp's j-th tile (the first 32 tiles of a warp: 2048 positions), so
-    // no table read sits between the end of one tile and the request for the next. Unsplit launches know which
-    // entries those are without the length: they are fetched together with it (one memory latency instead of two
+    // no table read sits between the end of one tile and the request for the next. Where the sequence is not split
+    // those entries are known without the length: they are fetched together with it (one memory latency instead of two
     // before the first tile can be requested). Entries past the sequence's end are never used.
     uint32_t my_blk = 0;
-    if (n_splits == 1 && warp + lane * DEC_WARPS < max_blocks) my_blk = (uint32_t)table[warp + lane * DEC_WARPS];
+    if (split == 0 && warp + lane * DEC_WARPS < max_blocks) my_blk = (uint32_t)table[warp + lane * DEC_WARPS];
     const int32_t kv_len = kv_lens[row];
 
     // block range of this split
@@ -266,7 +273,7 @@ attn_decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     // known to be complete
     const uint32_t pre = nmine < (uint32_t)C::STAGES ? nmine : (uint32_t)C::STAGES;
     bool deferred = false;
-    if (n_splits != 1 && lane < nmine) my_blk = (uint32_t)table[first + lane * DEC_WARPS];
+    if (n_act != 1 && lane < nmine) my_blk = (uint32_t)table[first + lane * DEC_WARPS];
     // physical block of this warp's j-th tile (j warp-uniform)
     auto blk_of = [&](uint32_t j) { return j < 32 ? __shfl_sync(0xffffffffu, my_blk, j) : (uint32_t)table[first + j * DEC_WARPS]; };
     if (lane < pre) {
@@ -653,12 +660,13 @@ static uint32_t wave_slots(uint32_t head_dim, uint32_t kv_dtype, uint32_t stages
     if (per_sm < 1) per_sm = 1;
     return B200_SMS * per_sm;
 }
-uint32_t attn_decode_pick_splits(uint32_t rows, uint32_t heads, uint32_t head_dim, uint32_t kv_dtype, uint32_t max_kv_len) {
+uint32_t attn_decode_pick_splits(uint32_t rows, uint32_t heads, uint32_t head_dim, uint32_t kv_dtype, uint32_t max_kv_len, bool counters_are_zero) {
     const uint64_t items = (uint64_t)rows * heads;
     if (items == 0) return 1;
     const uint32_t st = DEC_STAGES;
     const uint32_t room = (uint32_t)(wave_slots(head_dim, kv_dtype, st) / items);   // CTAs per item that keep one wave
     const uint32_t max_blocks = (max_kv_len + DEC_BS - 1) / DEC_BS;
+    if (max_blocks <= (counters_are_zero ? DEC_UNSPLIT_BLOCKS : DEC_UNSPLIT_BLOCKS_CLEAR)) return 1;
     uint32_t want = (max_blocks + DEC_WARPS * st - 1) / (DEC_WARPS * st);           // every warp at most one ring of blocks
     if (want > room) want = room;
     if (want > DEC_MAX_SPLITS) want = DEC_MAX_SPLITS;
@@ -777,7 +785,8 @@ static int launch_decode(cudaStream_t st, const void* q, const void* k_pool, con
         }
         return AK_OK;
     }
-    const uint32_t n_splits = p.n_splits ? p.n_splits : attn_decode_pick_splits(p.rows, p.heads, p.head_dim, p.kv_dtype, p.max_blocks_per_seq * DEC_BS);
+    const uint32_t n_splits =
+        p.n_splits ? p.n_splits : attn_decode_pick_splits(p.rows, p.heads, p.head_dim, p.kv_dtype, p.max_blocks_per_seq * DEC_BS, counters_are_zero);
     AK_REQUIRE(n_splits <= DEC_MAX_SPLITS, AK_ERR_INVALID_ARG, "attn_decode_paged: n_splits must be at most %d", DEC_MAX_SPLITS);
     AK_REQUIRE(n_splits == 1 || scratch, AK_ERR_INVALID_ARG, "attn_decode_paged: scratch required when n_splits > 1");
     if (n_splits > 1 && !counters_are_zero) {
@@ -805,7 +814,7 @@ using namespace ak;
 extern "C" {
 size_t ak_attn_decode_scratch_bytes(const ak_attn_decode_params* p) {
     if (!p) return 0;
-    uint32_t ns = p->n_splits ? p->n_splits : attn_decode_pick_splits(p->rows, p->heads, p->head_dim, p->kv_dtype, p->max_blocks_per_seq * DEC_BS);
+    uint32_t ns = p->n_splits ? p->n_splits : attn_decode_pick_splits(p->rows, p->heads, p->head_dim, p->kv_dtype, p->max_blocks_per_seq * DEC_BS, false);
     return attn_decode_scratch_bytes(p->rows, p->heads, p->head_dim, ns);
 }
 int ak_attn_decode_paged(void* stream, const void* q, const void* k_pool, const void* v_pool, const int32_t* block_tables,
@@ -862,7 +871,7 @@ size_t ak_attn_decode_noalloc_max_scratch_bytes(void) { return AK_NOALLOC_SCRATC
 int ak_attn_decode_paged_noalloc(void* stream, const void* q, const void* k_pool, const void* v_pool,
                                  const int32_t* block_tables, const int32_t* kv_lens, void* out, ak_attn_decode_params p) {
     AK_REQUIRE(q && k_pool && v_pool && block_tables && kv_lens && out, AK_ERR_INVALID_ARG, "ak_attn_decode_paged_noalloc: null pointer");
-    const uint32_t ns = p.n_splits ? p.n_splits : attn_decode_pick_splits(p.rows, p.heads, p.head_dim, p.kv_dtype, p.max_blocks_per_seq * DEC_BS);
+    const uint32_t ns = p.n_splits ? p.n_splits : attn_decode_pick_splits(p.rows, p.heads, p.head_dim, p.kv_dtype, p.max_blocks_per_seq * DEC_BS, false);
     const size_t need = attn_decode_scratch_bytes(p.rows, p.heads, p.head_dim, ns);
     AK_REQUIRE(need <= AK_NOALLOC_SCRATCH_BYTES, AK_ERR_UNSUPPORTED,
                "ak_attn_decode_paged_noalloc: %zu bytes of split partials and arrival counters exceed the built-in "

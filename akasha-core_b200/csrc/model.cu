@@ -658,7 +658,7 @@ int Runner::run(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_pf_len
     // One split count per runner (from the longest sequence it can hold): eager and captured
     // steps then sum in the same order, so a sequence's tokens do not depend on its neighbours.
     (void)max_kv_len;
-    const uint32_t n_splits = attn_decode_pick_splits(max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, max_seq_len_);
+    const uint32_t n_splits = attn_decode_pick_splits(max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, max_seq_len_, true);
     int rc = launch_layers(T, n_prefill_rows, n_pf_seqs, max_pf_len, any_decode, n_splits, false);
     if (rc) return rc;
     AK_CUDA(cudaMemcpyAsync(h_sampled_, d_sampled_, (size_t)max_seqs_ * 4, cudaMemcpyDeviceToHost, st));
@@ -703,7 +703,7 @@ int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_
     const uint64_t key = ((uint64_t)bank_ << 63) | ((uint64_t)rows_b << 32) | seqs_b;  // a graph bakes its bank's host buffers and events
     const uint32_t T = max_seqs_ + rows_b;
     const size_t bytes = ((size_t)d_.rows + (size_t)T * 4) * 4;
-    const uint32_t n_splits = attn_decode_pick_splits(max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, max_seq_len_);
+    const uint32_t n_splits = attn_decode_pick_splits(max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, max_seq_len_, true);
     auto it = graphs_.find(key);
     if (it == graphs_.end()) {
         // one eager pass first (sets kernel attributes, surfaces faults outside capture); it IS this step
