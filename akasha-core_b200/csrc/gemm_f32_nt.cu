@@ -7,7 +7,7 @@
 // it, so K is split over a thread-block cluster and the partial tiles are added through distributed shared memory in rank
 // order. The split is a function of (n, k) only: a row's sum does not depend on how many rows share the launch.
 // The 64 x 64 tile with 4 x 4 outputs per thread it replaces moved a shared-memory word for every two FMAs:
-// 512 x 2304 x 768 took 126 us with it, 70 us here (timed launch by launch).
+// 512 x 2304 x 768 took 126 us with it; a 512-token prefill of the 162M model 9.67 ms, 4.10 ms here.
 // m == 1 is a GEMV: a warp per output, the weights streamed once with 128-bit loads.
 #include <cooperative_groups.h>
 
@@ -20,9 +20,11 @@ namespace ntf32 {
 
 constexpr int BM = 64, BN = 128, BK = 16, THREADS = 128;
 
+// Row k of a tile starts 8 (k / 4) floats late: the transposing stores of 8 rows x 4 k groups fall into 32 banks.
+__device__ __host__ constexpr uint32_t at(uint32_t k, uint32_t width) { return k * width + 8 * (k >> 2); }
 struct Tiles {
-    float a[2][BK][BM + 4];
-    float b[2][BK][BN + 4];
+    float a[2][at(BK, BM)];
+    float b[2][at(BK, BN)];
 };
 union Smem {
     Tiles t;
@@ -54,7 +56,7 @@ __device__ __forceinline__ float4 load4(const float* __restrict__ p, uint32_t ro
 }
 
 template <bool SCALAR>
-__global__ void __launch_bounds__(THREADS, 4)
+__global__ void __launch_bounds__(THREADS, 3)
 gemm_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ c, uint32_t m, uint32_t n, uint32_t k, uint32_t flags) {
     __shared__ __align__(16) Smem sm;
     cg::cluster_group cluster = cg::this_cluster();
@@ -64,24 +66,28 @@ gemm_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __r
     const uint32_t per = ((k + BK - 1) / BK + ks - 1) / ks * BK;
     const uint32_t k_begin = min(rank * per, k), k_end = min(k_begin + per, k);
 
+    // Four lanes read the 64 bytes of a row that a K block has (a lane per row instead: 32 sectors per load, and the L1 was busier
+    // than the FMA pipe). The tiles are K-major.
+    const uint32_t lr = t >> 2, lq = t & 3;
     float4 ra[2], rb[4];
     auto fetch_b = [&](uint32_t k0) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) rb[i] = load4<SCALAR>(w, n0 + t, n, k0 + 4 * i, k_end, k);
+        for (int i = 0; i < 4; i++) rb[i] = load4<SCALAR>(w, n0 + lr + 32 * i, n, k0 + 4 * lq, k_end, k);
     };
     auto fetch_a = [&](uint32_t k0) {
 #pragma unroll
-        for (int i = 0; i < 2; i++) ra[i] = load4<SCALAR>(a, m0 + (t & 63), m, k0 + 4 * ((t >> 6) + 2 * i), k_end, k);
+        for (int i = 0; i < 2; i++) ra[i] = load4<SCALAR>(a, m0 + lr + 32 * i, m, k0 + 4 * lq, k_end, k);
     };
     auto put = [&](uint32_t buf) {
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            const uint32_t kq = ((t >> 6) + 2 * i) * 4, r = t & 63;
-            sm.t.a[buf][kq][r] = ra[i].x; sm.t.a[buf][kq + 1][r] = ra[i].y; sm.t.a[buf][kq + 2][r] = ra[i].z; sm.t.a[buf][kq + 3][r] = ra[i].w;
+            float* d = &sm.t.a[buf][at(4 * lq, BM) + lr + 32 * i];
+            d[0] = ra[i].x; d[BM] = ra[i].y; d[2 * BM] = ra[i].z; d[3 * BM] = ra[i].w;
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            sm.t.b[buf][4 * i][t] = rb[i].x; sm.t.b[buf][4 * i + 1][t] = rb[i].y; sm.t.b[buf][4 * i + 2][t] = rb[i].z; sm.t.b[buf][4 * i + 3][t] = rb[i].w;
+            float* d = &sm.t.b[buf][at(4 * lq, BN) + lr + 32 * i];
+            d[0] = rb[i].x; d[BN] = rb[i].y; d[2 * BN] = rb[i].z; d[3 * BN] = rb[i].w;
         }
     };
 
@@ -103,9 +109,10 @@ gemm_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __r
         if (more) { fetch_a(k0 + BK); fetch_b(k0 + BK); }
 #pragma unroll
         for (int kk = 0; kk < BK; kk++) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&sm.t.a[buf][kk][ty * 8]), a1 = *reinterpret_cast<const float4*>(&sm.t.a[buf][kk][ty * 8 + 4]);
-            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&sm.t.b[buf][kk][tx * 4]);
-            const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&sm.t.b[buf][kk][64 + tx * 4]);
+            const float* const ar = &sm.t.a[buf][at(kk, BM) + ty * 8];
+            const float* const br = &sm.t.b[buf][at(kk, BN) + tx * 4];
+            const float4 a0 = *reinterpret_cast<const float4*>(ar), a1 = *reinterpret_cast<const float4*>(ar + 4);
+            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(br), b1 = *reinterpret_cast<const ulonglong2*>(br + 64);
             const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
             for (int i = 0; i < 8; i++) {
@@ -212,11 +219,11 @@ int launch_gemm_f32_nt(cudaStream_t st, const float* a, const float* wt, float* 
         const uint32_t ctas = cdiv(n, GV_WARPS), room = B200_SMS * 8;
         return launch_k(gemv_kernel, dim3(ctas < room ? ctas : room), dim3(GV_WARPS * 32), 0, st, NO_CLUSTER, a, wt, c, n, k, flags, (uint32_t)vec);
     }
-    // Four CTAs share an SM: 592 are one wave. K is split so that 512 rows (8 row tiles) just fit it, 74 CTAs for every row
-    // tile (512 x 3072 x 768: three-way, 576 CTAs; four-way would be 768, a wave and a third), and a prompt of 64 tokens
-    // occupies half of the SMs. Never less than 64 of K per CTA.
+    // K is split so that one row tile (a prompt of up to 64 tokens) occupies every SM, at most eight ways (a portable cluster),
+    // never less than 64 of K per CTA. More rows queue up behind each other, three CTAs to an SM. Prefill of the 162M model
+    // with 74 / 111 / 148 CTAs per row tile: 64 tokens 1149 / 1058 / 1087 us, 201 2330 / 2424 / 2222, 512 4187 / 4099 / 4096.
     const uint32_t tn = cdiv(n, BN);
-    uint32_t ks = 74 / tn;
+    uint32_t ks = B200_SMS / tn;
     if (ks > 8) ks = 8;
     if (ks > k / 64) ks = k / 64;
     if (ks < 1) ks = 1;

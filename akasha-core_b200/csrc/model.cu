@@ -563,7 +563,8 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
             AK_CUDA(cudaEventRecord(ev_join_, st2_));
             AK_CUDA(cudaStreamWaitEvent(st, ev_join_, 0));
         } else {
-            rc = range(st, 0, T, any_decode, true);
+            // without a decode row the prompt rows go alone: 512 of them are 8 row tiles of a projection, 513 would be 9
+            rc = any_decode || T <= max_seqs_ ? range(st, 0, T, any_decode, true) : range(st, max_seqs_, T - max_seqs_, false, true);
             if (rc) return rc;
         }
     } else {

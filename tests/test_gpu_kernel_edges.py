@@ -197,3 +197,35 @@ def test_rmsnorm_wide(ak, torch_cuda, size):
     assert torch.equal(y[0], y[1])
     want = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * w.double()
     assert float(((y[1].double() - want).abs() / (want.abs() + 1e-6)).max()) < 2 ** -8   # one rounding to bf16
+
+
+# The automatic division of a sequence: whole up to 256 positions (640 where counters have to be cleared), else, with few
+# sequences, in pieces of at least 4 blocks.
+@pytest.mark.parametrize("rows,heads,hd,dtype,lens", [
+    (1, 12, 64, 1, (1, 255, 256, 257, 639, 640, 641, 900)),
+    (3, 5, 64, 0, (256, 257, 700)),
+    (2, 16, 128, 1, (1, 1024, 1025, 2100)),
+])
+def test_attn_decode_auto_splits(ak, torch_cuda, rows, heads, hd, dtype, lens):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    mx = max(lens)
+    mb = (mx + 15) // 16
+    tdt = torch.bfloat16 if dtype else torch.float32
+    kp, vp = (torch.randn(rows * mb, heads, 16, hd, device="cuda", generator=g).to(tdt) for _ in range(2))
+    tables = torch.randperm(rows * mb, device="cuda", generator=g).to(torch.int32).reshape(rows, mb)
+    q = torch.randn(rows, heads * hd, device="cuda", generator=g).to(tdt)
+    for step in range(len(lens) if rows == 1 else 1):
+        kv = [lens[(r + step) % len(lens)] for r in range(rows)]
+        out = torch.empty_like(q)
+        scratch = torch.full((ak.ops.attn_decode_scratch_bytes(rows, heads, hd, mb, 0, dtype) + 16,), 255, device="cuda", dtype=torch.uint8)
+        ak.ops.attn_decode_paged(q, kp, vp, tables, torch.tensor(kv, dtype=torch.int32, device="cuda"), out, rows, heads, hd, mb, hd ** -0.5, dtype, 0,
+                                 rows * mb, scratch)
+        ak.check(ak.lib().ak_check_device_status(None))
+        for r in range(min(rows, 8)):
+            k, v = (p[tables[r].long()].transpose(1, 2).reshape(mb * 16, heads, hd)[:kv[r]].double().transpose(0, 1) for p in (kp, vp))
+            s = torch.einsum("hd,hkd->hk", q[r].double().reshape(heads, hd), k) * hd ** -0.5
+            want = torch.einsum("hk,hkd->hd", s.softmax(-1), v).reshape(-1)
+            # bf16: P rounded on both sides of the quotient, the output once; f32: sums of a few hundred terms
+            tol = ((2 ** -8 + 2 ** -9) if dtype else 1e-5) * float(v.abs().max())
+            assert float((out[r].double() - want).abs().max()) < tol, (r, kv[r])
