@@ -11,27 +11,29 @@ constexpr int PF_BK = 64, PF_THREADS = 256, PF_BS = 16;
 
 // RPT = query rows per thread: the query tile is 16*RPT rows. RPT = 4 (64-row tiles) has the best
 // FMA-to-shared-load ratio; RPT = 1 (16-row tiles) makes four times as many CTAs, which is what a
-// single short prompt joining a decode batch needs to occupy the machine.
+// single short prompt needs to occupy the machine. What bounds a single prompt is the chain of key tiles of its last rows.
+// Row d of K^T starts 8 (d / 4) floats late: the transposing stores of 8 keys x 4 chunks fall into 32 banks.
+__device__ __host__ constexpr int pf_kt(int d) { return d * PF_BK + 8 * (d >> 2); }
 template <typename T, int HD, int RPT> struct PfSmem {
     static constexpr int BQ = 16 * RPT;
     float qt[HD][BQ + 4];   // Q^T
-    float kt[HD][PF_BK + 4];   // K^T
+    float kt[pf_kt(HD)];    // K^T
     float vs[PF_BK][HD + 4];   // V
     float pt[PF_BK][BQ + 4];  // P^T
 };
 
-template <typename T> __device__ __forceinline__ void load_chunk(const T* src, float* out);
-template <> __device__ __forceinline__ void load_chunk<float>(const float* src, float* out) {
-    float4 v = *reinterpret_cast<const float4*>(src);
-    out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
+// 16 bytes of T as floats
+template <typename T> __device__ __forceinline__ void expand(const uint4& raw, float* out);
+template <> __device__ __forceinline__ void expand<float>(const uint4& raw, float* out) {
+    out[0] = __uint_as_float(raw.x); out[1] = __uint_as_float(raw.y); out[2] = __uint_as_float(raw.z); out[3] = __uint_as_float(raw.w);
 }
-template <> __device__ __forceinline__ void load_chunk<bf16>(const bf16* src, float* out) {
-    uint4 raw = *reinterpret_cast<const uint4*>(src);
+template <> __device__ __forceinline__ void expand<bf16>(const uint4& raw, float* out) {
     out[0] = __uint_as_float(raw.x << 16); out[1] = __uint_as_float(raw.x & 0xffff0000u);
     out[2] = __uint_as_float(raw.y << 16); out[3] = __uint_as_float(raw.y & 0xffff0000u);
     out[4] = __uint_as_float(raw.z << 16); out[5] = __uint_as_float(raw.z & 0xffff0000u);
     out[6] = __uint_as_float(raw.w << 16); out[7] = __uint_as_float(raw.w & 0xffff0000u);
 }
+template <typename T> __device__ __forceinline__ void load_chunk(const T* src, float* out) { expand<T>(*reinterpret_cast<const uint4*>(src), out); }
 
 // grid: (q tiles, heads, sequences). PAGED: k/v are pools + block table; else contiguous rows.
 template <typename T, int HD, bool PAGED, int RPT>
@@ -49,7 +51,7 @@ attn_prefill_kernel(const T* __restrict__ q, const T* __restrict__ kbase, const 
     constexpr int PF_BQ = 16 * RPT;
     PfSmem<T, HD, RPT>& sm = *reinterpret_cast<PfSmem<T, HD, RPT>*>(smem_raw);
 
-    const uint32_t seq = blockIdx.z, h = blockIdx.y, qtile = blockIdx.x;
+    const uint32_t seq = blockIdx.z, h = blockIdx.y, qtile = gridDim.x - 1 - blockIdx.x;   // the last query tiles have the most keys: first
     const uint32_t dim = heads * HD;
     uint32_t row0, len;
     if (cu) { row0 = row_base + (uint32_t)cu[seq]; len = (uint32_t)(cu[seq + 1] - cu[seq]); }
@@ -80,41 +82,48 @@ attn_prefill_kernel(const T* __restrict__ q, const T* __restrict__ kbase, const 
     }
 
     const uint32_t q_last = (q0 + PF_BQ - 1 < len - 1) ? q0 + PF_BQ - 1 : len - 1;
+    // A tile's K and V pieces of this thread, all requested at once and one tile ahead: requested one after the other, each behind
+    // its block-table entry, they were 10,000 of a tile's 13,000 cycles. K: four lanes read 64 contiguous bytes of a key; V: CPR lanes
+    // read a whole row.
+    constexpr int NLD = PF_BK * CPR / PF_THREADS;
+    uint4 kr[NLD], vr[NLD];
+    auto k_piece = [&](int n, uint32_t& r, uint32_t& c) { const uint32_t e = tid + n * PF_THREADS; r = (e >> 2) % PF_BK; c = (e & 3) + 4 * (e / (4 * PF_BK)); };
+    auto v_piece = [&](int n, uint32_t& r, uint32_t& c) { const uint32_t e = tid + n * PF_THREADS; c = e % CPR; r = e / CPR; };
+    auto fetch = [&](uint32_t k0) {
+        auto piece = [&](const T* base, uint32_t r, uint32_t c) -> uint4 {
+            const uint32_t kj = k0 + r;
+            if (kj >= len) return make_uint4(0, 0, 0, 0);
+            const T* src = PAGED ? base + (((size_t)table[kj / PF_BS] * heads + h) * PF_BS + (kj % PF_BS)) * HD + c * EPC
+                                 : base + (size_t)(row0 + kj) * dim + (size_t)h * HD + c * EPC;
+            return *reinterpret_cast<const uint4*>(src);
+        };
+#pragma unroll
+        for (int n = 0; n < NLD; n++) {
+            uint32_t r, c;
+            k_piece(n, r, c);
+            kr[n] = piece(kbase, r, c);
+            v_piece(n, r, c);
+            vr[n] = piece(vbase, r, c);
+        }
+    };
+    fetch(0);
     for (uint32_t k0 = 0; k0 <= q_last; k0 += PF_BK) {
         __syncthreads();  // previous tile fully consumed (also orders the Q store before first use)
         // ---- K tile -> kt (transposed), V tile -> vs
-        for (uint32_t e = tid; e < PF_BK * CPR; e += PF_THREADS) {
-            uint32_t r = e % PF_BK, c = e / PF_BK;
-            uint32_t kj = k0 + r;
+#pragma unroll
+        for (int n = 0; n < NLD; n++) {
+            uint32_t r, c;
             float v[EPC];
-            if (kj < len) {
-                const T* src;
-                if (PAGED) src = kbase + (((size_t)table[kj / PF_BS] * heads + h) * PF_BS + (kj % PF_BS)) * HD + c * EPC;
-                else src = kbase + (size_t)(row0 + kj) * dim + (size_t)h * HD + c * EPC;
-                load_chunk<T>(src, v);
-            } else {
+            k_piece(n, r, c);
+            expand<T>(kr[n], v);
 #pragma unroll
-                for (int i = 0; i < EPC; i++) v[i] = 0.0f;
-            }
-#pragma unroll
-            for (int i = 0; i < EPC; i++) sm.kt[c * EPC + i][r] = v[i];
-        }
-        for (uint32_t e = tid; e < PF_BK * CPR; e += PF_THREADS) {
-            uint32_t c = e % CPR, r = e / CPR;
-            uint32_t kj = k0 + r;
-            float v[EPC];
-            if (kj < len) {
-                const T* src;
-                if (PAGED) src = vbase + (((size_t)table[kj / PF_BS] * heads + h) * PF_BS + (kj % PF_BS)) * HD + c * EPC;
-                else src = vbase + (size_t)(row0 + kj) * dim + (size_t)h * HD + c * EPC;
-                load_chunk<T>(src, v);
-            } else {
-#pragma unroll
-                for (int i = 0; i < EPC; i++) v[i] = 0.0f;
-            }
+            for (int i = 0; i < EPC; i++) sm.kt[pf_kt(c * EPC + i) + r] = v[i];
+            v_piece(n, r, c);
+            expand<T>(vr[n], v);
 #pragma unroll
             for (int i = 0; i < EPC; i++) sm.vs[r][c * EPC + i] = v[i];
         }
+        if (k0 + PF_BK <= q_last) fetch(k0 + PF_BK);
         __syncthreads();
 
         // ---- S = Q K^T for rows RPT*ty..RPT*ty+RPT-1, keys 4tx..4tx+3
@@ -128,7 +137,7 @@ attn_prefill_kernel(const T* __restrict__ q, const T* __restrict__ kbase, const 
             float qa_[RPT];
 #pragma unroll
             for (int i = 0; i < RPT; i++) qa_[i] = sm.qt[d][ty * RPT + i];
-            float4 kb = *reinterpret_cast<const float4*>(&sm.kt[d][tx * 4]);
+            float4 kb = *reinterpret_cast<const float4*>(&sm.kt[pf_kt(d) + tx * 4]);
             float kb_[4] = {kb.x, kb.y, kb.z, kb.w};
 #pragma unroll
             for (int i = 0; i < RPT; i++)
@@ -276,10 +285,13 @@ template <typename T, int HD, bool PAGED>
 static int launch_tiled(cudaStream_t st, const T* q, const T* k, const T* v, const int32_t* bt, uint32_t max_blocks,
                         const int32_t* cu, const int32_t* seq_slot, T* out, float* l_cache, uint32_t n_seqs,
                         uint32_t max_len, uint32_t row_base, uint32_t heads, float scale, uint32_t fixed_len) {
-    // 64-row query tiles when they already give two waves of CTAs, else 16-row tiles
+    // 64-row query tiles when they already give two waves of CTAs, 32-row tiles when those give half a wave, else 16-row tiles.
+    // One prompt x 12 heads (f32, head_dim 64) with 16 / 32 / 64 rows: 512 tokens 93 / 57 / 52 us, 300 37 / 26 / 34, 201 25 / 21 / 27.
     const uint64_t big = (uint64_t)cdiv(max_len, 64) * heads * n_seqs;
     if (big >= 296)
         return launch_tiled_rpt<T, HD, PAGED, 4>(st, q, k, v, bt, max_blocks, cu, seq_slot, out, l_cache, n_seqs, max_len, row_base, heads, scale, fixed_len);
+    if (2 * big >= 80)
+        return launch_tiled_rpt<T, HD, PAGED, 2>(st, q, k, v, bt, max_blocks, cu, seq_slot, out, l_cache, n_seqs, max_len, row_base, heads, scale, fixed_len);
     return launch_tiled_rpt<T, HD, PAGED, 1>(st, q, k, v, bt, max_blocks, cu, seq_slot, out, l_cache, n_seqs, max_len, row_base, heads, scale, fixed_len);
 }
 

@@ -229,3 +229,27 @@ def test_attn_decode_auto_splits(ak, torch_cuda, rows, heads, hd, dtype, lens):
             # bf16: P rounded on both sides of the quotient, the output once; f32: sums of a few hundred terms
             tol = ((2 ** -8 + 2 ** -9) if dtype else 1e-5) * float(v.abs().max())
             assert float((out[r].double() - want).abs().max()) < tol, (r, kv[r])
+
+
+# f32 prefill attention around the lines between 16-, 32- and 64-row query tiles, with lengths at the edges of a tile
+@pytest.mark.parametrize("heads,hd,lens", [(12, 64, (192,)), (12, 64, (193,)), (12, 64, (512, 31)), (12, 64, (65, 577, 1, 33, 640)), (5, 128, (512, 513))])
+def test_attn_prefill_f32_tiles(ak, torch_cuda, heads, hd, lens):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    n, mx = len(lens), max(lens)
+    mb = (mx + 15) // 16
+    kp, vp = (torch.randn(n * mb, heads, 16, hd, device="cuda", generator=g) for _ in range(2))
+    tables = torch.randperm(n * mb, device="cuda", generator=g).to(torch.int32).reshape(n, mb)
+    cu = np.zeros(n + 1, np.int32)
+    cu[1:] = np.cumsum(lens)
+    q = torch.randn(int(cu[-1]), heads * hd, device="cuda", generator=g)
+    out = torch.full_like(q, float("nan"))
+    ak.ops.attn_prefill_paged(q, kp, vp, tables, mb, torch.from_numpy(cu).cuda(), torch.arange(n, dtype=torch.int32, device="cuda"), out, n, mx, int(cu[-1]),
+                              heads, hd, hd ** -0.5, ak.AK_F32, n * mb)
+    for i, L in enumerate(lens):
+        r = slice(int(cu[i]), int(cu[i + 1]))
+        k, v = (p[tables[i].long()].transpose(1, 2).reshape(mb * 16, heads, hd)[:L].double().transpose(0, 1) for p in (kp, vp))
+        s = torch.einsum("lhd,hkd->hlk", q[r].double().reshape(L, heads, hd), k) * hd ** -0.5
+        s.masked_fill_(torch.ones(L, L, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+        want = torch.einsum("hlk,hkd->lhd", s.softmax(-1), v).reshape(L, -1)
+        assert float((out[r].double() - want).abs().max()) < 2e-5, (i, L)   # f32 sums of up to 640 terms
