@@ -277,8 +277,8 @@ __device__ __forceinline__ void epi_store16(const GemmEpi& ep, uint32_t row, boo
 template <int BN, int EPI, bool SPLIT>
 __global__ void __launch_bounds__(G_THREADS)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmEpi ep,
-                 uint32_t m, uint32_t n, uint32_t k, uint32_t stages, uint32_t kseg, uint32_t tmem_cols, uint32_t a_rows) {
-    // a_rows: rows of the activation box (128, or fewer when m is small: the MMA still reads 128 rows of
+                 uint32_t m, uint32_t n, uint32_t k, uint32_t stages, uint32_t kseg, uint32_t tmem_cols, uint32_t a_rows, uint32_t a_box) {
+    // a_rows: rows of an activation slot (128, or fewer when m is small: the MMA still reads 128 rows of
     // the stage, the rows past the box hold stale data and feed accumulator rows that are never stored).
     // kseg > 1 (only with a cluster of one CTA): the K range is accumulated in kseg separate TMEM
     // accumulators that the epilogue adds in order. It reproduces, bit for bit, what a cluster of
@@ -300,7 +300,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // tile is requested before the dependency wait. The MMA still reads 128 rows from a slot's base: what follows it
     // (later slots, the weight slots, padding when those are too few) feeds accumulator rows that are never stored.
     // The split-K exchange buffer holds a_rows rows per source CTA (rows past m are never exchanged).
-    const uint32_t a_bytes = a_rows * (GB_K * 2), stage_tx = a_bytes + C::B_BYTES;
+    const uint32_t a_bytes = a_rows * (GB_K * 2), stage_tx = a_box * (GB_K * 2) + C::B_BYTES;
     uint8_t* const b_base = smem + (size_t)stages * a_bytes;
     const uint32_t overrun = (GB_M - a_rows) * (GB_K * 2), b_total = stages * C::B_BYTES;
     float* red = reinterpret_cast<float*>(b_base + b_total + (overrun > b_total ? overrun - b_total : 0u));  // used when ks > 1
@@ -864,14 +864,21 @@ struct GemmPlan {
 static constexpr uint32_t SMEM_TWO_PER_SM = 112 * 1024;   // two CTAs fit one SM below this
 static constexpr uint32_t SMEM_ONE_PER_SM = 220 * 1024;
 static constexpr uint32_t SMEM_PAIR = 226 * 1024;         // the pair kernel: all a CTA may have but its few hundred static bytes
+// Launches of more than 48 rows claim at least this much: with small footprints the waiting CTAs of three or four launches of the
+// chain share an SM, and their activation traffic meets. Decode step of the 162M model, 64 rows: 515 -> 505 us. (40 rows: 441 ->
+// 445 us; there, and below, the deeper the chain stacks up the better.)
+static constexpr uint32_t SMEM_MIN_WIDE = 78 * 1024;
 static constexpr uint32_t SMEM_THREE_PER_SM = 74 * 1024;  // three CTAs fit one SM below this (228 KB, 1 KB reserved and ~0.25 KB static per CTA)
 
 // Rows of the activation TMA box: a decode batch fills only part of the 128-row MMA tile, and rows the
 // box does not fetch cost neither L2 requests nor zero-fill writes.
+// A long box that reaches past the last row is slow, the fill costs more than the rows would: 65 x 3072 x 768 took 8.6 us in a
+// chain of launches with a box of 128, 5.3 us with one of 65.
 static uint32_t a_box_rows(uint32_t m) {
-    if (m > 64) return GB_M;
+    if (m > 64) return m < (uint32_t)GB_M ? m : GB_M;
     return m > 32 ? 64 : (m > 16 ? 32 : 16);
 }
+static uint32_t a_slot_rows(uint32_t m) { return (a_box_rows(m) + 7) / 8 * 8; }   // whole swizzle atoms
 static uint32_t stage_bytes(uint32_t bn, uint32_t a_rows = GB_M) { return a_rows * GB_K * 2 + bn * GB_K * 2; }
 // shared memory of the one-CTA kernel: the ring, the rows an MMA reads past a short activation slot where the weight
 // slots do not cover them, the exchange buffer (a_rows rows per source CTA), alignment room
@@ -959,7 +966,7 @@ static GemmPlan plan_gemm(uint32_t m, uint32_t n, uint32_t k, bool allow_split, 
         for (int i = 0; i < 3; i++)
             if (cdiv(n, cands[i]) <= slots) { p.bn = cands[i]; break; }
         p.ks = 1;
-        const uint32_t ar = a_box_rows(m);
+        const uint32_t ar = a_slot_rows(m);
         uint32_t st = (SMEM_TWO_PER_SM - 1024 - (GB_M - ar) * GB_K * 2) / stage_bytes(p.bn, ar);
         if (st > G_MAX_STAGES) st = G_MAX_STAGES;
         if (st < 2) st = 2;
@@ -989,7 +996,7 @@ static GemmPlan plan_gemm(uint32_t m, uint32_t n, uint32_t k, bool allow_split, 
             if (better) { best_kb = per; best_ctas = ctas; p.bn = bn; p.ks = ks; }
         }
     const uint32_t per = cdiv(num_kb, p.ks) ? cdiv(num_kb, p.ks) : 1;
-    const uint32_t ar = a_box_rows(m);
+    const uint32_t ar = a_slot_rows(m);
     uint32_t st = gemm_fit_stages(per, p.bn, ar, p.ks > 1, SMEM_TWO_PER_SM);
     // A footprint that lets THREE CTAs share an SM is preferred when it costs at most one stage of the K range (that
     // K block then re-uses the first slot): the next launch's CTAs, and the attention CTAs behind the qkv projection,
@@ -1005,7 +1012,8 @@ static GemmPlan plan_gemm(uint32_t m, uint32_t n, uint32_t k, bool allow_split, 
 template <int BN, int EPI>
 static int launch_cfg(cudaStream_t st, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmEpi& ep, uint32_t m, uint32_t n,
                       uint32_t k, const GemmPlan& p) {
-    const size_t smem = gemm_smem_bytes(p.stages, BN, a_box_rows(m), p.ks > 1);
+    size_t smem = gemm_smem_bytes(p.stages, BN, a_slot_rows(m), p.ks > 1);
+    if (m > 48 && smem < SMEM_MIN_WIDE) smem = SMEM_MIN_WIDE;
     {
         // per-device "attribute set" flags; the library may be driven from one host thread per GPU
         static size_t attr_set[64] = {};
@@ -1023,9 +1031,9 @@ static int launch_cfg(cudaStream_t st, const CUtensorMap& tmA, const CUtensorMap
     AK_REQUIRE(cols <= 512, AK_ERR_UNSUPPORTED, "gemm_bf16: %u accumulator columns exceed TMEM", need);
     if (p.ks > 1)
         return launch_k(gemm_bf16_kernel<BN, EPI, true>, dim3(cdiv(n, BN), cdiv(m, GB_M), p.ks), dim3(G_THREADS), smem, st, dim3(1, 1, p.ks),
-                        tmA, tmB, ep, m, n, k, p.stages, p.kseg, cols, a_box_rows(m));
+                        tmA, tmB, ep, m, n, k, p.stages, p.kseg, cols, a_slot_rows(m), a_box_rows(m));
     return launch_k(gemm_bf16_kernel<BN, EPI, false>, dim3(cdiv(n, BN), cdiv(m, GB_M), 1), dim3(G_THREADS), smem, st, dim3(1, 1, 1),
-                    tmA, tmB, ep, m, n, k, p.stages, p.kseg, cols, a_box_rows(m));
+                    tmA, tmB, ep, m, n, k, p.stages, p.kseg, cols, a_slot_rows(m), a_box_rows(m));
 }
 
 template <int BN>

@@ -253,3 +253,19 @@ def test_attn_prefill_f32_tiles(ak, torch_cuda, heads, hd, lens):
         s.masked_fill_(torch.ones(L, L, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
         want = torch.einsum("hlk,hkd->lhd", s.softmax(-1), v).reshape(L, -1)
         assert float((out[r].double() - want).abs().max()) < 2e-5, (i, L)   # f32 sums of up to 640 terms
+
+
+# The activation box of a skinny GEMM: 16, 32, 64, then exactly the rows (slots of whole swizzle atoms), then 128
+@pytest.mark.parametrize("m", [1, 8, 16, 17, 33, 48, 49, 64, 65, 71, 72, 73, 100, 127, 128, 129])
+@pytest.mark.parametrize("n,k", [(2304, 768), (768, 3072)])
+def test_gemm_skinny_rows(ak, torch_cuda, m, n, k):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a, w = (torch.randn(r, k, device="cuda", generator=g).bfloat16() for r in (m, n))
+    c = torch.full((m + 1, n), 3.0, device="cuda")
+    ak.ops.gemm_bf16(a, w, c, m, n, k, ak.EPI_STORE_F32)
+    want = a.double() @ w.double().T
+    # exact products, k f32 additions of rounding 2^-24 each on partial sums of about sqrt(k): k^0.5 * k^0.5 * 2^-24, x8 for the extremes
+    assert float((c[:m].double() - want).abs().max()) < 8 * k * 2.0 ** -24
+    assert bool((c[m] == 3.0).all())
+    ak.check(ak.lib().ak_check_device_status(None))
