@@ -369,7 +369,7 @@ int Runner::init(ak_ctx* ctx, ak_weights* w, uint32_t max_seqs, uint32_t max_seq
     AK_CUDA(cudaStreamCreateWithFlags(&st_time_, cudaStreamNonBlocking));
     AK_CUDA(cudaEventCreateWithFlags(&ev_tfork_, cudaEventDisableTiming));
     AK_CUDA(cudaEventCreateWithFlags(&ev_tjoin_, cudaEventDisableTiming));
-    solo_ = max_seqs == 1 && tp_ == 1 && solo_supported(w->dtype, D, F, H, c.num_layers);
+    solo_ = max_seqs == 1 && tp_ == 1 && solo_supported(w->dtype, D, F, H, c.num_layers, V);
     if (solo_) {
         std::vector<SoloLayer> sl(c.num_layers);
         for (uint32_t l = 0; l < c.num_layers; l++) {

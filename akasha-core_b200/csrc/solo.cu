@@ -27,6 +27,7 @@
 // Nothing may spill: local memory is poison here (the ring leaves the L1 cache a few KB, every reload goes to L2; a 17-warp
 // version with 96 registers took 0.67 ms per step, and 44 bytes of spills at 128 registers cost 20 us).
 #include "solo.h"
+#include "solo_plan.h"
 
 namespace ak {
 
@@ -34,22 +35,16 @@ __device__ unsigned int g_solo_status = 0;
 
 namespace {
 
-constexpr int NW = 12;                   // compute warps
+using namespace solo;
+static_assert(CTAS == B200_SMS, "a block per SM");
 constexpr int NC = (NW + 1) * 32;        // threads of the compute and reducer warps (the block barrier's count)
 // Four warpgroups: the first holds the producer (warp 0) and the reducer (warp 1), the others the compute warps. 512 threads
 // launch with 128 registers each; the first group gives 48 of them to the others.
 constexpr int THREADS = 512, FIRST_COMPUTE = 4;
 constexpr int REGS_FIRST = 80, REGS_COMPUTE = 144;
 static_assert(REGS_FIRST * 128 + REGS_COMPUTE * 384 <= 65536, "the split draws on the registers of the launch");
-constexpr uint32_t SLOT = 12288;         // ring slot: one f32 row of 3072, four of 768
-constexpr uint32_t SLICE = 64;           // K elements of a slice
-constexpr uint32_t NQ = 6, BLK = 4 * NQ;  // most rows of a block: six per lane group
-constexpr uint32_t MAX_SLOTS = 12;
 constexpr uint32_t REPLICAS = 4;         // copies of every exchanged value: an SM polls copy (SM mod 4). 148 SMs polling one 128-byte line
                                          // occupy its L2 slice for ~300 cycles a round, and the store they wait for queues behind them
-constexpr uint32_t MAX_LAYERS = 48;
-constexpr uint32_t N_KINDS = 5;          // weight matrices: qkv, out-proj, ffn-up, ffn-down, lm_head
-constexpr size_t MAX_DYN_SMEM = 213 * 1024;   // 227 KB less the static variables
 
 // ---- flagged exchange: {value, step} in one 64-bit word
 __device__ __forceinline__ void ll_put(uint64_t* p, size_t copy_stride, float v, uint32_t ep) {
@@ -176,34 +171,6 @@ template <> struct Vec<bf16> {
         return make_uint4(o[0], o[1], o[2], o[3]);
     }
 };
-
-// One kind of weight matrix [n, k] as this SM sees it: its rows r0 .. r0 + rows, and how they travel through the ring: rpc
-// whole rows to a slot, or (rows wider than a slot) ppr pieces of `piece` elements. The compute warps work on blocks of blk
-// rows, a multiple of rpc (no chunk belongs to two blocks) whose chunks fit the ring. Divisions by rpc and piece are
-// multiplications by 65536 / d + 1 (exact for the row numbers of one SM and the slice numbers of one row).
-struct Kind {
-    uint32_t k, r0, rows, rpc, ppr, piece, blk, inv_rpc, inv_pslices;
-    uint32_t n0, chunks0, chunks; // rows and chunks of the first block, all chunks
-    uint32_t row_off[4][8];       // [r][i]: ring offset of row r + 4 i of a block, in bytes from the block's first chunk
-};
-__device__ __forceinline__ uint32_t div_inv(uint32_t v, uint32_t inv) { return (v * inv) >> 16; }
-__device__ __forceinline__ uint32_t row_begin(uint32_t n, uint32_t cta, uint32_t ctas) { return (uint32_t)(((uint64_t)n * cta) / ctas); }
-__device__ void make_kind(Kind& d, uint32_t n, uint32_t k, uint32_t esz, uint32_t slots, uint32_t cta, uint32_t ctas) {
-    d.k = k;
-    d.r0 = row_begin(n, cta, ctas);
-    d.rows = row_begin(n, cta + 1, ctas) - d.r0;
-    const uint32_t row = k * esz;
-    d.rpc = row <= SLOT ? min(SLOT / row, BLK) : 1;
-    d.piece = row <= SLOT ? k : SLOT / (SLICE * esz) * SLICE;
-    d.ppr = (k + d.piece - 1) / d.piece;
-    d.blk = max(1u, min(BLK / d.rpc, (slots - 2) / d.ppr)) * d.rpc;
-    d.n0 = min(d.blk, d.rows);
-    d.chunks0 = d.ppr > 1 ? d.n0 * d.ppr : (d.n0 + d.rpc - 1) / d.rpc;
-    d.chunks = d.ppr > 1 ? d.rows * d.ppr : (d.rows + d.rpc - 1) / d.rpc;
-    for (uint32_t r = 0; r < BLK; r++) d.row_off[r & 3][r >> 2] = d.ppr > 1 ? r * d.ppr * SLOT : r / d.rpc * SLOT + r % d.rpc * row;
-    d.inv_rpc = 65536 / d.rpc + 1;
-    d.inv_pslices = 65536 / ((d.piece + SLICE - 1) / SLICE) + 1;
-}
 
 struct Ring {
     uint8_t* base;
@@ -390,10 +357,6 @@ struct XchOff {   // word offsets inside a layer's exchange region
         total = hid2 + dim;
     }
 };
-
-// Compute warps that take part in attention: 48 KB of cache tiles for both types (a tile is 4 KB in f32, 2 KB in bf16), the
-// rest of shared memory is worth more to the weight ring.
-__host__ __device__ constexpr uint32_t att_warps(uint32_t esz) { return esz == 4 ? 6 : 12; }
 
 template <typename T, int HD>
 __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant__ SoloArgs a, const uint32_t slots) {
@@ -992,29 +955,12 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
     }
 }
 
-struct Plan {
-    uint32_t slots;
-    size_t smem;
-};
-bool make_plan(uint32_t esz, uint32_t D, uint32_t F, Plan& p) {
-    // beside the ring: the cache tiles of the compute warps, their slices of the residual stream and of a phase's input
-    const size_t rest = (size_t)att_warps(esz) * 2 * 1024 * esz + (size_t)NW * (cdiv(D / SLICE, NW) + cdiv(cdiv(F, SLICE), NW)) * SLICE * 4;
-    if (rest + 6 * SLOT > MAX_DYN_SMEM) return false;
-    p.slots = (uint32_t)((MAX_DYN_SMEM - rest) / SLOT);
-    if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
-    p.smem = p.slots * SLOT + rest;
-    return true;
-}
-
 }  // namespace
 
-bool solo_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers) {
-    const uint32_t esz = dtype == AK_F32 ? 4 : 2, hd = heads ? dim / heads : 0;
-    Plan p;
+bool solo_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers, uint32_t vocab) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
-    return (uint32_t)sms >= B200_SMS && (hd == 64 || hd == 128) && heads <= B200_SMS && n_layers <= MAX_LAYERS && (ffn * esz) % 16 == 0 && ffn >= B200_SMS &&
-           dim >= SLICE && dim * esz <= SLOT && ffn <= 32768 && make_plan(esz, dim, ffn, p);
+    return (uint32_t)sms >= B200_SMS && shape_supported(dtype == AK_F32 ? 4 : 2, dim, ffn, heads, n_layers, vocab);
 }
 
 size_t solo_xch_words(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers) {

@@ -37,7 +37,7 @@ struct SoloArgs {
     float eps, scale;
 };
 
-bool solo_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers);
+bool solo_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers, uint32_t vocab);
 size_t solo_xch_words(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers);
 int launch_solo(cudaStream_t st, uint32_t dtype, const SoloArgs& a);
 int solo_status(unsigned int* out);
