@@ -419,17 +419,23 @@ int Runner::solo_launch(int32_t tok_src, uint32_t pos, bool want_logits, bool ho
     return launch_solo(ctx_->stream, w_->dtype, a);
 }
 
+int Runner::solo_wait(uint32_t ticket, uint32_t& token) {
+    uint32_t v = 0;
+    AK_TRY(wait_word(h_solo_done_ + ticket % SOLO_AHEAD, ticket, v));
+    AK_REQUIRE(v != solo::STEP_FAILED, AK_ERR_DEVICE_WAIT, "batch-1 step: a bounded device-side wait expired");
+    token = v;
+    return AK_OK;
+}
+
 int Runner::wait_word(const uint64_t* w, uint32_t tag, uint32_t& value) {
     const volatile uint64_t* word = w;
-    for (uint64_t n = 1;; n++) {
-        const uint64_t v = *word;
-        if ((uint32_t)(v >> 32) == tag) { value = (uint32_t)v; break; }
+    for (uint64_t n = 1; !solo::read_word(*word, tag, value); n++) {
         if ((n & 0xfff) == 0) {   // now and then: has the stream stopped without reporting?
             const cudaError_t e = cudaStreamQuery(ctx_->stream);
             if (e == cudaErrorNotReady) continue;
             if (e != cudaSuccess) return cuda_fail(e, "batch-1 step", __FILE__, __LINE__);
-            const uint64_t last = *word;
-            AK_REQUIRE((uint32_t)(last >> 32) == tag, AK_ERR_CUDA, "batch-1 step ended without a result");
+            AK_REQUIRE(solo::read_word(*word, tag, value), AK_ERR_CUDA, "batch-1 step ended without a result");
+            break;
         }
     }
     std::atomic_thread_fence(std::memory_order_acquire);   // what was written before the word

@@ -7,6 +7,7 @@
 
 #include "kernels.h"
 #include "solo.h"
+#include "solo_plan.h"
 
 struct ak_ctx {
     int device = 0;
@@ -103,7 +104,7 @@ class Runner {
     static constexpr uint32_t SOLO_AHEAD = 4;
     bool solo() const { return solo_; }
     int solo_launch(int32_t tok_src, uint32_t pos, bool want_logits, bool host_logits, uint32_t& ticket);
-    int solo_wait(uint32_t ticket, uint32_t& token) { return wait_word(h_solo_done_ + ticket % SOLO_AHEAD, ticket, token); }
+    int solo_wait(uint32_t ticket, uint32_t& token);   // AK_ERR_DEVICE_WAIT: a wait of the step ran out, there is no token
     // spin until a device-written pinned word {value, tag} carries `tag`
     int wait_word(const uint64_t* word, uint32_t tag, uint32_t& value);
     const float* solo_logits_host() const { return h_logits_; }

@@ -23,6 +23,8 @@ struct ak_session {
     static constexpr uint32_t PICKS = 4;
     uint64_t* h_pick = nullptr;
     uint32_t pick_of[PICKS] = {}, pick_tag = 0;
+    uint32_t step_of[PICKS] = {};   // the decode step whose logits that token was sampled from
+    static_assert(PICKS <= Runner::SOLO_AHEAD, "a step's done word is read when its token is");
     ~ak_session() {
         if (d_hist) cudaFree(d_hist);
         if (h_pick) cudaFreeHost(h_pick);
@@ -121,9 +123,8 @@ static int decode_one(ak_session* s, int32_t tok_src) {   // models the persiste
 }
 
 // Launch the decode step that feeds tok_src (< 0: the device's last pick) at position pos; logits stay on the device.
-static int decode_launch(ak_session* s, int32_t tok_src, uint32_t pos) {
+static int decode_launch(ak_session* s, int32_t tok_src, uint32_t pos, uint32_t& ticket) {
     Runner& r = s->runner;
-    uint32_t ticket = 0;
     if (r.solo()) return r.solo_launch(tok_src, pos, true, false, ticket);
     s->cur_len = pos;
     AK_TRY(decode_one(s, tok_src));
@@ -268,7 +269,7 @@ int ak_session_generate(ak_session* s, const uint32_t* prompt, uint32_t n, uint3
     uint32_t launched = 0;
     const uint32_t ahead = r.solo() ? ak_session::PICKS - 1 : 1;
     auto launch = [&](uint32_t i) -> int {   // decode step i - 1 (i > 0), then the sampler of token i
-        if (i > 0) AK_TRY(decode_launch(s, -1, base + i - 1));
+        if (i > 0) AK_TRY(decode_launch(s, -1, base + i - 1, s->step_of[i % ak_session::PICKS]));
         if (++s->pick_tag == 0) s->pick_tag = 1;
         SampleSink sink;
         sink.hist = s->d_hist + n + i;
@@ -286,12 +287,18 @@ int ak_session_generate(ak_session* s, const uint32_t* prompt, uint32_t n, uint3
         }
         rc = r.wait_word(s->h_pick + i % ak_session::PICKS, s->pick_of[i % ak_session::PICKS], next);
         if (rc) return rc;
+        if (i > 0 && r.solo()) {   // (the step is done, the sampler ran behind it) were its logits good?
+            uint32_t greedy;
+            AK_TRY(r.solo_wait(s->step_of[i % ak_session::PICKS], greedy));
+        }
         out_tokens[(*n_out)++] = next;
         s->cur_len = base + i;
         if (stop_on_eos && next == eos) break;
         if (i >= most) break;                                // out of context mid-generation: return what we have
         if (i + 1 == max_new) {                              // the last token is fed too, as in the reference's loop
-            rc = decode_launch(s, -1, base + i);
+            uint32_t ticket = 0, greedy;
+            rc = decode_launch(s, -1, base + i, ticket);
+            if (rc == AK_OK && r.solo()) rc = r.solo_wait(ticket, greedy);
             if (rc) return rc;
             s->cur_len = base + i + 1;
         }

@@ -19,8 +19,9 @@
 // may still read it; the step number in the flags makes clearing them unnecessary.
 //
 // The grid is launched cooperatively (its blocks wait on one another): one block per SM, all resident. Every wait is
-// bounded: on expiry a status word is set, later waits of the block return at once, and the copies in flight are waited
-// for before the block leaves.
+// bounded: on expiry a status word is set, later waits of the block return at once, and the block reports the failure where it
+// would report its best logit, so that the step's done word says STEP_FAILED instead of a token. A warp whose wait for
+// a chunk ran out releases no more chunks, so no slot is written again, and the producer leaves only when every copy it started has landed.
 //
 // Arithmetic: f32 products and sums of f32 or bf16 weights with f32 activations (the multi-launch bf16 path rounds the
 // activations to bf16 for the tensor core; here they stay f32), keys and values rounded to the cache type.
@@ -43,6 +44,7 @@ constexpr int NC = (NW + 1) * 32;        // threads of the compute and reducer w
 constexpr int THREADS = 512, FIRST_COMPUTE = 4;
 constexpr int REGS_FIRST = 80, REGS_COMPUTE = 144;
 static_assert(REGS_FIRST * 128 + REGS_COMPUTE * 384 <= 65536, "the split draws on the registers of the launch");
+constexpr uint32_t BLOCK_FAILED = 0xfffffffeu;   // in the place of the index of a block's best logit (0xffffffff: it has none)
 constexpr uint32_t REPLICAS = 4;         // copies of every exchanged value: an SM polls copy (SM mod 4). 148 SMs polling one 128-byte line
                                          // occupy its L2 slice for ~300 cycles a round, and the store they wait for queues behind them
 
@@ -278,15 +280,16 @@ template <typename T> struct Block {
         }
     }
 
-    // wait for the block's chunks (from q on), take the first weights
-    __device__ __forceinline__ void fetch(const Ring& rg, const Cursor& q, const Kind& d, uint32_t n, uint32_t chunks, uint32_t warp, uint32_t lane, uint32_t* dead) {
+    // wait for the block's chunks (from q on), take the first weights; false: a wait ran out
+    __device__ __forceinline__ bool fetch(const Ring& rg, const Cursor& q, const Kind& d, uint32_t n, uint32_t chunks, uint32_t warp, uint32_t lane, uint32_t* dead) {
         base = q.s * SLOT;
+        bool got = true;
         if (lane < chunks) {
             Cursor mine = q;
             mine.advance(lane, rg.n);
-            wait_full(&rg.full[mine.s], mine.ph, dead);
+            got = wait_full(&rg.full[mine.s], mine.ph, dead);
         }
-        __syncwarp();
+        got = __all_sync(0xffffffffu, got) != 0;
         if (n <= 8) {
 #pragma unroll
             for (int s = 0; s < PQ / 2; s++) load<2>(rg, d, n, warp + NW * s, 0, lane, w + 2 * s * WP);
@@ -295,6 +298,7 @@ template <typename T> struct Block {
         }
 #pragma unroll
         for (int i = 0; i < 8; i++) acc[i] = 0.0f;
+        return got;
     }
     // add the warp's slice S (S == ANY: slice s > 0, nothing of it in registers), activations v
     static constexpr int ANY = 99;
@@ -448,14 +452,14 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
         }
-        if (!ok) {   // leaving early: the copies under way have to land first
-            if (lane_ < NA && kv_sent > 0) mbar_wait(&kv_full[lane_], (kv_sent - 1) & 1u);
-            if (lane_ == 0)
-                for (uint32_t i = 0; i < min(sent, slots); i++) {
-                    q.retreat(1, slots);
-                    mbar_wait(&full_bar[q.s], q.ph);
-                }
-        }
+        // every copy lands before the block's memory goes away: a slot is only written again when its last copy was waited for, so
+        // the latest one of each is enough
+        if (lane_ < NA && kv_sent > 0) mbar_wait(&kv_full[lane_], (kv_sent - 1) & 1u);
+        if (lane_ == 0)
+            for (uint32_t i = 0; i < min(sent, slots); i++) {
+                q.retreat(1, slots);
+                mbar_wait(&full_bar[q.s], q.ph);
+            }
         return;
     }
 
@@ -544,24 +548,27 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
         uint64_t* const fin = a.xch + (size_t)L * xo.total;
         if (lane == 0) {
             ll_put(fin + 2 * cta, copy, bv, ep);
-            ll_put(fin + 2 * cta + 1, copy, __uint_as_float(bi), ep);
+            ll_put(fin + 2 * cta + 1, copy, __uint_as_float(*(volatile uint32_t*)&dead ? BLOCK_FAILED : bi), ep);
         }
         if (cta != 0) return;
         bv = -INFINITY;
         bi = 0xffffffffu;
+        bool failed = false;
         for (uint32_t c = lane; c < ctas; c += 32) {
             float2 p[1];
             poll_pairs(fin + 2 * c, 0, 1, ep, wt, p);
+            failed = failed || __float_as_uint(p[0].y) == BLOCK_FAILED;
             better(bv, bi, p[0].x, __float_as_uint(p[0].y));
         }
         warp_best(bv, bi);
+        failed = __any_sync(0xffffffffu, failed || *(volatile uint32_t*)&dead);
         if (lane == 0) {
-            const uint32_t tok = bi == 0xffffffffu ? 0u : bi;
+            const uint32_t tok = bi < V ? bi : 0u;   // (no logit above -inf: 0)
             *a.sampled = tok;
             if (a.sampled_host) *(volatile uint32_t*)a.sampled_host = tok;
             if (a.done_host) {
                 __threadfence_system();
-                *(volatile uint64_t*)a.done_host = (uint64_t)tok | ((uint64_t)ep << 32);
+                *(volatile uint64_t*)a.done_host = (uint64_t)(failed ? STEP_FAILED : tok) | ((uint64_t)ep << 32);
             }
         }
         return;
@@ -592,6 +599,8 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
     // this is in the shadow of the reducer and the exchange), then wait for and take the first weights. In this order: the
     // two blocks together may be more than the ring.
     uint32_t to_release = 0;   // chunks before q that this warp is done with
+    bool alive = true;         // no wait of this warp for a copy has run out. After the first that did it releases nothing any more: a later
+                               // wait may take an old phase for its own, and the slot's copy may still be under way
     auto release = [&]() {
         if (lane < to_release) {
             Cursor c = q;
@@ -602,7 +611,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
     };
     auto begin = [&](Block<T>& blk, const Kind& d) {
         release();
-        blk.fetch(rg, q, d, d.n0, d.chunks0, warp, lane, &dead);
+        alive = blk.fetch(rg, q, d, d.n0, d.chunks0, warp, lane, &dead) && alive;
     };
     // After the first block's activations have been added: publish its partial sums, then work through the other row
     // blocks, activations from xs. A kind without rows on this SM has no block (and no barrier).
@@ -614,13 +623,13 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
             bar_block();
             buf ^= 1u;
             q.advance(chunks, rg.n);
-            to_release = chunks;
+            to_release = alive ? chunks : 0;
             if (j0 >= d.rows) break;
             release();
             const uint32_t n = min(d.blk, d.rows - j0);
             chunks = d.ppr > 1 ? n * d.ppr : div_inv(n + d.rpc - 1, d.inv_rpc);
             j0 += n;
-            blk.fetch(rg, q, d, n, chunks, warp, lane, &dead);
+            alive = blk.fetch(rg, q, d, n, chunks, warp, lane, &dead) && alive;
             if (nsl) blk.template add<0>(rg, d, n, 0, xs[0], warp, lane);
 #pragma unroll 1
             for (uint32_t i = 1; i < nsl; i++) blk.add_slice(rg, d, n, i, xs[i * 32], warp, lane);
@@ -695,8 +704,8 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
         auto release_to = [&](uint32_t c) {    // a chunk is waited for even where this warp has no row in it: only then is every arrival of the slot's last use in
             __syncwarp();
             for (; rel < c; rel++, cur.advance(1, rg.n)) {
-                wait_full(&rg.full[cur.s], cur.ph, &dead);
-                if (lane == 0) mbar_arrive(&rg.empty[cur.s]);
+                alive = __all_sync(0xffffffffu, wait_full(&rg.full[cur.s], cur.ph, &dead)) && alive;
+                if (alive && lane == 0) mbar_arrive(&rg.empty[cur.s]);
             }
         };
         const bool in_regs = D <= 32 * EPV * NV;
@@ -809,7 +818,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
 #pragma unroll 1
             for (uint32_t u = u0; u < u_end; u += NA, kv_use++) {
                 const uint32_t newest = a.pos - u * UP;   // the new position's row in this unit (>= UP: not here)
-                wait_full(&kv_full[warp], kv_use & 1u, &dead);
+                const bool got = wait_full(&kv_full[warp], kv_use & 1u, &dead);
                 float s[NL], mx = -INFINITY;
 #pragma unroll
                 for (int i = 0; i < NL; i++) {
@@ -850,8 +859,8 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
                 }
                 l_run = l_run * corr + ls;
                 m_run = m_new;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&kv_empty[warp]);
+                alive = __all_sync(0xffffffffu, got) && alive;
+                if (alive && lane == 0) mbar_arrive(&kv_empty[warp]);
             }
 #pragma unroll
             for (int o = VR; o < 32; o <<= 1) {

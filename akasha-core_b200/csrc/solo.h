@@ -29,7 +29,7 @@ struct SoloArgs {
     float* logits;               // [vocab] device, or nullptr
     float* logits_host;          // [vocab] mapped host memory, or nullptr
     uint32_t* sampled_host;      // mapped host word, or nullptr
-    uint64_t* done_host;         // mapped host word {token, step}: written after everything else, or nullptr
+    uint64_t* done_host;         // mapped host word {token, or solo::STEP_FAILED; step}: written after everything else, or nullptr
     uint32_t n_layers, dim, ffn, heads, vocab;
     uint32_t pos;                // position of the token fed in; positions 0 .. pos are attended to
     int32_t tok_src;             // >= 0 literal id; < 0: *sampled

@@ -96,5 +96,13 @@ inline bool shape_supported(uint32_t esz, uint32_t dim, uint32_t ffn, uint32_t h
     return rows * 4 <= kv_bytes(esz) && div_exact(head.rpc, rows);
 }
 
+// ---- the word {value, tag} in which the device reports that step `tag` is done
+constexpr uint32_t STEP_FAILED = 0xffffffffu;   // in the place of the token: a device-side wait ran out
+inline bool read_word(uint64_t word, uint32_t tag, uint32_t& value) {   // false: not written yet
+    if ((uint32_t)(word >> 32) != tag) return false;
+    value = (uint32_t)word;
+    return true;
+}
+
 }  // namespace solo
 }  // namespace ak

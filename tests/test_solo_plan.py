@@ -48,7 +48,22 @@ static void check(uint32_t esz, uint32_t dim, uint32_t ffn, uint32_t vocab) {
         }
     }
 }
+static uint64_t word(uint32_t value, uint32_t tag) { return (uint64_t)value | (uint64_t)tag << 32; }
+static int words() {   // the host's reading of a step's done word
+    uint32_t v = 7;
+    if (read_word(0, 1, v) || v != 7) return 1;                        // never written
+    if (read_word(word(5, 4), 8, v) || v != 7) return 2;               // an earlier step's
+    if (read_word(word(STEP_FAILED, 4), 8, v) || v != 7) return 3;
+    if (!read_word(word(5, 8), 8, v) || v != 5) return 4;
+    if (!read_word(word(0, 0xffffffffu), 0xffffffffu, v) || v != 0) return 5;
+    if (!read_word(word(STEP_FAILED, 8), 8, v) || v != STEP_FAILED) return 6;   // a wait of this step ran out: no vocabulary has that id
+    return 0;
+}
 int main(int argc, char** argv) {
+    if (argc == 2) {
+        printf("%d\n", words());
+        return 0;
+    }
     if (argc == 7) {   // one shape: esz dim ffn heads layers vocab
         uint32_t v[6];
         for (int i = 0; i < 6; i++) v[i] = (uint32_t)strtoul(argv[i + 1], 0, 10);
@@ -100,3 +115,7 @@ F32, BF16 = 4, 2
 ])
 def test_limits(plan, esz, dim, ffn, heads, layers, vocab, want):
     assert plan(esz, dim, ffn, heads, layers, vocab) == str(want)
+
+
+def test_done_word(plan):
+    assert plan("words") == "0"
