@@ -5,6 +5,7 @@
 #include <limits.h>
 #include <string.h>
 
+#include "ahead.h"
 #include "model.h"
 
 using namespace ak;
@@ -186,26 +187,24 @@ int ak_session_generate_greedy(ak_session* s, const uint32_t* prompt, uint32_t n
         // Steps are launched ahead of the tokens they produce (each feeds on the device's last pick), so the GPU goes from
         // one to the next. A step launched past an end-of-sequence token only writes cache rows beyond cur_len.
         Runner& r = s->runner;
-        uint32_t tickets[Runner::SOLO_AHEAD] = {}, launched = 0, done = 0;   // of the decode steps after `next`
+        if (max_new == 0) return AK_OK;
+        out_tokens[(*n_out)++] = next;
+        if (stop_on_eos && next == eos) return AK_OK;
+        uint32_t tickets[Runner::SOLO_AHEAD] = {};
         const uint32_t room = s->max_ctx - s->cur_len, base = s->cur_len;
-        const uint32_t most = max_new < room ? max_new : room;               // decode steps that may run
-        for (uint32_t i = 0; i < max_new; i++) {
-            out_tokens[(*n_out)++] = next;
-            if ((stop_on_eos && next == eos) || i >= most) break;            // also: out of context mid-generation
-            while (launched < most && launched - done < Runner::SOLO_AHEAD - 1) {
-                AK_TRY(r.solo_launch(-1, base + launched, false, false, tickets[launched % Runner::SOLO_AHEAD]));
-                launched++;
-            }
-            AK_TRY(r.solo_wait(tickets[done % Runner::SOLO_AHEAD], next));
-            done++;
-            s->cur_len = base + done;
-        }
-        while (done < launched) {   // steps past the end: let them finish before anyone else uses the cache
-            uint32_t unused;
-            AK_TRY(r.solo_wait(tickets[done % Runner::SOLO_AHEAD], unused));
-            done++;
-        }
-        return AK_OK;
+        return run_ahead(
+            max_new < room ? max_new : room, Runner::SOLO_AHEAD - 1,     // (out of context mid-generation: what there is)
+            [&](uint32_t j) { return r.solo_launch(-1, base + j, false, false, tickets[j % Runner::SOLO_AHEAD]); },
+            [&](uint32_t j, bool& stop) -> int {
+                AK_TRY(r.solo_wait(tickets[j % Runner::SOLO_AHEAD], next));
+                s->cur_len = base + j + 1;
+                if (j + 1 < max_new) {   // (the last token is fed too, as in the reference's loop)
+                    out_tokens[(*n_out)++] = next;
+                    stop = stop_on_eos && next == eos;
+                }
+                return AK_OK;
+            },
+            [&]() { return r.sync(); });   // no one else uses the cache before the steps past the end have finished
     }
     for (uint32_t i = 0; i < max_new; i++) {
         out_tokens[(*n_out)++] = next;
@@ -266,7 +265,6 @@ int ak_session_generate(ak_session* s, const uint32_t* prompt, uint32_t n, uint3
     // Token i is sampled from the logits of the step before it, replaces the greedy pick that step left for the next one and
     // joins the history, all on the device; the host learns it from a word the sampler writes last. Samplers and decode steps
     // are launched ahead of the tokens: a step past an end-of-sequence token only writes cache rows beyond cur_len.
-    uint32_t launched = 0;
     const uint32_t ahead = r.solo() ? ak_session::PICKS - 1 : 1;
     auto launch = [&](uint32_t i) -> int {   // decode step i - 1 (i > 0), then the sampler of token i
         if (i > 0) AK_TRY(decode_launch(s, -1, base + i - 1, s->step_of[i % ak_session::PICKS]));
@@ -279,31 +277,26 @@ int ak_session_generate(ak_session* s, const uint32_t* prompt, uint32_t n, uint3
         return launch_sample_rows(st, r.logits_dev(), 1, V, r.logits_ld(), s->d_hist, nullptr, n + i, repetition_penalty, temperature, top_k, top_p, seed,
                                   i, nullptr, r.sampled_dev(), sink);
     };
-    for (uint32_t i = 0; i < max_new; i++) {
-        while (launched < max_new && launched <= most && launched < i + ahead) {
-            rc = launch(launched);
-            if (rc) return rc;
-            launched++;
-        }
-        rc = r.wait_word(s->h_pick + i % ak_session::PICKS, s->pick_of[i % ak_session::PICKS], next);
-        if (rc) return rc;
+    auto wait = [&](uint32_t i, bool& stop) -> int {
+        AK_TRY(r.wait_word(s->h_pick + i % ak_session::PICKS, s->pick_of[i % ak_session::PICKS], next));
         if (i > 0 && r.solo()) {   // (the step is done, the sampler ran behind it) were its logits good?
             uint32_t greedy;
             AK_TRY(r.solo_wait(s->step_of[i % ak_session::PICKS], greedy));
         }
         out_tokens[(*n_out)++] = next;
         s->cur_len = base + i;
-        if (stop_on_eos && next == eos) break;
-        if (i >= most) break;                                // out of context mid-generation: return what we have
-        if (i + 1 == max_new) {                              // the last token is fed too, as in the reference's loop
+        stop = stop_on_eos && next == eos;
+        if (!stop && i < most && i + 1 == max_new) {             // the last token is fed too, as in the reference's loop
             uint32_t ticket = 0, greedy;
-            rc = decode_launch(s, -1, base + i, ticket);
-            if (rc == AK_OK && r.solo()) rc = r.solo_wait(ticket, greedy);
-            if (rc) return rc;
+            AK_TRY(decode_launch(s, -1, base + i, ticket));
+            if (r.solo()) AK_TRY(r.solo_wait(ticket, greedy));
             s->cur_len = base + i + 1;
         }
-    }
-    return r.sync();   // steps launched past the end have finished before anyone else uses the cache
+        return AK_OK;
+    };
+    // (token `most` is the last there is context for)
+    AK_TRY(run_ahead(max_new <= most ? max_new : most + 1, ahead, launch, wait, [&]() { return r.sync(); }));
+    return r.sync();
 }
 
 int ak_session_read_cache(ak_session* s, uint32_t layer, float* k_out, float* v_out) {
