@@ -23,3 +23,61 @@ def test_wide_ffn_falls_back(ak, ctx, dim, heads, ffn):
         assert np.linalg.norm(got - want) < 2e-5 * np.linalg.norm(want)   # f32 sums of up to 24000 terms in another order
     ctx.check_device_status()
     s.close(); ref.close(); w.close()
+
+
+# Generation that ends at an end-of-sequence token: decode steps (and samplers) were launched past it and have written cache rows beyond
+# cur_len. The same session then goes on as if they had never run: a decode step, a second generate, a generate on a new cache.
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("sampler", [{}, dict(temperature=0.9, top_k=12, top_p=0.95, repetition_penalty=1.1, seed=5)])
+@pytest.mark.parametrize("cfg_args", [(40, 64, 1, 1, 64), (40, 60, 1, 1, 64)])   # the persistent step; the launch chain (head_dim 60)
+def test_session_goes_on_after_an_early_stop(ak, ctx, cfg_args, sampler, dtype):
+    if dtype == 1 and cfg_args[1] == 60:
+        cfg_args = (40, 32, 1, 1, 64)   # (bf16 wants a width of whole 16-byte vectors)
+    params = ak.synthetic_weights(ak.ModelConfig(*cfg_args), seed=3, std=0.3)
+    prompt, more = ak.uniform_tokens(5, 40, seed=1), ak.uniform_tokens(3, 40, seed=2)
+    N = 40
+    free = ak.ModelConfig(*cfg_args)
+    w = ak.ModelWeights.from_params(ctx, free, params, dtype)
+    s = ak.InferenceSession(ctx, w, 64)
+    full = s.generate(prompt, N, stop_on_eos=False, **sampler).tolist()
+    s.close(); w.close()
+    # the tokens whose first appearance is at the start, a little later, and in the middle
+    stops = [full[0]] + [t for i, t in enumerate(full) if t not in full[:i] and 0 < i < N - 1][:3]
+    assert len(stops) >= 2
+    for eos in stops:
+        cfg = ak.ModelConfig(*cfg_args, eos_token=int(eos))
+        w = ak.ModelWeights.from_params(ctx, cfg, params, dtype)
+        s, ref = ak.InferenceSession(ctx, w, 64), ak.InferenceSession(ctx, w, 64)
+        first = full.index(eos)
+        out = s.generate(prompt, N, stop_on_eos=True, **sampler)
+        assert out.tolist() == full[:first + 1]
+        assert s.cur_len == prompt.size + first          # the last token is not in the cache
+        # a session that was only given the tokens
+        ref.replace_cache()
+        ref.prefill(prompt)
+        for t in out[:-1]:
+            ref.decode_step(int(t))
+        for layer in range(cfg.num_layers):
+            for a, b in zip(s.read_cache(layer), ref.read_cache(layer)):
+                assert np.array_equal(a, b)
+        for t in more:
+            (ga, ta), (gb, tb) = s.decode_step(int(t)), ref.decode_step(int(t))
+            assert np.array_equal(ga, gb) and ta == tb
+        assert np.array_equal(s.generate(more, 9, stop_on_eos=True, **sampler), ref.generate(more, 9, stop_on_eos=True, **sampler))
+        assert s.cur_len == ref.cur_len
+        s.replace_cache()
+        assert s.generate(prompt, N, stop_on_eos=False, **sampler).tolist() == full
+        s.close(); ref.close(); w.close()
+    ctx.check_device_status()
+
+
+# The context fills before max_new: one token more than there are steps, whether the steps run ahead or not.
+@pytest.mark.parametrize("sampler", [{}, dict(temperature=0.9, top_k=12, top_p=0.95, repetition_penalty=1.1, seed=5)])
+@pytest.mark.parametrize("max_ctx,max_new,tokens,cur", [(20, 100, 16, 20), (20, 16, 16, 20), (20, 15, 15, 20), (20, 14, 14, 19), (5, 3, 1, 5), (20, 0, 0, 5)])
+def test_generate_fills_the_context(ak, ctx, sampler, max_ctx, max_new, tokens, cur):
+    cfg = ak.ModelConfig(40, 64, 1, 1, 64)
+    w = ak.ModelWeights.from_params(ctx, cfg, ak.synthetic_weights(cfg, seed=3, std=0.3), 0)
+    s = ak.InferenceSession(ctx, w, max_ctx)
+    out = s.generate(ak.uniform_tokens(5, 40, seed=1), max_new, stop_on_eos=False, **sampler)
+    assert len(out) == tokens and s.cur_len == cur
+    s.close(); w.close()
