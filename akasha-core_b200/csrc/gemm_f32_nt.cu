@@ -5,10 +5,11 @@
 // multiply-adds per instruction), K blocks of 16 double-buffered in shared memory with the next block's global loads in
 // flight. What bounds it is the FMA pipe (128 per SM and cycle, ~74 TFLOP/s); a 64-query prompt has too few tiles to reach
 // it, so K is split over a thread-block cluster and the partial tiles are added through distributed shared memory in rank
-// order. The split is a function of (n, k) only: a row's sum does not depend on how many rows share the launch.
+// order. The split is a function of (n, k) only: a row's sum does not depend on how many rows share the launch, one included.
 // The 64 x 64 tile with 4 x 4 outputs per thread it replaces moved a shared-memory word for every two FMAs:
 // 512 x 2304 x 768 took 126 us with it; a 512-token prefill of the 162M model 9.67 ms, 4.10 ms here.
-// m == 1 is a GEMV: a warp per output, the weights streamed once with 128-bit loads.
+// GEMV: a warp per output, the weights streamed once with 128-bit loads. Its order of sums is another one, so it is only for rows that
+// never share a launch (GEMM_ALONE: the decode row of a runner with one slot).
 #include <cooperative_groups.h>
 
 #include "kernels.h"
@@ -215,7 +216,7 @@ int launch_gemm_f32_nt(cudaStream_t st, const float* a, const float* wt, float* 
     using namespace ntf32;
     if (m == 0 || n == 0) return AK_OK;
     const bool vec = (k & 3u) == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)wt % 16 == 0;
-    if (m == 1) {
+    if (m == 1 && (flags & GEMM_ALONE)) {
         const uint32_t ctas = cdiv(n, GV_WARPS), room = B200_SMS * 8;
         return launch_k(gemv_kernel, dim3(ctas < room ? ctas : room), dim3(GV_WARPS * 32), 0, st, NO_CLUSTER, a, wt, c, n, k, flags, (uint32_t)vec);
     }

@@ -58,11 +58,12 @@ int launch_gather_paged(cudaStream_t st, const void* pool, uint32_t kv_dtype, co
                         float* out, uint32_t len, uint32_t heads, uint32_t head_dim, uint32_t block_size);
 
 // ---- gemm_simt.cu (true fp32) ---------------------------------------------------------------
-enum { GEMM_ADD = 1, GEMM_SILU = 2 };
+enum { GEMM_ADD = 1, GEMM_SILU = 2, GEMM_ALONE = 4 };
 // C[m,n] (+)= A[m,k] @ B[k,n], row-major f32. m == 1 uses the cluster split-K GEMV.
 int launch_gemm_f32(cudaStream_t st, const float* a, const float* b, float* c, uint32_t m, uint32_t n,
                     uint32_t k, uint32_t flags);
-// C[m,n] (+)= A[m,k] @ Wt[n,k]^T, row-major f32 (gemm_f32_nt.cu): the runner's f32 projections, stored [out,in].
+// C[m,n] (+)= A[m,k] @ Wt[n,k]^T, row-major f32 (gemm_f32_nt.cu): the runner's f32 projections, stored [out,in]. A row's sum does not
+// depend on m, except with GEMM_ALONE: the row never shares a launch, so that m == 1 may be a GEMV (another order of sums).
 int launch_gemm_f32_nt(cudaStream_t st, const float* a, const float* wt, float* c, uint32_t m, uint32_t n, uint32_t k, uint32_t flags);
 
 // ---- gemm_tcgen05.cu (bf16 tensor cores) --------------------------------------------------------

@@ -446,7 +446,8 @@ int Runner::wait_word(const uint64_t* w, uint32_t tag, uint32_t& value) {
 int Runner::gemm(const void* a, const void* wt, void* c, uint32_t m, uint32_t n, uint32_t k, int mode) {
     cudaStream_t st = ctx_->stream;
     if (w_->dtype == AK_F32) {
-        uint32_t flags = mode == 1 ? GEMM_ADD : (mode == 2 ? GEMM_SILU : 0);
+        // (one row: the decode row of a runner with one slot, or its lm_head)
+        const uint32_t flags = (mode == 1 ? GEMM_ADD : (mode == 2 ? GEMM_SILU : 0)) | GEMM_ALONE;
         return launch_gemm_f32_nt(st, (const float*)a, (const float*)wt, (float*)c, m, n, k, flags);
     }
     uint32_t epi = mode == 1 ? AK_EPI_ADD_F32 : (mode == 2 ? AK_EPI_SILU_BF16 : AK_EPI_STORE_F32);
@@ -481,9 +482,10 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
         // follow; the two kinds never read each other's rows, so an admission step runs them as two
         // ranges on two streams, joined before the final norm.
         const size_t act = dt == AK_F32 ? 4 : 2;
-        auto gemm_s = [&](cudaStream_t s, const void* a, const void* wt, void* cc, uint32_t m, uint32_t n, uint32_t k, int mode) -> int {
+        // alone: the launch's rows are decode rows only. A prompt's row may be the only one of a step, and is not the only one of the next
+        auto gemm_s = [&](cudaStream_t s, const void* a, const void* wt, void* cc, uint32_t m, uint32_t n, uint32_t k, int mode, bool alone) -> int {
             if (dt == AK_F32) {
-                const uint32_t flags = mode == 1 ? GEMM_ADD : (mode == 2 ? GEMM_SILU : 0);
+                const uint32_t flags = (mode == 1 ? GEMM_ADD : (mode == 2 ? GEMM_SILU : 0)) | (alone ? GEMM_ALONE : 0);
                 return launch_gemm_f32_nt(s, (const float*)a, (const float*)wt, (float*)cc, m, n, k, flags);
             }
             const uint32_t epi = mode == 1 ? AK_EPI_ADD_F32 : (mode == 2 ? AK_EPI_SILU_BF16 : AK_EPI_STORE_F32);
@@ -500,7 +502,7 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
             for (uint32_t l = 0; l < c.num_layers; l++) {
                 const auto& b = w_->blocks[l];
                 RC(launch_rmsnorm(s, hid, b.norm_1, xn, dt, nullptr, nr, D, c.norm_eps));
-                RC(gemm_s(s, xn, b.qkv, qkv, nr, 3 * Dq, D, 0));
+                RC(gemm_s(s, xn, b.qkv, qkv, nr, 3 * Dq, D, 0, dec));
                 // Decode rows get their head split, RoPE and cache append inside the attention kernel (head sizes the
                 // TMA kernel handles); the separate kernel then only serves the prompt rows of the range.
                 const bool fuse = dec && attn_decode_fused_supported(hd);
@@ -549,10 +551,10 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
                                                  d_desc_ + d_.pf_slot, d_desc_ + d_.pf_pos0, attn_, n_pf_seqs, max_pf_len, max_seqs_, H, hd, 16, scale,
                                                  dt, max_rows_, n_blocks_));
                 }
-                RC(gemm_s(s, at, b.out, hid, nr, D, Dq, 1));
+                RC(gemm_s(s, at, b.out, hid, nr, D, Dq, 1, dec));
                 RC(launch_rmsnorm(s, hid, b.norm_2, xn, dt, nullptr, nr, D, c.norm_eps));
-                RC(gemm_s(s, xn, b.up, up, nr, F, D, 2));
-                RC(gemm_s(s, up, b.down, hid, nr, D, F, 1));
+                RC(gemm_s(s, xn, b.up, up, nr, F, D, 2, dec));
+                RC(gemm_s(s, up, b.down, hid, nr, D, F, 1, dec));
             }
             return AK_OK;
         };

@@ -81,3 +81,30 @@ def test_generate_fills_the_context(ak, ctx, sampler, max_ctx, max_new, tokens, 
     out = s.generate(ak.uniform_tokens(5, 40, seed=1), max_new, stop_on_eos=False, **sampler)
     assert len(out) == tokens and s.cur_len == cur
     s.close(); w.close()
+
+
+# f32: a prompt's row has the same bits whether it is prefilled alone or with others (one token: one row in the launch), in a session and
+# in an engine with and without the padding of captured steps.
+@pytest.mark.parametrize("dim,heads,ffn", [(320, 5, 1280), (768, 12, 3072)])
+def test_one_token_prompt_f32(ak, ctx, dim, heads, ffn):
+    cfg = ak.ModelConfig(500, dim, heads, 3, 64, ffn)
+    w = ak.ModelWeights(ctx, cfg, ak.AK_F32)
+    w.init_synthetic(3, 0.05)
+    rows = []
+    for n in (1, 2, 40):
+        s = ak.InferenceSession(ctx, w, 64)
+        s.replace_cache()
+        s.prefill(np.arange(7, 7 + n, dtype=np.uint32))
+        rows.append([a[0].copy() for layer in range(3) for a in s.read_cache(layer)])
+        s.close()
+    for other in rows[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(rows[0], other))
+    outs = []
+    for prompts, graph in (([[7]], False), ([[7]], True), ([[7], [9, 11, 13]], False)):
+        e = ak.Engine(ctx, w, max_seqs=3, max_seq_len=48, use_cuda_graph=graph)
+        ids = [e.submit(p, 48) for p in prompts]
+        e.run_to_completion()
+        outs.append(e.poll(ids[0])[0].tolist())
+        e.close()
+    assert outs[0] == outs[1] == outs[2]
+    w.close()
