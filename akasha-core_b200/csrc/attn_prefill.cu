@@ -285,12 +285,14 @@ template <typename T, int HD, bool PAGED>
 static int launch_tiled(cudaStream_t st, const T* q, const T* k, const T* v, const int32_t* bt, uint32_t max_blocks,
                         const int32_t* cu, const int32_t* seq_slot, T* out, float* l_cache, uint32_t n_seqs,
                         uint32_t max_len, uint32_t row_base, uint32_t heads, float scale, uint32_t fixed_len) {
-    // 64-row query tiles when they already give two waves of CTAs, 32-row tiles when those give half a wave, else 16-row tiles.
-    // One prompt x 12 heads (f32, head_dim 64) with 16 / 32 / 64 rows: 512 tokens 93 / 57 / 52 us, 300 37 / 26 / 34, 201 25 / 21 / 27.
-    const uint64_t big = (uint64_t)cdiv(max_len, 64) * heads * n_seqs;
-    if (big >= 296)
+    // The smallest query tile whose CTAs still get an SM each: a smaller tile has the shorter chain, but two of its CTAs on one SM take
+    // longer than one of twice the rows. f32 with 16 / 32 / 64 rows, one prompt x 12 heads of 64: 160 tokens 15 / 17 / 21 us, 201
+    // 26 / 22 / 27, 384 46 / 32 / 41, 448 81 / 53 / 47, 512 93 / 58 / 53, 768 150 / 113 / 78; x 16 heads of 128: 128 21 / 23 / 29, 256
+    // 70 / 43 / 51, 300 85 / 84 / 61, 512 196 / 138 / 97. A row's sums are the same with any of them.
+    auto ctas = [&](uint32_t tile) { return (uint64_t)cdiv(max_len, tile) * heads * n_seqs; };
+    if (ctas(32) > B200_SMS)
         return launch_tiled_rpt<T, HD, PAGED, 4>(st, q, k, v, bt, max_blocks, cu, seq_slot, out, l_cache, n_seqs, max_len, row_base, heads, scale, fixed_len);
-    if (2 * big >= 80)
+    if (ctas(16) > B200_SMS)
         return launch_tiled_rpt<T, HD, PAGED, 2>(st, q, k, v, bt, max_blocks, cu, seq_slot, out, l_cache, n_seqs, max_len, row_base, heads, scale, fixed_len);
     return launch_tiled_rpt<T, HD, PAGED, 1>(st, q, k, v, bt, max_blocks, cu, seq_slot, out, l_cache, n_seqs, max_len, row_base, heads, scale, fixed_len);
 }

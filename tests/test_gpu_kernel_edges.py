@@ -269,3 +269,28 @@ def test_gemm_skinny_rows(ak, torch_cuda, m, n, k):
     assert float((c[:m].double() - want).abs().max()) < 8 * k * 2.0 ** -24
     assert bool((c[m] == 3.0).all())
     ak.check(ak.lib().ak_check_device_status(None))
+
+
+# f32 prefill attention: 16-, 32- and 64-row query tiles, the choice going by the CTAs of the launch. A prompt alone (each tile in turn) and
+# with enough others for the largest tile: the same bits. The line between two tiles: 12 heads x 12 tiles are 144 CTAs, x 13 are 156.
+@pytest.mark.parametrize("heads,hd,L", [(12, 64, 192), (12, 64, 193), (12, 64, 384), (12, 64, 385), (5, 64, 464), (5, 64, 465), (16, 128, 144), (16, 128, 145), (16, 128, 289)])
+def test_attn_prefill_f32_tile_choice(ak, torch_cuda, heads, hd, L):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(L)
+    n, mb = 8, (L + 15) // 16
+    kp, vp = (torch.randn(n * mb, heads, 16, hd, device="cuda", generator=g) for _ in range(2))
+    tables = torch.randperm(n * mb, device="cuda", generator=g).to(torch.int32).reshape(n, mb)
+    q = torch.randn(n * L, heads * hd, device="cuda", generator=g)
+    outs = []
+    for k in (1, n):
+        cu = torch.arange(0, (k + 1) * L, L, dtype=torch.int32, device="cuda")
+        out = torch.full((k * L, heads * hd), float("nan"), device="cuda")
+        ak.ops.attn_prefill_paged(q[:k * L].contiguous(), kp, vp, tables, mb, cu, torch.arange(k, dtype=torch.int32, device="cuda"), out, k, L, k * L, heads, hd,
+                                  hd ** -0.5, ak.AK_F32, n * mb)
+        outs.append(out[:L])
+    assert torch.equal(outs[0], outs[1])
+    k, v = (p[tables[0].long()].transpose(1, 2).reshape(mb * 16, heads, hd)[:L].double().transpose(0, 1) for p in (kp, vp))
+    s = torch.einsum("lhd,hkd->hlk", q[:L].double().reshape(L, heads, hd), k) * hd ** -0.5
+    s.masked_fill_(torch.ones(L, L, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    want = torch.einsum("hlk,hkd->lhd", s.softmax(-1), v).reshape(L, -1)
+    assert float((outs[0].double() - want).abs().max()) < 2e-5   # f32 sums of up to 465 terms
