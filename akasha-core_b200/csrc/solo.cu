@@ -174,6 +174,13 @@ template <> struct Vec<bf16> {
     }
 };
 
+// 1 / sqrt(m): the hardware's approximation and one Newton step (below 1 ulp). The step has no value where m is 0 or infinite (a
+// residual stream whose squares overflow): there the approximation is exact.
+__device__ __forceinline__ float inv_rms(float m) {
+    const float y = rsqrtf(m);
+    return y > 0.0f && y < INFINITY ? y * fmaf(-0.5f * m * y, y, 1.5f) : y;
+}
+
 struct Ring {
     uint8_t* base;
     uint64_t *full, *empty;
@@ -508,9 +515,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
                 for (int i = 0; i < NW; i++) u[i] = part_ss[i];
 #pragma unroll
                 for (int i = 0; i < NW / 4; i++) u[i] = (u[4 * i] + u[4 * i + 1]) + (u[4 * i + 2] + u[4 * i + 3]);
-                // 1 / rms: the hardware's approximation and one Newton step (below 1 ulp)
-                const float m = ((u[0] + u[1]) + u[2]) * inv_d + a.eps, y = rsqrtf(m);
-                rs = y * fmaf(-0.5f * m * y, y, 1.5f);
+                rs = inv_rms(((u[0] + u[1]) + u[2]) * inv_d + a.eps);
             }
 #pragma unroll 1
             for (uint32_t j0 = 0; j0 < d.rows; j0 += d.blk, buf ^= 1u) {
@@ -695,7 +700,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
         ss = 0.0f;
 #pragma unroll
         for (int i = 0; i < NW; i++) ss += part_ss[i];
-        const float m = ss / (float)D + a.eps, y = rsqrtf(m), rs = y * fmaf(-0.5f * m * y, y, 1.5f);
+        const float rs = inv_rms(ss / (float)D + a.eps);
         const float* const x_all = reinterpret_cast<const float*>(kv_sm + NA * 2 * KV_TILE);
         float* const logit_sm = reinterpret_cast<float*>(kv_sm);   // (no cache tile is in use any more)
         float bv = -INFINITY;

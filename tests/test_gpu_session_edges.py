@@ -108,3 +108,19 @@ def test_one_token_prompt_f32(ak, ctx, dim, heads, ffn):
         e.close()
     assert outs[0] == outs[1] == outs[2]
     w.close()
+
+
+# A residual stream whose squares overflow f32: the norm's factor is 0 (1 / sqrt(inf)), so every logit is 0, in the step as in a prefill.
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_step_with_an_overflowing_norm(ak, ctx, dtype):
+    cfg = ak.ModelConfig(200, 128, 2, 2, 64)
+    params = ak.synthetic_weights(cfg, seed=1, std=0.05)
+    params[0] = params[0] * np.float32(1e22)
+    w = ak.ModelWeights.from_params(ctx, cfg, params, dtype)
+    s = ak.InferenceSession(ctx, w, 64)
+    s.replace_cache()
+    want, tok = s.prefill([3, 4, 5])
+    assert tok == 0 and np.array_equal(want, np.zeros(200, np.float32))
+    got, tok = s.decode_step(6)
+    assert tok == 0 and np.array_equal(got, want)
+    s.close(); w.close()
