@@ -210,14 +210,6 @@ rmsnorm_stream_kernel(float* __restrict__ x, const float* __restrict__ residual,
     const uint32_t step = rows_per_warp ? 4 : gridDim.x * 4;
     uint32_t row = blockIdx.x * 4 * (rows_per_warp ? rows_per_warp : 1) + (threadIdx.x >> 5);
     const uint32_t row_end = rows_per_warp ? min(rows, (blockIdx.x + 1) * 4 * rows_per_warp) : rows;
-    float4 g[AHEAD ? NV : 1];
-    if (AHEAD) {
-#pragma unroll
-        for (int c = 0; c < NV; c++) {
-            const uint32_t i = lane + 32u * c;
-            g[AHEAD ? c : 0] = i < nv ? reinterpret_cast<const float4*>(w)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
     // head_dim divides 128 (launcher), so all of a lane's float4 sit at the same offset d0 of their heads. head_dim <= 64:
     // lane j evaluates angle j mod (head_dim / 2) and lanes trade; head_dim = 128: every lane evaluates its own two.
     const uint32_t half = head_dim >> 1, d0 = ROPE ? (lane * 4) % head_dim : 0;
@@ -226,8 +218,11 @@ rmsnorm_stream_kernel(float* __restrict__ x, const float* __restrict__ residual,
         f0 = 1.0f / powf(10000.0f, (float)(head_dim <= 64 ? 2 * (lane & (half - 1)) : d0) / (float)head_dim);
         if (head_dim > 64) f1 = 1.0f / powf(10000.0f, (float)(d0 + 2) / (float)head_dim);
     }
+    // The weights may be the preceding kernel's output: read after the wait, but asked for from HBM before it (the L2 is coherent).
+    if (AHEAD && threadIdx.x * 32 < size) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + threadIdx.x * 32));
     pdl_wait();
     pdl_trigger();
+    float4 g[AHEAD ? NV : 1];
     float4 v[NV], nx[AHEAD ? NV : 1], nr[AHEAD && HAS_RES ? NV : 1];
     int32_t pos = 0, npos = 0;
     auto request = [&](uint32_t r) {   // the row's loads into the "next" registers
@@ -244,6 +239,13 @@ rmsnorm_stream_kernel(float* __restrict__ x, const float* __restrict__ residual,
         if (ROPE) npos = positions[r];
     };
     if (AHEAD && row < row_end) request(row);
+    if (AHEAD) {
+#pragma unroll
+        for (int c = 0; c < NV; c++) {
+            const uint32_t i = lane + 32u * c;
+            g[AHEAD ? c : 0] = i < nv ? reinterpret_cast<const float4*>(w)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
     for (; row < row_end; row += step) {
         float4* xr = reinterpret_cast<float4*>(x + (size_t)row * size);
         float ss = 0.0f;

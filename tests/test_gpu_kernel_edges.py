@@ -294,3 +294,25 @@ def test_attn_prefill_f32_tile_choice(ak, torch_cuda, heads, hd, L):
     s.masked_fill_(torch.ones(L, L, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
     want = torch.einsum("hlk,hkd->lhd", s.softmax(-1), v).reshape(L, -1)
     assert float((outs[0].double() - want).abs().max()) < 2e-5   # f32 sums of up to 465 terms
+
+
+# The streaming RMSNorm reads everything behind its dependency wait: norm weights that the launch before it has just written (a GEMM whose
+# dependents may start while it runs) are the new ones.
+@pytest.mark.parametrize("size,hd", [(320, 0), (768, 64), (1024, 128)])
+def test_rmsnorm_stream_weights_just_written(ak, torch_cuda, size, hd):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(size)
+    x = torch.randn(3000, size, device="cuda", generator=g)
+    a, wt = torch.randn(1, 8192, device="cuda", generator=g).bfloat16(), (0.01 * torch.randn(size, 8192, device="cuda", generator=g)).bfloat16()
+    pos = torch.arange(3000, device="cuda", dtype=torch.int32) if hd else None
+    y, want = (torch.empty(3000, size, device="cuda") for _ in range(2))
+    w = torch.empty(size, device="cuda")
+    ak.ops.gemm_bf16(a, wt, w, 1, size, 8192, ak.EPI_STORE_F32)
+    torch.cuda.synchronize()
+    ak.ops.rmsnorm_rope_residual(x, None, w, want, pos, 3000, size, 1e-5, hd, ak.AK_F32)
+    for _ in range(10):
+        w.fill_(float("nan"))
+        torch.cuda.synchronize()
+        ak.ops.gemm_bf16(a, wt, w, 1, size, 8192, ak.EPI_STORE_F32)
+        ak.ops.rmsnorm_rope_residual(x, None, w, y, pos, 3000, size, 1e-5, hd, ak.AK_F32)
+        assert torch.equal(y, want)
