@@ -434,8 +434,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
             const uint32_t u = u_begin + r * NA + lane_;
             if (lane_ >= NA || u >= u_end || !ok) return;
             const uint32_t p0 = u * UP;
-            const uint32_t blk = a.table ? (uint32_t)__ldg(a.table + (p0 >> 4)) : (p0 >> 4);
-            const size_t o = (((size_t)blk * H + head) * 16 + (p0 & 15)) * HD;
+            const size_t o = (((size_t)(p0 >> 4) * H + head) * 16 + (p0 & 15)) * HD;
             if (kv_sent > 0 && !wait_full(&kv_empty[lane_], (kv_sent - 1) & 1u, &dead)) { ok = false; return; }
             uint8_t* const dst = kv_sm + lane_ * 2 * KV_TILE;
             mbar_expect_tx(&kv_full[lane_], 2 * KV_TILE);
@@ -570,7 +569,6 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
         if (lane == 0) {
             const uint32_t tok = bi < V ? bi : 0u;   // (no logit above -inf: 0)
             *a.sampled = tok;
-            if (a.sampled_host) *(volatile uint32_t*)a.sampled_host = tok;
             if (a.done_host) {
                 __threadfence_system();
                 *(volatile uint64_t*)a.done_host = (uint64_t)(failed ? STEP_FAILED : tok) | ((uint64_t)ep << 32);
@@ -810,8 +808,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
                 vec_of(2, t);
                 vn = Vec<T>::put(t);
                 if (sub == 0) {
-                    const uint32_t blk = a.table ? (uint32_t)__ldg(a.table + (a.pos >> 4)) : (a.pos >> 4);
-                    const size_t o = (((size_t)blk * H + head) * 16 + (a.pos & 15)) * HD + lv * EPV;
+                    const size_t o = (((size_t)(a.pos >> 4) * H + head) * 16 + (a.pos & 15)) * HD + lv * EPV;
                     *reinterpret_cast<uint4*>(reinterpret_cast<T*>(w.k_pool) + o) = kn;
                     *reinterpret_cast<uint4*>(reinterpret_cast<T*>(w.v_pool) + o) = vn;
                 }

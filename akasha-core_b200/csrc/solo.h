@@ -13,7 +13,7 @@ struct SoloLayer {   // device array, one per layer; matrices [out, in]
     const float* norm_2;
     const void* up;
     const void* down;
-    void* k_pool;
+    void* k_pool;                // block i of the pools holds positions 16 i .. 16 i + 15 of the sequence
     void* v_pool;
 };
 
@@ -23,12 +23,10 @@ struct SoloArgs {
     const float* final_norm;
     const void* lm_head;
     const float2* rope;          // [rope_len][head_dim / 2] (cos, sin)
-    const int32_t* table;        // block table of the sequence on the device; nullptr = identity
     uint64_t* xch;               // solo_xch_words() 64-bit words, zero before the first launch
     uint32_t* sampled;           // device word: the token fed back when tok_src < 0, overwritten by the greedy pick
     float* logits;               // [vocab] device, or nullptr
     float* logits_host;          // [vocab] mapped host memory, or nullptr
-    uint32_t* sampled_host;      // mapped host word, or nullptr
     uint64_t* done_host;         // mapped host word {token, or solo::STEP_FAILED; step}: written after everything else, or nullptr
     uint32_t n_layers, dim, ffn, heads, vocab;
     uint32_t pos;                // position of the token fed in; positions 0 .. pos are attended to
