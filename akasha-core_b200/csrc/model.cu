@@ -369,23 +369,28 @@ int Runner::init(ak_ctx* ctx, ak_weights* w, uint32_t max_seqs, uint32_t max_seq
     AK_CUDA(cudaStreamCreateWithFlags(&st_time_, cudaStreamNonBlocking));
     AK_CUDA(cudaEventCreateWithFlags(&ev_tfork_, cudaEventDisableTiming));
     AK_CUDA(cudaEventCreateWithFlags(&ev_tjoin_, cudaEventDisableTiming));
-    solo_ = max_seqs == 1 && tp_ == 1 && solo_supported(w->dtype, D, F, H, c.num_layers, V);
-    if (solo_) {
-        std::vector<SoloLayer> sl(c.num_layers);
-        for (uint32_t l = 0; l < c.num_layers; l++) {
-            const auto& b = w->blocks[l];
-            sl[l] = {b.norm_1, b.qkv, b.out, b.norm_2, b.up, b.down, k_pool_[l], v_pool_[l]};
-        }
-        const size_t words = solo_xch_words(D, F, H, c.num_layers);
-        AK_CUDA(cudaMalloc((void**)&d_solo_layers_, sl.size() * sizeof(SoloLayer)));
-        AK_CUDA(cudaMemcpyAsync(d_solo_layers_, sl.data(), sl.size() * sizeof(SoloLayer), cudaMemcpyHostToDevice, ctx->stream));
-        AK_CUDA(cudaMalloc((void**)&d_solo_xch_, words * 8));
-        AK_CUDA(cudaMemsetAsync(d_solo_xch_, 0, words * 8, ctx->stream));
-        AK_CUDA(cudaMallocHost((void**)&h_solo_done_, SOLO_AHEAD * 8));
-        memset(h_solo_done_, 0, SOLO_AHEAD * 8);
-        AK_CUDA(cudaMallocHost((void**)&h_logits_, (size_t)V * 4));
-    }
     AK_CUDA(cudaStreamSynchronize(ctx->stream));
+    return AK_OK;
+}
+
+int Runner::init_solo() {
+    const ak_model_config& c = w_->cfg;
+    if (max_seqs_ != 1 || tp_ != 1 || !solo_supported(w_->dtype, c.dim, c.ffn_hidden, c.num_heads, c.num_layers, c.vocab_size)) return AK_OK;
+    std::vector<SoloLayer> sl(c.num_layers);
+    for (uint32_t l = 0; l < c.num_layers; l++) {
+        const auto& b = w_->blocks[l];
+        sl[l] = {b.norm_1, b.qkv, b.out, b.norm_2, b.up, b.down, k_pool_[l], v_pool_[l]};
+    }
+    const size_t words = solo_xch_words(c.dim, c.ffn_hidden, c.num_heads, c.num_layers);
+    AK_CUDA(cudaMalloc((void**)&d_solo_layers_, sl.size() * sizeof(SoloLayer)));
+    AK_CUDA(cudaMemcpyAsync(d_solo_layers_, sl.data(), sl.size() * sizeof(SoloLayer), cudaMemcpyHostToDevice, ctx_->stream));
+    AK_CUDA(cudaMalloc((void**)&d_solo_xch_, words * 8));
+    AK_CUDA(cudaMemsetAsync(d_solo_xch_, 0, words * 8, ctx_->stream));
+    AK_CUDA(cudaMallocHost((void**)&h_solo_done_, SOLO_AHEAD * 8));
+    memset(h_solo_done_, 0, SOLO_AHEAD * 8);
+    AK_CUDA(cudaMallocHost((void**)&h_logits_, (size_t)c.vocab_size * 4));
+    AK_CUDA(cudaStreamSynchronize(ctx_->stream));
+    solo_ = true;
     return AK_OK;
 }
 

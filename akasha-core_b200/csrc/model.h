@@ -102,6 +102,8 @@ class Runner {
     // blocks until step t (the value solo_launch gave) is done and returns its greedy token. At most SOLO_AHEAD steps may
     // be unwaited for. logits_host (with `want_logits`): the step's logits in pinned host memory, valid after solo_wait.
     static constexpr uint32_t SOLO_AHEAD = 4;
+    // init_solo() sets it up; only a session, whose blocks lie in order, calls it.
+    int init_solo();
     bool solo() const { return solo_; }
     int solo_launch(int32_t tok_src, uint32_t pos, bool want_logits, bool host_logits, uint32_t& ticket);
     int solo_wait(uint32_t ticket, uint32_t& token);   // AK_ERR_DEVICE_WAIT: a wait of the step ran out, there is no token

@@ -47,6 +47,7 @@ int ak_session_create(ak_ctx* ctx, ak_weights* w, uint32_t max_context_len, ak_s
     s->w = w;
     s->max_ctx = max_context_len;
     int rc = s->runner.init(ctx, w, 1, max_context_len, 0, max_context_len);
+    if (rc == AK_OK) rc = s->runner.init_solo();
     if (rc) {
         delete s;
         return rc;
