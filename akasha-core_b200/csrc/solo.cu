@@ -528,6 +528,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
                 for (int i = 0; i < NW / 4; i++) t[i] = (t[4 * i] + t[4 * i + 1]) + (t[4 * i + 2] + t[4 * i + 3]);
                 float v = ((t[0] + t[1]) + t[2]) * rs;
                 if (mine) {
+                    // (bf16 weights: off by 2^-17 of the value at most, and 0 below about -87)
                     if (ph == 2) v = sizeof(T) == 4 ? v / (1.0f + expf(-v)) : __fdividef(v, 1.0f + __expf(-v));
                     ll_put(dst, copy, v, ep);
                 }

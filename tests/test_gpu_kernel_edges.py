@@ -316,3 +316,23 @@ def test_rmsnorm_stream_weights_just_written(ak, torch_cuda, size, hd):
         ak.ops.gemm_bf16(a, wt, w, 1, size, 8192, ak.EPI_STORE_F32)
         ak.ops.rmsnorm_rope_residual(x, None, w, y, pos, 3000, size, 1e-5, hd, ak.AK_F32)
         assert torch.equal(y, want)
+
+
+# SiLU in the GEMM's epilogue over its whole range of arguments, both kernels: to half an ulp of bf16 (at most 2^-8 of the value; the quotient
+# itself is within 2^-16), and below 2e-36 where the denominator exp(-v) passes 2^126 (v < -87): there the result is 0.
+@pytest.mark.parametrize("m", [64, 1100])
+def test_gemm_silu_range(ak, torch_cuda, m):
+    torch = torch_cuda
+    n, k = 264, 8
+    c = torch.linspace(-110.0, 110.0, m).bfloat16()
+    d = torch.cat((torch.linspace(-1.0, 1.0, 200), torch.tensor([0.0, -0.0, 1e-30, -1e-30, 88.0, -88.0, 1000.0, -1000.0, 1e20, -1e20, 3e38, -3e38]),
+                   torch.linspace(-0.01, 0.01, 52))).bfloat16()
+    a, wt = torch.zeros(m, k, dtype=torch.bfloat16), torch.zeros(n, k, dtype=torch.bfloat16)
+    a[:, 0], a[:, 1], wt[:, 0], wt[:, 1] = c, 1.0, 1.0, d
+    out = torch.full((m, n), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ak.ops.gemm_bf16(a.cuda(), wt.cuda(), out, m, n, k, ak.EPI_SILU_BF16)
+    v = (c.double()[:, None] + d.double()[None, :]).float().double()      # the sum in f32
+    want = v / (1.0 + torch.exp(-v))
+    err = (out.cpu().double() - want).abs()
+    assert bool((err <= (2.0 ** -8 + 2.0 ** -16) * want.abs() + 2e-36).all())
+    assert bool((out.cpu()[v < -90.0] == 0.0).all()) and not bool(out.isnan().any())
