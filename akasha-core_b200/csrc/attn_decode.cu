@@ -48,6 +48,7 @@ constexpr int DEC_BS = 16;          // positions per KV block
 constexpr int DEC_MIN_BLOCKS = 4;   // a split never gets fewer KV blocks than this (one per warp)
 // Sequences of up to this many blocks stay in one CTA: four blocks per warp cost less than publishing, counting and merging
 // partials. Decode step of the 162M model, 8 sequences: 399 us unsplit against 415 us at 200 positions, 437 against 423 at 440.
+// (Longer sums per warp: f32 error against f64 2.2e-7 -> 2.8e-7 at 512 positions, bf16 1.01 to 1.06 times.)
 constexpr uint32_t DEC_UNSPLIT_BLOCKS = 16;
 // ... and a launch that would have to clear the arrival counters first (another ~2.5 us on the stream) splits later still: one
 // sequence x 12 heads, clearing included, 8.2 us unsplit against 10.1 us at 512 positions, 11.7 against 10.3 at 800.

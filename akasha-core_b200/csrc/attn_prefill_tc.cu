@@ -130,8 +130,10 @@ template <int HD, int QT> struct Cfg {
     static constexpr int THREADS = 64 + QT * 256;          // warp 0: TMA, warp 1: MMA; then two softmax warpgroups per query tile
 };
 // A row keeps the maximum its exponents are taken from until a tile exceeds it by more than this (in powers of two): the
-// probabilities then stay below 2^8, which costs bf16 and f32 no relative precision, and the output tile, which
-// accumulates in TMEM, is almost never rescaled.
+// probabilities then stay below 2^8 and the output tile, which accumulates in TMEM, is almost never rescaled. bf16's relative
+// rounding is the same at any size, but under a maximum that always follows the largest probability of a tile is 1, without rounding:
+// the output's error against f64 is 1.00 to 1.02 times as large for it (2.01e-3 -> 2.04e-3, 16 prompts of 128 to 3072, head_dim 128),
+// 1.07 for scores of standard deviation 4. Following always: 330 -> 349 us on those prompts.
 constexpr float RESCALE_LOG2 = 8.0f;
 
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {

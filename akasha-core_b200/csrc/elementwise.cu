@@ -1269,7 +1269,7 @@ sample_rows_kernel(const float* __restrict__ logits, uint32_t n, uint32_t ld, co
         return;
     }
     // ---- f64 softmax over the candidates (candidates that ran out end the list)
-    double* const e = reinterpret_cast<double*>(srow);   // the row is not needed any more: k <= n, and (n + bitmap) floats hold k doubles for n >= 2 k; else in place below
+    double* const e = reinterpret_cast<double*>(srow);   // the row is not needed any more; its n floats hold k doubles (room), or the values are formed again where they are used
     __shared__ double shared_sum;
     const bool room = 2 * k <= n;
     const double mx = (double)cand_v[0], T = (double)temperature;

@@ -867,7 +867,8 @@ static constexpr uint32_t SMEM_ONE_PER_SM = 220 * 1024;
 static constexpr uint32_t SMEM_PAIR = 226 * 1024;         // the pair kernel: all a CTA may have but its few hundred static bytes
 // Launches of more than 48 rows claim at least this much: with small footprints the waiting CTAs of three or four launches of the
 // chain share an SM, and their activation traffic meets. Decode step of the 162M model, 64 rows: 515 -> 505 us. (40 rows: 441 ->
-// 445 us; there, and below, the deeper the chain stacks up the better.)
+// 445 us; there, and below, the deeper the chain stacks up the better.) Measured at these two row counts of this model only; the
+// line between them, and other shapes, are not.
 static constexpr uint32_t SMEM_MIN_WIDE = 78 * 1024;
 static constexpr uint32_t SMEM_THREE_PER_SM = 74 * 1024;  // three CTAs fit one SM below this (228 KB, 1 KB reserved and ~0.25 KB static per CTA)
 
@@ -907,9 +908,10 @@ static GemmPlan plan_gemm(uint32_t m, uint32_t n, uint32_t k, bool allow_split, 
         if (sk.ks > 1) {
             const uint32_t mt = cdiv(m, GB_M);
             if (mt <= 4 && sk.ks == 2) {
-                // qkv / ffn-up with a prompt or two beside the decode rows: the two K halves as two accumulators
-                // of one CTA (same summation structure as the 2-CTA cluster exchange of the decode plan, without
-                // the exchange); measured 3-6 % off an admission step against the cluster form
+                // A projection whose K the skinny plan halves (qkv and ffn-up of the 1.4B model, qkv and out-proj of the 320-wide
+                // one), a prompt or two beside the decode rows: the two K halves as two accumulators of one CTA (same summation
+                // structure as the 2-CTA cluster exchange of the decode plan, without the exchange); it took 3-6 % off an
+                // admission step of the 162M model when that model's qkv and ffn-up were halved too
                 p.kseg = 2; p.ks = 1; p.bn = 64;
                 uint32_t st = (SMEM_THREE_PER_SM - 1024) / stage_bytes(p.bn);   // three per SM: these run beside the decode rows' chain
                 if (st > G_MAX_STAGES) st = G_MAX_STAGES;
@@ -985,7 +987,8 @@ static GemmPlan plan_gemm(uint32_t m, uint32_t n, uint32_t k, bool allow_split, 
             // occupies the tensor core 50 cycles for any N <= 64), a cluster exchange ~1.2 us. Split long K chains (K > 1024),
             // and short ones only when the unsplit grid would cover less than half of the SMs. Measured in a chain of
             // launches: 64 x 2304 x 768 4.4 us unsplit (144 CTAs of 16 columns), 5.6 us in two halves; 8 x 1280 x 320 3.1
-            // against 4.3 us; 8 x 768 x 768 3.4 us split four ways, 5.2 us unsplit.
+            // against 4.3 us; 8 x 768 x 768 3.4 us split four ways, 5.2 us unsplit. (f32 error against f64 at K = 768: 7.3e-7
+            // unsplit, as the large-m plans have it, 3.5e-7 in halves: the tensor core's sums are that much longer.)
             const bool short_k_ok = cdiv(n, 16) * 2 <= B200_SMS;
             if (ks > 1 && num_kb <= 16 && !short_k_ok) continue;
             if (ks > 1 && (!allow_split || ks * 2 > num_kb || (bn / ks) % 4 != 0)) continue;
