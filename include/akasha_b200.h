@@ -332,7 +332,8 @@ AK_API uint32_t ak_session_cur_len(const ak_session* s);
 /* prefill (src/nn/inference.rs:61-176). logits_out: host f32[vocab] or NULL;
  * argmax_out: host uint32 or NULL (greedy token of the returned logits, computed on device). */
 AK_API int ak_session_prefill(ak_session* s, const uint32_t* tokens, uint32_t n, float* logits_out, uint32_t* argmax_out);
-/* decode_step (src/nn/inference.rs:178-262). */
+/* decode_step (src/nn/inference.rs:178-262). It and generate return AK_ERR_DEVICE_WAIT where a device-side wait of the
+ * step ran out: that step gave no token and is not in the cache. */
 AK_API int ak_session_decode_step(ak_session* s, uint32_t token, float* logits_out, uint32_t* argmax_out);
 /* generate (src/nn/inference.rs:264-326) with temperature <= 0 and repetition_penalty == 1
  * (greedy, src/nn/sampling.rs:30-32): attaches a cache if none, prefill when the cache is empty
