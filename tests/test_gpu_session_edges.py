@@ -124,3 +124,61 @@ def test_step_with_an_overflowing_norm(ak, ctx, dtype):
     got, tok = s.decode_step(6)
     assert tok == 0 and np.array_equal(got, want)
     s.close(); w.close()
+
+
+# Two sessions on two contexts (streams) and an engine on a third, each in a thread of its own: a decode step needs every SM at once, the
+# others' kernels take them meanwhile. Every thread gets the tokens that it gets alone.
+def test_sessions_and_engine_in_threads(ak, ctx):
+    import threading
+    cfg = ak.ModelConfig(1000, 320, 5, 3, 256, 1280)
+    ctxs = [ak.Context(0) for _ in range(3)]
+    ws = [ak.ModelWeights(c, cfg, dt) for c, dt in zip(ctxs, (0, 1, 1))]
+    for w in ws:
+        w.init_synthetic(4, 0.05)
+    prompts = [ak.uniform_tokens(9 + 5 * i, 1000, seed=i) for i in range(6)]
+
+    def session(i):
+        s = ak.InferenceSession(ctxs[i], ws[i], 256)
+        out = []
+        for p in prompts[:4]:
+            s.replace_cache()
+            out.append(s.generate(p, 60, stop_on_eos=False).tolist())
+            s.replace_cache()
+            out.append(s.generate(p, 40, stop_on_eos=False, temperature=0.8, top_k=20, top_p=0.9, repetition_penalty=1.1, seed=i).tolist())
+        s.close()
+        return out
+
+    def engine(i):
+        e = ak.Engine(ctxs[i], ws[i], max_seqs=4, max_seq_len=128, use_cuda_graph=True)
+        out = []
+        for _ in range(3):
+            ids = [e.submit(p, 120) for p in prompts]
+            e.run_to_completion()
+            out += [e.poll(k)[0].tolist() for k in ids]
+            e.clear_finished()
+        e.close()
+        return out
+
+    jobs = [lambda: session(0), lambda: session(1), lambda: engine(2)]
+    alone = [j() for j in jobs]
+    for _ in range(2):
+        got, errors = [None] * 3, []
+
+        def work(k):
+            try:
+                got[k] = jobs[k]()
+            except Exception as e:   # noqa: BLE001
+                errors.append(e)
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not errors, errors
+        assert got == alone
+    for c in ctxs:
+        c.check_device_status()
+    for w in ws:
+        w.close()
+    for c in ctxs:
+        c.close()
