@@ -1,0 +1,1264 @@
+// One decode step of up to 32 sequences (bf16 weights and cache) as a single persistent kernel: embedding, every layer,
+// lm_head, greedy argmax.
+//
+// What bounds it. A decode-only step as a chain of 88 launches is bound by the launches: each is a boundary of ~2 us plus the latencies
+// of its first loads, 3 to 5 us for work of 0.1 to 1 us (162M model, 8 sequences of 300: 0.39 ms; the bytes take 0.05 ms). Here, as in the
+// batch-1 step (solo.cu), a layer is five phases of one kernel and only activations cross the chip:
+//   qkv rows -> attention (sequence, head) -> out-proj rows -> ffn-up rows -> ffn-down rows.
+// That step takes 0.205 ms (1 sequence 0.18, 16 of 350 0.27, 32 of 350 0.35; 320-wide model, 21 sequences 0.22 -> 0.143; 1.4B model, 16 of 1600
+// 2.5 -> 2.25). With 64 sequences a layer was slower than the chain's (every SM reads all activations: 0.58 against 0.49 ms), hence the limit of 32.
+// What is left is latency: per phase ~1 us from a store to the last SM's poll and ~1 us of dependent instructions, ~5 cycles each (with
+// everything between two phases done by the same warps it was 0.29 ms; with 40 bytes of spills 0.36).
+//   * A producer thread per SM walks the SM's weight tiles of all phases in order and keeps a shared-memory ring of tensor loads full.
+//   * A phase's rows are dealt to the SMs in tiles of 8, all of K: no sum crosses SMs. The 12 compute warps split K and leave partial tiles in
+//     shared memory; three epilogue warps add them in warp order and publish, while the compute warps are already at the next phase. The
+//     products are mma.m16n8k16 with 16 sequences on the M side and 8 weight rows on the N side: a tcgen05 tile (128 x 8 at least,
+//     operands through shared memory, the result back through tensor memory) costs more latency than these few products take.
+//   * Activations are published in the order of the MMA's A fragments (a lane's 8 consecutive k of a sequence are one 16-byte vector), so
+//     that a warp's fragment is one coalesced 512-byte load from L2 straight into registers. Both operands use the same order of k. What a
+//     tile publishes for 8 sequences is one 128-byte line (as 16-byte pieces of four lines: 1.6 us instead of 0.95 until the last SM had it).
+//   * A value is its own flag: an exchange buffer holds 0xffffffff words until it is written, a NaN no conversion and no arithmetic
+//     gives, and consumers poll the words they need. No fence and no second round trip between the value and its flag. Three sets of
+//     buffers are used in turn by the layers; the one of the layer before is filled with 0xff again after a layer's ffn-up (see clear).
+//   * RMS norm: the producer of the residual stream publishes x * gain rounded to bf16 (one rounding, as of the normalised value) and
+//     the sums of squares of its columns; 1 / rms is a factor of the row sums of the next phase, found by the epilogue warps meanwhile.
+//   * The residual stream stays in shared memory of the SM that owns its columns (out-proj and ffn-down have the same tiles).
+//   * Attention: a unit is (sequence, head, split of split_len positions); units are dealt to groups of 4 or 12 warps in order of length. Keys
+//     and values go through per-warp shared-memory buffers, the next layer's first tiles already while this layer's ffn runs. Scores are
+//     mma.m16n8k16 (7/8 of it for nothing, but an eighth of the instructions of f32 FMAs); P V is f32 FMAs, the transposing loads that an
+//     MMA would need have 8-way bank conflicts on unswizzled tiles (32 sequences: 0.41 ms instead of 0.35).
+//
+// Arithmetic: bf16 inputs rounded once, f32 products and sums, as in the launch chain; the probabilities stay f32. The order of every sum
+// depends on the model and on the number of slots only, never on which other sequences are there.
+//
+// The grid is launched cooperatively (its blocks wait on one another): one block per SM, all resident. Every wait is bounded: on expiry the block
+// is `dead` (later waits return at once), the status word is set and the host reports AK_ERR_DEVICE_WAIT. A warp whose wait for a
+// copy ran out releases no slot any more, and nobody leaves before the copies it started have landed.
+#include "batch.h"
+#include "tma.h"
+
+#include <type_traits>
+
+namespace ak {
+
+namespace {
+
+constexpr uint32_t NW = 12;               // compute warps
+constexpr uint32_t NH = 3;                // epilogue warps
+constexpr uint32_t NCT = NW * 32, NHT = NH * 32;   // threads of the compute and of the epilogue warps
+constexpr uint32_t THREADS = 512, FIRST_COMPUTE = 4;
+constexpr int REGS_FIRST = 80, REGS_COMPUTE = 144;
+static_assert(REGS_FIRST * 128 + REGS_COMPUTE * 384 <= 65536, "the split draws on the registers of the launch");
+constexpr uint32_t CHUNK = 24;            // K slices (of 32) of a ring slot at most
+constexpr uint32_t SLOT = 8 * CHUNK * 64; // 8 weight rows
+constexpr uint32_t MAX_SLOTS = 8, MAX_EXTRA = 6;
+constexpr uint32_t MAX_LAYERS = 48;
+constexpr uint32_t KV_BUF = 4096;         // bytes of a warp's key (and of its value) buffer: 2048 / head_dim positions
+constexpr uint32_t MAX_UNITS = 32;        // units of a group (a lane keeps one)
+constexpr uint32_t EMPTY = 0xffffffffu;   // an exchange word that is not written yet
+constexpr uint32_t MAX_DYN_SMEM = 216 * 1024;
+
+__host__ __device__ constexpr uint32_t m_tiles(uint32_t seqs) { return seqs <= 16 ? 1 : 2; }
+__host__ __device__ constexpr uint32_t tile_begin(uint32_t tiles, uint32_t cta) { return (tiles * cta) / B200_SMS; }
+// Positions of an attention unit. Sequences of up to 512 are whole (no merging); longer ones are cut small, so that the groups' shares come out even: of
+// 16 sequences of up to 3200 positions a layer took 57 us in units of 512, with half of the SMs done after 31 us.
+__host__ __device__ constexpr uint32_t split_len(uint32_t max_len) { return max_len <= 512 ? 512 : 256; }
+__host__ __device__ constexpr uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
+constexpr uint32_t TB = 3;                // weight tiles of a pass (accumulators, partial sums)
+
+// byte offsets inside an exchange set (and its size): x after ffn-down, attention, x after out-proj, ffn-up as A fragments; sums of squares; qkv and
+// the splits of the attention in f32; an SM's best logit of a row {value, index}
+struct SetOff {
+    uint32_t x1, at, x2, up, s1, s2, qkv, best, part;
+    size_t total;
+    SetOff() = default;
+    __host__ __device__ SetOff(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t mt, uint32_t splits) {
+        const uint32_t r = mt * 16, hd = dim / heads, cx = dim * r * 2, cs = dim / 8 * r * 4;
+        x1 = 0; at = x1 + cx; x2 = at + cx; up = x2 + cx;
+        s1 = up + ffn * r * 2; s2 = s1 + cs;
+        qkv = s2 + cs;
+        best = qkv + r * 3 * dim * 4;
+        part = best + B200_SMS * r * 8;
+        total = part + (splits > 1 ? (size_t)r * heads * splits * (hd + 4) * 4 : 0);
+    }
+};
+
+// Bounds the polling of one thread; `dead` is sticky for the block. A poll is a round trip to L2 (0.3 us or more), so the limit is a second or two.
+constexpr uint32_t MAX_POLLS = 1u << 22;
+struct Waiter {
+    uint32_t* dead;
+    __device__ __forceinline__ bool give_up(uint32_t& n) {
+        n++;
+        if ((n & 63u) == 0) {
+            if (*(volatile uint32_t*)dead) return true;
+            if (n > MAX_POLLS) {
+                *(volatile uint32_t*)dead = 1u;
+                return true;
+            }
+        }
+        return false;
+    }
+};
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, uint32_t* dead) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+#pragma unroll 1
+    for (;;) {
+#pragma unroll 1
+        for (uint32_t n = 0; n < 64; n++)
+            if (mbar_try_wait(bar, parity)) return true;
+        if (*(volatile uint32_t*)dead) return false;
+        if (clock64() - t0 > AK_WAIT_MAX_CYCLES) {
+            *(volatile uint32_t*)dead = 1u;
+            return false;
+        }
+    }
+}
+
+// ---- exchange words
+// (16 bytes in one piece: a vector that has any of its words has all of them)
+__device__ __forceinline__ uint4 xld4(const void* p) {
+    uint64_t a, b;
+    asm volatile("{\n.reg .b128 q;\nld.relaxed.gpu.global.b128 q, [%2];\nmov.b128 {%0, %1}, q;\n}\n" : "=l"(a), "=l"(b) : "l"(p));
+    return make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
+}
+__device__ __forceinline__ uint2 xld2(const void* p) {
+    uint2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void xst1(void* p, uint32_t v) { asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+__device__ __forceinline__ void xst2(void* p, uint32_t a, uint32_t b) { asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(a), "r"(b) : "memory"); }
+__device__ __forceinline__ void xst4(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    const uint64_t x = a | ((uint64_t)b << 32), y = c | ((uint64_t)d << 32);
+    asm volatile("{\n.reg .b128 q;\nmov.b128 q, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], q;\n}\n" ::"l"(p), "l"(x), "l"(y) : "memory");
+}
+// (the result of an operation is never EMPTY: a NaN comes out as 0x7fffffff)
+__device__ __forceinline__ uint32_t word(float v) { return __float_as_uint(v); }
+__device__ __forceinline__ uint32_t pack2(float a, float b) {   // (a NaN becomes 0x7fff)
+    const bf162 p = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&p);
+}
+template <uint32_t N> __device__ __forceinline__ void bar_sync(uint32_t id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(N) : "memory"); }
+__device__ __forceinline__ void bar_sync_n(uint32_t id, uint32_t n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+template <uint32_t N> __device__ __forceinline__ void bar_arrive(uint32_t id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(N) : "memory"); }
+enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_GROUP = 4 };   // BAR_GROUP and the next two: by group
+
+__device__ __forceinline__ uint64_t policy_evict_first() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float ex2(float x) {   // 2^x
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float redux_max(float v) {   // of the warp (no NaN)
+    float m;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
+    return m;
+}
+__device__ __forceinline__ void unpack8(const uint4& r, float (&o)[8]) {
+    o[0] = __uint_as_float(r.x << 16); o[1] = __uint_as_float(r.x & 0xffff0000u);
+    o[2] = __uint_as_float(r.y << 16); o[3] = __uint_as_float(r.y & 0xffff0000u);
+    o[4] = __uint_as_float(r.z << 16); o[5] = __uint_as_float(r.z & 0xffff0000u);
+    o[6] = __uint_as_float(r.w << 16); o[7] = __uint_as_float(r.w & 0xffff0000u);
+}
+// 1 / sqrt(m): the hardware's approximation and one Newton step, which has no value where m is 0 or infinite (there the approximation is exact)
+__device__ __forceinline__ float inv_rms(float m) {
+    const float y = rsqrtf(m);
+    return y > 0.0f && y < INFINITY ? y * fmaf(-0.5f * m * y, y, 1.5f) : y;
+}
+
+struct Cursor {   // a place in the ring: slot and the parity of its current use
+    uint32_t s = 0, ph = 0;
+    __device__ __forceinline__ void advance(uint32_t by, uint32_t n) {   // by <= n
+        s += by;
+        if (s >= n) { s -= n; ph ^= 1u; }
+    }
+};
+// A weight matrix [n, k] as this SM sees it (kept in shared memory: held in registers or recomputed, the four of them spill): its tiles of 8 rows, and K as
+// ring chunks of CHUNK slices of 32 (the last may have fewer).
+struct Kind {
+    uint32_t t0, n, slices, chunks, pitch, pieces;   // pitch: bytes of a row in a slot; pieces of a chunk in the tensor map
+    __device__ __forceinline__ uint32_t count(uint32_t c) const { return min(CHUNK, slices - c * CHUNK); }
+};
+// A weight row as pieces of the tensor map: 256 columns, or what divides the row
+__host__ __device__ constexpr uint32_t piece_of(uint32_t k) { return k % 256 == 0 ? 256 : k % 64 == 0 ? 64 : 32; }
+__host__ __device__ constexpr uint32_t chunk_cols(uint32_t k) { return k < CHUNK * 32 ? k : CHUNK * 32; }
+__device__ __forceinline__ void make_kind(Kind& d, uint32_t rows, uint32_t k, uint32_t cta) {
+    d.t0 = tile_begin(div_up(rows, 8), cta);
+    d.n = tile_begin(div_up(rows, 8), cta + 1) - d.t0;
+    d.slices = k >> 5;
+    d.chunks = div_up(d.slices, CHUNK);
+    d.pitch = chunk_cols(k) * 2;
+    d.pieces = CHUNK * 32 / piece_of(k);
+}
+// Byte offset of vector v (columns 8 v .. 8 v + 7) of a row among the A fragments. The eight vectors that a tile publishes for eight rows are one 128-byte
+// line: lane 4 g + t of a fragment reads vector 8 t + g of its 512 bytes.
+template <int MT> __device__ __forceinline__ uint32_t frag(uint32_t row, uint32_t v) {
+    return ((((v >> 2) * MT + (row >> 4)) * 2 + ((row >> 3) & 1)) * 32 + (v & 3) * 8 + (row & 7)) * 16;
+}
+struct Unit { uint32_t row, head, split, p0, n, nb; };   // attention unit: positions p0 .. p0 + n of (row, head), nb tiles
+// The tiles a warp has yet to request: tile b of unit j (u) of layer l, in the pool blocks pb0 (and pb1); nu: units of the warp's group.
+struct Walk {
+    Unit u;
+    uint32_t l, j, b, pb0, pb1, nu, more;
+};
+enum { QKV = 0, OUT = 1, FFN_UP = 2, FFN_DOWN = 3, HEAD = 4, N_KINDS = 5 };
+constexpr uint32_t NO_LOGIT = 0x7fffffffu;   // in the place of the index of a best logit
+
+// SPLIT: sequences may be longer than an attention unit
+template <int HD, int MT, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant__ BatchArgs a, const uint32_t slots, const uint32_t wpi) {
+    constexpr uint32_t R = MT * 16;               // rows of the exchange buffers
+    constexpr uint32_t PPC = CHUNK / NW;          // slices of a ring chunk that a warp has: 2
+    constexpr uint32_t Q = R / 4, TPL = 32 / Q;   // lanes that read a tile's sums of squares, tiles per load
+    constexpr uint32_t CH = HD / 8;               // 16-byte vectors of a cache row
+    constexpr uint32_t PPI = 32 / CH;             // positions a warp reads per instruction
+    constexpr uint32_t UP = 2048 / HD;            // positions of a tile buffer
+    extern __shared__ __align__(128) uint8_t smem[];
+    // (the bars and uses from MAX_SLOTS on belong to the extra slots that the lm_head has where the cache tiles were)
+    __shared__ uint64_t full_bar[MAX_SLOTS + MAX_EXTRA], empty_bar[MAX_SLOTS + MAX_EXTRA], k_bar[NW], v_bar[NW], free_bar, kv_free_bar;
+    __shared__ SoloLayer layers_sm[MAX_LAYERS];
+    __shared__ Kind kinds[N_KINDS];
+    __shared__ SetOff so;
+    __shared__ __align__(16) float ss_sm[2][NH][R];   // a norm phase's sums of squares, by epilogue warp
+    __shared__ float2 at_ml[2][NW];
+    __shared__ Walk walk_sm[NW];
+    __shared__ uint32_t units[NW][MAX_UNITS];
+    __shared__ uint32_t len_sm[32], by_len[32], pre_sm[33];
+    __shared__ uint32_t dead, live_sm, use_sm[MAX_SLOTS + MAX_EXTRA];   // use_sm: 1 + the number of the use a slot is in (lm_head only)
+
+    const uint32_t tid = threadIdx.x, warp_ = tid >> 5, lane = tid & 31;
+    const uint32_t cta = blockIdx.x;
+    const uint32_t D = a.dim, F = a.ffn, H = a.heads, L = a.n_layers;
+    uint8_t* const kv_sm = smem + slots * SLOT;
+    float* const part = reinterpret_cast<float*>(kv_sm + NW * 2 * KV_BUF);        // [NW][TB][R][8]
+    float* const at_acc = part + NW * TB * R * 8;                                 // [2][NW][HD]
+    float4* const res_sm = reinterpret_cast<float4*>(at_acc + 2 * NW * HD);       // [tile][R][2]: the residual stream of this SM's columns
+    float* const gain_sm = reinterpret_cast<float*>(res_sm + TB * R * 2);                // [2 L + 1][tiles][8]: the gains of its columns, by norm
+    const uint32_t SPLIT_LEN = SPLIT ? 256 : 512, splits = div_up(a.max_len, SPLIT_LEN);
+
+    if (tid == 160) so = SetOff(D, F, H, MT, splits);
+    if (tid == 0) {
+#pragma unroll 1
+        for (uint32_t s = 0; s < MAX_SLOTS + MAX_EXTRA; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], NW); use_sm[s] = 0; }
+#pragma unroll 1
+        for (uint32_t i = 0; i < NW; i++) { mbar_init(&k_bar[i], 1); mbar_init(&v_bar[i], 1); }
+        mbar_init(&free_bar, NH);
+        mbar_init(&kv_free_bar, NW);
+        dead = 0;
+        mbar_fence_init();
+    }
+    if (tid >= 32 && tid < 32 + N_KINDS) make_kind(kinds[tid - 32], tid == 32 ? 3 * D : tid == 34 ? F : tid == 36 ? a.vocab : D, tid == 35 ? F : D, cta);
+    if (warp_ == 2) {   // the rows' lengths, the rows by length (the longest first), the attention splits of the rows before by that rank
+        const uint32_t n = lane < a.seqs ? min((uint32_t)max(a.kv_lens[lane], 0), a.max_len) : 0u;
+        uint32_t rank = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 32; j++) {
+            const uint32_t o = __shfl_sync(0xffffffffu, n, j);
+            rank += o > n || (o == n && j < lane);
+        }
+        len_sm[lane] = n;
+        by_len[rank] = lane;
+        const uint32_t m = __ballot_sync(0xffffffffu, n > 0);
+        if (lane == 0) live_sm = m;
+        __syncwarp();
+        const uint32_t mine = div_up(len_sm[by_len[lane]], SPLIT_LEN);
+        uint32_t sum = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= (uint32_t)o) sum += t;
+        }
+        pre_sm[lane] = sum - mine;
+        if (lane == 31) pre_sm[32] = sum;
+    }
+#pragma unroll 1
+    for (uint32_t i = tid; i < L * (uint32_t)(sizeof(SoloLayer) / 8); i += THREADS)
+        reinterpret_cast<uint64_t*>(layers_sm)[i] = reinterpret_cast<const uint64_t*>(a.layers)[i];
+    const uint32_t e0 = *a.set0 % 3;
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t i = tid, n = kinds[OUT].n * 8; i < (2 * L + 1) * n; i += THREADS)
+        gain_sm[i] = (i / n == 2 * L ? a.final_norm : i / n & 1 ? layers_sm[i / (2 * n)].norm_2 : layers_sm[i / (2 * n)].norm_1)[kinds[OUT].t0 * 8 + i % n];
+    const uint32_t live = live_sm, n_act = __popc(live);
+    if (n_act == 0) return;   // (the host has not moved set0 for such a step either)
+    __syncthreads();   // the gains
+
+    // The lm_head keeps x where the cache tiles were, and extra slots behind it. Its chunk n is in slot n mod (slots + extra) of the two.
+    uint8_t* const extra_sm = kv_sm + D * R * 2;
+    const uint32_t extra = min(MAX_EXTRA, (NW * 2 * KV_BUF - D * R * 2) / SLOT), head_slots = slots + extra;
+    auto set_of = [&](uint32_t g) { return (g % 3) * (uint32_t)so.total; };   // byte offset; g = e0: the embedding, e0 + 1 + l: layer l
+    auto row_live = [&](uint32_t r) { return (live >> r) & 1u; };
+    auto eight_live = [&](uint32_t e) { return ((live >> (e * 8)) & 0xffu) != 0; };
+    const Waiter wt{&dead};
+    const float inv_dim = 1.0f / (float)D;
+
+    if (warp_ < FIRST_COMPUTE) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_FIRST));
+    if (warp_ == 0) {
+        // ---------------- producer: this SM's weight tiles in the order the compute warps use them, a chunk of a tile by one tensor load (its eight rows as
+        // bulk copies of their own took 0.6 us to issue: 3 TB/s over the chip)
+        if (lane != 0) return;
+        const CUtensorMap* const map = reinterpret_cast<const CUtensorMap*>(a.maps);
+        const uint64_t pol = policy_evict_first();
+        Cursor q;
+        uint32_t sent = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (uint32_t i = 0; i < 4 * L && ok; i++) {
+            const Kind& d = kinds[i & 3];
+#pragma unroll 1
+            for (uint32_t b = 0; b < d.n && ok; b += TB) {
+                const uint32_t nt = min(TB, d.n - b);
+#pragma unroll 1
+                for (uint32_t c = 0; c < d.chunks && ok; c++) {
+#pragma unroll 1
+                    for (uint32_t t = 0; t < nt; t++) {
+                        if (sent >= slots) ok = wait_bar(&empty_bar[q.s], q.ph ^ 1u, &dead);
+                        if (!ok) break;
+                        mbar_expect_tx(&full_bar[q.s], 8 * d.pitch);
+                        tma_load_rows(smem + q.s * SLOT, map + i, c * d.pieces, (d.t0 + b + t) * 8, &full_bar[q.s], pol);
+                        sent++;
+                        q.advance(1, slots);
+                    }
+                }
+            }
+        }
+        uint32_t head_sent = 0;
+        {
+            const Kind& d = kinds[HEAD];
+#pragma unroll 1
+            for (uint32_t t = 0, c = 0; t < d.n && ok; c = c + 1 < d.chunks ? c + 1 : 0, t += c == 0) {
+                const uint32_t lap = head_sent / head_slots, r = head_sent - lap * head_slots, x = r < slots ? 0 : MAX_SLOTS + r - slots;
+                const uint32_t bar = r < slots ? q.s : x;
+                if (r < slots) {
+                    if (sent >= slots) ok = wait_bar(&empty_bar[bar], q.ph ^ 1u, &dead);
+                } else {
+                    ok = lap ? wait_bar(&empty_bar[bar], (lap - 1) & 1u, &dead) : wait_bar(&kv_free_bar, 0, &dead);
+                }
+                if (!ok) break;
+                mbar_expect_tx(&full_bar[bar], 8 * d.pitch);
+                *(volatile uint32_t*)&use_sm[bar] = 1 + (r < slots ? sent / slots : lap);
+                tma_load_rows(r < slots ? smem + bar * SLOT : extra_sm + (r - slots) * SLOT, map + 4 * L, c * d.pieces, (d.t0 + t) * 8, &full_bar[bar], pol);
+                head_sent++;
+                if (r < slots) {
+                    sent++;
+                    q.advance(1, slots);
+                }
+            }
+        }
+        // leave when every copy has landed: the last use of each slot (q stands on the oldest)
+        const uint32_t n = min(sent, slots);
+#pragma unroll 1
+        for (uint32_t i = 0; i < n; i++) {
+            if (sent < slots) { q.s = i; q.ph = 1; }
+            mbar_wait(&full_bar[q.s], q.ph ^ 1u);
+            q.advance(1, slots);
+        }
+#pragma unroll 1
+        for (uint32_t r = slots; r < min(head_sent, head_slots); r++) mbar_wait(&full_bar[MAX_SLOTS + r - slots], ((head_sent - r - 1) / head_slots) & 1u);
+        return;
+    }
+    if (warp_ < FIRST_COMPUTE) {
+        // ---------------- epilogue: warp e has the e-th tile of a pass. It adds the compute warps' partial sums, applies the norm's factor or
+        // adds to the residual stream, and publishes; the compute warps are then already at the next phase. Also the embedding, the sums of
+        // squares of the norms, the clearing of exchange sets.
+        const uint32_t ht = tid - 32, e = warp_ - 1, h = lane & 1;   // lane: row 16 m + lane / 2, columns 4 h .. 4 h + 3 of the tile
+        const uint32_t rl = lane >> 1;
+        auto clear = [&](uint32_t g) {
+            uint4* p = reinterpret_cast<uint4*>(a.xch + set_of(g));
+            const uint32_t n = (uint32_t)(so.total / 16);
+#pragma unroll 1
+            for (uint32_t i = cta * NHT + ht; i < n; i += B200_SMS * NHT) p[i] = make_uint4(EMPTY, EMPTY, EMPTY, EMPTY);
+            __threadfence();
+        };
+        uint32_t nb = 0;
+        // 1 / rms of the lane's rows
+        auto factors = [&](uint32_t off, float (&f)[MT]) {   // lane (i / Q, i % Q) reads four rows of tile i / Q, + TPL, .. of this warp's
+            const uint32_t n = D / 8, step = NH * TPL;
+            const uint8_t* const sl = a.xch + off + lane % Q * 16;
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+            for (uint32_t t0 = e * TPL + lane / Q; t0 < n; t0 += 4 * step) {
+                uint4 y[4];
+                uint32_t polls = 0;
+                bool lack;
+                Waiter w = wt;
+#pragma unroll 1
+                do {
+#pragma unroll
+                    for (uint32_t d = 0; d < 4; d++) y[d] = t0 + d * step < n ? xld4(sl + (t0 + d * step) * (R * 4)) : make_uint4(0, 0, 0, 0);
+                    uint32_t mx = 0;
+#pragma unroll
+                    for (uint32_t d = 0; d < 4; d++) mx = max(max(mx, max(y[d].x, y[d].y)), max(y[d].z, y[d].w));
+                    lack = mx == EMPTY;
+                } while (lack && !w.give_up(polls));
+#pragma unroll
+                for (uint32_t d = 0; d < 4; d++) {
+                    sum.x += __uint_as_float(y[d].x); sum.y += __uint_as_float(y[d].y);
+                    sum.z += __uint_as_float(y[d].z); sum.w += __uint_as_float(y[d].w);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (uint32_t o = Q; o < 32; o <<= 1) {
+                sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o); sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+                sum.z += __shfl_xor_sync(0xffffffffu, sum.z, o); sum.w += __shfl_xor_sync(0xffffffffu, sum.w, o);
+            }
+            if (lane < Q) *reinterpret_cast<float4*>(&ss_sm[nb][e][lane * 4]) = sum;
+            bar_sync<NHT>(BAR_HELP);
+#pragma unroll
+            for (uint32_t m = 0; m < MT; m++) {
+                const float* const s = &ss_sm[nb][0][m * 16 + rl];
+                f[m] = inv_rms((s[0] + s[R] + s[2 * R]) * inv_dim + a.eps);
+            }
+            nb ^= 1u;
+        };
+        // publish 8 columns (the vector of a tile) held by two lanes; whole warps
+        auto put8 = [&](uint32_t dst, bool eight, const float4& v) {
+            const uint32_t w0 = pack2(v.x, v.y), w1 = pack2(v.z, v.w);
+            const uint32_t w2 = __shfl_down_sync(0xffffffffu, w0, 1), w3 = __shfl_down_sync(0xffffffffu, w1, 1);
+            if (h == 0 && eight) xst4(a.xch + dst, w0, w1, w2, w3);
+        };
+        // publish the residual stream, multiplied by the next norm's gain, and the sums of squares of whole tiles
+        auto put_x = [&](uint32_t xd, uint32_t sd, bool eight, const float4& x, const float4& g) {
+            put8(xd, eight, make_float4(x.x * g.x, x.y * g.y, x.z * g.z, x.w * g.w));
+            float s = (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            if (h == 0) xst1(a.xch + sd, word(s));   // (of every row: 0 where there is no sequence)
+        };
+        if (lane == 0) mbar_arrive(&free_bar);
+        // ---- embedding
+        if (e < kinds[OUT].n) {
+            const uint32_t tile = kinds[OUT].t0 + e;
+            const float4 g = *reinterpret_cast<const float4*>(gain_sm + e * 8 + h * 4);
+#pragma unroll
+            for (uint32_t m = 0; m < MT; m++) {
+                const uint32_t row = m * 16 + rl;
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (row_live(row)) {
+                    const int32_t ts = a.rows[row * 4];
+                    const uint32_t id = ts >= 0 ? (uint32_t)ts : a.sampled[(uint32_t)(-(ts + 1))];
+                    if (id < a.vocab) {
+                        const uint2 w = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(a.embedding) + (size_t)id * D + tile * 8 + h * 4);
+                        x = make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u));
+                    }
+                }
+                __syncwarp();
+                res_sm[(e * R + row) * 2 + h] = x;
+                put_x(set_of(e0) + so.x1 + frag<MT>(row, tile), set_of(e0) + so.s1 + (tile * R + row) * 4, eight_live(row >> 3), x, g);
+            }
+        }
+        // Set g may be cleared when everybody has read what there is in it, and has to be before anybody can be polling its next content.
+        // When ss2 of layer g + 1 is complete, out-proj of layer g + 1 is done, with it attention and qkv of that layer, so ffn-down of layer g (the
+        // last readers of set g but for x1 and ss1, which qkv of layer g + 1 has read). Its next content is layer g + 3's, polled first by an SM that has
+        // seen x1 of layer g + 3, so by then ffn-up of layer g + 2 has been published by every SM (each has tiles of it), by the threads that cleared,
+        // after the fence above. The set of the step's embedding stands for a layer. The last layer's set is cleared when the next step starts: it
+        // is used again in that step's second layer.
+        clear(e0 + 2);
+#pragma unroll 1
+        for (uint32_t i = 0; i < 4 * L; i++) {
+            const uint32_t l = i >> 2, ph = i & 3, set = set_of(e0 + 1 + l);
+            const Kind& d = kinds[ph];
+            const uint32_t tiles = d.n;
+            const bool norm = ph == QKV || ph == FFN_UP;
+            float f[MT];
+#pragma unroll
+            for (uint32_t m = 0; m < MT; m++) f[m] = 1.0f;
+            if (norm && tiles) factors(ph == QKV ? set_of(e0 + l) + so.s1 : set + so.s2, f);
+            // A row without a sequence is published as zeros where a row of its eight has one (the consumers look at whole eights only). Here its
+            // attention, by the SM with the row's number among its qkv tiles: it has just seen that the layer before is complete, so
+            // nobody's clearing of the set is still to come.
+            if (ph == QKV) {
+#pragma unroll 1
+                for (uint32_t r = d.t0; r < min(d.t0 + tiles, R); r++)
+                    if (!row_live(r) && eight_live(r >> 3)) {
+#pragma unroll 1
+                        for (uint32_t v = ht; v < D / 8; v += NHT) xst4(a.xch + set + so.at + frag<MT>(r, v), 0, 0, 0, 0);
+                    }
+            }
+#pragma unroll 1
+            for (uint32_t b = 0; b < tiles; b += TB) {
+                const bool has = b + e < tiles;
+                const uint32_t tile = d.t0 + b + e;
+                // all that does not need the sums
+                uint32_t dst[MT], sd[MT];
+                float4 res[MT], g = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (has) {
+                    if (!norm) g = *reinterpret_cast<const float4*>(gain_sm + ((2 * l + (ph == OUT ? 1 : 2)) * tiles + e) * 8 + h * 4);
+#pragma unroll
+                    for (uint32_t m = 0; m < MT; m++) {
+                        const uint32_t row = m * 16 + rl;
+                        res[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        sd[m] = 0;
+                        if (ph == QKV) dst[m] = set + so.qkv + (row * 3 * D + tile * 8 + h * 4) * 4;
+                        else dst[m] = set + (ph == OUT ? so.x2 : ph == FFN_UP ? so.up : so.x1) + frag<MT>(row, tile);
+                        if (!norm) {
+                            res[m] = res_sm[(e * R + row) * 2 + h];
+                            sd[m] = set + (ph == OUT ? so.s2 : so.s1) + (tile * R + row) * 4;
+                        }
+                    }
+                }
+                const float* const o = part + e * (R * 8) + lane * 4;
+                bar_sync<NCT + NHT>(BAR_PART);
+                if (has) {
+#pragma unroll
+                    for (uint32_t m = 0; m < MT; m++) {
+                        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                        for (uint32_t w0 = 0; w0 < NW; w0 += 4) {   // four at a time (registers), in pairs
+                            float4 y[4];
+#pragma unroll
+                            for (uint32_t w = 0; w < 4; w++) y[w] = *reinterpret_cast<const float4*>(o + (w0 + w) * (TB * R * 8) + m * 128);
+                            v.x += (y[0].x + y[1].x) + (y[2].x + y[3].x); v.y += (y[0].y + y[1].y) + (y[2].y + y[3].y);
+                            v.z += (y[0].z + y[1].z) + (y[2].z + y[3].z); v.w += (y[0].w + y[1].w) + (y[2].w + y[3].w);
+                        }
+                        const uint32_t row = m * 16 + rl;
+                        if (!norm) {
+                            v.x += res[m].x; v.y += res[m].y; v.z += res[m].z; v.w += res[m].w;
+                            put_x(dst[m], sd[m], eight_live(row >> 3), v, g);
+                            res_sm[(e * R + row) * 2 + h] = v;
+                            continue;
+                        }
+                        v.x *= f[m]; v.y *= f[m]; v.z *= f[m]; v.w *= f[m];
+                        if (ph == QKV) {
+                            if (row_live(row)) xst4(a.xch + dst[m], word(v.x), word(v.y), word(v.z), word(v.w));
+                            continue;
+                        }
+                        // SiLU (off by 2^-17 of the value at most, and 0 below about -87: far below the rounding to bf16)
+                        v.x = __fdividef(v.x, 1.0f + __expf(-v.x)); v.y = __fdividef(v.y, 1.0f + __expf(-v.y));
+                        v.z = __fdividef(v.z, 1.0f + __expf(-v.z)); v.w = __fdividef(v.w, 1.0f + __expf(-v.w));
+                        put8(dst[m], eight_live(row >> 3), v);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&free_bar);
+            }
+            if (ph == FFN_UP) clear(e0 + l);
+        }
+        return;
+    }
+
+    // ---------------- compute warps
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_COMPUTE));
+    const uint32_t cw = warp_ - FIRST_COMPUTE, ct = cw * 32 + lane;
+    bool alive = true;   // no wait of this warp for a copy has run out (after the first that did it releases no slot)
+    Cursor q;
+    const uint32_t frag_lane = (lane & 3) * 8 + (lane >> 2);
+    uint32_t part_ph = 0;           // parity of the use of the partial sums
+    uint32_t a_live = 0;            // the eights of the rows that have a sequence
+#pragma unroll
+    for (uint32_t e = 0; e < 2 * MT; e++) a_live |= (eight_live(e) ? 1u : 0u) << e;
+
+    // The warp's share of NT tiles of projection `kind`; x: A fragments. What a phase spends its time on is dependent instructions, ~5 cycles each, so
+    // all that can be is done before the activations arrive: the weights are in registers, addresses are known.
+    auto pass = [&](auto nt_c, uint32_t x, const Kind& kind) {
+        constexpr uint32_t NT = decltype(nt_c)::value;
+        constexpr uint32_t CPG = MT == 1 && NT == 1 ? 2 : 1, DEPTH = CPG * PPC;   // chunks of a group (what a warp requests together), slices
+        const uint32_t chunks = kind.chunks, slices = kind.slices, pitch = kind.pitch;
+        // the warp's slices cw + NW i, i < nsl
+        const uint32_t nsl = cw < slices ? (slices - cw + NW - 1) / NW : 0;
+        const uint8_t* xl = a.xch + (x + cw * (MT * 1024) + frag_lane * 16);
+        constexpr uint32_t STEP = NW * MT * 1024;
+        const uint32_t w_off = (lane >> 2) * pitch + cw * 64 + (lane & 3) * 16;
+        uint4 v[DEPTH][MT][2];
+        float acc[NT][MT][4];
+#pragma unroll
+        for (uint32_t t = 0; t < NT; t++)
+#pragma unroll
+            for (uint32_t m = 0; m < MT; m++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc[t][m][i] = 0.0f;
+#pragma unroll
+        for (uint32_t d = 0; d < DEPTH; d++)
+#pragma unroll
+            for (uint32_t e = 0; e < 2 * MT; e++) v[d][e >> 1][e & 1] = make_uint4(0, 0, 0, 0);
+        auto issue = [&](uint32_t i0) {
+#pragma unroll
+            for (uint32_t d = 0; d < DEPTH; d++)
+                if (i0 + d < nsl) {
+#pragma unroll
+                    for (uint32_t e = 0; e < 2 * MT; e++)
+                        if (a_live >> e & 1u) v[d][e >> 1][e & 1] = xld4(xl + d * STEP + e * 512);
+                }
+        };
+        issue(0);
+#pragma unroll 1
+        for (uint32_t c0 = 0;;) {
+            // the group's weights
+            Cursor first = q;
+            uint32_t used = 0;
+            uint4 w[DEPTH][NT];
+#pragma unroll
+            for (uint32_t cc = 0; cc < CPG; cc++)
+                if (cc == 0 || c0 + cc < chunks) {
+                    Cursor mine = q;
+                    mine.advance(lane < NT ? lane : 0, slots);
+                    const bool got = lane >= NT || wait_bar(&full_bar[mine.s], mine.ph, &dead);
+                    alive = __all_sync(0xffffffffu, got && alive) != 0;
+#pragma unroll
+                    for (uint32_t t = 0; t < NT; t++) {
+                        const uint32_t at = (q.s + t < slots ? q.s + t : q.s + t - slots) * SLOT + w_off;
+#pragma unroll
+                        for (uint32_t j = 0; j < PPC; j++)   // (past the end of K: what the slot held, for products that are left out)
+                            w[cc * PPC + j][t] = *reinterpret_cast<const uint4*>(smem + at + j * (NW * 64));
+                    }
+                    q.advance(NT, slots);
+                    used += NT;
+                }
+            // everything there?
+            const uint32_t left = nsl - min(nsl, c0 * PPC);
+            uint32_t polls = 0;
+#pragma unroll 1
+            for (;;) {
+                uint32_t mx = 0;   // EMPTY is the largest word
+#pragma unroll
+                for (uint32_t d = 0; d < DEPTH; d++)
+                    if (d < left) {
+#pragma unroll
+                        for (uint32_t e = 0; e < 2 * MT; e++) mx = max(mx, v[d][e >> 1][e & 1].x);
+                    }
+                Waiter wait = wt;
+                if (!__any_sync(0xffffffffu, mx == EMPTY) || __any_sync(0xffffffffu, wait.give_up(polls))) break;
+#pragma unroll
+                for (uint32_t d = 0; d < DEPTH; d++)
+                    if (d < left) {
+#pragma unroll
+                        for (uint32_t e = 0; e < 2 * MT; e++)
+                            if (a_live >> e & 1u) v[d][e >> 1][e & 1] = xld4(xl + d * STEP + e * 512);
+                    }
+            }
+#pragma unroll
+            for (uint32_t d = 0; d < DEPTH; d++)
+                if (d < left) {
+#pragma unroll
+                    for (uint32_t t = 0; t < NT; t++)
+#pragma unroll
+                        for (uint32_t m = 0; m < MT; m++) mma(acc[t][m], v[d][m][0].x, v[d][m][1].x, v[d][m][0].y, v[d][m][1].y, w[d][t].x, w[d][t].y);
+#pragma unroll
+                    for (uint32_t t = 0; t < NT; t++)
+#pragma unroll
+                        for (uint32_t m = 0; m < MT; m++) mma(acc[t][m], v[d][m][0].z, v[d][m][1].z, v[d][m][0].w, v[d][m][1].w, w[d][t].z, w[d][t].w);
+                }
+            // The group's slots go back, only now: a load from shared memory and an arrival on a barrier are not in order by themselves, so
+            // a slot could be overwritten under a load that the products have not waited for yet.
+            __syncwarp();
+            if (lane < used && alive) {
+                first.advance(lane, slots);
+                mbar_arrive(&empty_bar[first.s]);
+            }
+            c0 += CPG;
+            if (c0 >= chunks) break;
+            xl += DEPTH * STEP;
+            issue(c0 * PPC);
+        }
+        alive = wait_bar(&free_bar, part_ph, &dead) && alive;   // the sums that were there have been read
+        part_ph ^= 1u;
+        {
+            float* const o = part + (cw * TB * R + (lane >> 2)) * 8 + (lane & 3) * 2;
+#pragma unroll
+            for (uint32_t t = 0; t < NT; t++)
+#pragma unroll
+                for (uint32_t m = 0; m < MT; m++) {
+                    *reinterpret_cast<float2*>(o + (t * R + m * 16) * 8) = make_float2(acc[t][m][0], acc[t][m][1]);
+                    *reinterpret_cast<float2*>(o + (t * R + m * 16 + 8) * 8) = make_float2(acc[t][m][2], acc[t][m][3]);
+                }
+        }
+        __syncwarp();
+        bar_arrive<NCT + NHT>(BAR_PART);
+    };
+    auto gemm = [&](uint32_t x, const Kind& kind) {
+        const uint32_t tiles = kind.n;
+#pragma unroll 1
+        for (uint32_t b = 0; b < tiles; b += TB) {
+            const uint32_t nt = min(TB, tiles - b);
+            if (nt == 1) pass(std::integral_constant<uint32_t, 1>{}, x, kind);
+            else if (nt == 2) pass(std::integral_constant<uint32_t, 2>{}, x, kind);
+            else pass(std::integral_constant<uint32_t, 3>{}, x, kind);
+        }
+    };
+
+    uint32_t tiles_done = 0;   // parity of the tiles worked through
+    // ---- attention: units of this warp's group. What a warp keeps of it between layers is in shared memory (the projections need the registers).
+    auto group_of = [&]() { return wpi == NW ? 0u : cw >> 2; };     // wpi is 12 or 4
+    auto place_in = [&]() { return wpi == NW ? cw : cw & 3u; };
+    {   // unit j in lane j: row | head << 6 | split << 18
+        const uint32_t grp = group_of();
+        const uint32_t groups = B200_SMS * (NW / wpi), gid = grp * B200_SMS + cta;
+        const uint32_t u = lane * groups + ((lane & 1) ? groups - 1 - gid : gid);
+        uint32_t unit = EMPTY;
+        if (u < pre_sm[32] * H) {
+            const uint32_t v = u / H;
+            uint32_t lo = 0, hi = 32;   // the rank whose splits hold v
+#pragma unroll 1
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) / 2;
+                if (pre_sm[mid] <= v) lo = mid;
+                else hi = mid;
+            }
+            unit = by_len[lo] | ((u % H) << 6) | ((v - pre_sm[lo]) << 18);
+        }
+        units[cw][lane] = unit;
+        const uint32_t n = __popc(__ballot_sync(0xffffffffu, unit != EMPTY));
+        if (lane == 0) walk_sm[cw].nu = n;
+        __syncwarp();
+    }
+    auto unit_at = [&](uint32_t j) {
+        const uint32_t u = units[cw][j];
+        Unit o;
+        o.row = u & 63; o.head = (u >> 6) & 0xfff; o.split = u >> 18;
+        o.p0 = o.split * SPLIT_LEN;
+        o.n = min(SPLIT_LEN, len_sm[o.row] - o.p0);
+        o.nb = (o.n + UP - 1) / UP;
+        return o;
+    };
+    auto look_up = [&]() {   // the pool blocks of the walk's tile (lane 0)
+        Walk& k = walk_sm[cw];
+        const uint32_t p = k.b * UP;
+        const int32_t* bt = a.block_tables + (size_t)k.u.row * a.max_blocks + (k.u.p0 + p) / 16;
+        k.pb0 = (uint32_t)__ldg(bt);
+        k.pb1 = UP > 16 && p + 16 < k.u.n ? (uint32_t)__ldg(bt + 1) : EMPTY;
+    };
+    uint8_t* const kbuf = kv_sm + cw * 2 * KV_BUF;
+    uint8_t* const vbuf = kbuf + KV_BUF;
+    // Request the keys or the values of the walk's tile; with the values the walk moves on. Called by the whole warp after it has read the buffer;
+    // lane 0 does it, with the walk in shared memory.
+    auto request = [&](bool values) {
+        if (lane == 0 && walk_sm[cw].more) {
+            Walk& k = walk_sm[cw];
+            const SoloLayer& w = layers_sm[k.l];
+            const uint32_t pb0 = k.pb0, pb1 = k.pb1;
+            uint64_t* bar = values ? &v_bar[cw] : &k_bar[cw];
+            const bf16* pool = reinterpret_cast<const bf16*>(values ? w.v_pool : w.k_pool) + (size_t)k.u.head * (16 * HD);
+            uint8_t* dst = values ? vbuf : kbuf;
+            constexpr uint32_t TILE = 16 * HD * 2;
+            mbar_expect_tx(bar, UP > 16 && pb1 != EMPTY ? 2 * TILE : TILE);
+            bulk_g2s(dst, pool + (size_t)pb0 * H * (16 * HD), TILE, bar);
+            if (UP > 16 && pb1 != EMPTY) bulk_g2s(dst + TILE, pool + (size_t)pb1 * H * (16 * HD), TILE, bar);
+            if (values) {
+                k.b += wpi;
+#pragma unroll 1
+                while (k.b >= k.u.nb) {
+                    if (++k.j == k.nu) {
+                        k.j = 0;
+                        if (++k.l == L) { k.more = 0; break; }
+                    }
+                    k.u = unit_at(k.j);
+                    k.b = place_in();
+                }
+                look_up();
+            }
+        }
+        __syncwarp();
+    };
+    {
+        if (lane == 0) {
+            Walk& k = walk_sm[cw];
+            k.l = k.j = k.more = 0;
+            k.b = place_in();
+#pragma unroll 1
+            for (uint32_t j = k.nu; j-- > 0;)   // the first unit with a tile for this warp (if there is one there is one in every layer)
+                if (place_in() < unit_at(j).nb) { k.more = 1; k.j = j; }
+            if (k.more) {
+                k.u = unit_at(k.j);
+                look_up();
+            }
+        }
+        __syncwarp();
+        request(false);
+        request(true);
+    }
+
+    // publish a head of a row: lane i has its columns DL i .. DL i + DL - 1, to be divided by ls
+    constexpr uint32_t DL = HD / 32;
+    auto put_at = [&](uint32_t set, uint32_t row, uint32_t head, const float (&o)[DL], float ls) {
+        const float r = __fdividef(1.0f, ls);   // (2 ulp, before a rounding to bf16)
+        uint32_t w[4];
+        w[0] = pack2(o[0] * r, o[1] * r);
+        if constexpr (DL == 2) {
+#pragma unroll
+            for (int i = 1; i < 4; i++) w[i] = __shfl_down_sync(0xffffffffu, w[0], i);
+        } else {
+            w[1] = pack2(o[DL - 2] * r, o[DL - 1] * r);
+            w[2] = __shfl_down_sync(0xffffffffu, w[0], 1);
+            w[3] = __shfl_down_sync(0xffffffffu, w[1], 1);
+        }
+        if (lane % (8 / DL) == 0) {
+            uint8_t* const dst = a.xch + set + so.at + frag<MT>(row, (head * HD + lane * DL) >> 3);
+            xst4(dst, w[0], w[1], w[2], w[3]);
+        }
+    };
+
+    auto attention = [&](const SoloLayer& lw, uint32_t set) {
+        const uint32_t chunk = lane % CH;
+        const uint8_t* const qkv = a.xch + set + so.qkv;
+        const uint32_t grp = group_of(), wg = place_in(), nu = walk_sm[cw].nu;
+#pragma unroll 1
+        for (uint32_t j = 0; j < nu; j++) {
+            const Unit u = unit_at(j);
+            const uint32_t buf = j & 1, pos = len_sm[u.row] - 1;
+            const bool newest = u.p0 + u.n == pos + 1;   // the unit holds the sequence's new position
+            constexpr uint32_t KT = UP / 8, NS = HD / 32;   // eights of positions in a tile; k slices of a score
+            float m = -INFINITY, l = 0.0f, acc[8];   // this lane's 8 columns, of its share of the positions
+#pragma unroll
+            for (int e = 0; e < 8; e++) acc[e] = 0.0f;
+            if (wg < u.nb) {
+                // This lane's 8 columns of the new token's query; of the newest tile's warp also of its key and value, which go to the pools and
+                // (below) into the tile. All of it, the rotation's factors and the place in the pools are asked for together.
+                const bool owner = newest && wg == (wpi == NW ? (u.nb - 1) % NW : (u.nb - 1) & 3u);
+                const uint8_t* const src = qkv + ((size_t)u.row * 3 * D + u.head * HD + chunk * 8) * 4;
+                const float4* const rt = reinterpret_cast<const float4*>(a.rope + (size_t)pos * (HD / 2) + chunk * 4);
+                const float4 r0 = __ldg(rt), r1 = __ldg(rt + 1);
+                const uint32_t pb = owner ? (uint32_t)__ldg(a.block_tables + (size_t)u.row * a.max_blocks + pos / 16) : 0u;
+                uint4 qa[NS], kn = make_uint4(0, 0, 0, 0), vn = kn;
+                {
+                    uint4 x[6];
+                    uint32_t n = 0;
+                    Waiter w = wt;
+#pragma unroll
+                    for (int i = 0; i < 6; i++) x[i] = make_uint4(0, 0, 0, 0);
+                    bool lack;
+#pragma unroll 1
+                    do {
+#pragma unroll
+                        for (int i = 0; i < 6; i++)
+                            if (i < 2 || owner) x[i] = xld4(src + (size_t)(i >> 1) * D * 4 + (i & 1) * 16);
+                        lack = max(max(x[0].x, x[1].x), max(max(x[2].x, x[3].x), max(x[4].x, x[5].x))) == EMPTY;
+                    } while (__any_sync(0xffffffffu, lack) && !__any_sync(0xffffffffu, w.give_up(n)));
+                    auto packed = [&](const uint4& lo, const uint4& hi, bool rotate) {
+                        float o[8] = {__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z), __uint_as_float(lo.w),
+                                      __uint_as_float(hi.x), __uint_as_float(hi.y), __uint_as_float(hi.z), __uint_as_float(hi.w)};
+                        if (rotate) {
+                            rope_rotate(o[0], o[1], r0.x, r0.y, o[0], o[1]);
+                            rope_rotate(o[2], o[3], r0.z, r0.w, o[2], o[3]);
+                            rope_rotate(o[4], o[5], r1.x, r1.y, o[4], o[5]);
+                            rope_rotate(o[6], o[7], r1.z, r1.w, o[6], o[7]);
+                        }
+                        return make_uint4(pack2(o[0], o[1]), pack2(o[2], o[3]), pack2(o[4], o[5]), pack2(o[6], o[7]));
+                    };
+                    const uint4 qn = packed(x[0], x[1], true);
+                    // A fragments: slice s of lane (g, t) is vector 4 s + t, held by the lane of that chunk
+#pragma unroll
+                    for (uint32_t s = 0; s < NS; s++) {
+                        const uint32_t from = s * 4 + (lane & 3);
+                        qa[s] = make_uint4(__shfl_sync(0xffffffffu, qn.x, from), __shfl_sync(0xffffffffu, qn.y, from), __shfl_sync(0xffffffffu, qn.z, from),
+                                           __shfl_sync(0xffffffffu, qn.w, from));
+                    }
+                    if (owner) {
+                        kn = packed(x[2], x[3], true);
+                        vn = packed(x[4], x[5], false);
+                        if (lane < CH) {
+                            const size_t prow = (((size_t)pb * H + u.head) * 16 + (pos & 15)) * HD + chunk * 8;
+                            *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(lw.k_pool) + prow) = kn;
+                            *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(lw.v_pool) + prow) = vn;
+                        }
+                    }
+                }
+                const float sc = a.scale * 1.44269504088896f;   // scores in units of ln 2
+#pragma unroll 1
+                for (uint32_t b = wg; b < u.nb; b += wpi) {
+                    const uint32_t left = u.n - b * UP;   // positions of the tile that count, if fewer than UP
+                    const bool fresh = newest && left <= UP;
+                    const uint32_t at = (left - 1) * (HD * 2) + chunk * 16;   // the new position's row in the buffers
+                    alive = wait_bar(&k_bar[cw], tiles_done & 1u, &dead) && alive;
+                    if (fresh) {
+                        if (lane < CH) {
+                            *reinterpret_cast<uint4*>(kbuf + at) = kn;
+                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // before the next tile's copy into the buffer
+                        }
+                        __syncwarp();
+                    }
+                    float p[KT][2];   // positions 8 n + 2 t, + 1 (t = lane % 4)
+#pragma unroll
+                    for (uint32_t n = 0; n < KT; n++) {
+                        float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                        for (uint32_t s = 0; s < NS; s++) {
+                            const uint4 w = *reinterpret_cast<const uint4*>(kbuf + (n * 8 + (lane >> 2)) * (HD * 2) + s * 64 + (lane & 3) * 16);
+                            mma(c, qa[s].x, qa[s].x, qa[s].y, qa[s].y, w.x, w.y);
+                            mma(c, qa[s].z, qa[s].z, qa[s].w, qa[s].w, w.z, w.w);
+                        }
+                        p[n][0] = c[0];
+                        p[n][1] = c[1];
+                    }
+                    __syncwarp();
+                    request(false);
+                    float mx = -INFINITY;
+#pragma unroll
+                    for (uint32_t n = 0; n < KT; n++)
+#pragma unroll
+                        for (uint32_t e = 0; e < 2; e++) {
+                            if (n * 8 + (lane & 3) * 2 + e >= left) p[n][e] = -INFINITY;
+                            mx = fmaxf(mx, p[n][e]);
+                        }
+                    const float m2 = fmaxf(m, redux_max(mx) * sc), corr = ex2(m - m2);
+                    m = m2;
+                    l *= corr;
+                    // Every four lanes hold all probabilities; lane (g, t) keeps those of positions 8 n + 2 t + (g & 1) to hand out
+#pragma unroll
+                    for (uint32_t n = 0; n < KT; n++) {
+                        p[n][0] = ex2(fmaf(p[n][0], sc, -m2));
+                        p[n][1] = ex2(fmaf(p[n][1], sc, -m2));
+                        l += p[n][0] + p[n][1];
+                        p[n][0] = (lane & 4) ? p[n][1] : p[n][0];
+                    }
+#pragma unroll
+                    for (int e = 0; e < 8; e++) acc[e] *= corr;
+                    alive = wait_bar(&v_bar[cw], tiles_done & 1u, &dead) && alive;
+                    if (fresh) {   // what lies behind the sequence's end is anything, a NaN even
+                        if (lane < CH) *reinterpret_cast<uint4*>(vbuf + at) = vn;
+#pragma unroll 1
+                        for (uint32_t z = left * CH + lane; z < UP * CH; z += 32) *reinterpret_cast<uint4*>(vbuf + z * 16) = make_uint4(0, 0, 0, 0);
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        __syncwarp();
+                    }
+                    // values: this lane's vector i is of position PPI i + lane / CH
+#pragma unroll
+                    for (uint32_t i = 0; i < 8; i++) {
+                        const uint32_t r = (i * PPI & 7) + lane / CH;   // of the eight i PPI / 8
+                        const float pv = __shfl_sync(0xffffffffu, p[i * PPI / 8][0], (r & 1) * 4 + (r >> 1));
+                        float vx[8];
+                        unpack8(*reinterpret_cast<const uint4*>(vbuf + i * 512 + lane * 16), vx);
+#pragma unroll
+                        for (int e = 0; e < 8; e++) acc[e] = fmaf(pv, vx[e], acc[e]);
+                    }
+                    __syncwarp();
+                    request(true);
+                    tiles_done ^= 1u;
+                }
+            }
+            l += __shfl_xor_sync(0xffffffffu, l, 1);
+            l += __shfl_xor_sync(0xffffffffu, l, 2);
+            {   // the warp's sums over its shares of the positions (lanes with the same chunk)
+                float* const my_acc = at_acc + (buf * NW + cw) * HD + chunk * 8;
+                const bool h16 = lane & 16;
+                float t4[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) t4[i] = (h16 ? acc[4 + i] : acc[i]) + __shfl_xor_sync(0xffffffffu, h16 ? acc[i] : acc[4 + i], 16);
+                if (CH == 8) {
+                    const bool h8 = lane & 8;
+                    float t2[2];
+#pragma unroll
+                    for (int i = 0; i < 2; i++) t2[i] = (h8 ? t4[2 + i] : t4[i]) + __shfl_xor_sync(0xffffffffu, h8 ? t4[i] : t4[2 + i], 8);
+                    *reinterpret_cast<float2*>(my_acc + (h16 ? 4 : 0) + (h8 ? 2 : 0)) = make_float2(t2[0], t2[1]);
+                } else {
+                    *reinterpret_cast<float4*>(my_acc + (h16 ? 4 : 0)) = make_float4(t4[0], t4[1], t4[2], t4[3]);
+                }
+            }
+            if (lane == 0) at_ml[buf][cw] = make_float2(m, l);
+            bar_sync_n(BAR_GROUP + grp, wpi * 32);
+            if (wg == j % wpi) {   // one warp merges the group's, in warp order
+                const float2 ml = lane < wpi ? at_ml[buf][grp * wpi + lane] : make_float2(-INFINITY, 0.0f);
+                const float M = redux_max(ml.x), f = ex2(ml.x - M), ls = warp_sum(ml.y * f);
+                float o[DL];
+#pragma unroll
+                for (uint32_t e = 0; e < DL; e++) o[e] = 0.0f;
+                const float* src = at_acc + (buf * NW + grp * wpi) * HD + lane * DL;
+#pragma unroll 4
+                for (uint32_t w = 0; w < wpi; w++) {   // (wpi is 4 or 12)
+                    const float fw = __shfl_sync(0xffffffffu, f, w);
+#pragma unroll
+                    for (uint32_t e = 0; e < DL; e++) o[e] = fmaf(src[w * HD + e], fw, o[e]);
+                }
+                if (!SPLIT || len_sm[u.row] <= SPLIT_LEN) {
+                    put_at(set, u.row, u.head, o, ls);
+                } else {
+                    uint8_t* dst = a.xch + set + so.part + ((size_t)(u.row * H + u.head) * splits + u.split) * (HD + 4) * 4;
+                    if constexpr (DL == 2) xst2(dst + lane * 8, word(o[0]), word(o[1]));
+                    else xst4(dst + lane * 16, word(o[0]), word(o[1]), word(o[DL - 2]), word(o[DL - 1]));
+                    if (lane == 0) xst2(dst + HD * 4, word(M), word(ls));
+                }
+            }
+        }
+        // rows of several splits, each (row, head) by one warp of the chip: after all of its own units, so that nobody waits for a unit behind a merge
+        if (SPLIT) {
+#pragma unroll 1
+            for (uint32_t i = cw * B200_SMS + cta; i < n_act * H; i += NW * B200_SMS) {
+                const uint32_t row = by_len[i / H], head = i % H, n = len_sm[row], ns = div_up(n, SPLIT_LEN);
+                if (ns <= 1) break;   // (longest first)
+                const uint8_t* src = a.xch + set + so.part + (size_t)(row * H + head) * splits * (HD + 4) * 4;
+                float M = -INFINITY, ls = 0.0f, o[DL];
+#pragma unroll
+                for (uint32_t e = 0; e < DL; e++) o[e] = 0.0f;
+#pragma unroll 1
+                for (uint32_t s0 = 0; s0 < ns; s0 += 2) {
+                    uint2 ml[2], x[2][DL / 2];
+                    auto get = [&](int k) {
+                        const uint8_t* p = src + (size_t)(s0 + k) * (HD + 4) * 4;
+                        ml[k] = xld2(p + HD * 4);
+#pragma unroll
+                        for (uint32_t e = 0; e < DL / 2; e++) x[k][e] = xld2(p + lane * (DL * 4) + e * 8);
+                    };
+                    auto lacks = [&](int k) {
+                        bool b = ml[k].x == EMPTY || ml[k].y == EMPTY;
+#pragma unroll
+                        for (uint32_t e = 0; e < DL / 2; e++) b = b || x[k][e].x == EMPTY || x[k][e].y == EMPTY;
+                        return b;
+                    };
+#pragma unroll
+                    for (int k = 0; k < 2; k++)
+                        if (s0 + k < ns) get(k);
+                    uint32_t tries = 0;
+#pragma unroll 1
+                    for (;;) {
+                        bool again = false;
+#pragma unroll
+                        for (int k = 0; k < 2; k++)
+                            if (s0 + k < ns && lacks(k)) { get(k); again = true; }
+                        Waiter w = wt;
+                        if (!again || w.give_up(tries)) break;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 2; k++)
+                        if (s0 + k < ns) {
+                            const float pm = __uint_as_float(ml[k].x), m2 = fmaxf(M, pm), f0 = ex2(M - m2), f1 = ex2(pm - m2);
+                            M = m2;
+                            ls = ls * f0 + __uint_as_float(ml[k].y) * f1;
+#pragma unroll
+                            for (uint32_t e = 0; e < DL; e++) o[e] = o[e] * f0 + __uint_as_float(e & 1 ? x[k][e / 2].y : x[k][e / 2].x) * f1;
+                        }
+                }
+                put_at(set, row, head, o, ls);
+            }
+            __syncwarp();
+        }
+    };
+
+#pragma unroll 1
+    for (uint32_t i = 0; i < 4 * L; i++) {
+        const uint32_t l = i >> 2, ph = i & 3, set = set_of(e0 + 1 + l);
+        if (ph == OUT) {
+            attention(layers_sm[l], set);
+            if (l + 1 == L && lane == 0) mbar_arrive(&kv_free_bar);   // (its tiles have been read)
+        }
+        gemm(ph == QKV ? set_of(e0 + l) + so.x1 : set + (ph == OUT ? so.at : ph == FFN_UP ? so.x2 : so.up), kinds[ph]);
+    }
+    // ---- lm_head and greedy argmax. The last x goes to shared memory (where the cache tiles were), and a warp has a tile of the weights to itself: no
+    // sums across warps. A row's 1 / rms is left out, it does not change which logit is the largest.
+    {
+        const uint32_t fin = set_of(e0 + L) + so.best, x = set_of(e0 + L) + so.x1;
+        const Kind& d = kinds[HEAD];
+        uint4* const xs = reinterpret_cast<uint4*>(kv_sm);   // [slice][m][half][lane]
+#pragma unroll 1
+        for (uint32_t sl = cw; sl < d.slices; sl += NW)
+#pragma unroll
+            for (uint32_t p = 0; p < 2 * MT; p++) {
+                uint4 v = make_uint4(0, 0, 0, 0);
+                uint32_t n = 0;
+                Waiter w = wt;
+                if (a_live >> p & 1u)
+#pragma unroll 1
+                    do v = xld4(a.xch + x + (sl * (2 * MT) + p) * 512 + frag_lane * 16);
+                    while (v.x == EMPTY && !w.give_up(n));
+                xs[(sl * (2 * MT) + p) * 32 + lane] = v;
+            }
+        __syncwarp();
+        bar_sync<NCT>(BAR_HEAD);
+        float best_v[2 * MT];   // rows 8 p + lane / 4, of this lane's columns
+        uint32_t best_i[2 * MT];
+#pragma unroll
+        for (uint32_t p = 0; p < 2 * MT; p++) { best_v[p] = -INFINITY; best_i[p] = NO_LOGIT; }
+        // The chunks of tile t are numbers per t .. of the lm_head's; `base` chunks went through the ring before. Only the tile's warp waits for them, so it
+        // looks first whether the slot is in that use at all: a parity alone would take the use before the last for it.
+        const uint32_t per = d.chunks, busy = min(NW, max(1u, head_slots / per));   // (more warps than the ring holds tiles would only wait)
+        uint32_t base = 0;
+#pragma unroll 1
+        for (uint32_t k = 0; k < HEAD; k++) base += L * kinds[k].n * kinds[k].chunks;
+#pragma unroll 1
+        for (uint32_t t = cw; t < d.n && cw < busy; t += busy) {
+            float acc[MT][4], odd[MT][4];   // two chains of products
+#pragma unroll
+            for (uint32_t m = 0; m < MT; m++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) acc[m][k] = odd[m][k] = 0.0f;
+#pragma unroll 1
+            for (uint32_t c = 0; c < per; c++) {
+                const uint32_t at = t * per + c, lap = at / head_slots, r = at - lap * head_slots, ring = base + lap * slots + r;
+                const uint32_t use = r < slots ? ring / slots : lap, bar = r < slots ? ring % slots : MAX_SLOTS + r - slots;
+                uint32_t n = 0;
+                Waiter wait = wt;
+#pragma unroll 1
+                while (*(volatile uint32_t*)&use_sm[bar] != use + 1 && !wait.give_up(n)) {}
+                __syncwarp();
+                alive = __all_sync(0xffffffffu, *(volatile uint32_t*)&use_sm[bar] == use + 1 && wait_bar(&full_bar[bar], use & 1u, &dead) && alive) != 0;
+                const uint8_t* const wp = (r < slots ? smem + bar * SLOT : extra_sm + (r - slots) * SLOT) + (lane >> 2) * d.pitch + (lane & 3) * 16;
+                const uint4* const xp = xs + c * CHUNK * (2 * MT) * 32 + lane;
+                const uint32_t ns = d.count(c);
+#pragma unroll 4
+                for (uint32_t k = 0; k < ns; k++) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(wp + k * 64);
+#pragma unroll
+                    for (uint32_t m = 0; m < MT; m++) {
+                        const uint4 x0 = xp[(k * (2 * MT) + 2 * m) * 32], x1 = xp[(k * (2 * MT) + 2 * m + 1) * 32];
+                        mma(acc[m], x0.x, x1.x, x0.y, x1.y, w.x, w.y);
+                        mma(odd[m], x0.z, x1.z, x0.w, x1.w, w.z, w.w);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0 && alive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&empty_bar[bar])), "r"(NW) : "memory");
+            }
+#pragma unroll
+            for (uint32_t m = 0; m < MT; m++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) acc[m][k] += odd[m][k];
+            // columns 2 (lane % 4), + 1, in ascending order: the first of the largest stays
+            const uint32_t c0 = (d.t0 + t) * 8 + (lane & 3) * 2;
+#pragma unroll
+            for (uint32_t p = 0; p < 2 * MT; p++)
+#pragma unroll
+                for (uint32_t k = 0; k < 2; k++)
+                    if (c0 + k < a.vocab && acc[p >> 1][(p & 1) * 2 + k] > best_v[p]) { best_v[p] = acc[p >> 1][(p & 1) * 2 + k]; best_i[p] = c0 + k; }
+        }
+        // this SM's best of each row, then over the SMs, row r by SM r; the lowest index wins ties
+        auto better = [](float& v, uint32_t& n, float ov, uint32_t on) { if (ov > v || (ov == v && on < n)) { v = ov; n = on; } };
+        uint2* const best_sm = reinterpret_cast<uint2*>(at_acc);   // [R][NW]
+#pragma unroll
+        for (uint32_t p = 0; p < 2 * MT; p++) {
+#pragma unroll
+            for (int k = 1; k < 4; k <<= 1) {
+                const float ov = __shfl_xor_sync(0xffffffffu, best_v[p], k);
+                const uint32_t on = __shfl_xor_sync(0xffffffffu, best_i[p], k);
+                better(best_v[p], best_i[p], ov, on);
+            }
+            if ((lane & 3) == 0) best_sm[(p * 8 + (lane >> 2)) * NW + cw] = make_uint2(__float_as_uint(best_v[p]), best_i[p]);
+        }
+        bar_sync<NCT>(BAR_HEAD);
+        if (ct < R && row_live(ct)) {
+            float v = -INFINITY;
+            uint32_t n = NO_LOGIT;
+#pragma unroll
+            for (uint32_t k = 0; k < NW; k++) {
+                const uint2 o = best_sm[ct * NW + k];
+                better(v, n, __uint_as_float(o.x), o.y);
+            }
+            xst2(a.xch + fin + (ct * B200_SMS + cta) * 8, word(v), n);
+        }
+        if (cta < R && row_live(cta) && cw == 0) {
+            __syncwarp();
+            float v = -INFINITY;
+            uint32_t n = NO_LOGIT;
+#pragma unroll 1
+            for (uint32_t c = lane; c < B200_SMS; c += 32) {
+                uint2 o;
+                uint32_t polls = 0;
+                Waiter w = wt;
+#pragma unroll 1
+                do o = xld2(a.xch + fin + (cta * B200_SMS + c) * 8);
+                while ((o.x == EMPTY || o.y == EMPTY) && !w.give_up(polls));
+                better(v, n, __uint_as_float(o.x), o.y);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 16; k > 0; k >>= 1) {
+                const float ov = __shfl_xor_sync(0xffffffffu, v, k);
+                const uint32_t on = __shfl_xor_sync(0xffffffffu, n, k);
+                better(v, n, ov, on);
+            }
+            if (lane == 0) a.sampled[cta] = n < a.vocab ? n : 0u;   // (no logit above -inf: 0)
+        }
+    }
+    if (!alive || *(volatile uint32_t*)&dead) {
+        // tiles this warp requested and may not have waited for (their copies end by themselves)
+        mbar_wait(&k_bar[cw], tiles_done & 1u);
+        mbar_wait(&v_bar[cw], tiles_done & 1u);
+        if (lane == 0) atomicExch(a.status, 1u);
+    }
+}
+
+struct Plan {
+    uint32_t slots, wpi;
+    size_t smem;
+};
+Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len) {
+    const uint32_t hd = dim / heads;
+    const size_t rest = NW * 2 * KV_BUF + (size_t)NW * TB * m_tiles(seqs) * 16 * 32 + 2 * NW * hd * 4 + TB * 32 * 2 * 16 + (size_t)(2 * n_layers + 1) * div_up(dim / 8, B200_SMS) * 32;
+    Plan p;
+    p.slots = (uint32_t)((MAX_DYN_SMEM - rest) / SLOT);
+    if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
+    p.smem = p.slots * SLOT + rest;
+    // Few units: all warps of an SM work on one; else four, so that an SM's units overlap.
+    p.wpi = seqs * heads * div_up(max_len, split_len(max_len)) <= B200_SMS ? 12 : 4;
+    return p;
+}
+
+template <int HD, int MT, bool SPLIT>
+int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p) {
+    {
+        static bool attr_set[64] = {};
+        int dev = 0;
+        AK_CUDA(cudaGetDevice(&dev));
+        std::lock_guard<std::mutex> lock(device_cache_mutex());
+        if (!attr_set[dev & 63]) {
+            AK_CUDA(cudaFuncSetAttribute(batch_kernel<HD, MT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
+            attr_set[dev & 63] = true;
+        }
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(B200_SMS);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    AK_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel<HD, MT, SPLIT>, a, p.slots, p.wpi));
+    AK_COUNT_LAUNCH();
+    return AK_OK;
+}
+
+}  // namespace
+
+int batch_maps(void* out, const SoloLayer* layers, const void* lm_head, uint32_t n_layers, uint32_t dim, uint32_t ffn, uint32_t vocab) {
+    CUtensorMap* m = reinterpret_cast<CUtensorMap*>(out);
+    auto put = [&](const void* w, uint32_t rows, uint32_t k) { return make_tmap_rows(m++, w, rows, k, piece_of(k), chunk_cols(k) / piece_of(k), 8); };
+    for (uint32_t l = 0; l < n_layers; l++) {
+        AK_TRY(put(layers[l].qkv, 3 * dim, dim));
+        AK_TRY(put(layers[l].out, dim, dim));
+        AK_TRY(put(layers[l].up, ffn, dim));
+        AK_TRY(put(layers[l].down, dim, ffn));
+    }
+    return put(lm_head, vocab, dim);
+}
+
+bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers, uint32_t seqs, uint32_t max_len) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+    const uint32_t hd = heads ? dim / heads : 0;
+    if ((uint32_t)sms < B200_SMS || dtype != AK_BF16 || (hd != 64 && hd != 128) || dim != heads * hd || heads > 4095) return false;
+    if (seqs < 1 || seqs > 32 || n_layers < 1 || n_layers > MAX_LAYERS || dim < 96 || dim % 32 || ffn % 32 || ffn > 65536) return false;
+    if (ffn / 8 < B200_SMS) return false;                                        // every SM has ffn-up rows (the clearing of the sets counts on it)
+    if (div_up(dim / 8, B200_SMS) > TB) return false;                            // the residual stream is worked on in one pass
+    if (dim * m_tiles(seqs) * 16 * 2 > NW * 2 * KV_BUF) return false;             // the lm_head keeps x where the cache tiles were
+    const uint32_t splits = div_up(max_len, split_len(max_len));
+    const Plan p = make_plan(dim, n_layers, heads, seqs, max_len);
+    if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * B200_SMS * (NW / p.wpi)) return false;
+    const SetOff so(dim, ffn, heads, m_tiles(seqs), splits);
+    return p.slots >= 4 && 3 * so.total < (1ull << 32);
+}
+
+size_t batch_xch_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) {
+    return 3 * SetOff(dim, ffn, heads, m_tiles(seqs), div_up(max_len, split_len(max_len))).total;
+}
+
+int launch_batch(cudaStream_t st, const BatchArgs& a) {
+    const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.seqs, a.max_len);
+    const bool two = m_tiles(a.seqs) == 2, split = a.max_len > split_len(a.max_len);
+    if (a.dim / a.heads == 64) {
+        if (split) return two ? launch_batch_t<64, 2, true>(st, a, p) : launch_batch_t<64, 1, true>(st, a, p);
+        return two ? launch_batch_t<64, 2, false>(st, a, p) : launch_batch_t<64, 1, false>(st, a, p);
+    }
+    if (split) return two ? launch_batch_t<128, 2, true>(st, a, p) : launch_batch_t<128, 1, true>(st, a, p);
+    return two ? launch_batch_t<128, 2, false>(st, a, p) : launch_batch_t<128, 1, false>(st, a, p);
+}
+
+}  // namespace ak

@@ -137,6 +137,11 @@ int ak_engine_create(ak_ctx* ctx, ak_weights* w, const ak_engine_config* cfg, ak
     }
     e->chunk_rows = e->runner.chunked_prefill_supported() ? cfg->prefill_chunk_rows : 0;
     if (e->chunk_rows > e->runner.max_prefill_tokens()) e->chunk_rows = e->runner.max_prefill_tokens();
+    // (with attn_timing the decode attention has to be a launch of its own)
+    if (!cfg->attn_timing) {
+        rc = e->runner.init_batch();
+        if (rc) { delete e; return rc; }
+    }
     e->runner.enable_attn_timing(cfg->attn_timing != 0);
     e->runner.set_keep_logits(false);
     for (const auto& pr : w->params)
@@ -261,7 +266,7 @@ int ak_engine_step(ak_engine* e, uint32_t* n_running, uint32_t* n_waiting) {
             const uint32_t pos = s->cached;
             rows[i] = {-(int32_t)(i + 1), (int32_t)pos, s->blocks[pos / 16] * 16 + (int32_t)(pos % 16), (int32_t)i};
             kv[i] = (int32_t)(pos + 1);
-            outr[i] = (int32_t)i;
+            outr[i] = r.batch() ? -1 : (int32_t)i;
             any_decode = true;
             n_dec++;
             if (pos + 1 > max_kv) max_kv = pos + 1;

@@ -252,7 +252,7 @@ Runner::~Runner() {
     cudaFree(amax_val_); cudaFree(amax_idx_); cudaFree(tp_tmp_);
     cudaFree(xf_); cudaFree(logits_); cudaFree(attn_scratch_); cudaFree(rope_table_);
     cudaFree(d_desc_); cudaFree(d_sampled_);
-    cudaFree(d_solo_layers_); cudaFree(d_solo_xch_);
+    cudaFree(d_solo_layers_); cudaFree(d_solo_xch_); cudaFree(d_batch_layers_); cudaFree(d_batch_maps_); cudaFree(d_batch_xch_);
     if (h_solo_done_) cudaFreeHost(h_solo_done_);
     if (h_logits_) cudaFreeHost(h_logits_);
     for (Bank& b : banks_) {
@@ -286,14 +286,15 @@ int Runner::init(ak_ctx* ctx, ak_weights* w, uint32_t max_seqs, uint32_t max_seq
     d_.pf_cu = d_.row_order + max_seqs;
     d_.pf_slot = d_.pf_cu + max_seqs + 1;
     d_.pf_pos0 = d_.pf_slot + max_seqs;
-    d_.block_tables = d_.pf_pos0 + max_seqs;
+    d_.batch_set = d_.pf_pos0 + max_seqs;
+    d_.block_tables = d_.batch_set + 1;
     d_.rows = align_up(d_.block_tables + max_seqs * max_blocks_, 4);
     d_.total = d_.rows + max_rows_ * 4;
     for (Bank& b : banks_) {
         AK_CUDA(cudaMallocHost((void**)&b.h_desc, (size_t)d_.total * 4));
         memset(b.h_desc, 0, (size_t)d_.total * 4);
-        AK_CUDA(cudaMallocHost((void**)&b.h_sampled, (size_t)max_seqs * 4));
-        memset(b.h_sampled, 0, (size_t)max_seqs * 4);
+        AK_CUDA(cudaMallocHost((void**)&b.h_sampled, sampled_words() * 4));
+        memset(b.h_sampled, 0, sampled_words() * 4);
     }
     bank_ = 0;
     h_desc_ = banks_[0].h_desc;
@@ -301,8 +302,8 @@ int Runner::init(ak_ctx* ctx, ak_weights* w, uint32_t max_seqs, uint32_t max_seq
     AK_CUDA(cudaMalloc((void**)&d_desc_, (size_t)d_.total * 4));
     AK_CUDA(cudaMemset(d_desc_, 0, (size_t)d_.total * 4));
 
-    AK_CUDA(cudaMalloc((void**)&d_sampled_, (size_t)max_seqs * 4));
-    AK_CUDA(cudaMemset(d_sampled_, 0, (size_t)max_seqs * 4));
+    AK_CUDA(cudaMalloc((void**)&d_sampled_, sampled_words() * 4));
+    AK_CUDA(cudaMemset(d_sampled_, 0, sampled_words() * 4));
 
     const size_t pool_bytes = (size_t)n_blocks_ * heads_l_ * 16 * hd * act;  // each rank caches its own heads
     k_pool_.assign(c.num_layers, nullptr);
@@ -373,17 +374,76 @@ int Runner::init(ak_ctx* ctx, ak_weights* w, uint32_t max_seqs, uint32_t max_seq
     return AK_OK;
 }
 
-int Runner::init_solo() {
-    const ak_model_config& c = w_->cfg;
-    if (max_seqs_ != 1 || tp_ != 1 || !solo_supported(w_->dtype, c.dim, c.ffn_hidden, c.num_heads, c.num_layers, c.vocab_size)) return AK_OK;
-    std::vector<SoloLayer> sl(c.num_layers);
-    for (uint32_t l = 0; l < c.num_layers; l++) {
+// the layers as the persistent kernels want them
+std::vector<SoloLayer> Runner::solo_layers() const {
+    std::vector<SoloLayer> sl(w_->cfg.num_layers);
+    for (uint32_t l = 0; l < w_->cfg.num_layers; l++) {
         const auto& b = w_->blocks[l];
         sl[l] = {b.norm_1, b.qkv, b.out, b.norm_2, b.up, b.down, k_pool_[l], v_pool_[l]};
     }
+    return sl;
+}
+int Runner::upload_layers(SoloLayer** out) {
+    const std::vector<SoloLayer> sl = solo_layers();
+    AK_CUDA(cudaMalloc((void**)out, sl.size() * sizeof(SoloLayer)));
+    AK_CUDA(cudaMemcpyAsync(*out, sl.data(), sl.size() * sizeof(SoloLayer), cudaMemcpyHostToDevice, ctx_->stream));
+    AK_CUDA(cudaStreamSynchronize(ctx_->stream));
+    return AK_OK;
+}
+
+int Runner::init_batch() {
+    const ak_model_config& c = w_->cfg;
+    if (tp_ != 1 || !batch_supported(w_->dtype, c.dim, c.ffn_hidden, c.num_heads, c.num_layers, max_seqs_, max_seq_len_)) return AK_OK;
+    AK_TRY(upload_layers(&d_batch_layers_));
+    std::vector<char> maps((4 * c.num_layers + 1) * 128 + 64);
+    void* const host = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(maps.data()) + 63) & ~(uintptr_t)63);   // (a map's alignment)
+    AK_TRY(batch_maps(host, solo_layers().data(), w_->lm_head, c.num_layers, c.dim, c.ffn_hidden, c.vocab_size));
+    AK_CUDA(cudaMalloc(&d_batch_maps_, (4 * c.num_layers + 1) * 128));
+    AK_CUDA(cudaMemcpyAsync(d_batch_maps_, host, (4 * c.num_layers + 1) * 128, cudaMemcpyHostToDevice, ctx_->stream));
+    const size_t bytes = batch_xch_bytes(c.dim, c.ffn_hidden, c.num_heads, max_seqs_, max_seq_len_);
+    AK_CUDA(cudaMalloc((void**)&d_batch_xch_, bytes));
+    AK_CUDA(cudaMemsetAsync(d_batch_xch_, 0xff, bytes, ctx_->stream));
+    AK_CUDA(cudaStreamSynchronize(ctx_->stream));
+    batch_ = true;
+    return AK_OK;
+}
+
+// The step's words of the descriptor. The exchange sets move on by a set per layer and one for the embedding, if there is a decode row.
+void Runner::describe_batch() {
+    if (!batch_) return;
+    h_desc_[d_.batch_set] = (int32_t)batch_set_;
+    bool any = false;
+    for (uint32_t i = 0; i < max_seqs_; i++) any = any || h_kv_lens()[i] > 0;
+    if (any) batch_set_ = (batch_set_ + w_->cfg.num_layers + 1) % 3;
+}
+
+int Runner::launch_decode_batch() {
+    const ak_model_config& c = w_->cfg;
+    BatchArgs a{};
+    a.layers = d_batch_layers_;
+    a.embedding = w_->embedding;
+    a.final_norm = w_->final_norm;
+    a.maps = d_batch_maps_;
+    a.rope = rope_table_;
+    a.xch = d_batch_xch_;
+    a.sampled = d_sampled_;
+    a.rows = d_desc_ + d_.rows;
+    a.kv_lens = d_desc_ + d_.kv_lens;
+    a.block_tables = d_desc_ + d_.block_tables;
+    a.set0 = reinterpret_cast<const uint32_t*>(d_desc_ + d_.batch_set);
+    a.status = d_sampled_ + max_seqs_;
+    a.n_layers = c.num_layers; a.dim = c.dim; a.ffn = c.ffn_hidden; a.heads = c.num_heads; a.vocab = c.vocab_size;
+    a.seqs = max_seqs_; a.max_blocks = max_blocks_; a.max_len = max_seq_len_;
+    a.eps = c.norm_eps;
+    a.scale = 1.0f / sqrtf((float)(c.dim / c.num_heads));
+    return launch_batch(ctx_->stream, a);
+}
+
+int Runner::init_solo() {
+    const ak_model_config& c = w_->cfg;
+    if (max_seqs_ != 1 || tp_ != 1 || !solo_supported(w_->dtype, c.dim, c.ffn_hidden, c.num_heads, c.num_layers, c.vocab_size)) return AK_OK;
+    AK_TRY(upload_layers(&d_solo_layers_));
     const size_t words = solo_xch_words(c.dim, c.ffn_hidden, c.num_heads, c.num_layers);
-    AK_CUDA(cudaMalloc((void**)&d_solo_layers_, sl.size() * sizeof(SoloLayer)));
-    AK_CUDA(cudaMemcpyAsync(d_solo_layers_, sl.data(), sl.size() * sizeof(SoloLayer), cudaMemcpyHostToDevice, ctx_->stream));
     AK_CUDA(cudaMalloc((void**)&d_solo_xch_, words * 8));
     AK_CUDA(cudaMemsetAsync(d_solo_xch_, 0, words * 8, ctx_->stream));
     AK_CUDA(cudaMallocHost((void**)&h_solo_done_, SOLO_AHEAD * 8));
@@ -566,7 +626,14 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
         // A step of at most 128 rows (the decode rows plus one prompt chunk) is ONE row tile of every projection: the
         // prompt rows ride in the decode launches for free. Larger admission steps run the two kinds of rows as two
         // ranges on two streams.
-        if (two_streams_ && any_decode && T > max_seqs_ && n_pf_seqs && T > 128) {
+        if (batch_) {
+            // The persistent kernel takes the whole chip, so the prompt rows follow it. It samples the decode rows' tokens itself (their out_rows
+            // are -1); what comes after the ranges is for the prompts' last rows.
+            if (any_decode) RC(launch_decode_batch());
+            if (T == max_seqs_) return AK_OK;
+            rc = range(st, max_seqs_, T - max_seqs_, false, true);
+            if (rc) return rc;
+        } else if (two_streams_ && any_decode && T > max_seqs_ && n_pf_seqs && T > 128) {
             AK_CUDA(cudaEventRecord(ev_fork_, st));
             AK_CUDA(cudaStreamWaitEvent(st2_, ev_fork_, 0));
             rc = range(st, 0, max_seqs_, true, false);
@@ -667,7 +734,8 @@ int Runner::run(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_pf_len
     cudaStream_t st = ctx_->stream;
     const uint32_t T = max_seqs_ + n_prefill_rows;
     const size_t bytes = ((size_t)d_.rows + (size_t)T * 4) * 4;
-    attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
+    if (batch_) describe_batch();
+    else attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
     AK_CUDA(cudaMemcpyAsync(d_desc_, h_desc_, bytes, cudaMemcpyHostToDevice, st));
     // One split count per runner (from the longest sequence it can hold): eager and captured
     // steps then sum in the same order, so a sequence's tokens do not depend on its neighbours.
@@ -675,10 +743,10 @@ int Runner::run(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_pf_len
     const uint32_t n_splits = attn_decode_pick_splits(max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, max_seq_len_, true);
     int rc = launch_layers(T, n_prefill_rows, n_pf_seqs, max_pf_len, any_decode, n_splits, false);
     if (rc) return rc;
-    AK_CUDA(cudaMemcpyAsync(h_sampled_, d_sampled_, (size_t)max_seqs_ * 4, cudaMemcpyDeviceToHost, st));
+    AK_CUDA(cudaMemcpyAsync(h_sampled_, d_sampled_, sampled_words() * 4, cudaMemcpyDeviceToHost, st));
     eager_steps++;
     h2d_bytes += bytes;
-    d2h_bytes += (size_t)max_seqs_ * 4;
+    d2h_bytes += sampled_words() * 4;
     return AK_OK;
 }
 
@@ -713,7 +781,8 @@ int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_
         int32_t* p0 = h_pf_pos0();
         for (uint32_t i = n_pf_seqs; i < seqs_b; i++) { cu[i + 1] = cu[n_pf_seqs]; pfs[i] = 0; p0[i] = 0; }
     }
-    attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
+    if (batch_) describe_batch();
+    else attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
     const uint64_t key = ((uint64_t)bank_ << 63) | ((uint64_t)rows_b << 32) | seqs_b;  // a graph bakes its bank's host buffers and events
     const uint32_t T = max_seqs_ + rows_b;
     const size_t bytes = ((size_t)d_.rows + (size_t)T * 4) * 4;
@@ -724,11 +793,11 @@ int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_
         AK_CUDA(cudaMemcpyAsync(d_desc_, h_desc_, bytes, cudaMemcpyHostToDevice, st));
         int rc = launch_layers(T, rows_b, seqs_b, len_b, true, n_splits, false);
         if (rc) return rc;
-        AK_CUDA(cudaMemcpyAsync(h_sampled_, d_sampled_, (size_t)max_seqs_ * 4, cudaMemcpyDeviceToHost, st));
+        AK_CUDA(cudaMemcpyAsync(h_sampled_, d_sampled_, sampled_words() * 4, cudaMemcpyDeviceToHost, st));
         AK_CUDA(cudaStreamSynchronize(st));
         eager_steps++;
         h2d_bytes += bytes;
-        d2h_bytes += (size_t)max_seqs_ * 4;
+        d2h_bytes += sampled_words() * 4;
         cudaGraph_t graph = nullptr;
         AK_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaMemcpyAsync(d_desc_, h_desc_, bytes, cudaMemcpyHostToDevice, st);
@@ -738,7 +807,7 @@ int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_
         g.kernels = g_launch_count - l0;
         g.h2d = bytes;
         g_launch_count = l0;  // recorded into the graph, not launched
-        if (rc == AK_OK) e = cudaMemcpyAsync(h_sampled_, d_sampled_, (size_t)max_seqs_ * 4, cudaMemcpyDeviceToHost, st);
+        if (rc == AK_OK) e = cudaMemcpyAsync(h_sampled_, d_sampled_, sampled_words() * 4, cudaMemcpyDeviceToHost, st);
         cudaError_t e2 = cudaStreamEndCapture(st, &graph);
         if (rc) return rc;
         if (e != cudaSuccess) return cuda_fail(e, "capture memcpy", __FILE__, __LINE__);
@@ -758,7 +827,7 @@ int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_
     graph_launches++;
     g_launch_count += it->second.kernels;
     h2d_bytes += it->second.h2d;
-    d2h_bytes += (size_t)max_seqs_ * 4;
+    d2h_bytes += sampled_words() * 4;
     return AK_OK;
 }
 
@@ -782,6 +851,7 @@ int Runner::mark_done() {
 int Runner::wait_bank(uint32_t b) {
     trace_dump();
     AK_CUDA(cudaEventSynchronize(banks_[b & 1u].ev_done));
+    AK_REQUIRE(banks_[b & 1u].h_sampled[max_seqs_] == 0, AK_ERR_DEVICE_WAIT, "decode step: a bounded device-side wait expired");
     return AK_OK;
 }
 

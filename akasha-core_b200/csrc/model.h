@@ -5,6 +5,7 @@
 #include <map>
 #include <vector>
 
+#include "batch.h"
 #include "kernels.h"
 #include "solo.h"
 #include "solo_plan.h"
@@ -65,7 +66,7 @@ struct RowInfo {
 };
 
 struct StepDesc {  // offsets (in int32 units) into the descriptor buffer
-    uint32_t kv_lens, out_rows, row_order, pf_cu, pf_slot, pf_pos0, block_tables, rows, total;
+    uint32_t kv_lens, out_rows, row_order, pf_cu, pf_slot, pf_pos0, batch_set, block_tables, rows, total;
 };
 
 class Runner {
@@ -107,6 +108,10 @@ class Runner {
     bool solo() const { return solo_; }
     int solo_launch(int32_t tok_src, uint32_t pos, bool want_logits, bool host_logits, uint32_t& ticket);
     int solo_wait(uint32_t ticket, uint32_t& token);   // AK_ERR_DEVICE_WAIT: a wait of the step ran out, there is no token
+    // Decode rows through one persistent kernel (batch.cu) instead of the launch chain, where model and slots allow it. A row's sums are not in
+    // the chain's order, so all decode rows of a runner's life take one of the two.
+    int init_batch();
+    bool batch() const { return batch_; }   // its decode rows are sampled by the kernel: their out_rows are -1
     // spin until a device-written pinned word {value, tag} carries `tag`
     int wait_word(const uint64_t* word, uint32_t tag, uint32_t& value);
     const float* solo_logits_host() const { return h_logits_; }
@@ -203,6 +208,16 @@ class Runner {
     uint64_t* h_solo_done_ = nullptr;   // pinned: one word per step in flight
     float* h_logits_ = nullptr;         // pinned, [vocab]
     uint32_t solo_step_ = 0;
+    bool batch_ = false;
+    uint8_t* d_batch_xch_ = nullptr;
+    SoloLayer* d_batch_layers_ = nullptr;
+    void* d_batch_maps_ = nullptr;
+    uint32_t batch_set_ = 0;            // exchange set of the next step's embedding
+    std::vector<SoloLayer> solo_layers() const;
+    int upload_layers(SoloLayer** out);
+    int launch_decode_batch();
+    void describe_batch();              // the step's words of the descriptor
+    size_t sampled_words() const { return max_seqs_ + 1; }   // the tokens, and the status word of the persistent step
     SoloArgs solo_args(int32_t tok_src, uint32_t pos);
     // Admission steps: the admitted prompts' rows run on a second stream, concurrently with the decode
     // rows (different sequences: they share nothing until the final norm).

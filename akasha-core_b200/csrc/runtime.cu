@@ -57,6 +57,22 @@ static EncodeTiledFn get_encode() {
     return fn;
 }
 
+int make_tmap_rows(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t inner, uint32_t box_pieces, uint32_t box_rows) {
+    EncodeTiledFn enc = get_encode();
+    AK_REQUIRE(enc, AK_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available from this driver");
+    AK_REQUIRE(((uintptr_t)base % 16) == 0 && inner % 8 == 0 && inner <= 256 && cols % inner == 0 && box_pieces <= 256 && box_rows <= 256, AK_ERR_INVALID_ARG,
+               "tensor map: bad rows (base %p, %llu columns in pieces of %u)", base, (unsigned long long)cols, inner);
+    cuuint64_t gdim[3] = {inner, cols / inner, rows};
+    cuuint64_t gstride[2] = {(cuuint64_t)inner * 2, cols * 2};
+    cuuint32_t box[3] = {inner, box_pieces, box_rows};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    AK_REQUIRE(r == CUDA_SUCCESS, AK_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d (rows %llu cols %llu)", (int)r, (unsigned long long)rows,
+               (unsigned long long)cols);
+    return AK_OK;
+}
+
 int make_tmap_2d(CUtensorMap* out, const void* base, uint32_t elem_bytes, uint64_t cols, uint64_t rows,
                  uint64_t row_stride_bytes, uint32_t box_cols, uint32_t box_rows, TmaSwizzle swizzle) {
     EncodeTiledFn enc = get_encode();

@@ -15,6 +15,10 @@ enum TmaSwizzle { TMA_SWIZZLE_NONE = 0, TMA_SWIZZLE_128B = 3 };
 int make_tmap_2d(CUtensorMap* out, const void* base, uint32_t elem_bytes, uint64_t cols, uint64_t rows,
                  uint64_t row_stride_bytes, uint32_t box_cols, uint32_t box_rows, TmaSwizzle swizzle);
 
+// bf16 [rows, cols] seen as [rows, cols / inner, inner], so that one box may hold more than 256 columns of its rows: box_pieces * inner of
+// them, row after row. What lies outside reads 0.
+int make_tmap_rows(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t inner, uint32_t box_pieces, uint32_t box_rows);
+
 #ifdef __CUDACC__
 // Tiled 2-D load, completion counted in bytes on `bar`. x (the innermost coordinate) times the
 // element size must be a multiple of 16 bytes.
@@ -23,6 +27,14 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* t
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
             smem_u32(smem_dst)),
         "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(y)
+        : "memory");
+}
+// A box of make_tmap_rows(): pieces from `piece` on of the rows from `row` on. `pol`: L2 cache policy.
+__device__ __forceinline__ void tma_load_rows(void* smem_dst, const CUtensorMap* tmap, int32_t piece, int32_t row, uint64_t* bar, uint64_t pol) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;" ::"r"(
+            smem_u32(smem_dst)),
+        "l"(tmap), "r"(smem_u32(bar)), "r"(0), "r"(piece), "r"(row), "l"(pol)
         : "memory");
 }
 // Tiled 2-D store from shared memory (elements outside the tensor are not written), and the same adding into f32. The

@@ -368,7 +368,8 @@ typedef struct ak_engine_config {
     uint32_t max_batch_tokens; /* token budget of one step (prefill + decode rows)  */
     uint32_t use_cuda_graph;   /* capture the decode-only step in a CUDA graph      */
     uint32_t stop_on_eos;      /* 0: run every sequence to its max_len              */
-    uint32_t attn_timing;      /* record CUDA events around layer 0's decode attention */
+    uint32_t attn_timing;      /* record CUDA events around layer 0's decode attention (which is then a launch of its own also with up
+                                  to 32 slots, where a decode step is otherwise one kernel) */
     uint32_t async_steps;      /* 1: ak_engine_step returns once step N is LAUNCHED and step N-1's tokens are on the
                                 * host, so describing and launching a step overlaps the previous step's GPU time.
                                 * Needs stop_on_eos == 0 (sequence ends must be known without the tokens);
