@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     }
     if (tid >= 32 && tid < 32 + N_KINDS) make_kind(kinds[tid - 32], tid == 32 ? 3 * D : tid == 34 ? F : tid == 36 ? a.vocab : D, tid == 35 ? F : D, cta);
     if (warp_ == 2) {   // the rows' lengths, the rows by length (the longest first), the attention splits of the rows before by that rank
-        const uint32_t n = lane < a.seqs ? min((uint32_t)max(a.kv_lens[lane], 0), a.max_len) : 0u;
+        const uint32_t n = lane < a.seqs ? min((uint32_t)max(a.rows ? a.kv_lens[lane] : a.lens[lane], 0), a.max_len) : 0u;
         uint32_t rank = 0;
 #pragma unroll
         for (uint32_t j = 0; j < 32; j++) {
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll 1
     for (uint32_t i = tid; i < L * (uint32_t)(sizeof(SoloLayer) / 8); i += THREADS)
         reinterpret_cast<uint64_t*>(layers_sm)[i] = reinterpret_cast<const uint64_t*>(a.layers)[i];
-    const uint32_t e0 = *a.set0 % 3;
+    const uint32_t e0 = (a.rows ? *a.set0 : a.set) % 3;
     __syncthreads();
 #pragma unroll 1
     for (uint32_t i = tid, n = kinds[OUT].n * 8; i < (2 * L + 1) * n; i += THREADS)
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 const uint32_t row = m * 16 + rl;
                 float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (row_live(row)) {
-                    const int32_t ts = a.rows[row * 4];
+                    const int32_t ts = a.rows ? a.rows[row * 4] : a.tok_src[row];
                     const uint32_t id = ts >= 0 ? (uint32_t)ts : a.sampled[(uint32_t)(-(ts + 1))];
                     if (id < a.vocab) {
                         const uint2 w = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(a.embedding) + (size_t)id * D + tile * 8 + h * 4);
@@ -1145,16 +1145,21 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             __syncwarp();
             float v = -INFINITY;
             uint32_t n = NO_LOGIT;
+            constexpr uint32_t PER = (B200_SMS + 31) / 32;
+            uint2 o[PER];
+            uint32_t polls = 0;
+            Waiter w = wt;
+            bool lack;
 #pragma unroll 1
-            for (uint32_t c = lane; c < B200_SMS; c += 32) {
-                uint2 o;
-                uint32_t polls = 0;
-                Waiter w = wt;
-#pragma unroll 1
-                do o = xld2(a.xch + fin + (cta * B200_SMS + c) * 8);
-                while ((o.x == EMPTY || o.y == EMPTY) && !w.give_up(polls));
-                better(v, n, __uint_as_float(o.x), o.y);
-            }
+            do {
+                lack = false;
+#pragma unroll
+                for (uint32_t k = 0; k < PER; k++) o[k] = lane + 32 * k < B200_SMS ? xld2(a.xch + fin + (cta * B200_SMS + lane + 32 * k) * 8) : make_uint2(0xff800000u, NO_LOGIT);
+#pragma unroll
+                for (uint32_t k = 0; k < PER; k++) lack = lack || o[k].x == EMPTY || o[k].y == EMPTY;
+            } while (lack && !w.give_up(polls));
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++) better(v, n, __uint_as_float(o[k].x), o[k].y);
             __syncwarp();
 #pragma unroll
             for (int k = 16; k > 0; k >>= 1) {
@@ -1162,14 +1167,21 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 const uint32_t on = __shfl_xor_sync(0xffffffffu, n, k);
                 better(v, n, ov, on);
             }
-            if (lane == 0) a.sampled[cta] = n < a.vocab ? n : 0u;   // (no logit above -inf: 0)
+            if (lane == 0) {
+                const uint32_t tok = n < a.vocab ? n : 0u;   // (no logit above -inf: 0)
+                a.sampled[cta] = tok;
+                if (a.sampled_host) a.sampled_host[cta] = tok;
+            }
         }
     }
     if (!alive || *(volatile uint32_t*)&dead) {
         // tiles this warp requested and may not have waited for (their copies end by themselves)
         mbar_wait(&k_bar[cw], tiles_done & 1u);
         mbar_wait(&v_bar[cw], tiles_done & 1u);
-        if (lane == 0) atomicExch(a.status, 1u);
+        if (lane == 0) {
+            atomicExch(a.status, 1u);
+            if (a.sampled_host) *(volatile uint32_t*)(a.sampled_host + a.seqs) = 1u;
+        }
     }
 }
 
@@ -1235,7 +1247,7 @@ bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads,
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
     const uint32_t hd = heads ? dim / heads : 0;
     if ((uint32_t)sms < B200_SMS || dtype != AK_BF16 || (hd != 64 && hd != 128) || dim != heads * hd || heads > 4095) return false;
-    if (seqs < 1 || seqs > 32 || n_layers < 1 || n_layers > MAX_LAYERS || dim < 96 || dim % 32 || ffn % 32 || ffn > 65536) return false;
+    if (seqs < 1 || seqs > BATCH_ROWS || n_layers < 1 || n_layers > MAX_LAYERS || dim < 96 || dim % 32 || ffn % 32 || ffn > 65536) return false;
     if (ffn / 8 < B200_SMS) return false;                                        // every SM has ffn-up rows (the clearing of the sets counts on it)
     if (div_up(dim / 8, B200_SMS) > TB) return false;                            // the residual stream is worked on in one pass
     if (dim * m_tiles(seqs) * 16 * 2 > NW * 2 * KV_BUF) return false;             // the lm_head keeps x where the cache tiles were

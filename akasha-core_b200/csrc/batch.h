@@ -5,6 +5,8 @@
 
 namespace ak {
 
+constexpr uint32_t BATCH_ROWS = 32;
+
 struct BatchArgs {
     const SoloLayer* layers;     // device array, one per layer; matrices [out, in] bf16
     const void* maps;            // device array of CUtensorMap (batch_maps): qkv, out, up, down of each layer, lm_head
@@ -13,10 +15,14 @@ struct BatchArgs {
     const float2* rope;          // [max_len][head_dim / 2] (cos, sin)
     uint8_t* xch;                // batch_xch_bytes(), all 0xff before the first launch
     uint32_t* sampled;           // [seqs]: the token fed back to a row with tok_src < 0, overwritten by the row's greedy pick
+    // The step, in device memory or (rows == nullptr) by value
     const int32_t* rows;         // [seqs] of int4 {tok_src, pos, slot, seq}
     const int32_t* kv_lens;      // [seqs]: positions attended to, the new one included; 0: the row is not there
-    const int32_t* block_tables; // [seqs][max_blocks]
     const uint32_t* set0;        // device word: exchange set of the step's embedding, advances by n_layers + 1 (mod 3) from step to step
+    int32_t tok_src[BATCH_ROWS], lens[BATCH_ROWS];
+    uint32_t set;
+    const int32_t* block_tables; // [seqs][max_blocks]
+    uint32_t* sampled_host;      // where else the picks go: [seqs] in mapped host memory and behind them the status word, or nullptr
     uint32_t* status;            // device word: made non-zero when a wait runs out
     uint32_t n_layers, dim, ffn, heads, vocab, seqs, max_blocks, max_len;
     float eps, scale;

@@ -417,7 +417,7 @@ void Runner::describe_batch() {
     if (any) batch_set_ = (batch_set_ + w_->cfg.num_layers + 1) % 3;
 }
 
-int Runner::launch_decode_batch() {
+BatchArgs Runner::batch_args() const {
     const ak_model_config& c = w_->cfg;
     BatchArgs a{};
     a.layers = d_batch_layers_;
@@ -427,16 +427,32 @@ int Runner::launch_decode_batch() {
     a.rope = rope_table_;
     a.xch = d_batch_xch_;
     a.sampled = d_sampled_;
-    a.rows = d_desc_ + d_.rows;
-    a.kv_lens = d_desc_ + d_.kv_lens;
     a.block_tables = d_desc_ + d_.block_tables;
-    a.set0 = reinterpret_cast<const uint32_t*>(d_desc_ + d_.batch_set);
     a.status = d_sampled_ + max_seqs_;
     a.n_layers = c.num_layers; a.dim = c.dim; a.ffn = c.ffn_hidden; a.heads = c.num_heads; a.vocab = c.vocab_size;
     a.seqs = max_seqs_; a.max_blocks = max_blocks_; a.max_len = max_seq_len_;
     a.eps = c.norm_eps;
     a.scale = 1.0f / sqrtf((float)(c.dim / c.num_heads));
-    return launch_batch(ctx_->stream, a);
+    return a;
+}
+
+// The block tables are on the device already: a sequence's were uploaded with its prompt's step, and they do not change. So neither a copy to
+// the device nor one back stands between two steps (162M model, 8 sequences: as a graph of copy, kernel, copy 15 us more per step).
+int Runner::run_decode_batch() {
+    AK_CUDA(cudaSetDevice(ctx_->device));
+    BatchArgs a = batch_args();
+    a.set = (uint32_t)h_desc_[d_.batch_set];
+    for (uint32_t i = 0; i < max_seqs_; i++) {
+        a.tok_src[i] = h_rows()[i].tok_src;
+        a.lens[i] = h_kv_lens()[i];
+    }
+    a.sampled_host = h_sampled_;
+    const auto h0 = std::chrono::steady_clock::now();
+    AK_TRY(launch_batch(ctx_->stream, a));
+    launch_host_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - h0).count();
+    h2d_bytes += (size_t)max_seqs_ * 8;
+    d2h_bytes += (size_t)max_seqs_ * 4;
+    return AK_OK;
 }
 
 int Runner::init_solo() {
@@ -629,8 +645,13 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
         if (batch_) {
             // The persistent kernel takes the whole chip, so the prompt rows follow it. It samples the decode rows' tokens itself (their out_rows
             // are -1); what comes after the ranges is for the prompts' last rows.
-            if (any_decode) RC(launch_decode_batch());
-            if (T == max_seqs_) return AK_OK;
+            if (any_decode) {
+                BatchArgs a = batch_args();
+                a.rows = rows;
+                a.kv_lens = d_desc_ + d_.kv_lens;
+                a.set0 = reinterpret_cast<const uint32_t*>(d_desc_ + d_.batch_set);
+                RC(launch_batch(st, a));
+            }
             rc = range(st, max_seqs_, T - max_seqs_, false, true);
             if (rc) return rc;
         } else if (two_streams_ && any_decode && T > max_seqs_ && n_pf_seqs && T > 128) {
@@ -734,8 +755,12 @@ int Runner::run(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_pf_len
     cudaStream_t st = ctx_->stream;
     const uint32_t T = max_seqs_ + n_prefill_rows;
     const size_t bytes = ((size_t)d_.rows + (size_t)T * 4) * 4;
-    if (batch_) describe_batch();
-    else attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
+    if (batch_) {
+        describe_batch();
+        if (n_prefill_rows == 0) return run_decode_batch();
+    } else {
+        attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
+    }
     AK_CUDA(cudaMemcpyAsync(d_desc_, h_desc_, bytes, cudaMemcpyHostToDevice, st));
     // One split count per runner (from the longest sequence it can hold): eager and captured
     // steps then sum in the same order, so a sequence's tokens do not depend on its neighbours.
@@ -781,8 +806,12 @@ int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_
         int32_t* p0 = h_pf_pos0();
         for (uint32_t i = n_pf_seqs; i < seqs_b; i++) { cu[i + 1] = cu[n_pf_seqs]; pfs[i] = 0; p0[i] = 0; }
     }
-    if (batch_) describe_batch();
-    else attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
+    if (batch_) {
+        describe_batch();
+        if (n_prefill_rows == 0) return run_decode_batch();
+    } else {
+        attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
+    }
     const uint64_t key = ((uint64_t)bank_ << 63) | ((uint64_t)rows_b << 32) | seqs_b;  // a graph bakes its bank's host buffers and events
     const uint32_t T = max_seqs_ + rows_b;
     const size_t bytes = ((size_t)d_.rows + (size_t)T * 4) * 4;

@@ -215,7 +215,8 @@ class Runner {
     uint32_t batch_set_ = 0;            // exchange set of the next step's embedding
     std::vector<SoloLayer> solo_layers() const;
     int upload_layers(SoloLayer** out);
-    int launch_decode_batch();
+    BatchArgs batch_args() const;
+    int run_decode_batch();             // a decode-only step: one launch, the step by value, the picks straight to the host
     void describe_batch();              // the step's words of the descriptor
     size_t sampled_words() const { return max_seqs_ + 1; }   // the tokens, and the status word of the persistent step
     SoloArgs solo_args(int32_t tok_src, uint32_t pos);
