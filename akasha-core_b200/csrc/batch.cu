@@ -176,6 +176,11 @@ __device__ __forceinline__ float inv_rms(float m) {
     return y > 0.0f && y < INFINITY ? y * fmaf(-0.5f * m * y, y, 1.5f) : y;
 }
 
+// A load from shared memory and a later arrival on a barrier (or the request of a copy) are not in order by themselves: a buffer could be overwritten
+// under a load that nothing has waited for yet. True for every value, but known only when v, and with it all that v was computed from, is there in
+// every lane.
+__device__ __forceinline__ bool settled(float v) { return __any_sync(0xffffffffu, __float_as_uint(v) != EMPTY) != 0; }
+
 struct Cursor {   // a place in the ring: slot and the parity of its current use
     uint32_t s = 0, ph = 0;
     __device__ __forceinline__ void advance(uint32_t by, uint32_t n) {   // by <= n
@@ -590,12 +595,18 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                         if (a_live >> e & 1u) v[d][e >> 1][e & 1] = xld4(xl + d * STEP + e * 512);
                 }
         };
+        uint32_t used = 0;   // slots before q that are not given back yet (a group's)
+        auto release = [&]() {
+            if (lane < used && alive) {
+                const uint32_t back = used - lane;
+                mbar_arrive(&empty_bar[q.s >= back ? q.s - back : q.s + slots - back]);
+            }
+        };
         issue(0);
 #pragma unroll 1
         for (uint32_t c0 = 0;;) {
             // the group's weights
-            Cursor first = q;
-            uint32_t used = 0;
+            used = 0;
             uint4 w[DEPTH][NT];
 #pragma unroll
             for (uint32_t cc = 0; cc < CPG; cc++)
@@ -648,15 +659,12 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll
                         for (uint32_t m = 0; m < MT; m++) mma(acc[t][m], v[d][m][0].z, v[d][m][1].z, v[d][m][0].w, v[d][m][1].w, w[d][t].z, w[d][t].w);
                 }
-            // The group's slots go back, only now: a load from shared memory and an arrival on a barrier are not in order by themselves, so
-            // a slot could be overwritten under a load that the products have not waited for yet.
-            __syncwarp();
-            if (lane < used && alive) {
-                first.advance(lane, slots);
-                mbar_arrive(&empty_bar[first.s]);
-            }
             c0 += CPG;
             if (c0 >= chunks) break;
+            float all = acc[0][0][0];
+#pragma unroll
+            for (uint32_t t = 1; t < NT; t++) all += acc[t][0][0];
+            if (settled(all)) release();
             xl += DEPTH * STEP;
             issue(c0 * PPC);
         }
@@ -674,6 +682,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         }
         __syncwarp();
         bar_arrive<NCT + NHT>(BAR_PART);
+        release();   // (behind the stores, which waited for the products and so for the weights)
     };
     auto gemm = [&](uint32_t x, const Kind& kind) {
         const uint32_t tiles = kind.n;
@@ -889,8 +898,6 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                         p[n][0] = c[0];
                         p[n][1] = c[1];
                     }
-                    __syncwarp();
-                    request(false);
                     float mx = -INFINITY;
 #pragma unroll
                     for (uint32_t n = 0; n < KT; n++)
@@ -900,6 +907,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                             mx = fmaxf(mx, p[n][e]);
                         }
                     const float m2 = fmaxf(m, redux_max(mx) * sc), corr = ex2(m - m2);
+                    if (__float_as_uint(m2) != EMPTY) request(false);   // (always, but with all lanes' scores there: see settled)
                     m = m2;
                     l *= corr;
                     // Every four lanes hold all probabilities; lane (g, t) keeps those of positions 8 n + 2 t + (g & 1) to hand out
@@ -930,8 +938,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll
                         for (int e = 0; e < 8; e++) acc[e] = fmaf(pv, vx[e], acc[e]);
                     }
-                    __syncwarp();
-                    request(true);
+                    if (settled(acc[0])) request(true);
                     tiles_done ^= 1u;
                 }
             }
@@ -1102,8 +1109,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                         mma(odd[m], x0.z, x1.z, x0.w, x1.w, w.z, w.w);
                     }
                 }
-                __syncwarp();
-                if (lane == 0 && alive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&empty_bar[bar])), "r"(NW) : "memory");
+                if (settled(fmaxf(acc[0][0], odd[0][0])) && lane == 0 && alive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&empty_bar[bar])), "r"(NW) : "memory");
             }
 #pragma unroll
             for (uint32_t m = 0; m < MT; m++)
