@@ -5,8 +5,8 @@
 // of its first loads, 3 to 5 us for work of 0.1 to 1 us (162M model, 8 sequences of 300: 0.39 ms; the bytes take 0.05 ms). Here, as in the
 // batch-1 step (solo.cu), a layer is five phases of one kernel and only activations cross the chip:
 //   qkv rows -> attention (sequence, head) -> out-proj rows -> ffn-up rows -> ffn-down rows.
-// That step takes 0.205 ms (1 sequence 0.18, 16 of 350 0.27, 32 of 350 0.35; 320-wide model, 21 sequences 0.22 -> 0.143; 1.4B model, 16 of 1600
-// 2.5 -> 2.25). With 64 sequences a layer was slower than the chain's (every SM reads all activations: 0.58 against 0.49 ms), hence the limit of 32.
+// That step takes 0.187 ms (1 sequence 0.17, 16 of 350 0.25, 32 of 350 0.334; 320-wide model, 21 sequences 0.22 -> 0.127; 1.4B model, 16 of 1600
+// 2.5 -> 2.1). With 64 sequences an early form was slower than the chain (every SM reads all activations: 0.58 against 0.49 ms), hence the limit of 32.
 // What is left is latency: per phase ~1 us from a store to the last SM's poll and ~1 us of dependent instructions, ~5 cycles each (with
 // everything between two phases done by the same warps it was 0.29 ms; with 40 bytes of spills 0.36).
 //   * A producer thread per SM walks the SM's weight tiles of all phases in order and keeps a shared-memory ring of tensor loads full.
