@@ -35,6 +35,7 @@
 // is `dead` (later waits return at once), the status word is set and the host reports AK_ERR_DEVICE_WAIT. A warp whose wait for a
 // copy ran out releases no slot any more, and nobody leaves before the copies it started have landed.
 #include "batch.h"
+#include "batch_plan.h"
 #include "tma.h"
 
 #include <type_traits>
@@ -43,45 +44,13 @@ namespace ak {
 
 namespace {
 
-constexpr uint32_t NW = 12;               // compute warps
-constexpr uint32_t NH = 3;                // epilogue warps
+using namespace batch;
+static_assert(SMS == B200_SMS, "a block per SM");
 constexpr uint32_t NCT = NW * 32, NHT = NH * 32;   // threads of the compute and of the epilogue warps
 constexpr uint32_t THREADS = 512, FIRST_COMPUTE = 4;
 constexpr int REGS_FIRST = 80, REGS_COMPUTE = 144;
 static_assert(REGS_FIRST * 128 + REGS_COMPUTE * 384 <= 65536, "the split draws on the registers of the launch");
-constexpr uint32_t CHUNK = 24;            // K slices (of 32) of a ring slot at most
-constexpr uint32_t SLOT = 8 * CHUNK * 64; // 8 weight rows
-constexpr uint32_t MAX_SLOTS = 8, MAX_EXTRA = 6;
-constexpr uint32_t MAX_LAYERS = 48;
-constexpr uint32_t KV_BUF = 4096;         // bytes of a warp's key (and of its value) buffer: 2048 / head_dim positions
-constexpr uint32_t MAX_UNITS = 32;        // units of a group (a lane keeps one)
 constexpr uint32_t EMPTY = 0xffffffffu;   // an exchange word that is not written yet
-constexpr uint32_t MAX_DYN_SMEM = 216 * 1024;
-
-__host__ __device__ constexpr uint32_t m_tiles(uint32_t seqs) { return seqs <= 16 ? 1 : 2; }
-__host__ __device__ constexpr uint32_t tile_begin(uint32_t tiles, uint32_t cta) { return (tiles * cta) / B200_SMS; }
-// Positions of an attention unit. Sequences of up to 512 are whole (no merging); longer ones are cut small, so that the groups' shares come out even: of
-// 16 sequences of up to 3200 positions a layer took 57 us in units of 512, with half of the SMs done after 31 us.
-__host__ __device__ constexpr uint32_t split_len(uint32_t max_len) { return max_len <= 512 ? 512 : 256; }
-__host__ __device__ constexpr uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
-constexpr uint32_t TB = 3;                // weight tiles of a pass (accumulators, partial sums)
-
-// byte offsets inside an exchange set (and its size): x after ffn-down, attention, x after out-proj, ffn-up as A fragments; sums of squares; qkv and
-// the splits of the attention in f32; an SM's best logit of a row {value, index}
-struct SetOff {
-    uint32_t x1, at, x2, up, s1, s2, qkv, best, part;
-    size_t total;
-    SetOff() = default;
-    __host__ __device__ SetOff(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t mt, uint32_t splits) {
-        const uint32_t r = mt * 16, hd = dim / heads, cx = dim * r * 2, cs = dim / 8 * r * 4;
-        x1 = 0; at = x1 + cx; x2 = at + cx; up = x2 + cx;
-        s1 = up + ffn * r * 2; s2 = s1 + cs;
-        qkv = s2 + cs;
-        best = qkv + r * 3 * dim * 4;
-        part = best + B200_SMS * r * 8;
-        total = part + (splits > 1 ? (size_t)r * heads * splits * (hd + 4) * 4 : 0);
-    }
-};
 
 // Bounds the polling of one thread; `dead` is sticky for the block. A poll is a round trip to L2 (0.3 us or more), so the limit is a second or two.
 constexpr uint32_t MAX_POLLS = 1u << 22;
@@ -194,9 +163,6 @@ struct Kind {
     uint32_t t0, n, slices, chunks, pitch, pieces;   // pitch: bytes of a row in a slot; pieces of a chunk in the tensor map
     __device__ __forceinline__ uint32_t count(uint32_t c) const { return min(CHUNK, slices - c * CHUNK); }
 };
-// A weight row as pieces of the tensor map: 256 columns, or what divides the row
-__host__ __device__ constexpr uint32_t piece_of(uint32_t k) { return k % 256 == 0 ? 256 : k % 64 == 0 ? 64 : 32; }
-__host__ __device__ constexpr uint32_t chunk_cols(uint32_t k) { return k < CHUNK * 32 ? k : CHUNK * 32; }
 __device__ __forceinline__ void make_kind(Kind& d, uint32_t rows, uint32_t k, uint32_t cta) {
     d.t0 = tile_begin(div_up(rows, 8), cta);
     d.n = tile_begin(div_up(rows, 8), cta + 1) - d.t0;
@@ -249,7 +215,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     float* const at_acc = part + NW * TB * R * 8;                                 // [2][NW][HD]
     float4* const res_sm = reinterpret_cast<float4*>(at_acc + 2 * NW * HD);       // [tile][R][2]: the residual stream of this SM's columns
     float* const gain_sm = reinterpret_cast<float*>(res_sm + TB * R * 2);                // [2 L + 1][tiles][8]: the gains of its columns, by norm
-    const uint32_t SPLIT_LEN = SPLIT ? 256 : 512, splits = div_up(a.max_len, SPLIT_LEN);
+    const uint32_t SPLIT_LEN = unit_len(SPLIT), splits = div_up(a.max_len, SPLIT_LEN);
 
     if (tid == 160) so = SetOff(D, F, H, MT, splits);
     if (tid == 0) {
@@ -1191,22 +1157,6 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     }
 }
 
-struct Plan {
-    uint32_t slots, wpi;
-    size_t smem;
-};
-Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len) {
-    const uint32_t hd = dim / heads;
-    const size_t rest = NW * 2 * KV_BUF + (size_t)NW * TB * m_tiles(seqs) * 16 * 32 + 2 * NW * hd * 4 + TB * 32 * 2 * 16 + (size_t)(2 * n_layers + 1) * div_up(dim / 8, B200_SMS) * 32;
-    Plan p;
-    p.slots = (uint32_t)((MAX_DYN_SMEM - rest) / SLOT);
-    if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
-    p.smem = p.slots * SLOT + rest;
-    // Few units: all warps of an SM work on one; else four, so that an SM's units overlap.
-    p.wpi = seqs * heads * div_up(max_len, split_len(max_len)) <= B200_SMS ? 12 : 4;
-    return p;
-}
-
 template <int HD, int MT, bool SPLIT>
 int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p) {
     {
@@ -1251,26 +1201,14 @@ int batch_maps(void* out, const SoloLayer* layers, const void* lm_head, uint32_t
 bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers, uint32_t seqs, uint32_t max_len) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
-    const uint32_t hd = heads ? dim / heads : 0;
-    if ((uint32_t)sms < B200_SMS || dtype != AK_BF16 || (hd != 64 && hd != 128) || dim != heads * hd || heads > 4095) return false;
-    if (seqs < 1 || seqs > BATCH_ROWS || n_layers < 1 || n_layers > MAX_LAYERS || dim < 96 || dim % 32 || ffn % 32 || ffn > 65536) return false;
-    if (ffn / 8 < B200_SMS) return false;                                        // every SM has ffn-up rows (the clearing of the sets counts on it)
-    if (div_up(dim / 8, B200_SMS) > TB) return false;                            // the residual stream is worked on in one pass
-    if (dim * m_tiles(seqs) * 16 * 2 > NW * 2 * KV_BUF) return false;             // the lm_head keeps x where the cache tiles were
-    const uint32_t splits = div_up(max_len, split_len(max_len));
-    const Plan p = make_plan(dim, n_layers, heads, seqs, max_len);
-    if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * B200_SMS * (NW / p.wpi)) return false;
-    const SetOff so(dim, ffn, heads, m_tiles(seqs), splits);
-    return p.slots >= 4 && 3 * so.total < (1ull << 32);
+    return (uint32_t)sms >= B200_SMS && dtype == AK_BF16 && shape_supported(dim, ffn, heads, n_layers, seqs, max_len);
 }
 
-size_t batch_xch_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) {
-    return 3 * SetOff(dim, ffn, heads, m_tiles(seqs), div_up(max_len, split_len(max_len))).total;
-}
+size_t batch_xch_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) { return xch_bytes(dim, ffn, heads, seqs, max_len); }
 
 int launch_batch(cudaStream_t st, const BatchArgs& a) {
     const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.seqs, a.max_len);
-    const bool two = m_tiles(a.seqs) == 2, split = a.max_len > split_len(a.max_len);
+    const bool two = m_tiles(a.seqs) == 2, split = has_splits(a.max_len);
     if (a.dim / a.heads == 64) {
         if (split) return two ? launch_batch_t<64, 2, true>(st, a, p) : launch_batch_t<64, 1, true>(st, a, p);
         return two ? launch_batch_t<64, 2, false>(st, a, p) : launch_batch_t<64, 1, false>(st, a, p);

@@ -1,11 +1,12 @@
 // Decode step of up to 32 sequences as one persistent kernel (batch.cu): launch interface.
 #pragma once
+#include "batch_plan.h"
 #include "kernels.h"
 #include "solo.h"
 
 namespace ak {
 
-constexpr uint32_t BATCH_ROWS = 32;
+constexpr uint32_t BATCH_ROWS = batch::ROWS;
 
 struct BatchArgs {
     const SoloLayer* layers;     // device array, one per layer; matrices [out, in] bf16

@@ -1,0 +1,97 @@
+// Decode step of up to 32 sequences (batch.cu): tiles, exchange buffers and shared memory, and which models they fit.
+// Plain C++ (no CUDA header), so that the plan can be checked on the host.
+#pragma once
+#include <stddef.h>
+#include <stdint.h>
+
+#ifndef AK_PLAN_FN
+#ifdef __CUDACC__
+#define AK_PLAN_FN __host__ __device__ inline
+#else
+#define AK_PLAN_FN inline
+#endif
+#endif
+
+namespace ak {
+namespace batch {
+
+constexpr uint32_t SMS = 148;             // one block per SM
+constexpr uint32_t ROWS = 32;             // most sequences of a step
+constexpr uint32_t NW = 12;               // compute warps
+constexpr uint32_t NH = 3;                // epilogue warps
+constexpr uint32_t TB = 3;                // weight tiles of a pass (accumulators, partial sums)
+constexpr uint32_t CHUNK = 24;            // K slices (of 32) of a ring slot at most
+constexpr uint32_t SLOT = 8 * CHUNK * 64; // 8 weight rows
+constexpr uint32_t MAX_SLOTS = 8, MAX_EXTRA = 6;
+constexpr uint32_t MAX_LAYERS = 48;
+constexpr uint32_t KV_BUF = 4096;         // bytes of a warp's key (and of its value) buffer: 2048 / head_dim positions
+constexpr uint32_t MAX_UNITS = 32;        // attention units of a group (a lane keeps one)
+constexpr uint32_t MAX_DYN_SMEM = 216 * 1024;
+
+AK_PLAN_FN constexpr uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
+AK_PLAN_FN constexpr uint32_t m_tiles(uint32_t seqs) { return seqs <= 16 ? 1 : 2; }
+AK_PLAN_FN constexpr uint32_t tile_begin(uint32_t tiles, uint32_t cta) { return (tiles * cta) / SMS; }
+// Positions of an attention unit. Sequences of up to 512 are whole (no merging); longer ones are cut small, so that the groups' shares come out even: of
+// 16 sequences of up to 3200 positions a layer took 57 us in units of 512, with half of the SMs done after 31 us.
+AK_PLAN_FN constexpr bool has_splits(uint32_t max_len) { return max_len > 512; }
+AK_PLAN_FN constexpr uint32_t unit_len(bool splits) { return splits ? 256 : 512; }
+AK_PLAN_FN constexpr uint32_t split_len(uint32_t max_len) { return unit_len(has_splits(max_len)); }
+// A weight row as pieces of the tensor map: 256 columns, or what divides the row
+AK_PLAN_FN constexpr uint32_t piece_of(uint32_t k) { return k % 256 == 0 ? 256 : k % 64 == 0 ? 64 : 32; }
+AK_PLAN_FN constexpr uint32_t chunk_cols(uint32_t k) { return k < CHUNK * 32 ? k : CHUNK * 32; }
+
+// byte offsets inside an exchange set (and its size): x after ffn-down, attention, x after out-proj, ffn-up as A fragments; sums of squares; qkv and
+// the splits of the attention in f32; an SM's best logit of a row {value, index}
+struct SetOff {
+    uint32_t x1, at, x2, up, s1, s2, qkv, best, part;
+    size_t total;
+    SetOff() = default;
+    AK_PLAN_FN SetOff(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t mt, uint32_t splits) {
+        const uint32_t r = mt * 16, hd = dim / heads, cx = dim * r * 2, cs = dim / 8 * r * 4;
+        x1 = 0; at = x1 + cx; x2 = at + cx; up = x2 + cx;
+        s1 = up + ffn * r * 2; s2 = s1 + cs;
+        qkv = s2 + cs;
+        best = qkv + r * 3 * dim * 4;
+        part = best + SMS * r * 8;
+        total = part + (splits > 1 ? (size_t)r * heads * splits * (hd + 4) * 4 : 0);
+    }
+};
+
+// The exchange sets, used in turn: the step's embedding has set e0, layer l set e0 + 1 + l (mod SETS), the next step starts with the set behind.
+constexpr uint32_t SETS = 3;
+
+inline size_t xch_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) {
+    return SETS * SetOff(dim, ffn, heads, m_tiles(seqs), div_up(max_len, split_len(max_len))).total;
+}
+
+struct Plan {
+    uint32_t slots, wpi;
+    size_t smem;
+};
+inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len) {
+    const uint32_t hd = dim / heads;
+    const size_t rest = NW * 2 * KV_BUF + (size_t)NW * TB * m_tiles(seqs) * 16 * 32 + 2 * NW * hd * 4 + TB * 32 * 2 * 16 + (size_t)(2 * n_layers + 1) * div_up(dim / 8, SMS) * 32;
+    Plan p;
+    p.slots = (uint32_t)((MAX_DYN_SMEM - rest) / SLOT);
+    if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
+    p.smem = p.slots * SLOT + rest;
+    // Few units: all warps of an SM work on one; else four, so that an SM's units overlap.
+    p.wpi = seqs * heads * div_up(max_len, split_len(max_len)) <= SMS ? 12 : 4;
+    return p;
+}
+
+inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers, uint32_t seqs, uint32_t max_len) {
+    const uint32_t hd = heads ? dim / heads : 0;
+    if ((hd != 64 && hd != 128) || dim != heads * hd || heads > 4095) return false;
+    if (seqs < 1 || seqs > ROWS || n_layers < 1 || n_layers > MAX_LAYERS || dim < 96 || dim % 32 || ffn % 32 || ffn > 65536) return false;
+    if (ffn / 8 < SMS) return false;                                       // every SM has ffn-up rows (the clearing of the sets counts on it)
+    if (div_up(dim / 8, SMS) > TB) return false;                           // the residual stream is worked on in one pass
+    if (dim * m_tiles(seqs) * 16 * 2 > NW * 2 * KV_BUF) return false;      // the lm_head keeps x where the cache tiles were
+    const uint32_t splits = div_up(max_len, split_len(max_len));
+    const Plan p = make_plan(dim, n_layers, heads, seqs, max_len);
+    if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * SMS * (NW / p.wpi)) return false;
+    return p.slots >= 4 && xch_bytes(dim, ffn, heads, seqs, max_len) < (1ull << 32);
+}
+
+}  // namespace batch
+}  // namespace ak
