@@ -255,19 +255,19 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll 1
     for (uint32_t i = tid; i < L * (uint32_t)(sizeof(SoloLayer) / 8); i += THREADS)
         reinterpret_cast<uint64_t*>(layers_sm)[i] = reinterpret_cast<const uint64_t*>(a.layers)[i];
-    const uint32_t e0 = (a.rows ? *a.set0 : a.set) % 3;
+    const uint32_t e0 = *(const volatile uint32_t*)&a.state->set;   // (before the block's barrier, so before this SM publishes anything)
     __syncthreads();
 #pragma unroll 1
     for (uint32_t i = tid, n = kinds[OUT].n * 8; i < (2 * L + 1) * n; i += THREADS)
         gain_sm[i] = (i / n == 2 * L ? a.final_norm : i / n & 1 ? layers_sm[i / (2 * n)].norm_2 : layers_sm[i / (2 * n)].norm_1)[kinds[OUT].t0 * 8 + i % n];
     const uint32_t live = live_sm, n_act = __popc(live);
-    if (n_act == 0) return;   // (the host has not moved set0 for such a step either)
+    if (n_act == 0) return;
     __syncthreads();   // the gains
 
     // The lm_head keeps x where the cache tiles were, and extra slots behind it. Its chunk n is in slot n mod (slots + extra) of the two.
     uint8_t* const extra_sm = kv_sm + D * R * 2;
     const uint32_t extra = min(MAX_EXTRA, (NW * 2 * KV_BUF - D * R * 2) / SLOT), head_slots = slots + extra;
-    auto set_of = [&](uint32_t g) { return (g % 3) * (uint32_t)so.total; };   // byte offset; g = e0: the embedding, e0 + 1 + l: layer l
+    auto set_of = [&](uint32_t g) { return (g % SETS) * (uint32_t)so.total; };   // byte offset; g = e0: the embedding, e0 + 1 + l: layer l
     auto row_live = [&](uint32_t r) { return (live >> r) & 1u; };
     auto eight_live = [&](uint32_t e) { return ((live >> (e * 8)) & 0xffu) != 0; };
     const Waiter wt{&dead};
@@ -1143,6 +1143,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 const uint32_t tok = n < a.vocab ? n : 0u;   // (no logit above -inf: 0)
                 a.sampled[cta] = tok;
                 if (a.sampled_host) a.sampled_host[cta] = tok;
+                if (cta == (uint32_t)__ffs(live) - 1) a.state->set = (e0 + L + 1) % SETS;   // every SM has published its best, so has read it
             }
         }
     }
@@ -1204,7 +1205,7 @@ bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads,
     return (uint32_t)sms >= B200_SMS && dtype == AK_BF16 && shape_supported(dim, ffn, heads, n_layers, seqs, max_len);
 }
 
-size_t batch_xch_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) { return xch_bytes(dim, ffn, heads, seqs, max_len); }
+size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) { return sets_bytes(dim, ffn, heads, seqs, max_len); }
 
 int launch_batch(cudaStream_t st, const BatchArgs& a) {
     const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.seqs, a.max_len);

@@ -14,14 +14,13 @@ struct BatchArgs {
     const void* embedding;
     const float* final_norm;
     const float2* rope;          // [max_len][head_dim / 2] (cos, sin)
-    uint8_t* xch;                // batch_xch_bytes(), all 0xff before the first launch
+    uint8_t* xch;                // exchange sets, batch_sets_bytes(): all 0xff before the first launch
+    batch::State* state;         // zero before the first launch
     uint32_t* sampled;           // [seqs]: the token fed back to a row with tok_src < 0, overwritten by the row's greedy pick
     // The step, in device memory or (rows == nullptr) by value
     const int32_t* rows;         // [seqs] of int4 {tok_src, pos, slot, seq}
     const int32_t* kv_lens;      // [seqs]: positions attended to, the new one included; 0: the row is not there
-    const uint32_t* set0;        // device word: exchange set of the step's embedding, advances by n_layers + 1 (mod 3) from step to step
     int32_t tok_src[BATCH_ROWS], lens[BATCH_ROWS];
-    uint32_t set;
     const int32_t* block_tables; // [seqs][max_blocks]
     uint32_t* sampled_host;      // where else the picks go: [seqs] in mapped host memory and behind them the status word, or nullptr
     uint32_t* status;            // device word: made non-zero when a wait runs out
@@ -32,7 +31,7 @@ struct BatchArgs {
 bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers, uint32_t seqs, uint32_t max_len);
 // the weights' tensor maps, 4 n_layers + 1 of 128 bytes in host memory (layers: host array)
 int batch_maps(void* out, const SoloLayer* layers, const void* lm_head, uint32_t n_layers, uint32_t dim, uint32_t ffn, uint32_t vocab);
-size_t batch_xch_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len);
+size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len);
 int launch_batch(cudaStream_t st, const BatchArgs& a);
 
 }  // namespace ak

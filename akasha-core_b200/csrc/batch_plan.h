@@ -60,8 +60,14 @@ struct SetOff {
 // The exchange sets, used in turn: the step's embedding has set e0, layer l set e0 + 1 + l (mod SETS), the next step starts with the set behind.
 constexpr uint32_t SETS = 3;
 
-inline size_t xch_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) {
-    return SETS * SetOff(dim, ffn, heads, m_tiles(seqs), div_up(max_len, split_len(max_len))).total;
+// What steps hand on to each other, behind the sets. Only the kernel writes it, at the end of a step: a launch that failed changes nothing.
+struct State {
+    uint32_t set;   // e0 of the next step
+    uint32_t pad[31];
+};
+
+inline size_t sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) {
+    return (SETS * SetOff(dim, ffn, heads, m_tiles(seqs), div_up(max_len, split_len(max_len))).total + 127) / 128 * 128;
 }
 
 struct Plan {
@@ -90,7 +96,7 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
     const uint32_t splits = div_up(max_len, split_len(max_len));
     const Plan p = make_plan(dim, n_layers, heads, seqs, max_len);
     if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * SMS * (NW / p.wpi)) return false;
-    return p.slots >= 4 && xch_bytes(dim, ffn, heads, seqs, max_len) < (1ull << 32);
+    return p.slots >= 4 && sets_bytes(dim, ffn, heads, seqs, max_len) < (1ull << 32);
 }
 
 }  // namespace batch

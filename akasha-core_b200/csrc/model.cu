@@ -286,8 +286,7 @@ int Runner::init(ak_ctx* ctx, ak_weights* w, uint32_t max_seqs, uint32_t max_seq
     d_.pf_cu = d_.row_order + max_seqs;
     d_.pf_slot = d_.pf_cu + max_seqs + 1;
     d_.pf_pos0 = d_.pf_slot + max_seqs;
-    d_.batch_set = d_.pf_pos0 + max_seqs;
-    d_.block_tables = d_.batch_set + 1;
+    d_.block_tables = d_.pf_pos0 + max_seqs;
     d_.rows = align_up(d_.block_tables + max_seqs * max_blocks_, 4);
     d_.total = d_.rows + max_rows_ * 4;
     for (Bank& b : banks_) {
@@ -400,21 +399,14 @@ int Runner::init_batch() {
     AK_TRY(batch_maps(host, solo_layers().data(), w_->lm_head, c.num_layers, c.dim, c.ffn_hidden, c.vocab_size));
     AK_CUDA(cudaMalloc(&d_batch_maps_, (4 * c.num_layers + 1) * 128));
     AK_CUDA(cudaMemcpyAsync(d_batch_maps_, host, (4 * c.num_layers + 1) * 128, cudaMemcpyHostToDevice, ctx_->stream));
-    const size_t bytes = batch_xch_bytes(c.dim, c.ffn_hidden, c.num_heads, max_seqs_, max_seq_len_);
-    AK_CUDA(cudaMalloc((void**)&d_batch_xch_, bytes));
+    const size_t bytes = batch_sets_bytes(c.dim, c.ffn_hidden, c.num_heads, max_seqs_, max_seq_len_);
+    AK_CUDA(cudaMalloc((void**)&d_batch_xch_, bytes + sizeof(batch::State)));
+    d_batch_state_ = reinterpret_cast<batch::State*>(d_batch_xch_ + bytes);
     AK_CUDA(cudaMemsetAsync(d_batch_xch_, 0xff, bytes, ctx_->stream));
+    AK_CUDA(cudaMemsetAsync(d_batch_state_, 0, sizeof(batch::State), ctx_->stream));
     AK_CUDA(cudaStreamSynchronize(ctx_->stream));
     batch_ = true;
     return AK_OK;
-}
-
-// The step's words of the descriptor. The exchange sets move on by a set per layer and one for the embedding, if there is a decode row.
-void Runner::describe_batch() {
-    if (!batch_) return;
-    h_desc_[d_.batch_set] = (int32_t)batch_set_;
-    bool any = false;
-    for (uint32_t i = 0; i < max_seqs_; i++) any = any || h_kv_lens()[i] > 0;
-    if (any) batch_set_ = (batch_set_ + w_->cfg.num_layers + 1) % 3;
 }
 
 BatchArgs Runner::batch_args() const {
@@ -426,6 +418,7 @@ BatchArgs Runner::batch_args() const {
     a.maps = d_batch_maps_;
     a.rope = rope_table_;
     a.xch = d_batch_xch_;
+    a.state = d_batch_state_;
     a.sampled = d_sampled_;
     a.block_tables = d_desc_ + d_.block_tables;
     a.status = d_sampled_ + max_seqs_;
@@ -441,7 +434,6 @@ BatchArgs Runner::batch_args() const {
 int Runner::run_decode_batch() {
     AK_CUDA(cudaSetDevice(ctx_->device));
     BatchArgs a = batch_args();
-    a.set = (uint32_t)h_desc_[d_.batch_set];
     for (uint32_t i = 0; i < max_seqs_; i++) {
         a.tok_src[i] = h_rows()[i].tok_src;
         a.lens[i] = h_kv_lens()[i];
@@ -649,8 +641,8 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
                 BatchArgs a = batch_args();
                 a.rows = rows;
                 a.kv_lens = d_desc_ + d_.kv_lens;
-                a.set0 = reinterpret_cast<const uint32_t*>(d_desc_ + d_.batch_set);
                 RC(launch_batch(st, a));
+                batch_ran_ = !capturing;
             }
             rc = range(st, max_seqs_, T - max_seqs_, false, true);
             if (rc) return rc;
@@ -750,28 +742,65 @@ int Runner::attn_time_mark(cudaStream_t s, cudaEvent_t ev, bool capturing) {
 }
 
 int Runner::run(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_pf_len, bool any_decode, uint32_t max_kv_len) {
+    AK_REQUIRE(!failed_, failed_, "runner: a step before failed half way");
     AK_REQUIRE(n_prefill_rows <= max_pf_tokens_, AK_ERR_INVALID_ARG, "runner: %u prefill rows exceed the step budget %u", n_prefill_rows, max_pf_tokens_);
     AK_CUDA(cudaSetDevice(ctx_->device));
     cudaStream_t st = ctx_->stream;
     const uint32_t T = max_seqs_ + n_prefill_rows;
     const size_t bytes = ((size_t)d_.rows + (size_t)T * 4) * 4;
     if (batch_) {
-        describe_batch();
         if (n_prefill_rows == 0) return run_decode_batch();
     } else {
         attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
     }
-    AK_CUDA(cudaMemcpyAsync(d_desc_, h_desc_, bytes, cudaMemcpyHostToDevice, st));
     // One split count per runner (from the longest sequence it can hold): eager and captured
     // steps then sum in the same order, so a sequence's tokens do not depend on its neighbours.
     (void)max_kv_len;
     const uint32_t n_splits = attn_decode_pick_splits(max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, max_seq_len_, true);
-    int rc = launch_layers(T, n_prefill_rows, n_pf_seqs, max_pf_len, any_decode, n_splits, false);
-    if (rc) return rc;
-    AK_CUDA(cudaMemcpyAsync(h_sampled_, d_sampled_, sampled_words() * 4, cudaMemcpyDeviceToHost, st));
+    return launch_step(T, n_prefill_rows, n_pf_seqs, max_pf_len, any_decode, n_splits, bytes);
+}
+
+// A step launch by launch: descriptor, kernels, tokens. One that fails may be launched again, unless its persistent step is on the stream: that
+// one feeds its tokens to the next.
+int Runner::launch_step(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, uint32_t max_pf_len, bool any_decode, uint32_t n_splits, size_t desc_bytes) {
+    batch_ran_ = false;
+    AK_CUDA(cudaMemcpyAsync(d_desc_, h_desc_, desc_bytes, cudaMemcpyHostToDevice, ctx_->stream));
+    int rc = launch_layers(T, n_pf_rows, n_pf_seqs, max_pf_len, any_decode, n_splits, false);
+    if (rc == AK_OK) {
+        const cudaError_t e = cudaMemcpyAsync(h_sampled_, d_sampled_, sampled_words() * 4, cudaMemcpyDeviceToHost, ctx_->stream);
+        if (e != cudaSuccess) rc = cuda_fail(e, "copy of the sampled tokens", __FILE__, __LINE__);
+    }
+    if (rc) {
+        if (batch_ran_) failed_ = rc;
+        return rc;
+    }
     eager_steps++;
-    h2d_bytes += bytes;
+    h2d_bytes += desc_bytes;
     d2h_bytes += sampled_words() * 4;
+    return AK_OK;
+}
+
+// The step just launched as a graph, for the next of its shape.
+int Runner::capture_step(uint64_t key, uint32_t T, uint32_t rows_b, uint32_t seqs_b, uint32_t len_b, uint32_t n_splits, size_t bytes) {
+    cudaStream_t st = ctx_->stream;
+    cudaGraph_t graph = nullptr;
+    AK_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    cudaError_t e = cudaMemcpyAsync(d_desc_, h_desc_, bytes, cudaMemcpyHostToDevice, st);
+    const unsigned long long l0 = g_launch_count;
+    const int rc = (e == cudaSuccess) ? launch_layers(T, rows_b, seqs_b, len_b, true, n_splits, true) : AK_ERR_CUDA;
+    StepGraph g;
+    g.kernels = g_launch_count - l0;
+    g.h2d = bytes;
+    g_launch_count = l0;  // recorded into the graph, not launched
+    if (rc == AK_OK) e = cudaMemcpyAsync(h_sampled_, d_sampled_, sampled_words() * 4, cudaMemcpyDeviceToHost, st);
+    cudaError_t e2 = cudaStreamEndCapture(st, &graph);
+    if (rc) return rc;
+    if (e != cudaSuccess) return cuda_fail(e, "capture memcpy", __FILE__, __LINE__);
+    if (e2 != cudaSuccess) return cuda_fail(e2, "cudaStreamEndCapture", __FILE__, __LINE__);
+    AK_CUDA(cudaGraphInstantiate(&g.exec, graph, 0));
+    cudaGraphDestroy(graph);
+    graphs_[key] = g;
+    if ((key << 1) == 0) graph_kernels = g.kernels;
     return AK_OK;
 }
 
@@ -787,6 +816,7 @@ static uint32_t pow2_bucket(uint32_t v, uint32_t lo) {
 // graph per bucket is captured on first use. Row results do not depend on the bucket (every
 // kernel treats rows independently and the GEMM's K order is fixed per (n, k)).
 int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_pf_len) {
+    AK_REQUIRE(!failed_, failed_, "runner: a step before failed half way");
     AK_REQUIRE(n_prefill_rows <= max_pf_tokens_ && n_pf_seqs <= max_seqs_, AK_ERR_INVALID_ARG, "runner: step exceeds its budget");
     AK_CUDA(cudaSetDevice(ctx_->device));
     cudaStream_t st = ctx_->stream;
@@ -807,7 +837,6 @@ int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_
         for (uint32_t i = n_pf_seqs; i < seqs_b; i++) { cu[i + 1] = cu[n_pf_seqs]; pfs[i] = 0; p0[i] = 0; }
     }
     if (batch_) {
-        describe_batch();
         if (n_prefill_rows == 0) return run_decode_batch();
     } else {
         attn_decode_row_order(h_kv_lens(), max_seqs_, heads_l_, w_->cfg.dim / w_->cfg.num_heads, w_->dtype, h_row_order());
@@ -819,33 +848,12 @@ int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_
     auto it = graphs_.find(key);
     if (it == graphs_.end()) {
         // one eager pass first (sets kernel attributes, surfaces faults outside capture); it IS this step
-        AK_CUDA(cudaMemcpyAsync(d_desc_, h_desc_, bytes, cudaMemcpyHostToDevice, st));
-        int rc = launch_layers(T, rows_b, seqs_b, len_b, true, n_splits, false);
+        int rc = launch_step(T, rows_b, seqs_b, len_b, true, n_splits, bytes);
         if (rc) return rc;
-        AK_CUDA(cudaMemcpyAsync(h_sampled_, d_sampled_, sampled_words() * 4, cudaMemcpyDeviceToHost, st));
         AK_CUDA(cudaStreamSynchronize(st));
-        eager_steps++;
-        h2d_bytes += bytes;
-        d2h_bytes += sampled_words() * 4;
-        cudaGraph_t graph = nullptr;
-        AK_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = cudaMemcpyAsync(d_desc_, h_desc_, bytes, cudaMemcpyHostToDevice, st);
-        const unsigned long long l0 = g_launch_count;
-        rc = (e == cudaSuccess) ? launch_layers(T, rows_b, seqs_b, len_b, true, n_splits, true) : AK_ERR_CUDA;
-        StepGraph g;
-        g.kernels = g_launch_count - l0;
-        g.h2d = bytes;
-        g_launch_count = l0;  // recorded into the graph, not launched
-        if (rc == AK_OK) e = cudaMemcpyAsync(h_sampled_, d_sampled_, sampled_words() * 4, cudaMemcpyDeviceToHost, st);
-        cudaError_t e2 = cudaStreamEndCapture(st, &graph);
-        if (rc) return rc;
-        if (e != cudaSuccess) return cuda_fail(e, "capture memcpy", __FILE__, __LINE__);
-        if (e2 != cudaSuccess) return cuda_fail(e2, "cudaStreamEndCapture", __FILE__, __LINE__);
-        AK_CUDA(cudaGraphInstantiate(&g.exec, graph, 0));
-        cudaGraphDestroy(graph);
-        graphs_[key] = g;
-        if ((key << 1) == 0) graph_kernels = g.kernels;
-        return AK_OK;
+        rc = capture_step(key, T, rows_b, seqs_b, len_b, n_splits, bytes);
+        if (rc) failed_ = rc;   // (the step itself has run)
+        return rc;
     }
     if (attn_timing_) AK_CUDA(cudaEventRecord(ev_g0_, st));
     const auto h0 = std::chrono::steady_clock::now();

@@ -66,7 +66,7 @@ struct RowInfo {
 };
 
 struct StepDesc {  // offsets (in int32 units) into the descriptor buffer
-    uint32_t kv_lens, out_rows, row_order, pf_cu, pf_slot, pf_pos0, batch_set, block_tables, rows, total;
+    uint32_t kv_lens, out_rows, row_order, pf_cu, pf_slot, pf_pos0, block_tables, rows, total;
 };
 
 class Runner {
@@ -212,12 +212,15 @@ class Runner {
     uint8_t* d_batch_xch_ = nullptr;
     SoloLayer* d_batch_layers_ = nullptr;
     void* d_batch_maps_ = nullptr;
-    uint32_t batch_set_ = 0;            // exchange set of the next step's embedding
+    batch::State* d_batch_state_ = nullptr;   // behind the exchange sets
+    bool batch_ran_ = false;            // a persistent step of the step being launched is on the stream
+    int failed_ = 0;                    // the error after which this runner takes no step any more
+    int capture_step(uint64_t key, uint32_t T, uint32_t rows_b, uint32_t seqs_b, uint32_t len_b, uint32_t n_splits, size_t bytes);
+    int launch_step(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, uint32_t max_pf_len, bool any_decode, uint32_t n_splits, size_t desc_bytes);
     std::vector<SoloLayer> solo_layers() const;
     int upload_layers(SoloLayer** out);
     BatchArgs batch_args() const;
     int run_decode_batch();             // a decode-only step: one launch, the step by value, the picks straight to the host
-    void describe_batch();              // the step's words of the descriptor
     size_t sampled_words() const { return max_seqs_ + 1; }   // the tokens, and the status word of the persistent step
     SoloArgs solo_args(int32_t tok_src, uint32_t pos);
     // Admission steps: the admitted prompts' rows run on a second stream, concurrently with the decode
