@@ -18,7 +18,7 @@
 //     that a warp's fragment is one coalesced 512-byte load from L2 straight into registers. Both operands use the same order of k. What a
 //     tile publishes for 8 sequences is one 128-byte line (as 16-byte pieces of four lines: 1.6 us instead of 0.95 until the last SM had it).
 //   * A value is its own flag: an exchange buffer holds 0xffffffff words until it is written, a NaN no conversion and no arithmetic
-//     gives, and consumers poll the words they need. No fence and no second round trip between the value and its flag. Three sets of
+//     gives, and consumers poll the words they need. No fence and no second round trip between the value and its flag. Four sets of
 //     buffers are used in turn by the layers; the one of the layer before is filled with 0xff again after a layer's ffn-up (see clear).
 //   * RMS norm: the producer of the residual stream publishes x * gain rounded to bf16 (one rounding, as of the normalised value) and
 //     the sums of squares of its columns; 1 / rms is a factor of the row sums of the next phase, found by the epilogue warps meanwhile.
@@ -349,7 +349,18 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             const uint32_t n = (uint32_t)(so.total / 16);
 #pragma unroll 1
             for (uint32_t i = cta * NHT + ht; i < n; i += B200_SMS * NHT) p[i] = make_uint4(EMPTY, EMPTY, EMPTY, EMPTY);
-            __threadfence();
+            bar_sync<NHT>(BAR_HELP);
+            if (ht == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&a.state->cleared) : "memory");
+        };
+        const uint32_t counted = *(const volatile uint32_t*)&a.state->counted;
+        auto wait_cleared = [&](uint32_t clears) {
+            if (lane == 0) {
+                uint32_t n = 0, v;
+                Waiter w = wt;
+                do asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&a.state->cleared) : "memory");
+                while ((int32_t)(v - counted - clears * B200_SMS) < 0 && !w.give_up(n));
+            }
+            __syncwarp();
         };
         uint32_t nb = 0;
         // 1 / rms of the lane's rows
@@ -428,13 +439,13 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 put_x(set_of(e0) + so.x1 + frag<MT>(row, tile), set_of(e0) + so.s1 + (tile * R + row) * 4, eight_live(row >> 3), x, g);
             }
         }
-        // Set g may be cleared when everybody has read what there is in it, and has to be before anybody can be polling its next content.
-        // When ss2 of layer g + 1 is complete, out-proj of layer g + 1 is done, with it attention and qkv of that layer, so ffn-down of layer g (the
-        // last readers of set g but for x1 and ss1, which qkv of layer g + 1 has read). Its next content is layer g + 3's, polled first by an SM that has
-        // seen x1 of layer g + 3, so by then ffn-up of layer g + 2 has been published by every SM (each has tiles of it), by the threads that cleared,
-        // after the fence above. The set of the step's embedding stands for a layer. The last layer's set is cleared when the next step starts: it
-        // is used again in that step's second layer.
-        clear(e0 + 2);
+        // Set g may be cleared when everybody has read what there is in it: when ss2 of layer g + 1 is complete, out-proj of layer g + 1 is done, with
+        // it attention and qkv of that layer, so ffn-down of layer g (the last readers of set g but for x1 and ss1, which qkv of layer g + 1
+        // has read). And it has to be cleared before anybody polls its next content or writes it: see clears_before_out(). The count goes up by a
+        // release behind all stores of an SM's epilogue and is awaited with an acquire that the compute warps get with the next free_bar, so
+        // the clears are ordered before those polls whatever was read in between. Nothing waits here in earnest: the count is two phases old.
+        // The set of the step's embedding stands for a layer. The last layer's set is cleared when the next step starts.
+        clear(e0 + SETS - 1);
 #pragma unroll 1
         for (uint32_t i = 0; i < 4 * L; i++) {
             const uint32_t l = i >> 2, ph = i & 3, set = set_of(e0 + 1 + l);
@@ -445,9 +456,9 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll
             for (uint32_t m = 0; m < MT; m++) f[m] = 1.0f;
             if (norm && tiles) factors(ph == QKV ? set_of(e0 + l) + so.s1 : set + so.s2, f);
+            if (ph == OUT) wait_cleared(clears_before_out(l));
             // A row without a sequence is published as zeros where a row of its eight has one (the consumers look at whole eights only). Here its
-            // attention, by the SM with the row's number among its qkv tiles: it has just seen that the layer before is complete, so
-            // nobody's clearing of the set is still to come.
+            // attention, by the SM with the row's number among its qkv tiles.
             if (ph == QKV) {
 #pragma unroll 1
                 for (uint32_t r = d.t0; r < min(d.t0 + tiles, R); r++)
@@ -1143,7 +1154,10 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 const uint32_t tok = n < a.vocab ? n : 0u;   // (no logit above -inf: 0)
                 a.sampled[cta] = tok;
                 if (a.sampled_host) a.sampled_host[cta] = tok;
-                if (cta == (uint32_t)__ffs(live) - 1) a.state->set = (e0 + L + 1) % SETS;   // every SM has published its best, so has read it
+                if (cta == (uint32_t)__ffs(live) - 1) {   // every SM has published its best, so has read them
+                    a.state->set = (e0 + L + 1) % SETS;
+                    a.state->counted += clears_of_step(L) * B200_SMS;
+                }
             }
         }
     }

@@ -58,12 +58,23 @@ struct SetOff {
 };
 
 // The exchange sets, used in turn: the step's embedding has set e0, layer l set e0 + 1 + l (mod SETS), the next step starts with the set behind.
-constexpr uint32_t SETS = 3;
+// A set is cleared, by all SMs together, when what it holds has been read by everybody: the set of layer l - 1 (the embedding's for l = 0) once an SM
+// has published its ffn-up of layer l, and the last layer's at the start of the next step. An SM counts itself in behind each of its clears.
+constexpr uint32_t SETS = 4;
+// Clears that every SM has counted itself in for before an SM's epilogue goes on to the out-proj of layer l: the one at the start and those behind
+// the ffn-up of layers 0 .. l - 1. So the set of layer l + 2 is clean before anybody looks at it: the warp furthest ahead (one without
+// a slice of x, on an SM that has ffn-up tiles only) comes to the attention of layer l + 2 knowing that its epilogue is through ffn-up of layer l.
+// With three sets, and known by what was read only, such a warp could see a set before another SM had cleared it.
+AK_PLAN_FN constexpr uint32_t clears_before_out(uint32_t l) { return 1 + l; }
+AK_PLAN_FN constexpr uint32_t clears_of_step(uint32_t n_layers) { return 1 + n_layers; }
 
 // What steps hand on to each other, behind the sets. Only the kernel writes it, at the end of a step: a launch that failed changes nothing.
 struct State {
-    uint32_t set;   // e0 of the next step
-    uint32_t pad[31];
+    uint32_t set;       // e0 of the next step
+    uint32_t counted;   // what `cleared` is when the next step starts
+    uint32_t pad0[30];
+    uint32_t cleared;   // SMs counted in for clears since the beginning (mod 2^32)
+    uint32_t pad1[31];
 };
 
 inline size_t sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) {
