@@ -152,6 +152,7 @@ _PROTOS = {
     "ak_engine_poll": [vp, C.c_uint64, u32p, C.c_uint32, u32p, C.POINTER(C.c_int)],
     "ak_engine_block_table": [vp, C.c_uint64, i32p, C.c_uint32, u32p],
     "ak_engine_clear_finished": [vp],
+    "ak_engine_drill_wait": [vp, C.c_uint64],
     "ak_session_generate": [vp, u32p, C.c_uint32, C.c_uint32, C.c_float, C.c_uint32, C.c_float, C.c_float, C.c_uint64, C.c_int, u32p,
                             u32p],
     "ak_engine_get_stats": [vp, C.POINTER(EngineStats)],
@@ -529,6 +530,10 @@ class Engine:
 
     def clear_finished(self):
         check(lib().ak_engine_clear_finished(self.h))
+
+    def drill_wait(self, cycles: int):
+        """Failure drill: the next decode-only step's waits run out after `cycles` (engines whose decode step is one kernel)."""
+        check(lib().ak_engine_drill_wait(self.h, cycles))
 
     def stats(self) -> dict:
         s = EngineStats()

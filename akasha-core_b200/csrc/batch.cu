@@ -31,9 +31,11 @@
 // Arithmetic: bf16 inputs rounded once, f32 products and sums, as in the launch chain; the probabilities stay f32. The order of every sum
 // depends on the model and on the number of slots only, never on which other sequences are there.
 //
-// The grid is launched cooperatively (its blocks wait on one another): one block per SM, all resident. Every wait is bounded: on expiry the block
-// is `dead` (later waits return at once), the status word is set and the host reports AK_ERR_DEVICE_WAIT. A warp whose wait for a
-// copy ran out releases no slot any more, and nobody leaves before the copies it started have landed.
+// The grid is launched cooperatively (its blocks wait on one another): one block per SM, all resident. The step has a time limit; a wait that goes on
+// past it gives up and the block is `dead` (later waits give up soon). Its warps go through the rest of the step all the same, so that
+// the barriers between them come out even, but a warp whose wait for a copy ran out releases no slot and requests no copy any more, and
+// nobody leaves before the copies it started have landed. The status word is set, the host reports AK_ERR_DEVICE_WAIT, and a step
+// launched behind it returns at once: the exchange sets are not clean.
 #include "batch.h"
 #include "batch_plan.h"
 #include "tma.h"
@@ -41,6 +43,8 @@
 #include <type_traits>
 
 namespace ak {
+
+__device__ unsigned int g_batch_status = 0;
 
 namespace {
 
@@ -52,36 +56,39 @@ constexpr int REGS_FIRST = 80, REGS_COMPUTE = 144;
 static_assert(REGS_FIRST * 128 + REGS_COMPUTE * 384 <= 65536, "the split draws on the registers of the launch");
 constexpr uint32_t EMPTY = 0xffffffffu;   // an exchange word that is not written yet
 
-// Bounds the polling of one thread; `dead` is sticky for the block. A poll is a round trip to L2 (0.3 us or more), so the limit is a second or two.
-constexpr uint32_t MAX_POLLS = 1u << 22;
-struct Waiter {
-    uint32_t* dead;
-    __device__ __forceinline__ bool give_up(uint32_t& n) {
-        n++;
-        if ((n & 63u) == 0) {
-            if (*(volatile uint32_t*)dead) return true;
-            if (n > MAX_POLLS) {
-                *(volatile uint32_t*)dead = 1u;
-                return true;
-            }
-        }
-        return false;
+// Bounds the waits of a block (in shared memory): `dead` is sticky and set when a wait goes on past the deadline, a time limit of the whole step.
+struct Expiry {
+    long long deadline;
+    uint32_t dead;
+    __device__ __forceinline__ bool is_dead() const { return *(const volatile uint32_t*)&dead != 0; }
+    __device__ __forceinline__ bool expired() {
+        if (is_dead()) return true;
+        if (clock64() <= *(const volatile long long*)&deadline) return false;
+        *(volatile uint32_t*)&dead = 1u;
+        return true;
     }
 };
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, uint32_t* dead) {
+struct Waiter {   // of one thread that polls
+    Expiry* x;
+    __device__ __forceinline__ bool give_up(uint32_t& n) { return (++n & 63u) == 0 && x->expired(); }
+};
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, Expiry& x) {
     if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
 #pragma unroll 1
     for (;;) {
 #pragma unroll 1
         for (uint32_t n = 0; n < 64; n++)
             if (mbar_try_wait(bar, parity)) return true;
-        if (*(volatile uint32_t*)dead) return false;
-        if (clock64() - t0 > AK_WAIT_MAX_CYCLES) {
-            *(volatile uint32_t*)dead = 1u;
-            return false;
-        }
+        if (x.expired()) return false;
     }
+}
+// For warps of the same block. They always come, late when their own waits run out, so this one does not give up with them: a warp that went on without them
+// would arrive at BAR_PART twice in one use. (2^33 cycles behind the deadline it ends all the same.)
+__device__ __forceinline__ void wait_block(uint64_t* bar, uint32_t parity, const Expiry& x) {
+    if (mbar_try_wait(bar, parity)) return;
+#pragma unroll 1
+    while (!mbar_try_wait(bar, parity))
+        if (clock64() > *(const volatile long long*)&x.deadline + (1ll << 33)) return;
 }
 
 // ---- exchange words
@@ -180,7 +187,7 @@ struct Unit { uint32_t row, head, split, p0, n, nb; };   // attention unit: posi
 // The tiles a warp has yet to request: tile b of unit j (u) of layer l, in the pool blocks pb0 (and pb1); nu: units of the warp's group.
 struct Walk {
     Unit u;
-    uint32_t l, j, b, pb0, pb1, nu, more;
+    uint32_t l, j, b, pb0, pb1, nu, more, asked, sent;   // asked: its keys are requested; sent: requests made for values
 };
 enum { QKV = 0, OUT = 1, FFN_UP = 2, FFN_DOWN = 3, HEAD = 4, N_KINDS = 5 };
 constexpr uint32_t NO_LOGIT = 0x7fffffffu;   // in the place of the index of a best logit
@@ -205,7 +212,8 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     __shared__ Walk walk_sm[NW];
     __shared__ uint32_t units[NW][MAX_UNITS];
     __shared__ uint32_t len_sm[32], by_len[32], pre_sm[33];
-    __shared__ uint32_t dead, live_sm, use_sm[MAX_SLOTS + MAX_EXTRA];   // use_sm: 1 + the number of the use a slot is in (lm_head only)
+    __shared__ Expiry expiry;
+    __shared__ uint32_t failed_sm, live_sm, use_sm[MAX_SLOTS + MAX_EXTRA];   // use_sm: 1 + the number of the use a slot is in (lm_head only)
 
     const uint32_t tid = threadIdx.x, warp_ = tid >> 5, lane = tid & 31;
     const uint32_t cta = blockIdx.x;
@@ -225,7 +233,9 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         for (uint32_t i = 0; i < NW; i++) { mbar_init(&k_bar[i], 1); mbar_init(&v_bar[i], 1); }
         mbar_init(&free_bar, NH);
         mbar_init(&kv_free_bar, NW);
-        dead = 0;
+        expiry.deadline = clock64() + (long long)a.max_cycles;
+        expiry.dead = 0;
+        failed_sm = *(const volatile uint32_t*)a.status;
         mbar_fence_init();
     }
     if (tid >= 32 && tid < 32 + N_KINDS) make_kind(kinds[tid - 32], tid == 32 ? 3 * D : tid == 34 ? F : tid == 36 ? a.vocab : D, tid == 35 ? F : D, cta);
@@ -257,6 +267,15 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         reinterpret_cast<uint64_t*>(layers_sm)[i] = reinterpret_cast<const uint64_t*>(a.layers)[i];
     const uint32_t e0 = *(const volatile uint32_t*)&a.state->set;   // (before the block's barrier, so before this SM publishes anything)
     __syncthreads();
+    auto report = [&]() {
+        atomicExch(a.status, 1u);
+        atomicExch(&g_batch_status, 1u);
+        if (a.sampled_host) *(volatile uint32_t*)(a.sampled_host + a.seqs) = 1u;
+    };
+    if (failed_sm) {   // a step before this one failed
+        if (tid == 0) report();
+        return;
+    }
 #pragma unroll 1
     for (uint32_t i = tid, n = kinds[OUT].n * 8; i < (2 * L + 1) * n; i += THREADS)
         gain_sm[i] = (i / n == 2 * L ? a.final_norm : i / n & 1 ? layers_sm[i / (2 * n)].norm_2 : layers_sm[i / (2 * n)].norm_1)[kinds[OUT].t0 * 8 + i % n];
@@ -270,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     auto set_of = [&](uint32_t g) { return (g % SETS) * (uint32_t)so.total; };   // byte offset; g = e0: the embedding, e0 + 1 + l: layer l
     auto row_live = [&](uint32_t r) { return (live >> r) & 1u; };
     auto eight_live = [&](uint32_t e) { return ((live >> (e * 8)) & 0xffu) != 0; };
-    const Waiter wt{&dead};
+    const Waiter wt{&expiry};
     const float inv_dim = 1.0f / (float)D;
 
     if (warp_ < FIRST_COMPUTE) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_FIRST));
@@ -293,7 +312,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 for (uint32_t c = 0; c < d.chunks && ok; c++) {
 #pragma unroll 1
                     for (uint32_t t = 0; t < nt; t++) {
-                        if (sent >= slots) ok = wait_bar(&empty_bar[q.s], q.ph ^ 1u, &dead);
+                        if (sent >= slots) ok = wait_bar(&empty_bar[q.s], q.ph ^ 1u, expiry);
                         if (!ok) break;
                         mbar_expect_tx(&full_bar[q.s], 8 * d.pitch);
                         tma_load_rows(smem + q.s * SLOT, map + i, c * d.pieces, (d.t0 + b + t) * 8, &full_bar[q.s], pol);
@@ -311,9 +330,9 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 const uint32_t lap = head_sent / head_slots, r = head_sent - lap * head_slots, x = r < slots ? 0 : MAX_SLOTS + r - slots;
                 const uint32_t bar = r < slots ? q.s : x;
                 if (r < slots) {
-                    if (sent >= slots) ok = wait_bar(&empty_bar[bar], q.ph ^ 1u, &dead);
+                    if (sent >= slots) ok = wait_bar(&empty_bar[bar], q.ph ^ 1u, expiry);
                 } else {
-                    ok = lap ? wait_bar(&empty_bar[bar], (lap - 1) & 1u, &dead) : wait_bar(&kv_free_bar, 0, &dead);
+                    ok = lap ? wait_bar(&empty_bar[bar], (lap - 1) & 1u, expiry) : wait_bar(&kv_free_bar, 0, expiry);
                 }
                 if (!ok) break;
                 mbar_expect_tx(&full_bar[bar], 8 * d.pitch);
@@ -336,6 +355,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         }
 #pragma unroll 1
         for (uint32_t r = slots; r < min(head_sent, head_slots); r++) mbar_wait(&full_bar[MAX_SLOTS + r - slots], ((head_sent - r - 1) / head_slots) & 1u);
+        if (expiry.is_dead()) report();
         return;
     }
     if (warp_ < FIRST_COMPUTE) {
@@ -526,6 +546,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             }
             if (ph == FFN_UP) clear(e0 + l);
         }
+        if (lane == 0 && expiry.is_dead()) report();
         return;
     }
 
@@ -590,7 +611,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 if (cc == 0 || c0 + cc < chunks) {
                     Cursor mine = q;
                     mine.advance(lane < NT ? lane : 0, slots);
-                    const bool got = lane >= NT || wait_bar(&full_bar[mine.s], mine.ph, &dead);
+                    const bool got = lane >= NT || wait_bar(&full_bar[mine.s], mine.ph, expiry);
                     alive = __all_sync(0xffffffffu, got && alive) != 0;
 #pragma unroll
                     for (uint32_t t = 0; t < NT; t++) {
@@ -645,7 +666,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             xl += DEPTH * STEP;
             issue(c0 * PPC);
         }
-        alive = wait_bar(&free_bar, part_ph, &dead) && alive;   // the sums that were there have been read
+        wait_block(&free_bar, part_ph, expiry);   // the sums that were there have been read
         part_ph ^= 1u;
         {
             float* const o = part + (cw * TB * R + (lane >> 2)) * 8 + (lane & 3) * 2;
@@ -718,7 +739,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     // Request the keys or the values of the walk's tile; with the values the walk moves on. Called by the whole warp after it has read the buffer;
     // lane 0 does it, with the walk in shared memory.
     auto request = [&](bool values) {
-        if (lane == 0 && walk_sm[cw].more) {
+        if (lane == 0 && alive && walk_sm[cw].more) {
             Walk& k = walk_sm[cw];
             const SoloLayer& w = layers_sm[k.l];
             const uint32_t pb0 = k.pb0, pb1 = k.pb1;
@@ -729,7 +750,9 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             mbar_expect_tx(bar, UP > 16 && pb1 != EMPTY ? 2 * TILE : TILE);
             bulk_g2s(dst, pool + (size_t)pb0 * H * (16 * HD), TILE, bar);
             if (UP > 16 && pb1 != EMPTY) bulk_g2s(dst + TILE, pool + (size_t)pb1 * H * (16 * HD), TILE, bar);
+            k.asked = !values;
             if (values) {
+                k.sent++;
                 k.b += wpi;
 #pragma unroll 1
                 while (k.b >= k.u.nb) {
@@ -748,7 +771,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     {
         if (lane == 0) {
             Walk& k = walk_sm[cw];
-            k.l = k.j = k.more = 0;
+            k.l = k.j = k.more = k.asked = k.sent = 0;
             k.b = place_in();
 #pragma unroll 1
             for (uint32_t j = k.nu; j-- > 0;)   // the first unit with a tile for this warp (if there is one there is one in every layer)
@@ -854,7 +877,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                     const uint32_t left = u.n - b * UP;   // positions of the tile that count, if fewer than UP
                     const bool fresh = newest && left <= UP;
                     const uint32_t at = (left - 1) * (HD * 2) + chunk * 16;   // the new position's row in the buffers
-                    alive = wait_bar(&k_bar[cw], tiles_done & 1u, &dead) && alive;
+                    alive = wait_bar(&k_bar[cw], tiles_done & 1u, expiry) && alive;
                     if (fresh) {
                         if (lane < CH) {
                             *reinterpret_cast<uint4*>(kbuf + at) = kn;
@@ -897,7 +920,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                     }
 #pragma unroll
                     for (int e = 0; e < 8; e++) acc[e] *= corr;
-                    alive = wait_bar(&v_bar[cw], tiles_done & 1u, &dead) && alive;
+                    alive = wait_bar(&v_bar[cw], tiles_done & 1u, expiry) && alive;
                     if (fresh) {   // what lies behind the sequence's end is anything, a NaN even
                         if (lane < CH) *reinterpret_cast<uint4*>(vbuf + at) = vn;
 #pragma unroll 1
@@ -1072,7 +1095,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll 1
                 while (*(volatile uint32_t*)&use_sm[bar] != use + 1 && !wait.give_up(n)) {}
                 __syncwarp();
-                alive = __all_sync(0xffffffffu, *(volatile uint32_t*)&use_sm[bar] == use + 1 && wait_bar(&full_bar[bar], use & 1u, &dead) && alive) != 0;
+                alive = __all_sync(0xffffffffu, *(volatile uint32_t*)&use_sm[bar] == use + 1 && wait_bar(&full_bar[bar], use & 1u, expiry) && alive) != 0;
                 const uint8_t* const wp = (r < slots ? smem + bar * SLOT : extra_sm + (r - slots) * SLOT) + (lane >> 2) * d.pitch + (lane & 3) * 16;
                 const uint4* const xp = xs + c * CHUNK * (2 * MT) * 32 + lane;
                 const uint32_t ns = d.count(c);
@@ -1161,19 +1184,17 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             }
         }
     }
-    if (!alive || *(volatile uint32_t*)&dead) {
-        // tiles this warp requested and may not have waited for (their copies end by themselves)
-        mbar_wait(&k_bar[cw], tiles_done & 1u);
-        mbar_wait(&v_bar[cw], tiles_done & 1u);
-        if (lane == 0) {
-            atomicExch(a.status, 1u);
-            if (a.sampled_host) *(volatile uint32_t*)(a.sampled_host + a.seqs) = 1u;
-        }
+    if (expiry.is_dead()) {
+        // the latest copy into each buffer may not have been waited for (a copy was only requested when the one before was)
+        const uint32_t nv = walk_sm[cw].sent, nk = nv + walk_sm[cw].asked;
+        if (nk) mbar_wait(&k_bar[cw], (nk - 1) & 1u);
+        if (nv) mbar_wait(&v_bar[cw], (nv - 1) & 1u);
+        if (lane == 0) report();
     }
 }
 
 template <int HD, int MT, bool SPLIT>
-int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p) {
+int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p, uint32_t blocks) {
     {
         static bool attr_set[64] = {};
         int dev = 0;
@@ -1185,7 +1206,7 @@ int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p) {
         }
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(B200_SMS);
+    cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
@@ -1221,15 +1242,21 @@ bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads,
 
 size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) { return sets_bytes(dim, ffn, heads, seqs, max_len); }
 
-int launch_batch(cudaStream_t st, const BatchArgs& a) {
+int launch_batch(cudaStream_t st, const BatchArgs& a, uint32_t missing) {
+    const uint32_t blocks = B200_SMS - missing;
     const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.seqs, a.max_len);
     const bool two = m_tiles(a.seqs) == 2, split = has_splits(a.max_len);
     if (a.dim / a.heads == 64) {
-        if (split) return two ? launch_batch_t<64, 2, true>(st, a, p) : launch_batch_t<64, 1, true>(st, a, p);
-        return two ? launch_batch_t<64, 2, false>(st, a, p) : launch_batch_t<64, 1, false>(st, a, p);
+        if (split) return two ? launch_batch_t<64, 2, true>(st, a, p, blocks) : launch_batch_t<64, 1, true>(st, a, p, blocks);
+        return two ? launch_batch_t<64, 2, false>(st, a, p, blocks) : launch_batch_t<64, 1, false>(st, a, p, blocks);
     }
-    if (split) return two ? launch_batch_t<128, 2, true>(st, a, p) : launch_batch_t<128, 1, true>(st, a, p);
-    return two ? launch_batch_t<128, 2, false>(st, a, p) : launch_batch_t<128, 1, false>(st, a, p);
+    if (split) return two ? launch_batch_t<128, 2, true>(st, a, p, blocks) : launch_batch_t<128, 1, true>(st, a, p, blocks);
+    return two ? launch_batch_t<128, 2, false>(st, a, p, blocks) : launch_batch_t<128, 1, false>(st, a, p, blocks);
+}
+
+int batch_status(unsigned int* out) {
+    AK_CUDA(cudaMemcpyFromSymbol(out, g_batch_status, sizeof(unsigned int)));
+    return AK_OK;
 }
 
 }  // namespace ak

@@ -23,7 +23,8 @@ struct BatchArgs {
     int32_t tok_src[BATCH_ROWS], lens[BATCH_ROWS];
     const int32_t* block_tables; // [seqs][max_blocks]
     uint32_t* sampled_host;      // where else the picks go: [seqs] in mapped host memory and behind them the status word, or nullptr
-    uint32_t* status;            // device word: made non-zero when a wait runs out
+    uint32_t* status;            // device word: made non-zero when a wait runs out; a step that finds it so does nothing
+    uint64_t max_cycles;         // time limit of the step, in SM clocks
     uint32_t n_layers, dim, ffn, heads, vocab, seqs, max_blocks, max_len;
     float eps, scale;
 };
@@ -32,6 +33,9 @@ bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads,
 // the weights' tensor maps, 4 n_layers + 1 of 128 bytes in host memory (layers: host array)
 int batch_maps(void* out, const SoloLayer* layers, const void* lm_head, uint32_t n_layers, uint32_t dim, uint32_t ffn, uint32_t vocab);
 size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len);
-int launch_batch(cudaStream_t st, const BatchArgs& a);
+constexpr uint64_t BATCH_MAX_CYCLES = 1ull << 32;   // two seconds or so, for a step of milliseconds
+// missing: blocks left out, so that the others' waits run out (a drill)
+int launch_batch(cudaStream_t st, const BatchArgs& a, uint32_t missing = 0);
+int batch_status(unsigned int* out);
 
 }  // namespace ak

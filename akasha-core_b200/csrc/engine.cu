@@ -421,6 +421,11 @@ int ak_engine_block_table(ak_engine* e, uint64_t seq_id, int32_t* out, uint32_t 
     return AK_OK;
 }
 
+int ak_engine_drill_wait(ak_engine* e, uint64_t cycles) {
+    AK_REQUIRE(e, AK_ERR_INVALID_ARG, "ak_engine_drill_wait: null engine");
+    return e->runner.drill_wait(cycles);
+}
+
 int ak_engine_clear_finished(ak_engine* e) {
     AK_REQUIRE(e, AK_ERR_INVALID_ARG, "ak_engine_clear_finished: null engine");
     { int rcf = collect(e); if (rcf) return rcf; }

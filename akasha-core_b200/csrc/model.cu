@@ -422,6 +422,7 @@ BatchArgs Runner::batch_args() const {
     a.sampled = d_sampled_;
     a.block_tables = d_desc_ + d_.block_tables;
     a.status = d_sampled_ + max_seqs_;
+    a.max_cycles = BATCH_MAX_CYCLES;
     a.n_layers = c.num_layers; a.dim = c.dim; a.ffn = c.ffn_hidden; a.heads = c.num_heads; a.vocab = c.vocab_size;
     a.seqs = max_seqs_; a.max_blocks = max_blocks_; a.max_len = max_seq_len_;
     a.eps = c.norm_eps;
@@ -439,11 +440,20 @@ int Runner::run_decode_batch() {
         a.lens[i] = h_kv_lens()[i];
     }
     a.sampled_host = h_sampled_;
+    if (drill_cycles_) a.max_cycles = drill_cycles_;
     const auto h0 = std::chrono::steady_clock::now();
-    AK_TRY(launch_batch(ctx_->stream, a));
+    AK_TRY(launch_batch(ctx_->stream, a, drill_cycles_ ? 1 : 0));
+    drill_cycles_ = 0;
     launch_host_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - h0).count();
     h2d_bytes += (size_t)max_seqs_ * 8;
     d2h_bytes += (size_t)max_seqs_ * 4;
+    return AK_OK;
+}
+
+int Runner::drill_wait(uint64_t cycles) {
+    AK_REQUIRE(batch_, AK_ERR_UNSUPPORTED, "drill: the decode steps are launch chains");
+    AK_REQUIRE(cycles > 0 && cycles <= BATCH_MAX_CYCLES, AK_ERR_INVALID_ARG, "drill: 1 to %llu cycles", (unsigned long long)BATCH_MAX_CYCLES);
+    drill_cycles_ = cycles;
     return AK_OK;
 }
 

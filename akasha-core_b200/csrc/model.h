@@ -111,6 +111,7 @@ class Runner {
     // Decode rows through one persistent kernel (batch.cu) instead of the launch chain, where model and slots allow it. A row's sums are not in
     // the chain's order, so all decode rows of a runner's life take one of the two.
     int init_batch();
+    int drill_wait(uint64_t cycles);        // the next decode-only step runs a block short and for `cycles` at most
     bool batch() const { return batch_; }   // its decode rows are sampled by the kernel: their out_rows are -1
     // spin until a device-written pinned word {value, tag} carries `tag`
     int wait_word(const uint64_t* word, uint32_t tag, uint32_t& value);
@@ -213,6 +214,7 @@ class Runner {
     SoloLayer* d_batch_layers_ = nullptr;
     void* d_batch_maps_ = nullptr;
     batch::State* d_batch_state_ = nullptr;   // behind the exchange sets
+    uint64_t drill_cycles_ = 0;
     bool batch_ran_ = false;            // a persistent step of the step being launched is on the stream
     int failed_ = 0;                    // the error after which this runner takes no step any more
     int capture_step(uint64_t key, uint32_t T, uint32_t rows_b, uint32_t seqs_b, uint32_t len_b, uint32_t n_splits, size_t bytes);

@@ -404,6 +404,9 @@ AK_API int ak_engine_poll(ak_engine* e, uint64_t seq_id, uint32_t* out, uint32_t
 AK_API int ak_engine_block_table(ak_engine* e, uint64_t seq_id, int32_t* out, uint32_t cap, uint32_t* n_out);
 /* Forget finished sequences' records. */
 AK_API int ak_engine_clear_finished(ak_engine* e);
+/* Failure drill, for decode steps that are one kernel (AK_ERR_UNSUPPORTED otherwise): the next decode-only step runs without one of
+ * its blocks, so that the other blocks' waits run out, `cycles` SM clocks after its start. */
+AK_API int ak_engine_drill_wait(ak_engine* e, uint64_t cycles);
 typedef struct ak_engine_stats {
     uint64_t steps, decode_tokens, prefill_tokens, graph_launches, eager_steps, kernel_launches;
     double attn_ms_total;        /* sum of timed layer-0 decode-attention launches (attn_timing) */

@@ -204,6 +204,7 @@ extern "C" {
     pub fn ak_engine_poll(e: *mut AkEngine, seq_id: u64, out: *mut u32, cap: u32, n_out: *mut u32, finished: *mut c_int) -> c_int;
     pub fn ak_engine_block_table(e: *mut AkEngine, seq_id: u64, out: *mut i32, cap: u32, n_out: *mut u32) -> c_int;
     pub fn ak_engine_clear_finished(e: *mut AkEngine) -> c_int;
+    pub fn ak_engine_drill_wait(e: *mut AkEngine, cycles: u64) -> c_int;
     pub fn ak_engine_get_stats(e: *mut AkEngine, out: *mut AkEngineStats) -> c_int;
     pub fn ak_engine_reset_stats(e: *mut AkEngine) -> c_int;
 }
