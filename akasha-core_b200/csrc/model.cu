@@ -752,7 +752,7 @@ int Runner::attn_time_mark(cudaStream_t s, cudaEvent_t ev, bool capturing) {
 }
 
 int Runner::run(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_pf_len, bool any_decode, uint32_t max_kv_len) {
-    AK_REQUIRE(!failed_, failed_, "runner: a step before failed half way");
+    AK_REQUIRE(!failed_, failed_, "runner: no step after one that failed half way");
     AK_REQUIRE(n_prefill_rows <= max_pf_tokens_, AK_ERR_INVALID_ARG, "runner: %u prefill rows exceed the step budget %u", n_prefill_rows, max_pf_tokens_);
     AK_CUDA(cudaSetDevice(ctx_->device));
     cudaStream_t st = ctx_->stream;
@@ -826,7 +826,7 @@ static uint32_t pow2_bucket(uint32_t v, uint32_t lo) {
 // graph per bucket is captured on first use. Row results do not depend on the bucket (every
 // kernel treats rows independently and the GEMM's K order is fixed per (n, k)).
 int Runner::run_graph(uint32_t n_prefill_rows, uint32_t n_pf_seqs, uint32_t max_pf_len) {
-    AK_REQUIRE(!failed_, failed_, "runner: a step before failed half way");
+    AK_REQUIRE(!failed_, failed_, "runner: no step after one that failed half way");
     AK_REQUIRE(n_prefill_rows <= max_pf_tokens_ && n_pf_seqs <= max_seqs_, AK_ERR_INVALID_ARG, "runner: step exceeds its budget");
     AK_CUDA(cudaSetDevice(ctx_->device));
     cudaStream_t st = ctx_->stream;
@@ -898,7 +898,8 @@ int Runner::mark_done() {
 int Runner::wait_bank(uint32_t b) {
     trace_dump();
     AK_CUDA(cudaEventSynchronize(banks_[b & 1u].ev_done));
-    AK_REQUIRE(banks_[b & 1u].h_sampled[max_seqs_] == 0, AK_ERR_DEVICE_WAIT, "decode step: a bounded device-side wait expired");
+    if (banks_[b & 1u].h_sampled[max_seqs_] != 0) failed_ = AK_ERR_DEVICE_WAIT;   // its exchange sets are not clean any more
+    AK_REQUIRE(failed_ != AK_ERR_DEVICE_WAIT, failed_, "decode step: a bounded device-side wait expired");
     return AK_OK;
 }
 

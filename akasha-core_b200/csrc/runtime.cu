@@ -4,6 +4,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "batch.h"
 #include "kernels.h"
 #include "solo.h"
 #include "tma.h"
@@ -174,6 +175,9 @@ int ak_check_device_status(void* stream) {
     rc = solo_status(&v);
     if (rc) return rc;
     AK_REQUIRE(v == 0, AK_ERR_DEVICE_WAIT, "batch-1 decode step: a bounded device-side wait expired (code %u)", v);
+    rc = batch_status(&v);
+    if (rc) return rc;
+    AK_REQUIRE(v == 0, AK_ERR_DEVICE_WAIT, "decode step of several sequences: a bounded device-side wait expired (code %u)", v);
     return AK_OK;
 }
 

@@ -391,7 +391,9 @@ AK_API int ak_engine_destroy(ak_engine* e);
 AK_API int ak_engine_submit(ak_engine* e, const uint32_t* prompt, uint32_t n, uint32_t max_total_len, uint64_t* seq_id);
 /* One scheduler step: admit waiting sequences into free slots (their prompts are prefilled in
  * this step's ragged batch), run one token for every running sequence, retire finished ones.
- * n_running / n_finished_total may be NULL. Returns after the step's token ids are on the host. */
+ * n_running / n_finished_total may be NULL. Returns after the step's token ids are on the host. AK_ERR_DEVICE_WAIT where a
+ * device-side wait of a step ran out: its tokens, and with them the engine's running sequences, are lost. It launches no step any
+ * more, this call and poll go on to report the error; destroy it. */
 AK_API int ak_engine_step(ak_engine* e, uint32_t* n_running, uint32_t* n_waiting);
 /* Steps until nothing is running or waiting (at most max_steps; 0 = no limit), then waits for the last
  * step. steps_done may be NULL. The loop the reference's `generate` runs per sequence

@@ -62,6 +62,21 @@ def child(shape, more=""):
 SHAPES = [(320, 5, 1280, 2, 3, 96, True), (256, 2, 1184, 3, 20, 700, False), (768, 12, 3072, 2, 8, 512, True), (512, 4, 2048, 2, 32, 96, False)]
 
 
+def test_the_engine_takes_no_further_step():
+    """Every later call reports the error without launching anything, and so does the device status, which knows the kernel."""
+    for shape in SHAPES[:2]:
+        child(shape, """
+assert all(c == 104 for c in codes[first:]), codes
+for call in (e.step, e.run_to_completion, lambda: e.poll(ids[0]), ctx.check_device_status):
+    n0 = ak.lib().ak_launch_count()
+    try:
+        call()
+        raise SystemExit("no error")
+    except ak.AkashaError as x:
+        assert x.code == 104 and ak.lib().ak_launch_count() == n0, x
+""")
+
+
 @pytest.mark.parametrize("shape", SHAPES)
 def test_a_wait_that_runs_out_is_an_error(shape):
     child(shape)
