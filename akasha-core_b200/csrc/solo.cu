@@ -862,7 +862,9 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
                 }
                 l_run = l_run * corr + ls;
                 m_run = m_new;
-                alive = __all_sync(0xffffffffu, got) && alive;
+                // The buffer goes back behind a value that all of this tile's loads went into, in every lane: a load from shared memory and a later
+                // arrival on a barrier are not in order by themselves (the comparison is true of every sum: a NaN comes out as 0x7fffffff).
+                alive = __all_sync(0xffffffffu, got && __float_as_uint(acc[0]) != 0xffffffffu) && alive;
                 if (alive && lane == 0) mbar_arrive(&kv_empty[warp]);
             }
 #pragma unroll
