@@ -183,12 +183,6 @@ __device__ __forceinline__ void make_kind(Kind& d, uint32_t rows, uint32_t k, ui
 template <int MT> __device__ __forceinline__ uint32_t frag(uint32_t row, uint32_t v) {
     return ((((v >> 2) * MT + (row >> 4)) * 2 + ((row >> 3) & 1)) * 32 + (v & 3) * 8 + (row & 7)) * 16;
 }
-struct Unit { uint32_t row, head, split, p0, n, nb; };   // attention unit: positions p0 .. p0 + n of (row, head), nb tiles
-// The tiles a warp has yet to request: tile b of unit j (u) of layer l, in the pool blocks pb0 (and pb1); nu: units of the warp's group.
-struct Walk {
-    Unit u;
-    uint32_t l, j, b, pb0, pb1, nu, more, asked, sent;   // asked: its keys are requested; sent: requests made for values
-};
 enum { QKV = 0, OUT = 1, FFN_UP = 2, FFN_DOWN = 3, HEAD = 4, N_KINDS = 5 };
 constexpr uint32_t NO_LOGIT = 0x7fffffffu;   // in the place of the index of a best logit
 
@@ -753,17 +747,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             k.asked = !values;
             if (values) {
                 k.sent++;
-                k.b += wpi;
-#pragma unroll 1
-                while (k.b >= k.u.nb) {
-                    if (++k.j == k.nu) {
-                        k.j = 0;
-                        if (++k.l == L) { k.more = 0; break; }
-                    }
-                    k.u = unit_at(k.j);
-                    k.b = place_in();
-                }
-                look_up();
+                walk_on(k, wpi, place_in(), L, unit_at, look_up);
             }
         }
         __syncwarp();

@@ -97,6 +97,35 @@ inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t 
     return p;
 }
 
+// An attention unit: positions p0 .. p0 + n of (row, head), nb tiles.
+struct Unit { uint32_t row, head, split, p0, n, nb; };
+// The tiles a warp has yet to request, in order: tile b of unit j (u) of layer l, in the pool blocks pb0 (and pb1); nu: units of the warp's group.
+struct Walk {
+    Unit u;
+    uint32_t l, j, b, pb0, pb1, nu, more, asked, sent;   // more: there is such a tile; asked: its keys are requested; sent: requests made for values
+};
+// To the next tile of the warp, the place-th of the wpi of its group, which has a tile in some unit. unit_at(j): unit j of the group. look_up(): the
+// tile's pool blocks; asked for tiles that exist only.
+template <class UnitAt, class LookUp>
+AK_PLAN_FN void walk_on(Walk& k, uint32_t wpi, uint32_t place, uint32_t n_layers, UnitAt unit_at, LookUp look_up) {
+    k.b += wpi;
+#ifdef __CUDACC__
+#pragma unroll 1
+#endif
+    while (k.b >= k.u.nb) {
+        if (++k.j == k.nu) {
+            k.j = 0;
+            if (++k.l == n_layers) {
+                k.more = 0;
+                return;
+            }
+        }
+        k.u = unit_at(k.j);
+        k.b = place;
+    }
+    look_up();
+}
+
 inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers, uint32_t seqs, uint32_t max_len) {
     const uint32_t hd = heads ? dim / heads : 0;
     if ((hd != 64 && hd != 128) || dim != heads * hd || heads > 4095) return false;

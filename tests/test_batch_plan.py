@@ -130,15 +130,64 @@ int main(int argc, char** argv) {
 """
 
 
-@pytest.fixture(scope="module")
-def plan(tmp_path_factory):
+# A warp's walk over its cache tiles, for every length of a unit: the block table is read for the sequence's own blocks only, every tile is met
+# once in its order, in every layer.
+WALK = r"""
+#include <stdio.h>
+#include <initializer_list>
+#include "batch_plan.h"
+using namespace ak::batch;
+int main() {
+    int bad = 0, walks = 0;
+    for (uint32_t up : {16u, 32u})
+        for (uint32_t wpi : {4u, 12u})
+            for (uint32_t place = 0; place < wpi; place++)
+                for (uint32_t n0 = 1; n0 <= 512; n0 += n0 < 70 ? 1 : 61)
+                    for (uint32_t n1 : {0u, 1u, 17u, 33u, 512u}) {
+                        const uint32_t lens[2] = {n0, n1}, nu = n1 ? 2 : 1, L = 3;
+                        auto unit_at = [&](uint32_t j) { return Unit{0, 0, 0, 0, lens[j], div_up(lens[j], up)}; };
+                        Walk k{};
+                        k.nu = nu;
+                        k.b = place;
+                        uint32_t want = 0, met = 0;
+                        for (uint32_t j = nu; j-- > 0;) {
+                            for (uint32_t b = place; b < unit_at(j).nb; b += wpi) want++;
+                            if (place < unit_at(j).nb) { k.more = 1; k.j = j; }
+                        }
+                        if (!k.more) continue;
+                        k.u = unit_at(k.j);
+                        uint32_t last = 0;
+                        auto look = [&]() {
+                            if (k.b * up >= k.u.n) bad++;
+                            const uint32_t at = (k.l * 2 + k.j) * 64 + k.b + 1;
+                            if (at <= last || k.b % wpi != place) bad++;
+                            last = at;
+                            met++;
+                        };
+                        look();
+                        while (k.more && met <= 3 * want) walk_on(k, wpi, place, L, unit_at, look);
+                        if (met != 3 * want) bad++;
+                        walks++;
+                    }
+    printf(bad ? "%d bad\n" : "ok %d\n", bad ? bad : walks);
+    return 0;
+}
+"""
+
+
+def build(tmp_path_factory, text):
     gxx = shutil.which("g++")
     if not gxx:
         pytest.skip("no g++")
     d = tmp_path_factory.mktemp("batch_plan")
-    (d / "check.cpp").write_text(CHECK)
+    (d / "check.cpp").write_text(text)
     subprocess.run([gxx, "-std=c++17", "-O2", "-I", os.path.join(ROOT, "akasha-core_b200", "csrc"), str(d / "check.cpp"), "-o", str(d / "check")], check=True)
     return lambda *a: subprocess.run([str(d / "check"), *map(str, a)], capture_output=True, text=True).stdout.strip()
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    return build(tmp_path_factory, CHECK)
 
 
 # dim 96 .. 320: SMs without rows of qkv, out-proj and ffn-down, warps without a slice of x; 768 and 2048: every SM has all kinds of rows
@@ -147,3 +196,8 @@ def plan(tmp_path_factory):
 def test_sets_are_clean_and_unread(plan, dim, ffn, heads, rows, max_len):
     for layers in (1, 2, 3, 4, 7):
         assert plan(dim, ffn, heads, layers, rows, max_len) == "ok"
+
+
+def test_walk_stays_in_the_block_table(tmp_path_factory):
+    out = build(tmp_path_factory, WALK)()
+    assert out.startswith("ok") and int(out.split()[1]) > 1000, out
