@@ -98,6 +98,11 @@ __device__ __forceinline__ uint4 xld4(const void* p) {
     asm volatile("{\n.reg .b128 q;\nld.relaxed.gpu.global.b128 q, [%2];\nmov.b128 {%0, %1}, q;\n}\n" : "=l"(a), "=l"(b) : "l"(p));
     return make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
 }
+__device__ __forceinline__ uint32_t xld1(const void* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ uint2 xld2(const void* p) {
     uint2 v;
     asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
@@ -118,7 +123,7 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {   // (a NaN become
 template <uint32_t N> __device__ __forceinline__ void bar_sync(uint32_t id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(N) : "memory"); }
 __device__ __forceinline__ void bar_sync_n(uint32_t id, uint32_t n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 template <uint32_t N> __device__ __forceinline__ void bar_arrive(uint32_t id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(N) : "memory"); }
-enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_GROUP = 4 };   // BAR_GROUP and the next two: by group
+enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_GROUP = 4, BAR_FLAT = 7 };   // BAR_GROUP and the next two: by group
 
 __device__ __forceinline__ uint64_t policy_evict_first() {
     uint64_t p;
@@ -207,7 +212,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     __shared__ uint32_t units[NW][MAX_UNITS];
     __shared__ uint32_t len_sm[32], by_len[32], pre_sm[33];
     __shared__ Expiry expiry;
-    __shared__ uint32_t failed_sm, live_sm, use_sm[MAX_SLOTS + MAX_EXTRA];   // use_sm: 1 + the number of the use a slot is in (lm_head only)
+    __shared__ uint32_t failed_sm, flat_sm, live_sm, use_sm[MAX_SLOTS + MAX_EXTRA];   // use_sm: 1 + the number of the use a slot is in (lm_head only)
 
     const uint32_t tid = threadIdx.x, warp_ = tid >> 5, lane = tid & 31;
     const uint32_t cta = blockIdx.x;
@@ -539,6 +544,24 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 if (lane == 0) mbar_arrive(&free_bar);
             }
             if (ph == FFN_UP) clear(e0 + l);
+        }
+        // The picks leave out 1 / rms, which changes no order, but for a row whose sum of squares overflowed: there it is 0, and so are all logits.
+        if (e == 0 && cta < R && row_live(cta)) {
+            float sum = 0.0f;
+#pragma unroll 1
+            for (uint32_t t = lane; t < D / 8; t += 32) {
+                uint32_t y, n = 0;
+                Waiter w = wt;
+#pragma unroll 1
+                do y = xld1(a.xch + set_of(e0 + L) + so.s1 + (t * R + cta) * 4);
+                while (y == EMPTY && !w.give_up(n));
+                sum += __uint_as_float(y);
+            }
+            __syncwarp();
+            sum = warp_sum(sum);
+            if (lane == 0) flat_sm = sum == INFINITY;
+            __syncwarp();
+            bar_arrive<64>(BAR_FLAT);
         }
         if (lane == 0 && expiry.is_dead()) report();
         return;
@@ -1157,8 +1180,9 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 const uint32_t on = __shfl_xor_sync(0xffffffffu, n, k);
                 better(v, n, ov, on);
             }
+            bar_sync<64>(BAR_FLAT);
             if (lane == 0) {
-                const uint32_t tok = n < a.vocab ? n : 0u;   // (no logit above -inf: 0)
+                const uint32_t tok = n < a.vocab && !flat_sm ? n : 0u;   // (no logit above -inf, or all 0: 0)
                 a.sampled[cta] = tok;
                 if (a.sampled_host) a.sampled_host[cta] = tok;
                 if (cta == (uint32_t)__ffs(live) - 1) {   // every SM has published its best, so has read them

@@ -75,6 +75,20 @@ def test_rows_that_are_not_finite(ak, ctx, slots):
     w.close()
 
 
+def test_sums_of_squares_that_overflow(ak, ctx):
+    """1 / rms is 0 there, so every logit is 0 and the first token is picked, as by the launch chain."""
+    cfg = ak.ModelConfig(997, 320, 5, 2, 96, 1280)
+    params = ak.synthetic_weights(cfg, seed=4, std=0.05)
+    params[0] *= np.float32(1e25)
+    w = ak.ModelWeights.from_params(ctx, cfg, params, ak.AK_BF16)
+    for slots in (3, 20):
+        prompts = [ak.uniform_tokens(4 + i, 997, seed=i) for i in range(slots)]
+        out = engine(ak, ctx, w, prompts, slots, 96, 6, False)
+        assert out == engine(ak, ctx, w, prompts, slots, 96, 6, True) and out == [[0] * 6] * slots
+    ctx.check_device_status()
+    w.close()
+
+
 def test_many_runs_give_the_same_tokens(ak, ctx):
     for dim, heads, slots, total in ((320, 5, 21, 512), (256, 2, 8, 620), (768, 12, 32, 512)):
         cfg = ak.ModelConfig(1000, dim, heads, 4, total, 4 * dim if dim > 300 else 1184)
