@@ -630,6 +630,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                     mine.advance(lane < NT ? lane : 0, slots);
                     const bool got = lane >= NT || wait_bar(&full_bar[mine.s], mine.ph, expiry);
                     alive = __all_sync(0xffffffffu, got && alive) != 0;
+                    __syncwarp();   // (a vote orders no memory: without this the lanes that do not wait may read before the weights are there)
 #pragma unroll
                     for (uint32_t t = 0; t < NT; t++) {
                         const uint32_t at = (q.s + t < slots ? q.s + t : q.s + t - slots) * SLOT + w_off;
