@@ -297,6 +297,7 @@ template <typename T> struct Block {
             got = wait_full(&rg.full[mine.s], mine.ph, dead);
         }
         got = __all_sync(0xffffffffu, got) != 0;
+        __syncwarp();   // (a vote orders no memory: without this the lanes that do not wait might read before the weights are there)
         if (n <= 8) {
 #pragma unroll
             for (int s = 0; s < PQ / 2; s++) load<2>(rg, d, n, warp + NW * s, 0, lane, w + 2 * s * WP);
