@@ -175,9 +175,9 @@ struct Kind {
     uint32_t t0, n, slices, chunks, pitch, pieces;   // pitch: bytes of a row in a slot; pieces of a chunk in the tensor map
     __device__ __forceinline__ uint32_t count(uint32_t c) const { return min(CHUNK, slices - c * CHUNK); }
 };
-__device__ __forceinline__ void make_kind(Kind& d, uint32_t rows, uint32_t k, uint32_t cta) {
-    d.t0 = tile_begin(div_up(rows, 8), cta);
-    d.n = tile_begin(div_up(rows, 8), cta + 1) - d.t0;
+__device__ __forceinline__ void make_kind(Kind& d, uint32_t rows, uint32_t k, uint32_t cta, uint32_t sms) {
+    d.t0 = tile_begin(div_up(rows, 8), cta, sms);
+    d.n = tile_begin(div_up(rows, 8), cta + 1, sms) - d.t0;
     d.slices = k >> 5;
     d.chunks = div_up(d.slices, CHUNK);
     d.pitch = chunk_cols(k) * 2;
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         failed_sm = *(const volatile uint32_t*)a.status;
         mbar_fence_init();
     }
-    if (tid >= 32 && tid < 32 + N_KINDS) make_kind(kinds[tid - 32], tid == 32 ? 3 * D : tid == 34 ? F : tid == 36 ? a.vocab : D, tid == 35 ? F : D, cta);
+    if (tid >= 32 && tid < 32 + N_KINDS) make_kind(kinds[tid - 32], tid == 32 ? 3 * D : tid == 34 ? F : tid == 36 ? a.vocab : D, tid == 35 ? F : D, cta, a.sms);
     if (warp_ == 2) {   // the rows' lengths, the rows by length (the longest first), the attention splits of the rows before by that rank
         const uint32_t n = lane < a.seqs ? min((uint32_t)max(a.rows ? a.kv_lens[lane] : a.lens[lane], 0), a.max_len) : 0u;
         uint32_t rank = 0;
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             uint4* p = reinterpret_cast<uint4*>(a.xch + set_of(g));
             const uint32_t n = (uint32_t)(so.total / 16);
 #pragma unroll 1
-            for (uint32_t i = cta * NHT + ht; i < n; i += B200_SMS * NHT) p[i] = make_uint4(EMPTY, EMPTY, EMPTY, EMPTY);
+            for (uint32_t i = cta * NHT + ht; i < n; i += a.sms * NHT) p[i] = make_uint4(EMPTY, EMPTY, EMPTY, EMPTY);
             bar_sync<NHT>(BAR_HELP);
             if (ht == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&a.state->cleared) : "memory");
         };
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 uint32_t n = 0, v;
                 Waiter w = wt;
                 do asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&a.state->cleared) : "memory");
-                while ((int32_t)(v - counted - clears * B200_SMS) < 0 && !w.give_up(n));
+                while ((int32_t)(v - counted - clears * a.sms) < 0 && !w.give_up(n));
             }
             __syncwarp();
         };
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     auto place_in = [&]() { return wpi == NW ? cw : cw & 3u; };
     {   // unit j in lane j: row | head << 6 | split << 18
         const uint32_t grp = group_of();
-        const uint32_t groups = B200_SMS * (NW / wpi), gid = grp * B200_SMS + cta;
+        const uint32_t groups = a.sms * (NW / wpi), gid = grp * a.sms + cta;
         const uint32_t u = lane * groups + ((lane & 1) ? groups - 1 - gid : gid);
         uint32_t unit = EMPTY;
         if (u < pre_sm[32] * H) {
@@ -996,7 +996,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         // rows of several splits, each (row, head) by one warp of the chip: after all of its own units, so that nobody waits for a unit behind a merge
         if (SPLIT) {
 #pragma unroll 1
-            for (uint32_t i = cw * B200_SMS + cta; i < n_act * H; i += NW * B200_SMS) {
+            for (uint32_t i = cw * a.sms + cta; i < n_act * H; i += NW * a.sms) {
                 const uint32_t row = by_len[i / H], head = i % H, n = len_sm[row], ns = div_up(n, SPLIT_LEN);
                 if (ns <= 1) break;   // (longest first)
                 const uint8_t* src = a.xch + set + so.part + (size_t)(row * H + head) * splits * (HD + 4) * 4;
@@ -1168,7 +1168,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             do {
                 lack = false;
 #pragma unroll
-                for (uint32_t k = 0; k < PER; k++) o[k] = lane + 32 * k < B200_SMS ? xld2(a.xch + fin + (cta * B200_SMS + lane + 32 * k) * 8) : make_uint2(0xff800000u, NO_LOGIT);
+                for (uint32_t k = 0; k < PER; k++) o[k] = lane + 32 * k < a.sms ? xld2(a.xch + fin + (cta * B200_SMS + lane + 32 * k) * 8) : make_uint2(0xff800000u, NO_LOGIT);
 #pragma unroll
                 for (uint32_t k = 0; k < PER; k++) lack = lack || o[k].x == EMPTY || o[k].y == EMPTY;
             } while (lack && !w.give_up(polls));
@@ -1188,7 +1188,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 if (a.sampled_host) a.sampled_host[cta] = tok;
                 if (cta == (uint32_t)__ffs(live) - 1) {   // every SM has published its best, so has read them
                     a.state->set = (e0 + L + 1) % SETS;
-                    a.state->counted += clears_of_step(L) * B200_SMS;
+                    a.state->counted += clears_of_step(L) * a.sms;
                 }
             }
         }
@@ -1252,8 +1252,8 @@ bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads,
 size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) { return sets_bytes(dim, ffn, heads, seqs, max_len); }
 
 int launch_batch(cudaStream_t st, const BatchArgs& a, uint32_t missing) {
-    const uint32_t blocks = B200_SMS - missing;
-    const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.seqs, a.max_len);
+    const uint32_t blocks = a.sms - missing;
+    const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.seqs, a.max_len, a.sms);
     const bool two = m_tiles(a.seqs) == 2, split = has_splits(a.max_len);
     if (a.dim / a.heads == 64) {
         if (split) return two ? launch_batch_t<64, 2, true>(st, a, p, blocks) : launch_batch_t<64, 1, true>(st, a, p, blocks);

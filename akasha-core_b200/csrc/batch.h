@@ -26,6 +26,7 @@ struct BatchArgs {
     uint32_t* status;            // device word: made non-zero when a wait runs out; a step that finds it so does nothing
     uint64_t max_cycles;         // time limit of the step, in SM clocks
     uint32_t n_layers, dim, ffn, heads, vocab, seqs, max_blocks, max_len;
+    uint32_t sms;                // blocks the step is divided over
     float eps, scale;
 };
 

@@ -16,7 +16,9 @@ namespace ak {
 namespace batch {
 
 constexpr uint32_t SMS = 148;             // one block per SM
+constexpr uint32_t SMS_BESIDE = 48;       // the fewest blocks of a step beside prompts
 constexpr uint32_t ROWS = 32;             // most sequences of a step
+static_assert(SMS_BESIDE >= ROWS, "block r picks the token of row r");
 constexpr uint32_t NW = 12;               // compute warps
 constexpr uint32_t NH = 3;                // epilogue warps
 constexpr uint32_t TB = 3;                // weight tiles of a pass (accumulators, partial sums)
@@ -30,7 +32,7 @@ constexpr uint32_t MAX_DYN_SMEM = 216 * 1024;
 
 AK_PLAN_FN constexpr uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 AK_PLAN_FN constexpr uint32_t m_tiles(uint32_t seqs) { return seqs <= 16 ? 1 : 2; }
-AK_PLAN_FN constexpr uint32_t tile_begin(uint32_t tiles, uint32_t cta) { return (tiles * cta) / SMS; }
+AK_PLAN_FN constexpr uint32_t tile_begin(uint32_t tiles, uint32_t cta, uint32_t sms) { return (tiles * cta) / sms; }   // of the step's sms blocks
 // Positions of an attention unit. Sequences of up to 512 are whole (no merging); longer ones are cut small, so that the groups' shares come out even: of
 // 16 sequences of up to 3200 positions a layer took 57 us in units of 512, with half of the SMs done after 31 us.
 AK_PLAN_FN constexpr bool has_splits(uint32_t max_len) { return max_len > 512; }
@@ -85,14 +87,14 @@ struct Plan {
     uint32_t slots, wpi;
     size_t smem;
 };
-inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len) {
+inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len, uint32_t sms = SMS) {
     const uint32_t hd = dim / heads;
-    const size_t rest = NW * 2 * KV_BUF + (size_t)NW * TB * m_tiles(seqs) * 16 * 32 + 2 * NW * hd * 4 + TB * 32 * 2 * 16 + (size_t)(2 * n_layers + 1) * div_up(dim / 8, SMS) * 32;
+    const size_t rest = NW * 2 * KV_BUF + (size_t)NW * TB * m_tiles(seqs) * 16 * 32 + 2 * NW * hd * 4 + TB * 32 * 2 * 16 + (size_t)(2 * n_layers + 1) * div_up(dim / 8, sms) * 32;
     Plan p;
     p.slots = (uint32_t)((MAX_DYN_SMEM - rest) / SLOT);
     if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
     p.smem = p.slots * SLOT + rest;
-    // Few units: all warps of an SM work on one; else four, so that an SM's units overlap.
+    // Few units: all warps of an SM work on one; else four, so that an SM's units overlap. (Not by the step's blocks: a unit's sums depend on it.)
     p.wpi = seqs * heads * div_up(max_len, split_len(max_len)) <= SMS ? 12 : 4;
     return p;
 }
@@ -137,6 +139,21 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
     const Plan p = make_plan(dim, n_layers, heads, seqs, max_len);
     if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * SMS * (NW / p.wpi)) return false;
     return p.slots >= 4 && sets_bytes(dim, ffn, heads, seqs, max_len) < (1ull << 32);
+}
+
+// SMs of a step with prompts beside it, whose chain of launches gets the others. The chain is the longer of the two in almost every such step, so the step
+// takes as few as its plan allows (what it computes does not depend on the number of its blocks). Jobs with prompts in most steps, ms: 162M model, 32
+// slots, prompts of 1 to 24, 8 tokens on average: step and chain one after the other on all SMs 39.3, beside each other on 90 SMs 34.9, 74
+// 33.1, 60 32.7, 48 30.7 (all rows through the chain, which shares its launches then: 31.2); 8 slots, prompts of 16 to 448, 2 tokens: 20.8, 19.2, 18.9,
+// 18.9, 18.5 (19.8); 320-wide model, 32 slots: 20.8, 16.7, 16.0, 15.9, 15.9 (17.2); 1.4B model (86 SMs at least), 16 slots, prompts of 1 to
+// 64, 4 tokens: 57.5, 55.8, 54.9 (53.9: both read all weights), prompts of 128 to 1024: 128.7, 129.3, 127.9 (128.8).
+inline uint32_t sms_beside(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len) {
+    const uint64_t units = (uint64_t)seqs * heads * div_up(max_len, split_len(max_len));
+    for (uint32_t sms = SMS_BESIDE; sms < SMS; sms++) {
+        const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms);
+        if (div_up(dim / 8, sms) <= TB && units <= (uint64_t)MAX_UNITS * sms * (NW / p.wpi) && p.slots >= 4) return sms;
+    }
+    return SMS;
 }
 
 }  // namespace batch

@@ -425,6 +425,7 @@ BatchArgs Runner::batch_args() const {
     a.max_cycles = BATCH_MAX_CYCLES;
     a.n_layers = c.num_layers; a.dim = c.dim; a.ffn = c.ffn_hidden; a.heads = c.num_heads; a.vocab = c.vocab_size;
     a.seqs = max_seqs_; a.max_blocks = max_blocks_; a.max_len = max_seq_len_;
+    a.sms = B200_SMS;
     a.eps = c.norm_eps;
     a.scale = 1.0f / sqrtf((float)(c.dim / c.num_heads));
     return a;
@@ -644,18 +645,24 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
         // A step of at most 128 rows (the decode rows plus one prompt chunk) is ONE row tile of every projection: the
         // prompt rows ride in the decode launches for free. Larger admission steps run the two kinds of rows as two
         // ranges on two streams.
-        if (batch_) {
-            // The persistent kernel takes the whole chip, so the prompt rows follow it. It samples the decode rows' tokens itself (their out_rows
-            // are -1); what comes after the ranges is for the prompts' last rows.
-            if (any_decode) {
+        if (batch_ && any_decode) {
+            // The decode rows' persistent kernel on some of the SMs, the prompt rows' chain on the others (first, so that its first launches find
+            // room). The kernel samples its tokens itself (the rows' out_rows are -1); what comes after the ranges is for the prompts' last rows.
+            AK_CUDA(cudaEventRecord(ev_fork_, st));
+            AK_CUDA(cudaStreamWaitEvent(st2_, ev_fork_, 0));
+            rc = range(st2_, max_seqs_, T - max_seqs_, false, true);
+            if (rc == AK_OK) {
                 BatchArgs a = batch_args();
                 a.rows = rows;
                 a.kv_lens = d_desc_ + d_.kv_lens;
-                RC(launch_batch(st, a));
-                batch_ran_ = !capturing;
+                a.sms = batch::sms_beside(c.dim, c.num_layers, c.num_heads, max_seqs_, max_seq_len_);
+                rc = launch_batch(st, a);
+                batch_ran_ = rc == AK_OK && !capturing;
             }
-            rc = range(st, max_seqs_, T - max_seqs_, false, true);
+            AK_CUDA(cudaEventRecord(ev_join_, st2_));   // (what was launched is waited for whatever failed)
+            AK_CUDA(cudaStreamWaitEvent(st, ev_join_, 0));
             if (rc) return rc;
+            trace_mark("batch");
         } else if (two_streams_ && any_decode && T > max_seqs_ && n_pf_seqs && T > 128) {
             AK_CUDA(cudaEventRecord(ev_fork_, st));
             AK_CUDA(cudaStreamWaitEvent(st2_, ev_fork_, 0));

@@ -18,11 +18,12 @@ CHECK = r"""
 #include <vector>
 #include "batch_plan.h"
 using namespace ak::batch;
+static uint32_t sms = SMS;   // blocks of the step
 struct Known {
     int clears[SMS], phase[SMS];   // (phase: 5 * layer + 0 qkv, 1 attention, 2 out-proj, 3 ffn-up, 4 ffn-down; -1: none)
-    Known() { memset(clears, 0, sizeof clears); for (uint32_t t = 0; t < SMS; t++) phase[t] = -1; }
+    Known() { memset(clears, 0, sizeof clears); for (uint32_t t = 0; t < sms; t++) phase[t] = -1; }
     void join(const Known& o) {
-        for (uint32_t t = 0; t < SMS; t++) {
+        for (uint32_t t = 0; t < sms; t++) {
             if (o.clears[t] > clears[t]) clears[t] = o.clears[t];
             if (o.phase[t] > phase[t]) phase[t] = o.phase[t];
         }
@@ -35,18 +36,18 @@ static int bad;
 static void look(const Known& k, int l, const char* what, uint32_t sm) {
     const int need = l + 3 - (int)SETS;   // clears: the one at the start, then one behind each ffn-up
     if (need <= 0) return;                // that content was a launch before
-    for (uint32_t t = 0; t < SMS; t++)
+    for (uint32_t t = 0; t < sms; t++)
         if (k.clears[t] < need) {
             if (!bad++) printf("layer %d %s on SM %u: SM %u has counted %d of %d clears\n", l, what, sm, t, k.clears[t], need);
             return;
         }
 }
-static uint32_t n_tiles(uint32_t rows, uint32_t sm) { return tile_begin(div_up(rows, 8), sm + 1) - tile_begin(div_up(rows, 8), sm); }
+static uint32_t n_tiles(uint32_t rows, uint32_t sm) { return tile_begin(div_up(rows, 8), sm + 1, sms) - tile_begin(div_up(rows, 8), sm, sms); }
 // publishers of columns [c0, c1) of a matrix's product
 static Known publishers(const std::vector<Known>& pub, uint32_t rows, uint32_t c0, uint32_t c1) {
     Known k;
-    for (uint32_t t = 0; t < SMS; t++) {
-        const uint32_t a = tile_begin(div_up(rows, 8), t) * 8, b = tile_begin(div_up(rows, 8), t + 1) * 8;
+    for (uint32_t t = 0; t < sms; t++) {
+        const uint32_t a = tile_begin(div_up(rows, 8), t, sms) * 8, b = tile_begin(div_up(rows, 8), t + 1, sms) * 8;
         if (a < c1 && c0 < b) k.join(pub[t]);
     }
     return k;
@@ -55,21 +56,22 @@ int main(int argc, char** argv) {
     if (argc < 7) return 2;
     dim = atoi(argv[1]); ffn = atoi(argv[2]); heads = atoi(argv[3]); L = atoi(argv[4]);
     const uint32_t rows = atoi(argv[5]), max_len = atoi(argv[6]);
-    counter = argc < 8 || atoi(argv[7]);
+    counter = argc < 9 || atoi(argv[8]);
+    if (argc >= 8 && atoi(argv[7])) sms = sms_beside(dim, L, heads, rows, max_len);
     if (!shape_supported(dim, ffn, heads, L, rows, max_len)) { printf("refused\n"); return 0; }
     const Plan p = make_plan(dim, L, heads, rows, max_len);
     std::vector<std::vector<Known>> w(SMS, std::vector<Known>(NW));   // compute warps
     std::vector<Known> e(SMS), freed(SMS), x1(SMS), qkv(SMS), x2(SMS), up(SMS);
     std::vector<Known> at(rows * heads);
-    for (uint32_t s = 0; s < SMS; s++) { freed[s] = e[s]; e[s].clears[s] = 1; x1[s] = e[s]; }   // embedding; the clear at the start
+    for (uint32_t s = 0; s < sms; s++) { freed[s] = e[s]; e[s].clears[s] = 1; x1[s] = e[s]; }   // embedding; the clear at the start
     const uint32_t n_of[4] = {3 * dim, dim, ffn, dim}, k_of[4] = {dim, dim, dim, ffn};
-    const uint32_t groups = SMS * (NW / p.wpi), splits = div_up(max_len, split_len(max_len));
+    const uint32_t groups = sms * (NW / p.wpi), splits = div_up(max_len, split_len(max_len));
     for (uint32_t l = 0; l < L; l++)
         for (uint32_t ph = 0; ph < 4; ph++) {
             if (ph == 1) {   // attention: every unit, its warps together; one publishes
                 std::vector<Known> part(rows * heads * splits);
                 for (uint32_t u = 0; u < rows * heads * splits; u++) {
-                    const uint32_t j = u / groups, x = u % groups, g = j & 1 ? groups - 1 - x : x, s = g % SMS, w0 = g / SMS * p.wpi, head = u / splits % heads;
+                    const uint32_t j = u / groups, x = u % groups, g = j & 1 ? groups - 1 - x : x, s = g % sms, w0 = g / sms * p.wpi, head = u / splits % heads;
                     Known all;
                     for (uint32_t i = w0; i < w0 + p.wpi; i++) {
                         look(w[s][i], l, "attention", s);
@@ -87,7 +89,7 @@ int main(int argc, char** argv) {
             std::vector<Known>& out = ph == 0 ? qkv : ph == 1 ? x2 : ph == 2 ? up : x1;
             const std::vector<Known> in = ph == 0 ? x1 : ph == 2 ? x2 : up;
             std::vector<Known> next(SMS);
-            for (uint32_t s = 0; s < SMS; s++) {
+            for (uint32_t s = 0; s < sms; s++) {
                 const uint32_t n = n_tiles(n_of[ph], s);
                 const int src = ph == 0 ? (int)l - 1 : (int)l;
                 if ((ph == 0 || ph == 2) && n) {   // sums of squares
@@ -95,7 +97,7 @@ int main(int argc, char** argv) {
                     e[s].join(publishers(in, dim, 0, dim));
                 }
                 if (ph == 1 && counter)
-                    for (uint32_t t = 0; t < SMS; t++)
+                    for (uint32_t t = 0; t < sms; t++)
                         if (e[s].clears[t] < (int)clears_before_out(l)) e[s].clears[t] = clears_before_out(l);
                 for (uint32_t b = 0; b < n; b += TB) {
                     for (uint32_t i = 0; i < NW; i++) {
@@ -113,7 +115,7 @@ int main(int argc, char** argv) {
                 if (n) { look(e[s], l, "publish", s); next[s].phase[s] = 5 * l + (ph ? ph + 1 : 0); }
                 if (ph == 2) {
                     // the set of layer l - 1 is cleared: who reads it (to the end: qkv of layer l) has published that phase, which is behind its reads
-                    for (uint32_t t = 0; t < SMS; t++) {
+                    for (uint32_t t = 0; t < sms; t++) {
                         const int last = n_tiles(3 * dim, t) ? 5 * (int)l : 5 * (int)(l - 1) + (n_tiles(dim, t) ? 4 : 3);
                         if (l && t != s && e[s].phase[t] < last) {
                             if (!bad++) printf("layer %u: SM %u clears the set of layer %u, SM %u is known to be through phase %d, not %d\n", l, s, l - 1, t, e[s].phase[t], last);
@@ -195,7 +197,8 @@ def plan(tmp_path_factory):
 @pytest.mark.parametrize("rows,max_len", [(1, 512), (8, 512), (16, 1200)])
 def test_sets_are_clean_and_unread(plan, dim, ffn, heads, rows, max_len):
     for layers in (1, 2, 3, 4, 7):
-        assert plan(dim, ffn, heads, layers, rows, max_len) == "ok"
+        for beside in (0, 1):
+            assert plan(dim, ffn, heads, layers, rows, max_len, beside) == "ok"
 
 
 def test_walk_stays_in_the_block_table(tmp_path_factory):

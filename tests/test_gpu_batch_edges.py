@@ -44,6 +44,31 @@ def test_every_sequence_is_the_oracles(ak, orc, ctx, slots, dim, heads, ffn, voc
     w.close()
 
 
+@pytest.mark.parametrize("slots,dim,heads,ffn,layers,total", [
+    (5, 320, 5, 1280, 3, 300), (20, 320, 5, 1280, 2, 700), (4, 768, 12, 3072, 2, 300), (3, 2048, 16, 8192, 1, 200), (16, 3072, 24, 3072, 1, 200)])
+def test_prompts_beside_the_step(ak, ctx, slots, dim, heads, ffn, layers, total):
+    """Steps with prompts run on fewer SMs: a sequence's tokens are those it has alone, with whole prompts and with chunks."""
+    cfg = ak.ModelConfig(997, dim, heads, layers, total, ffn)
+    w = ak.ModelWeights(ctx, cfg, ak.AK_BF16)
+    w.init_synthetic(5, 0.05)
+    prompts = [ak.uniform_tokens(1 + 29 * i % 150, 997, seed=i) for i in range(3 * slots)]
+    new = [1 + 7 * i % 12 for i in range(len(prompts))]
+    def job(which, chunk):
+        e = ak.Engine(ctx, w, max_seqs=slots, max_seq_len=total, async_steps=True, prefill_chunk_rows=chunk)
+        ids = [e.submit(prompts[i], len(prompts[i]) + new[i]) for i in which]
+        e.run_to_completion()
+        out = [e.poll(i)[0].tolist() for i in ids]
+        e.close()
+        return out
+    everything = range(len(prompts))
+    out = job(everything, 0)
+    assert job(everything, 0) == out and job(everything, 24) == out
+    for i in list(everything)[:: max(1, slots // 3)]:
+        assert job([i], 0) == [out[i]], i
+    ctx.check_device_status()
+    w.close()
+
+
 def engine(ak, ctx, w, prompts, slots, total, new, chain):
     e = ak.Engine(ctx, w, max_seqs=slots, max_seq_len=total, attn_timing=chain)   # with attn_timing a step is a chain of launches
     ids = [e.submit(p, len(p) + new) for p in prompts]
