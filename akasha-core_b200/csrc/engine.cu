@@ -223,8 +223,9 @@ int ak_engine_step(ak_engine* e, uint32_t* n_running, uint32_t* n_waiting) {
     // Whole prompts (as many as fit the step budget) when nobody is decoding or a lot of prompt is pending. Otherwise
     // chunks: while other sequences decode, a prompt is prefilled `chunk_rows` rows per step, so that decode rows and
     // prompt rows together stay within ONE 128-row tile of every projection and the prompt rides in the decode
-    // launches; its sequence samples its first token in the step that holds its last chunk. Chunk boundaries depend on
-    // the prompt alone, and a row's arithmetic does not depend on which rows share its launch.
+    // launches (or, beside a persistent decode step, its own chain stays short); its sequence samples its first token in the
+    // step that holds its last chunk. Chunk boundaries depend on the prompt alone, and a row's arithmetic does not
+    // depend on which rows share its launch.
     bool decoding_now = false;
     for (uint32_t i = 0; i < S; i++) decoding_now |= (e->slots[i] && !e->slots[i]->finished && !e->slots[i]->in_prefill);
     uint64_t pending_rows = 0;
@@ -363,7 +364,7 @@ int ak_engine_step(ak_engine* e, uint32_t* n_running, uint32_t* n_waiting) {
     e->stats.steps++;
     e->stats.decode_tokens += n_dec;
     e->stats.prefill_tokens += pf_rows;
-    if (graph) e->stats.graph_launches++; else e->stats.eager_steps++;
+    if (graph && !(r.batch() && pf_rows == 0)) e->stats.graph_launches++; else e->stats.eager_steps++;   // (the latter: one launch)
     e->stats.kernel_launches += (g_launch_count - launches0);
     e->stats.h2d_bytes = r.h2d_bytes;
     e->stats.launch_host_ms_total = r.launch_host_ms - e->launch_host_base;

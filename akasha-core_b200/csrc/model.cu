@@ -642,9 +642,9 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
             }
             return AK_OK;
         };
-        // A step of at most 128 rows (the decode rows plus one prompt chunk) is ONE row tile of every projection: the
-        // prompt rows ride in the decode launches for free. Larger admission steps run the two kinds of rows as two
-        // ranges on two streams.
+        // In a launch chain a step of at most 128 rows (the decode rows plus one prompt chunk) is ONE row tile of every
+        // projection: the prompt rows ride in the decode launches for free. Larger admission steps run the two kinds of rows as
+        // two ranges on two streams.
         if (batch_ && any_decode) {
             // The decode rows' persistent kernel on some of the SMs, the prompt rows' chain on the others (first, so that its first launches find
             // room). The kernel samples its tokens itself (the rows' out_rows are -1); what comes after the ranges is for the prompts' last rows.
@@ -817,7 +817,6 @@ int Runner::capture_step(uint64_t key, uint32_t T, uint32_t rows_b, uint32_t seq
     AK_CUDA(cudaGraphInstantiate(&g.exec, graph, 0));
     cudaGraphDestroy(graph);
     graphs_[key] = g;
-    if ((key << 1) == 0) graph_kernels = g.kernels;
     return AK_OK;
 }
 

@@ -143,7 +143,6 @@ class Runner {
     double launch_host_ms = 0.0;       // host time spent inside cudaGraphLaunch, accumulated
     uint64_t graph_launches = 0, eager_steps = 0;
     uint64_t h2d_bytes = 0, d2h_bytes = 0;   // bytes copied by run() / run_decode_graph()
-    uint64_t graph_kernels = 0;              // kernel launches recorded in the captured decode step
 
    private:
     int launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, uint32_t max_pf_len, bool any_decode, uint32_t n_splits, bool capturing);

@@ -366,10 +366,11 @@ typedef struct ak_engine_config {
     uint32_t kv_blocks;        /* KV pool size in blocks (0 = max_seqs * ceil(max_seq_len/16)) */
     uint32_t block_size;       /* must be 16 */
     uint32_t max_batch_tokens; /* token budget of one step (prefill + decode rows)  */
-    uint32_t use_cuda_graph;   /* capture the decode-only step in a CUDA graph      */
+    uint32_t use_cuda_graph;   /* capture steps in CUDA graphs, one per shape (a decode-only step that is one kernel is launched as such) */
     uint32_t stop_on_eos;      /* 0: run every sequence to its max_len              */
-    uint32_t attn_timing;      /* record CUDA events around layer 0's decode attention (which is then a launch of its own also with up
-                                  to 32 slots, where a decode step is otherwise one kernel) */
+    uint32_t attn_timing;      /* record CUDA events around layer 0's decode attention and the captured steps. With bf16 weights and up to
+                                * 32 slots a decode step is otherwise one kernel; with this it is the launch chain of larger
+                                * engines, whose sums are in another order (tokens may differ where two logits are all but equal) */
     uint32_t async_steps;      /* 1: ak_engine_step returns once step N is LAUNCHED and step N-1's tokens are on the
                                 * host, so describing and launching a step overlaps the previous step's GPU time.
                                 * Needs stop_on_eos == 0 (sequence ends must be known without the tokens);
@@ -379,7 +380,8 @@ typedef struct ak_engine_config {
                                   * admits it. N > 0: while other sequences are decoding, an admitted prompt is prefilled N rows
                                   * per step and its sequence samples its first token in the step that holds its last chunk; with
                                   * max_seqs + N <= 128 decode rows and prompt rows share ONE 128-row tile of every projection and
-                                  * the prompt rides in the decode launches (no step is stretched by a long prompt). Needs bf16
+                                  * the prompt rides in the decode launches (no step is stretched by a long prompt); where the decode
+                                  * step is one kernel the chunk's launches run beside it. Needs bf16
                                   * weights, head_dim 64 or 128, no tensor parallelism; ignored otherwise. Tokens per sequence are
                                   * the same either way; admission times, hence block tables, differ. With nobody decoding, or more
                                   * than 8 chunks of prompt pending, prompts are prefilled whole. */
@@ -410,7 +412,9 @@ AK_API int ak_engine_clear_finished(ak_engine* e);
  * its blocks, so that the other blocks' waits run out, `cycles` SM clocks after its start. */
 AK_API int ak_engine_drill_wait(ak_engine* e, uint64_t cycles);
 typedef struct ak_engine_stats {
-    uint64_t steps, decode_tokens, prefill_tokens, graph_launches, eager_steps, kernel_launches;
+    uint64_t steps, decode_tokens, prefill_tokens;
+    uint64_t graph_launches, eager_steps; /* steps as a graph (with use_cuda_graph), and launch by launch or as one kernel */
+    uint64_t kernel_launches;
     double attn_ms_total;        /* sum of timed layer-0 decode-attention launches (attn_timing) */
     uint64_t attn_launches_timed;
     uint64_t attn_bytes_total;   /* algorithmic bytes of those launches */

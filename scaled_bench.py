@@ -51,8 +51,10 @@ def main():
     mine = list(range(n_seqs)) if tp > 1 else sharding.shard_round_robin(n_seqs, rank, world)
     prompts = [ak.uniform_tokens(int(lens[i]), cfg.vocab_size, seed=50_000 + i) for i in mine]
     max_len = 3072 + gen
+    # up to 32 slots a decode step is one kernel, unless its attention is to be timed
+    timing = max_seqs > 32 or tp > 1
     eng = ak.Engine(ctx, w, max_seqs=max_seqs, max_seq_len=max_len, max_batch_tokens=max_seqs + 16384,
-                    use_cuda_graph=True, attn_timing=True, async_steps=(tp == 1))
+                    use_cuda_graph=True, attn_timing=timing, async_steps=(tp == 1))
 
     def job():
         ids = [eng.submit(p, len(p) + gen) for p in prompts]
@@ -86,10 +88,10 @@ def main():
             "mode": f"tp{tp}" if tp > 1 else f"dp{world}", "n_gpus": world, "generated_tokens": units, "seconds": secs,
             "tok/s": thr, "prompt_tokens_rank0": int(sum(len(p) for p in prompts)),
             "rank0": {"steps": st["steps"], "decode_tokens": st["decode_tokens"], "prefill_tokens": st["prefill_tokens"],
-                      "attn_GB/s": st["attn_bytes_total"] / max(1e-9, st["attn_ms_total"] * 1e-3) / 1e9,
-                      "attn_us_layer0": 1e3 * st["attn_ms_total"] / max(1, st["attn_launches_timed"]),
+                      "attn_GB/s": st["attn_bytes_total"] / max(1e-9, st["attn_ms_total"] * 1e-3) / 1e9 if timing else None,
+                      "attn_us_layer0": 1e3 * st["attn_ms_total"] / max(1, st["attn_launches_timed"]) if timing else None,
                       # where rank 0's time goes: device time of its steps, host time spent launching them
-                      "gpu_ms_total": st["step_gpu_ms_total"], "launch_host_ms_total": st["launch_host_ms_total"]}}))
+                      "gpu_ms_total": st["step_gpu_ms_total"] if timing else None, "launch_host_ms_total": st["launch_host_ms_total"]}}))
     eng.close(); w.close(); ctx.close()
     if world > 1:
         dist.barrier()

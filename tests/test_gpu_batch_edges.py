@@ -131,3 +131,22 @@ def test_many_runs_give_the_same_tokens(ak, ctx):
             want = out
         e.close(); w.close()
     ctx.check_device_status()
+
+
+def test_steps_are_counted_as_they_are_launched(ak, ctx):
+    """A decode-only step of the persistent kernel is one launch and no graph, a step with prompts is a graph."""
+    cfg = ak.ModelConfig(997, 320, 5, 2, 96, 1280)
+    w = ak.ModelWeights(ctx, cfg, ak.AK_BF16)
+    w.init_synthetic(3, 0.05)
+    for async_steps in (False, True):
+        e = ak.Engine(ctx, w, max_seqs=4, max_seq_len=96, use_cuda_graph=True, async_steps=async_steps)
+        for rep in range(2):
+            for i in range(4):
+                e.submit(ak.uniform_tokens(5, 997, seed=i), 25)
+            e.run_to_completion()
+            st = e.stats()
+            e.reset_stats()
+            assert (st["steps"], st["graph_launches"], st["eager_steps"]) == (20, 1, 19)
+        assert st["kernel_launches"] <= 19 + 30
+        e.close()
+    w.close()
