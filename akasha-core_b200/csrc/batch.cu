@@ -6,9 +6,9 @@
 // batch-1 step (solo.cu), a layer is five phases of one kernel and only activations cross the chip:
 //   qkv rows -> attention (sequence, head) -> out-proj rows -> ffn-up rows -> ffn-down rows.
 // That step takes 0.187 ms (1 sequence 0.17, 16 of 350 0.25, 32 of 350 0.334; 320-wide model, 21 sequences 0.22 -> 0.127; 1.4B model, 16 of 1600
-// 2.5 -> 2.1). With 64 sequences an early form was slower than the chain (every SM reads all activations: 0.58 against 0.49 ms), hence the limit of 32.
-// What is left is latency: per phase ~1 us from a store to the last SM's poll and ~1 us of dependent instructions, ~5 cycles each (with
-// everything between two phases done by the same warps it was 0.29 ms; with 40 bytes of spills 0.36).
+// 2.5 -> 2.1). With 64 sequences a form of it (since deleted) was slower than the chain: every SM reads all activations, 0.58 against 0.49 ms. Hence the
+// limit of 32. What is left is latency: per phase the way from a store to the last SM's poll, and dependent instructions (with everything
+// between two phases done by the same warps it was 0.29 ms).
 //   * A producer thread per SM walks the SM's weight tiles of all phases in order and keeps a shared-memory ring of tensor loads full.
 //   * A phase's rows are dealt to the SMs in tiles of 8, all of K: no sum crosses SMs. The 12 compute warps split K and leave partial tiles in
 //     shared memory; three epilogue warps add them in warp order and publish, while the compute warps are already at the next phase. The
@@ -16,7 +16,7 @@
 //     operands through shared memory, the result back through tensor memory) costs more latency than these few products take.
 //   * Activations are published in the order of the MMA's A fragments (a lane's 8 consecutive k of a sequence are one 16-byte vector), so
 //     that a warp's fragment is one coalesced 512-byte load from L2 straight into registers. Both operands use the same order of k. What a
-//     tile publishes for 8 sequences is one 128-byte line (as 16-byte pieces of four lines: 1.6 us instead of 0.95 until the last SM had it).
+//     tile publishes for 8 sequences is one 128-byte line.
 //   * A value is its own flag: an exchange buffer holds 0xffffffff words until it is written, a NaN no conversion and no arithmetic
 //     gives, and consumers poll the words they need. No fence and no second round trip between the value and its flag. Four sets of
 //     buffers are used in turn by the layers; the one of the layer before is filled with 0xff again after a layer's ffn-up (see clear).
@@ -222,7 +222,8 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     float* const at_acc = part + NW * TB * R * 8;                                 // [2][NW][HD]
     float4* const res_sm = reinterpret_cast<float4*>(at_acc + 2 * NW * HD);       // [tile][R][2]: the residual stream of this SM's columns
     float* const gain_sm = reinterpret_cast<float*>(res_sm + TB * R * 2);                // [2 L + 1][tiles][8]: the gains of its columns, by norm
-    const uint32_t SPLIT_LEN = unit_len(SPLIT), splits = div_up(a.max_len, SPLIT_LEN);
+    constexpr uint32_t SPLIT_LEN = unit_len(SPLIT, HD);
+    const uint32_t splits = div_up(a.max_len, SPLIT_LEN);
 
     if (tid == 160) so = SetOff(D, F, H, MT, splits);
     if (tid == 0) {
@@ -1254,7 +1255,7 @@ size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seq
 int launch_batch(cudaStream_t st, const BatchArgs& a, uint32_t missing) {
     const uint32_t blocks = a.sms - missing;
     const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.seqs, a.max_len, a.sms);
-    const bool two = m_tiles(a.seqs) == 2, split = has_splits(a.max_len);
+    const bool two = m_tiles(a.seqs) == 2, split = has_splits(a.max_len, a.dim / a.heads);
     if (a.dim / a.heads == 64) {
         if (split) return two ? launch_batch_t<64, 2, true>(st, a, p, blocks) : launch_batch_t<64, 1, true>(st, a, p, blocks);
         return two ? launch_batch_t<64, 2, false>(st, a, p, blocks) : launch_batch_t<64, 1, false>(st, a, p, blocks);

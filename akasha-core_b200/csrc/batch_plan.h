@@ -33,11 +33,14 @@ constexpr uint32_t MAX_DYN_SMEM = 216 * 1024;
 AK_PLAN_FN constexpr uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 AK_PLAN_FN constexpr uint32_t m_tiles(uint32_t seqs) { return seqs <= 16 ? 1 : 2; }
 AK_PLAN_FN constexpr uint32_t tile_begin(uint32_t tiles, uint32_t cta, uint32_t sms) { return (tiles * cta) / sms; }   // of the step's sms blocks
-// Positions of an attention unit. Sequences of up to 512 are whole (no merging); longer ones are cut small, so that the groups' shares come out even: of
-// 16 sequences of up to 3200 positions a layer took 57 us in units of 512, with half of the SMs done after 31 us.
-AK_PLAN_FN constexpr bool has_splits(uint32_t max_len) { return max_len > 512; }
-AK_PLAN_FN constexpr uint32_t unit_len(bool splits) { return splits ? 256 : 512; }
-AK_PLAN_FN constexpr uint32_t split_len(uint32_t max_len) { return unit_len(has_splits(max_len)); }
+// Positions of an attention unit. Where all sequences fit in 128 KB of keys (1024 positions of head size 64, 512 of 128) they are whole, which saves
+// publishing and merging; longer ones are cut into 256 positions, so that the groups' shares come out even. Jobs of 30 to 40 steps near the
+// capacity, ms, cut / whole: 162M model 8 slots, 520 positions 9.70 / 9.18, 768 10.31 / 9.82, 1024 11.32 / 11.10, 2048 16.3 / 15.3; 32 slots, 768 23.5 / 21.5,
+// 1024 28.1 / 25.8, 2048 46.7 / 44.1; 320-wide model 21 slots, 1024 7.83 / 7.75, 4 slots, 2048 6.11 / 7.19; 1.4B model (head size 128) 4 slots, 1024
+// 38.7 / 39.1, 16 slots, 1024 89.0 / 90.0, 2048 148 / 160. In units of 512 instead of 256: 0.92 to 1.06 of the speed; of 128: 0.87 to 1.03.
+AK_PLAN_FN constexpr uint32_t unit_len(bool splits, uint32_t hd) { return splits ? 256 : 65536 / hd; }
+AK_PLAN_FN constexpr bool has_splits(uint32_t max_len, uint32_t hd) { return max_len > unit_len(false, hd); }
+AK_PLAN_FN constexpr uint32_t split_len(uint32_t max_len, uint32_t hd) { return unit_len(has_splits(max_len, hd), hd); }
 // A weight row as pieces of the tensor map: 256 columns, or what divides the row
 AK_PLAN_FN constexpr uint32_t piece_of(uint32_t k) { return k % 256 == 0 ? 256 : k % 64 == 0 ? 64 : 32; }
 AK_PLAN_FN constexpr uint32_t chunk_cols(uint32_t k) { return k < CHUNK * 32 ? k : CHUNK * 32; }
@@ -80,7 +83,7 @@ struct State {
 };
 
 inline size_t sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) {
-    return (SETS * SetOff(dim, ffn, heads, m_tiles(seqs), div_up(max_len, split_len(max_len))).total + 127) / 128 * 128;
+    return (SETS * SetOff(dim, ffn, heads, m_tiles(seqs), div_up(max_len, split_len(max_len, dim / heads))).total + 127) / 128 * 128;
 }
 
 struct Plan {
@@ -95,7 +98,7 @@ inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t 
     if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
     p.smem = p.slots * SLOT + rest;
     // Few units: all warps of an SM work on one; else four, so that an SM's units overlap. (Not by the step's blocks: a unit's sums depend on it.)
-    p.wpi = seqs * heads * div_up(max_len, split_len(max_len)) <= SMS ? 12 : 4;
+    p.wpi = seqs * heads * div_up(max_len, split_len(max_len, hd)) <= SMS ? 12 : 4;
     return p;
 }
 
@@ -135,7 +138,7 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
     if (ffn / 8 < SMS) return false;                                       // every SM has ffn-up rows (the clearing of the sets counts on it)
     if (div_up(dim / 8, SMS) > TB) return false;                           // the residual stream is worked on in one pass
     if (dim * m_tiles(seqs) * 16 * 2 > NW * 2 * KV_BUF) return false;      // the lm_head keeps x where the cache tiles were
-    const uint32_t splits = div_up(max_len, split_len(max_len));
+    const uint32_t splits = div_up(max_len, split_len(max_len, hd));
     const Plan p = make_plan(dim, n_layers, heads, seqs, max_len);
     if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * SMS * (NW / p.wpi)) return false;
     return p.slots >= 4 && sets_bytes(dim, ffn, heads, seqs, max_len) < (1ull << 32);
@@ -148,7 +151,7 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
 // 18.9, 18.5 (19.8); 320-wide model, 32 slots: 20.8, 16.7, 16.0, 15.9, 15.9 (17.2); 1.4B model (86 SMs at least), 16 slots, prompts of 1 to
 // 64, 4 tokens: 57.5, 55.8, 54.9 (53.9: both read all weights), prompts of 128 to 1024: 128.7, 129.3, 127.9 (128.8).
 inline uint32_t sms_beside(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len) {
-    const uint64_t units = (uint64_t)seqs * heads * div_up(max_len, split_len(max_len));
+    const uint64_t units = (uint64_t)seqs * heads * div_up(max_len, split_len(max_len, dim / heads));
     for (uint32_t sms = SMS_BESIDE; sms < SMS; sms++) {
         const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms);
         if (div_up(dim / 8, sms) <= TB && units <= (uint64_t)MAX_UNITS * sms * (NW / p.wpi) && p.slots >= 4) return sms;

@@ -65,7 +65,7 @@ int main(int argc, char** argv) {
     std::vector<Known> at(rows * heads);
     for (uint32_t s = 0; s < sms; s++) { freed[s] = e[s]; e[s].clears[s] = 1; x1[s] = e[s]; }   // embedding; the clear at the start
     const uint32_t n_of[4] = {3 * dim, dim, ffn, dim}, k_of[4] = {dim, dim, dim, ffn};
-    const uint32_t groups = sms * (NW / p.wpi), splits = div_up(max_len, split_len(max_len));
+    const uint32_t groups = sms * (NW / p.wpi), splits = div_up(max_len, split_len(max_len, dim / heads));
     for (uint32_t l = 0; l < L; l++)
         for (uint32_t ph = 0; ph < 4; ph++) {
             if (ph == 1) {   // attention: every unit, its warps together; one publishes
@@ -194,7 +194,7 @@ def plan(tmp_path_factory):
 
 # dim 96 .. 320: SMs without rows of qkv, out-proj and ffn-down, warps without a slice of x; 768 and 2048: every SM has all kinds of rows
 @pytest.mark.parametrize("dim,ffn,heads", [(128, 1184, 1), (256, 1216, 2), (320, 1280, 5), (768, 3072, 12), (1280, 2560, 10), (2048, 8192, 16)])
-@pytest.mark.parametrize("rows,max_len", [(1, 512), (8, 512), (16, 1200)])
+@pytest.mark.parametrize("rows,max_len", [(1, 512), (8, 1024), (16, 1200)])
 def test_sets_are_clean_and_unread(plan, dim, ffn, heads, rows, max_len):
     for layers in (1, 2, 3, 4, 7):
         for beside in (0, 1):

@@ -15,7 +15,10 @@ TILES = (127, 128, 129, 255, 383, 385, 480, 500)   # around the 4 and 12 tiles o
     (32, 320, 5, 1280, 997, 2, 512, (TILES + EDGES) * 2),               # four warps a unit; rows 16 .. 31 in the second tile of rows
     (8, 256, 2, 1184, 997, 2, 512, TILES),                              # the same for head size 128
     (32, 640, 5, 1280, 997, 2, 512, EDGES + TILES + TILES[:8]),
-    (32, 320, 5, 1280, 997, 2, 620, LONG * 3),                          # splits with 32 slots
+    (32, 320, 5, 1280, 997, 2, 1024, LONG * 2 + (1000, 1010, 800) + EDGES[:9]),   # the longest whole sequences of head size 64
+    (4, 320, 5, 1280, 997, 2, 1040, (1018, 1030, 767, 300)),            # splits from there on, with one tile of rows and with two
+    (32, 320, 5, 1280, 997, 2, 1200, LONG * 2 + (1000, 1024, 1100) + EDGES[:9]),
+    (32, 256, 2, 1184, 997, 2, 620, LONG * 3),                          # for head size 128 from 512 on
     (4, 320, 5, 1280, 997, 1, 96, (1, 16, 33, 60)),                     # one layer: a set is used again two steps later
     (6, 2048, 16, 8192, 997, 2, 96, (1, 16, 33, 48, 7, 12)),            # two tiles of the residual stream on an SM, K of several ring chunks
     (5, 2048, 16, 8192, 1000, 1, 700, (1, 255, 257, 600, 33)),
@@ -45,7 +48,7 @@ def test_every_sequence_is_the_oracles(ak, orc, ctx, slots, dim, heads, ffn, voc
 
 
 @pytest.mark.parametrize("slots,dim,heads,ffn,layers,total", [
-    (5, 320, 5, 1280, 3, 300), (20, 320, 5, 1280, 2, 700), (4, 768, 12, 3072, 2, 300), (3, 2048, 16, 8192, 1, 200), (16, 3072, 24, 3072, 1, 200)])
+    (5, 320, 5, 1280, 3, 300), (20, 320, 5, 1280, 2, 1100), (4, 768, 12, 3072, 2, 300), (3, 2048, 16, 8192, 1, 200), (16, 3072, 24, 3072, 1, 200)])
 def test_prompts_beside_the_step(ak, ctx, slots, dim, heads, ffn, layers, total):
     """Steps with prompts run on fewer SMs: a sequence's tokens are those it has alone, with whole prompts and with chunks."""
     cfg = ak.ModelConfig(997, dim, heads, layers, total, ffn)
@@ -115,7 +118,7 @@ def test_sums_of_squares_that_overflow(ak, ctx):
 
 
 def test_many_runs_give_the_same_tokens(ak, ctx):
-    for dim, heads, slots, total in ((320, 5, 21, 512), (256, 2, 8, 620), (768, 12, 32, 512), (768, 12, 32, 768), (320, 5, 32, 768), (256, 2, 20, 768)):
+    for dim, heads, slots, total in ((320, 5, 21, 512), (256, 2, 8, 620), (768, 12, 32, 512), (768, 12, 32, 1200), (320, 5, 32, 1200), (320, 5, 9, 1200), (256, 2, 20, 768)):
         cfg = ak.ModelConfig(1000, dim, heads, 4, total, 4 * dim if dim > 300 else 1184)
         w = ak.ModelWeights(ctx, cfg, ak.AK_BF16)
         w.init_synthetic(3, 0.05)

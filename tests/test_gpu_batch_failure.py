@@ -59,7 +59,7 @@ def child(shape, more=""):
 
 
 # one and two tiles of rows, with and without splits, SMs with all and with few kinds of rows
-SHAPES = [(320, 5, 1280, 2, 3, 96, True), (256, 2, 1184, 3, 20, 700, False), (768, 12, 3072, 2, 8, 512, True), (512, 4, 2048, 2, 32, 96, False)]
+SHAPES = [(320, 5, 1280, 2, 3, 96, True), (256, 2, 1184, 3, 20, 700, False), (768, 12, 3072, 2, 8, 512, True), (512, 4, 2048, 2, 32, 96, False), (320, 5, 1280, 2, 20, 1100, True)]
 
 
 def test_the_engine_takes_no_further_step():
