@@ -65,6 +65,9 @@ int launch_gemm_f32(cudaStream_t st, const float* a, const float* b, float* c, u
 // C[m,n] (+)= A[m,k] @ Wt[n,k]^T, row-major f32 (gemm_f32_nt.cu): the runner's f32 projections, stored [out,in]. A row's sum does not
 // depend on m, except with GEMM_ALONE: the row never shares a launch, so that m == 1 may be a GEMV (another order of sums).
 int launch_gemm_f32_nt(cudaStream_t st, const float* a, const float* wt, float* c, uint32_t m, uint32_t n, uint32_t k, uint32_t flags);
+// gemm_f32_tc.cu: the same product from split operands on the tensor cores (16-byte rows and operands)
+int launch_gemm_f32_tc(cudaStream_t st, const float* a, const float* wt, float* c, uint32_t m, uint32_t n, uint32_t k, uint32_t flags);
+int gemm_f32_tc_status(unsigned int* out);
 
 // ---- gemm_tcgen05.cu (bf16 tensor cores) --------------------------------------------------------
 // invariant: keep the K summation structure a function of (n, k) only, so a row's result is the

@@ -172,6 +172,9 @@ int ak_check_device_status(void* stream) {
     rc = prefill_tc_status(&v);
     if (rc) return rc;
     AK_REQUIRE(v == 0, AK_ERR_DEVICE_WAIT, "attn_prefill (tensor cores): a bounded device-side wait expired (code %u)", v);
+    rc = gemm_f32_tc_status(&v);
+    if (rc) return rc;
+    AK_REQUIRE(v == 0, AK_ERR_DEVICE_WAIT, "f32 product (tensor cores): a bounded device-side wait expired (code %u)", v);
     rc = solo_status(&v);
     if (rc) return rc;
     AK_REQUIRE(v == 0, AK_ERR_DEVICE_WAIT, "batch-1 decode step: a bounded device-side wait expired (code %u)", v);

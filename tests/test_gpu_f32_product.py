@@ -1,0 +1,78 @@
+"""GPU: the f32 product from split operands on the tensor cores (csrc/gemm_f32_tc.cu), through prompts of f32 sessions against 64-bit arithmetic."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def forward64(cfg, params, toks):
+    """Keys and values of every layer and the last row's logits, in float64."""
+    import torch
+    P = [torch.from_numpy(np.asarray(p)).double() for p in params]
+    D, H, L = cfg.dim, cfg.num_heads, cfg.num_layers
+    hd, n = D // H, len(toks)
+    norm = lambda x, g: x / torch.sqrt((x * x).mean(-1, keepdim=True) + cfg.norm_eps) * g
+    freq = 1.0 / torch.pow(torch.tensor(10000.0), torch.arange(0, hd, 2, dtype=torch.float32) / hd)
+    ang = (torch.arange(n, dtype=torch.float32)[:, None] * freq[None]).double()
+    cs, sn = torch.cos(ang)[:, None], torch.sin(ang)[:, None]
+    def rope(x):
+        a, b = x[..., 0::2], x[..., 1::2]
+        return torch.stack((a * cs - b * sn, a * sn + b * cs), -1).reshape(x.shape)
+    h = P[0][torch.from_numpy(np.asarray(toks).astype(np.int64))]
+    mask = torch.ones(n, n, dtype=torch.bool).tril()
+    ks, vs = [], []
+    for l in range(L):
+        n1, qkv, out, n2, up, down = P[1 + 6 * l:7 + 6 * l]
+        q, k, v = (norm(h, n1) @ qkv).reshape(n, 3, H, hd).unbind(1)
+        q, k = rope(q), rope(k)
+        s = torch.einsum("ihd,jhd->hij", q, k) / np.sqrt(hd)
+        p = torch.softmax(s.masked_fill(~mask, -np.inf), -1)
+        h = h + torch.einsum("hij,jhd->ihd", p, v).reshape(n, D) @ out
+        u = norm(h, n2) @ up
+        h = h + (u * torch.sigmoid(u)) @ down
+        ks.append(k.reshape(n, D).numpy())
+        vs.append(v.reshape(n, D).numpy())
+    return ks, vs, (norm(h[-1:], P[1 + 6 * L]) @ P[2 + 6 * L])[0].numpy()
+
+
+# K of one block and of several, not a multiple of a block (64) nor of a half (32); one segment to five, in one group and in two; columns that end inside
+# a tile; rows at the edges of the 128-row tile and of the eight rows a warp splits
+@pytest.mark.parametrize("dim,heads,ffn,vocab", [(64, 1, 100, 33), (132, 3, 260, 129), (320, 5, 1280, 997), (768, 12, 3072, 1000), (1088, 17, 36, 64)])
+def test_prompt_against_64_bits(ak, ctx, dim, heads, ffn, vocab):
+    cfg = ak.ModelConfig(vocab, dim, heads, 2, 600, ffn)
+    params = ak.synthetic_weights(cfg, seed=dim, std=0.05)
+    w = ak.ModelWeights.from_params(ctx, cfg, params, ak.AK_F32)
+    s = ak.InferenceSession(ctx, w, 600)
+    for n in (1, 2, 9, 63, 127, 128, 129, 300, 520):
+        toks = ak.uniform_tokens(n, vocab, seed=n)
+        ks, vs, want = forward64(cfg, params, toks)
+        s.replace_cache()
+        logits, _ = s.prefill(toks)
+        # Sums of up to 3072 terms, each rounded to 2^-24 of a partial sum a few dozen times: 2e-7 in the norm; about ten such products one behind another
+        err = lambda a, b: np.linalg.norm(np.asarray(a, np.float64).ravel() - b.ravel()) / np.linalg.norm(b)
+        for l in range(2):
+            k, v = s.read_cache(l)
+            assert err(k, ks[l]) < 2e-6 and err(v, vs[l]) < 2e-6, (n, l)
+        assert err(logits, want) < 2e-6, n
+    ctx.check_device_status()
+    s.close(); w.close()
+
+
+def test_rows_that_are_not_finite(ak, ctx):
+    """Rows before an infinite one are what they are without it; the row itself is not finite (its norm has no value)."""
+    cfg = ak.ModelConfig(50, 320, 5, 1, 200, 1280)
+    params = ak.synthetic_weights(cfg, seed=2, std=0.05)
+    params[0][7, 3] = np.inf
+    w = ak.ModelWeights.from_params(ctx, cfg, params, ak.AK_F32)
+    s = ak.InferenceSession(ctx, w, 200)
+    toks = 8 + ak.uniform_tokens(150, 42, seed=1)
+    s.replace_cache(); s.prefill(toks)
+    clean = s.read_cache(0)
+    toks[130] = 7
+    s.replace_cache(); s.prefill(toks)
+    for a, b in zip(clean, s.read_cache(0)):
+        a, b = np.asarray(a).reshape(150, -1), np.asarray(b).reshape(150, -1)
+        rows = np.arange(150) != 130
+        assert np.array_equal(a[rows], b[rows]) and not np.isfinite(b[130]).any()
+    ctx.check_device_status()
+    s.close(); w.close()
