@@ -191,9 +191,11 @@ template <int MT> __device__ __forceinline__ uint32_t frag(uint32_t row, uint32_
 enum { QKV = 0, OUT = 1, FFN_UP = 2, FFN_DOWN = 3, HEAD = 4, N_KINDS = 5 };
 constexpr uint32_t NO_LOGIT = 0x7fffffffu;   // in the place of the index of a best logit
 
+template <int PARTS> struct Parts { BatchArgs part[PARTS]; };
+
 // SPLIT: sequences may be longer than an attention unit
-template <int HD, int MT, bool SPLIT>
-__global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant__ BatchArgs a, const uint32_t slots, const uint32_t wpi) {
+template <int HD, int MT, bool SPLIT, int PARTS>
+__global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant__ Parts<PARTS> step, const uint32_t slots, const uint32_t wpi) {
     constexpr uint32_t R = MT * 16;               // rows of the exchange buffers
     constexpr uint32_t PPC = CHUNK / NW;          // slices of a ring chunk that a warp has: 2
     constexpr uint32_t Q = R / 4, TPL = 32 / Q;   // lanes that read a tile's sums of squares, tiles per load
@@ -215,7 +217,10 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     __shared__ uint32_t failed_sm, flat_sm, live_sm, use_sm[MAX_SLOTS + MAX_EXTRA];   // use_sm: 1 + the number of the use a slot is in (lm_head only)
 
     const uint32_t tid = threadIdx.x, warp_ = tid >> 5, lane = tid & 31;
-    const uint32_t cta = blockIdx.x;
+    // (of the first part all blocks are there, if any is left out)
+    const uint32_t part_no = PARTS > 1 && blockIdx.x >= step.part[0].sms ? 1u : 0u;
+    const BatchArgs& a = step.part[PARTS > 1 ? part_no : 0];
+    const uint32_t cta = PARTS > 1 ? blockIdx.x - part_no * step.part[0].sms : blockIdx.x;
     const uint32_t D = a.dim, F = a.ffn, H = a.heads, L = a.n_layers;
     uint8_t* const kv_sm = smem + slots * SLOT;
     float* const part = reinterpret_cast<float*>(kv_sm + NW * 2 * KV_BUF);        // [NW][TB][R][8]
@@ -240,7 +245,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     }
     if (tid >= 32 && tid < 32 + N_KINDS) make_kind(kinds[tid - 32], tid == 32 ? 3 * D : tid == 34 ? F : tid == 36 ? a.vocab : D, tid == 35 ? F : D, cta, a.sms);
     if (warp_ == 2) {   // the rows' lengths, the rows by length (the longest first), the attention splits of the rows before by that rank
-        const uint32_t n = lane < a.seqs ? min((uint32_t)max(a.rows ? a.kv_lens[lane] : a.lens[lane], 0), a.max_len) : 0u;
+        const uint32_t n = lane < a.present ? min((uint32_t)max(a.rows ? a.kv_lens[lane] : a.lens[lane], 0), a.max_len) : 0u;
         uint32_t rank = 0;
 #pragma unroll
         for (uint32_t j = 0; j < 32; j++) {
@@ -270,7 +275,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     auto report = [&]() {
         atomicExch(a.status, 1u);
         atomicExch(&g_batch_status, 1u);
-        if (a.sampled_host) *(volatile uint32_t*)(a.sampled_host + a.seqs) = 1u;
+        if (a.status_host) *(volatile uint32_t*)a.status_host = 1u;
     };
     if (failed_sm) {   // a step before this one failed
         if (tid == 0) report();
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (row_live(row)) {
                     const int32_t ts = a.rows ? a.rows[row * 4] : a.tok_src[row];
-                    const uint32_t id = ts >= 0 ? (uint32_t)ts : a.sampled[(uint32_t)(-(ts + 1))];
+                    const uint32_t id = ts >= 0 ? (uint32_t)ts : a.sampled[row];
                     if (id < a.vocab) {
                         const uint2 w = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(a.embedding) + (size_t)id * D + tile * 8 + h * 4);
                         x = make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u));
@@ -1203,18 +1208,20 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     }
 }
 
-template <int HD, int MT, bool SPLIT>
-int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p, uint32_t blocks) {
+template <int HD, int MT, bool SPLIT, int PARTS>
+int launch_batch_t(cudaStream_t st, const BatchArgs* parts, const Plan& p, uint32_t blocks) {
     {
         static bool attr_set[64] = {};
         int dev = 0;
         AK_CUDA(cudaGetDevice(&dev));
         std::lock_guard<std::mutex> lock(device_cache_mutex());
         if (!attr_set[dev & 63]) {
-            AK_CUDA(cudaFuncSetAttribute(batch_kernel<HD, MT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
+            AK_CUDA(cudaFuncSetAttribute(batch_kernel<HD, MT, SPLIT, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
             attr_set[dev & 63] = true;
         }
     }
+    Parts<PARTS> step;
+    for (int i = 0; i < PARTS; i++) step.part[i] = parts[i];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(THREADS);
@@ -1225,7 +1232,7 @@ int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p, uint32_t 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    AK_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel<HD, MT, SPLIT>, a, p.slots, p.wpi));
+    AK_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel<HD, MT, SPLIT, PARTS>, step, p.slots, p.wpi));
     AK_COUNT_LAUNCH();
     return AK_OK;
 }
@@ -1252,16 +1259,21 @@ bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads,
 
 size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) { return sets_bytes(dim, ffn, heads, seqs, max_len); }
 
-int launch_batch(cudaStream_t st, const BatchArgs& a, uint32_t missing) {
-    const uint32_t blocks = a.sms - missing;
+int launch_batch(cudaStream_t st, const BatchArgs* parts, uint32_t n, uint32_t missing) {
+    const BatchArgs& a = parts[0];
+    const uint32_t blocks = n * a.sms - missing;
     const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.seqs, a.max_len, a.sms);
-    const bool two = m_tiles(a.seqs) == 2, split = has_splits(a.max_len, a.dim / a.heads);
-    if (a.dim / a.heads == 64) {
-        if (split) return two ? launch_batch_t<64, 2, true>(st, a, p, blocks) : launch_batch_t<64, 1, true>(st, a, p, blocks);
-        return two ? launch_batch_t<64, 2, false>(st, a, p, blocks) : launch_batch_t<64, 1, false>(st, a, p, blocks);
+    const bool two = m_tiles(a.seqs) == 2, split = has_splits(a.max_len, a.dim / a.heads), hd64 = a.dim / a.heads == 64;
+    if (n == 2) {   // (17 to 32 rows each)
+        if (hd64) return split ? launch_batch_t<64, 2, true, 2>(st, parts, p, blocks) : launch_batch_t<64, 2, false, 2>(st, parts, p, blocks);
+        return split ? launch_batch_t<128, 2, true, 2>(st, parts, p, blocks) : launch_batch_t<128, 2, false, 2>(st, parts, p, blocks);
     }
-    if (split) return two ? launch_batch_t<128, 2, true>(st, a, p, blocks) : launch_batch_t<128, 1, true>(st, a, p, blocks);
-    return two ? launch_batch_t<128, 2, false>(st, a, p, blocks) : launch_batch_t<128, 1, false>(st, a, p, blocks);
+    if (hd64) {
+        if (split) return two ? launch_batch_t<64, 2, true, 1>(st, parts, p, blocks) : launch_batch_t<64, 1, true, 1>(st, parts, p, blocks);
+        return two ? launch_batch_t<64, 2, false, 1>(st, parts, p, blocks) : launch_batch_t<64, 1, false, 1>(st, parts, p, blocks);
+    }
+    if (split) return two ? launch_batch_t<128, 2, true, 1>(st, parts, p, blocks) : launch_batch_t<128, 1, true, 1>(st, parts, p, blocks);
+    return two ? launch_batch_t<128, 2, false, 1>(st, parts, p, blocks) : launch_batch_t<128, 1, false, 1>(st, parts, p, blocks);
 }
 
 int batch_status(unsigned int* out) {

@@ -1,4 +1,4 @@
-// Decode step of up to 32 sequences as one persistent kernel (batch.cu): launch interface.
+// Decode step of up to 64 sequences as one persistent kernel (batch.cu): launch interface.
 #pragma once
 #include "batch_plan.h"
 #include "kernels.h"
@@ -8,6 +8,7 @@ namespace ak {
 
 constexpr uint32_t BATCH_ROWS = batch::ROWS;
 
+// One part of a step: up to 32 of its sequences, on SMs of its own (batch_plan.h). The parts of a step differ in what belongs to their rows and sets.
 struct BatchArgs {
     const SoloLayer* layers;     // device array, one per layer; matrices [out, in] bf16
     const void* maps;            // device array of CUtensorMap (batch_maps): qkv, out, up, down of each layer, lm_head
@@ -16,27 +17,30 @@ struct BatchArgs {
     const float2* rope;          // [max_len][head_dim / 2] (cos, sin)
     uint8_t* xch;                // exchange sets, batch_sets_bytes(): all 0xff before the first launch
     batch::State* state;         // zero before the first launch
-    uint32_t* sampled;           // [seqs]: the token fed back to a row with tok_src < 0, overwritten by the row's greedy pick
+    uint32_t* sampled;           // [present]: the token fed back to a row with tok_src < 0 (its own last pick), overwritten by the row's greedy pick
     // The step, in device memory or (rows == nullptr) by value
-    const int32_t* rows;         // [seqs] of int4 {tok_src, pos, slot, seq}
-    const int32_t* kv_lens;      // [seqs]: positions attended to, the new one included; 0: the row is not there
+    const int32_t* rows;         // [present] of int4 {tok_src, pos, slot, seq}
+    const int32_t* kv_lens;      // [present]: positions attended to, the new one included; 0: the row is not there
     int32_t tok_src[BATCH_ROWS], lens[BATCH_ROWS];
-    const int32_t* block_tables; // [seqs][max_blocks]
-    uint32_t* sampled_host;      // where else the picks go: [seqs] in mapped host memory and behind them the status word, or nullptr
+    const int32_t* block_tables; // [present][max_blocks]
+    uint32_t* sampled_host;      // where else the picks go: [present] in mapped host memory, or nullptr
     uint32_t* status;            // device word: made non-zero when a wait runs out; a step that finds it so does nothing
+    uint32_t* status_host;       // the same for the host, or nullptr
     uint64_t max_cycles;         // time limit of the step, in SM clocks
-    uint32_t n_layers, dim, ffn, heads, vocab, seqs, max_blocks, max_len;
-    uint32_t sms;                // blocks the step is divided over
+    uint32_t n_layers, dim, ffn, heads, vocab, max_blocks, max_len;
+    uint32_t seqs, present;      // rows of a part (the plan goes by them), rows that this one has
+    uint32_t sms;                // blocks the part is divided over
     float eps, scale;
 };
 
 bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers, uint32_t seqs, uint32_t max_len);
 // the weights' tensor maps, 4 n_layers + 1 of 128 bytes in host memory (layers: host array)
 int batch_maps(void* out, const SoloLayer* layers, const void* lm_head, uint32_t n_layers, uint32_t dim, uint32_t ffn, uint32_t vocab);
+// a part's sets; seqs: of a part
 size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len);
 constexpr uint64_t BATCH_MAX_CYCLES = 1ull << 32;   // two seconds or so, for a step of milliseconds
-// missing: blocks left out, so that the others' waits run out (a drill)
-int launch_batch(cudaStream_t st, const BatchArgs& a, uint32_t missing = 0);
+// n parts. missing: blocks left out, so that the others' waits run out (a drill)
+int launch_batch(cudaStream_t st, const BatchArgs* parts, uint32_t n, uint32_t missing = 0);
 int batch_status(unsigned int* out);
 
 }  // namespace ak

@@ -1,4 +1,4 @@
-// Decode step of up to 32 sequences (batch.cu): tiles, exchange buffers and shared memory, and which models they fit.
+// Decode step of up to 64 sequences (batch.cu): tiles, exchange buffers and shared memory, and which models they fit.
 // Plain C++ (no CUDA header), so that the plan can be checked on the host.
 #pragma once
 #include <stddef.h>
@@ -17,7 +17,8 @@ namespace batch {
 
 constexpr uint32_t SMS = 148;             // one block per SM
 constexpr uint32_t SMS_BESIDE = 48;       // the fewest blocks of a step beside prompts
-constexpr uint32_t ROWS = 32;             // most sequences of a step
+constexpr uint32_t ROWS = 32;             // most sequences of a part
+constexpr uint32_t MAX_PARTS = 2;
 static_assert(SMS_BESIDE >= ROWS, "block r picks the token of row r");
 constexpr uint32_t NW = 12;               // compute warps
 constexpr uint32_t NH = 3;                // epilogue warps
@@ -31,6 +32,9 @@ constexpr uint32_t MAX_UNITS = 32;        // attention units of a group (a lane 
 constexpr uint32_t MAX_DYN_SMEM = 216 * 1024;
 
 AK_PLAN_FN constexpr uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
+// More than 32 sequences are two parts, each with half of the sequences and half of the SMs, that have nothing to do with each other
+AK_PLAN_FN constexpr uint32_t parts_of(uint32_t seqs) { return seqs <= ROWS ? 1 : MAX_PARTS; }
+AK_PLAN_FN constexpr uint32_t part_seqs(uint32_t seqs) { return div_up(seqs, parts_of(seqs)); }
 AK_PLAN_FN constexpr uint32_t m_tiles(uint32_t seqs) { return seqs <= 16 ? 1 : 2; }
 AK_PLAN_FN constexpr uint32_t tile_begin(uint32_t tiles, uint32_t cta, uint32_t sms) { return (tiles * cta) / sms; }   // of the step's sms blocks
 // Positions of an attention unit. Where all sequences fit in 128 KB of keys (1024 positions of head size 64, 512 of 128) they are whole, which saves
@@ -134,13 +138,15 @@ AK_PLAN_FN void walk_on(Walk& k, uint32_t wpi, uint32_t place, uint32_t n_layers
 inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers, uint32_t seqs, uint32_t max_len) {
     const uint32_t hd = heads ? dim / heads : 0;
     if ((hd != 64 && hd != 128) || dim != heads * hd || heads > 4095) return false;
-    if (seqs < 1 || seqs > ROWS || n_layers < 1 || n_layers > MAX_LAYERS || dim < 96 || dim % 32 || ffn % 32 || ffn > 65536) return false;
+    if (seqs < 1 || seqs > ROWS * MAX_PARTS || n_layers < 1 || n_layers > MAX_LAYERS || dim < 96 || dim % 32 || ffn % 32 || ffn > 65536) return false;
+    const uint32_t sms = SMS / parts_of(seqs);
+    seqs = part_seqs(seqs);
     if (ffn / 8 < SMS) return false;                                       // every SM has ffn-up rows (the clearing of the sets counts on it)
-    if (div_up(dim / 8, SMS) > TB) return false;                           // the residual stream is worked on in one pass
+    if (div_up(dim / 8, sms) > TB) return false;                           // the residual stream is worked on in one pass
     if (dim * m_tiles(seqs) * 16 * 2 > NW * 2 * KV_BUF) return false;      // the lm_head keeps x where the cache tiles were
     const uint32_t splits = div_up(max_len, split_len(max_len, hd));
-    const Plan p = make_plan(dim, n_layers, heads, seqs, max_len);
-    if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * SMS * (NW / p.wpi)) return false;
+    const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms);
+    if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * sms * (NW / p.wpi)) return false;
     return p.slots >= 4 && sets_bytes(dim, ffn, heads, seqs, max_len) < (1ull << 32);
 }
 
@@ -150,13 +156,14 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
 // 33.1, 60 32.7, 48 30.7 (all rows through the chain, which shares its launches then: 31.2); 8 slots, prompts of 16 to 448, 2 tokens: 20.8, 19.2, 18.9,
 // 18.9, 18.5 (19.8); 320-wide model, 32 slots: 20.8, 16.7, 16.0, 15.9, 15.9 (17.2); 1.4B model (86 SMs at least), 16 slots, prompts of 1 to
 // 64, 4 tokens: 57.5, 55.8, 54.9 (53.9: both read all weights), prompts of 128 to 1024: 128.7, 129.3, 127.9 (128.8).
-inline uint32_t sms_beside(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len) {
+// (of a part; seqs: the part's)
+inline uint32_t sms_beside(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len, uint32_t parts = 1) {
     const uint64_t units = (uint64_t)seqs * heads * div_up(max_len, split_len(max_len, dim / heads));
-    for (uint32_t sms = SMS_BESIDE; sms < SMS; sms++) {
+    for (uint32_t sms = SMS_BESIDE; sms < SMS / parts; sms++) {
         const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms);
         if (div_up(dim / 8, sms) <= TB && units <= (uint64_t)MAX_UNITS * sms * (NW / p.wpi) && p.slots >= 4) return sms;
     }
-    return SMS;
+    return SMS / parts;
 }
 
 }  // namespace batch

@@ -1,0 +1,36 @@
+"""CPU: a step of 33 to 64 sequences as two parts (csrc/batch_plan.h): the exchange sets of a part, on half of the SMs, and which models fit."""
+import pytest
+
+from test_batch_plan import CHECK, build
+
+HALF = CHECK.replace("sms_beside(dim, L, heads, rows, max_len)", "atoi(argv[7]) == 1 ? SMS / 2 : sms_beside(dim, L, heads, rows, max_len, 2)")
+SHAPES = r"""
+#include <stdio.h>
+#include <stdlib.h>
+#include "batch_plan.h"
+using namespace ak::batch;
+int main(int argc, char** argv) {
+    const uint32_t v[] = {(uint32_t)atoi(argv[1]), (uint32_t)atoi(argv[2]), (uint32_t)atoi(argv[3]), (uint32_t)atoi(argv[4]), (uint32_t)atoi(argv[5]), (uint32_t)atoi(argv[6])};
+    printf("%d %u %u", shape_supported(v[0], v[1], v[2], v[3], v[4], v[5]), parts_of(v[4]), part_seqs(v[4]));
+    return 0;
+}
+"""
+
+
+@pytest.mark.parametrize("dim,ffn,heads", [(128, 1184, 1), (320, 1280, 5), (768, 3072, 12), (1280, 2560, 10), (1536, 6144, 12)])
+@pytest.mark.parametrize("rows,max_len", [(17, 512), (32, 1200)])
+def test_sets_of_a_part_are_clean_and_unread(tmp_path_factory, dim, ffn, heads, rows, max_len):
+    plan = build(tmp_path_factory, HALF)
+    for layers in (1, 2, 5):
+        for sms in (1, 2):   # half of the SMs; those of a step beside prompts
+            assert plan(dim, ffn, heads, layers, rows, max_len, sms) == "ok"
+
+
+def test_which_shapes_are_two_parts(tmp_path_factory):
+    shapes = build(tmp_path_factory, SHAPES)
+    assert shapes(768, 3072, 12, 12, 32, 512) == "1 1 32"
+    assert shapes(768, 3072, 12, 12, 33, 512) == "1 2 17"
+    assert shapes(768, 3072, 12, 12, 64, 512) == "1 2 32"
+    assert shapes(768, 3072, 12, 12, 65, 512).startswith("0")
+    assert shapes(1536, 6144, 12, 24, 64, 512).startswith("1")
+    assert shapes(2048, 8192, 16, 24, 64, 512).startswith("0")   # 32 rows of x do not fit where the cache tiles were
