@@ -65,8 +65,9 @@ struct ak_engine {
     bool async_ok() const { return cfg.async_steps != 0 && cfg.stop_on_eos == 0; }
 };
 
-// Wait for the step in flight and write its tokens into their sequences.
-static int collect(ak_engine* e) {
+// Wait for the step in flight and write its tokens into their sequences. `next`: the step launched behind it, if any: a sequence that turns out to
+// have ended has a row there that counts for nothing (it wrote into blocks that are still the sequence's).
+static int collect(ak_engine* e, ak_engine::Pending* next = nullptr) {
     ak_engine::Pending& p = e->pending;
     if (!p.active) return AK_OK;
     Runner& r = e->runner;
@@ -80,7 +81,16 @@ static int collect(ak_engine* e) {
         Seq* s = p.fill[i].first;
         const uint32_t tok = sampled[p.fill_slot[i]];
         s->generated[p.fill[i].second] = tok;
-        if (e->cfg.stop_on_eos && tok == mc.eos_token) s->finished = true;
+        if (!e->cfg.stop_on_eos || tok != mc.eos_token) continue;
+        s->finished = true;
+        for (size_t j = 0; next && j < next->fill.size(); j++)
+            if (next->fill[j].first == s) {
+                next->fill.erase(next->fill.begin() + j);
+                next->fill_slot.erase(next->fill_slot.begin() + j);
+                s->generated.pop_back();
+                e->stats.decode_tokens--;
+                break;
+            }
     }
     const float step_ms = e->cfg.attn_timing ? r.last_step_gpu_ms() : 0.0f;
     e->stats.step_gpu_ms_total += step_ms;
@@ -181,17 +191,18 @@ int ak_engine_submit(ak_engine* e, const uint32_t* prompt, uint32_t n, uint32_t 
     return AK_OK;
 }
 
-int ak_engine_step(ak_engine* e, uint32_t* n_running, uint32_t* n_waiting) {
-    AK_REQUIRE(e, AK_ERR_INVALID_ARG, "ak_engine_step: null engine");
+}  // extern "C"
+
+// ahead: launch this step before the tokens of the one before it are read (ends by length are known in time, an end-of-sequence token a step late)
+static int engine_step(ak_engine* e, bool ahead, uint32_t* n_running, uint32_t* n_waiting) {
     Runner& r = e->runner;
     const uint32_t S = e->cfg.max_seqs;
     const ak_model_config& mc = e->w->cfg;
     const unsigned long long launches0 = g_launch_count;
-    // Without async steps the previous step's tokens decide who has finished: read them first.
-    // With async steps sequence ends depend on lengths only, so this step is planned and launched
-    // while the previous one still runs, and the previous one's tokens are read afterwards.
-    if (!e->async_ok()) { int rc0 = collect(e); if (rc0) return rc0; }
-    r.set_bank(e->async_ok() ? (uint32_t)(e->step_index & 1u) : 0u);
+    // Not ahead, the previous step's tokens decide who has finished: read them first. Ahead, this step is planned and launched while the previous
+    // one still runs, and the previous one's tokens are read afterwards.
+    if (!ahead) AK_TRY(collect(e));
+    r.set_bank(ahead ? (uint32_t)(e->step_index & 1u) : 0u);
 
     // 1. retire sequences that finished in the previous step (their blocks go back first)
     for (uint32_t i = 0; i < S; i++)
@@ -347,22 +358,19 @@ int ak_engine_step(ak_engine* e, uint32_t* n_running, uint32_t* n_waiting) {
         emit_token(wk.s);
     }
     while (!e->prefill_queue.empty() && !e->prefill_queue.front()->in_prefill) e->prefill_queue.pop_front();
-    uint32_t running = 0;
-    for (uint32_t i = 0; i < S; i++) if (e->slots[i] && !e->slots[i]->finished) running++;
+    e->stats.decode_tokens += n_dec;
     // the previous step (other bank) has had this step's host work to finish in: read its tokens now
-    rc = collect(e);
+    rc = collect(e, &now);
     if (rc) return rc;
     e->pending = std::move(now);
     e->step_index++;
-    if (!e->async_ok()) {
+    if (!ahead) {
         rc = collect(e);
         if (rc) return rc;
-        // an end-of-sequence token may have finished sequences that the length rule left running
-        running = 0;
-        for (uint32_t i = 0; i < S; i++) if (e->slots[i] && !e->slots[i]->finished) running++;
     }
+    uint32_t running = 0;   // (an end-of-sequence token may have finished sequences that the length rule left running)
+    for (uint32_t i = 0; i < S; i++) if (e->slots[i] && !e->slots[i]->finished) running++;
     e->stats.steps++;
-    e->stats.decode_tokens += n_dec;
     e->stats.prefill_tokens += pf_rows;
     if (graph && !(r.batch() && pf_rows == 0)) e->stats.graph_launches++; else e->stats.eager_steps++;   // (the latter: one launch)
     e->stats.kernel_launches += (g_launch_count - launches0);
@@ -374,14 +382,28 @@ int ak_engine_step(ak_engine* e, uint32_t* n_running, uint32_t* n_waiting) {
     return AK_OK;
 }
 
+extern "C" {
+
+int ak_engine_step(ak_engine* e, uint32_t* n_running, uint32_t* n_waiting) {
+    AK_REQUIRE(e, AK_ERR_INVALID_ARG, "ak_engine_step: null engine");
+    return engine_step(e, e->async_ok(), n_running, n_waiting);
+}
+
 int ak_engine_run(ak_engine* e, uint64_t max_steps, uint64_t* steps_done) {
     AK_REQUIRE(e, AK_ERR_INVALID_ARG, "ak_engine_run: null engine");
     uint64_t n = 0;
+    // To the end, nobody looks at the tokens between two steps: every step is launched ahead. The host's turn between two of them (wait, read,
+    // describe, launch) took 20 us; a sequence that ends at a token keeps its slot a step longer. Tokens do not depend on who shares a step.
+    // (A limit that the queue cannot reach is none: a step takes at least one sequence on by a token, in its prompt or behind it.)
+    uint64_t most = 1;
+    for (const auto& kv : e->all)
+        if (!kv.second->finished) most += kv.second->prompt.size() + kv.second->max_total + 1;
+    const bool ahead = max_steps == 0 || max_steps >= most || e->async_ok();
     for (;;) {
         if (max_steps && n >= max_steps) break;
         uint32_t running = 0, waiting = 0;
         const uint64_t launched0 = e->stats.steps;
-        int rc = ak_engine_step(e, &running, &waiting);
+        int rc = engine_step(e, ahead, &running, &waiting);
         if (rc) return rc;
         n++;
         if (running == 0 && waiting == 0) break;
