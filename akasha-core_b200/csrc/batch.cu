@@ -52,7 +52,7 @@ using namespace batch;
 static_assert(SMS == B200_SMS, "a block per SM");
 constexpr uint32_t NCT = NW * 32, NHT = NH * 32;   // threads of the compute and of the epilogue warps
 constexpr uint32_t THREADS = 512, FIRST_COMPUTE = 4;
-constexpr int REGS_FIRST = 80, REGS_COMPUTE = 144;
+constexpr int REGS_FIRST = 104, REGS_COMPUTE = 136;
 static_assert(REGS_FIRST * 128 + REGS_COMPUTE * 384 <= 65536, "the split draws on the registers of the launch");
 constexpr uint32_t EMPTY = 0xffffffffu;   // an exchange word that is not written yet
 
@@ -191,13 +191,12 @@ template <int MT> __device__ __forceinline__ uint32_t frag(uint32_t row, uint32_
 enum { QKV = 0, OUT = 1, FFN_UP = 2, FFN_DOWN = 3, HEAD = 4, N_KINDS = 5 };
 constexpr uint32_t NO_LOGIT = 0x7fffffffu;   // in the place of the index of a best logit
 
-template <int PARTS> struct Parts { BatchArgs part[PARTS]; };
-
 // SPLIT: sequences may be longer than an attention unit
 template <int HD, int MT, bool SPLIT, int PARTS>
-__global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant__ Parts<PARTS> step, const uint32_t slots, const uint32_t wpi) {
+__global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant__ BatchArgs a, const uint32_t slots, const uint32_t wpi) {
     constexpr uint32_t R = MT * 16;               // rows of the exchange buffers
     constexpr uint32_t PPC = CHUNK / NW;          // slices of a ring chunk that a warp has: 2
+    constexpr bool KEEP = PARTS > 1;              // activations stay in registers for the passes of a phase (half of the SMs have twice the tiles)
     constexpr uint32_t Q = R / 4, TPL = 32 / Q;   // lanes that read a tile's sums of squares, tiles per load
     constexpr uint32_t CH = HD / 8;               // 16-byte vectors of a cache row
     constexpr uint32_t PPI = 32 / CH;             // positions a warp reads per instruction
@@ -217,10 +216,10 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     __shared__ uint32_t failed_sm, flat_sm, live_sm, use_sm[MAX_SLOTS + MAX_EXTRA];   // use_sm: 1 + the number of the use a slot is in (lm_head only)
 
     const uint32_t tid = threadIdx.x, warp_ = tid >> 5, lane = tid & 31;
-    // (of the first part all blocks are there, if any is left out)
-    const uint32_t part_no = PARTS > 1 && blockIdx.x >= step.part[0].sms ? 1u : 0u;
-    const BatchArgs& a = step.part[PARTS > 1 ? part_no : 0];
-    const uint32_t cta = PARTS > 1 ? blockIdx.x - part_no * step.part[0].sms : blockIdx.x;
+    // What tells the parts apart: rows, sets (an offset that set_of() adds), state. (As arguments of their own, chosen by the block, they cost 5 % of a step.)
+    const uint32_t part_no = PARTS > 1 && blockIdx.x >= a.sms ? 1u : 0u, row0 = PARTS > 1 ? part_no * a.part_seqs : 0u;
+    const uint32_t cta = PARTS > 1 ? blockIdx.x - part_no * a.sms : blockIdx.x;
+    State* const state = PARTS > 1 ? a.state + part_no : a.state;
     const uint32_t D = a.dim, F = a.ffn, H = a.heads, L = a.n_layers;
     uint8_t* const kv_sm = smem + slots * SLOT;
     float* const part = reinterpret_cast<float*>(kv_sm + NW * 2 * KV_BUF);        // [NW][TB][R][8]
@@ -245,7 +244,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     }
     if (tid >= 32 && tid < 32 + N_KINDS) make_kind(kinds[tid - 32], tid == 32 ? 3 * D : tid == 34 ? F : tid == 36 ? a.vocab : D, tid == 35 ? F : D, cta, a.sms);
     if (warp_ == 2) {   // the rows' lengths, the rows by length (the longest first), the attention splits of the rows before by that rank
-        const uint32_t n = lane < a.present ? min((uint32_t)max(a.rows ? a.kv_lens[lane] : a.lens[lane], 0), a.max_len) : 0u;
+        const uint32_t n = lane < a.part_seqs && row0 + lane < a.seqs ? min((uint32_t)max(a.rows ? a.kv_lens[row0 + lane] : a.lens[row0 + lane], 0), a.max_len) : 0u;
         uint32_t rank = 0;
 #pragma unroll
         for (uint32_t j = 0; j < 32; j++) {
@@ -270,12 +269,12 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll 1
     for (uint32_t i = tid; i < L * (uint32_t)(sizeof(SoloLayer) / 8); i += THREADS)
         reinterpret_cast<uint64_t*>(layers_sm)[i] = reinterpret_cast<const uint64_t*>(a.layers)[i];
-    const uint32_t e0 = *(const volatile uint32_t*)&a.state->set;   // (before the block's barrier, so before this SM publishes anything)
+    const uint32_t e0 = *(const volatile uint32_t*)&state->set;   // (before the block's barrier, so before this SM publishes anything)
     __syncthreads();
     auto report = [&]() {
         atomicExch(a.status, 1u);
         atomicExch(&g_batch_status, 1u);
-        if (a.status_host) *(volatile uint32_t*)a.status_host = 1u;
+        if (a.sampled_host) *(volatile uint32_t*)(a.sampled_host + a.seqs) = 1u;
     };
     if (failed_sm) {   // a step before this one failed
         if (tid == 0) report();
@@ -291,7 +290,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     // The lm_head keeps x where the cache tiles were, and extra slots behind it. Its chunk n is in slot n mod (slots + extra) of the two.
     uint8_t* const extra_sm = kv_sm + D * R * 2;
     const uint32_t extra = min(MAX_EXTRA, (NW * 2 * KV_BUF - D * R * 2) / SLOT), head_slots = slots + extra;
-    auto set_of = [&](uint32_t g) { return (g % SETS) * (uint32_t)so.total; };   // byte offset; g = e0: the embedding, e0 + 1 + l: layer l
+    auto set_of = [&](uint32_t g) { return (g % SETS) * (uint32_t)so.total + (PARTS > 1 ? part_no * a.part_bytes : 0u); };   // byte offset; g = e0: the embedding, e0 + 1 + l: layer l
     auto row_live = [&](uint32_t r) { return (live >> r) & 1u; };
     auto eight_live = [&](uint32_t e) { return ((live >> (e * 8)) & 0xffu) != 0; };
     const Waiter wt{&expiry};
@@ -375,14 +374,14 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll 1
             for (uint32_t i = cta * NHT + ht; i < n; i += a.sms * NHT) p[i] = make_uint4(EMPTY, EMPTY, EMPTY, EMPTY);
             bar_sync<NHT>(BAR_HELP);
-            if (ht == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&a.state->cleared) : "memory");
+            if (ht == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&state->cleared) : "memory");
         };
-        const uint32_t counted = *(const volatile uint32_t*)&a.state->counted;
+        const uint32_t counted = *(const volatile uint32_t*)&state->counted;
         auto wait_cleared = [&](uint32_t clears) {
             if (lane == 0) {
                 uint32_t n = 0, v;
                 Waiter w = wt;
-                do asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&a.state->cleared) : "memory");
+                do asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&state->cleared) : "memory");
                 while ((int32_t)(v - counted - clears * a.sms) < 0 && !w.give_up(n));
             }
             __syncwarp();
@@ -399,10 +398,13 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 uint32_t polls = 0;
                 bool lack;
                 Waiter w = wt;
+#pragma unroll
+                for (uint32_t d = 0; d < 4; d++) y[d].x = y[d].y = y[d].z = y[d].w = t0 + d * step < n ? EMPTY : 0u;
 #pragma unroll 1
                 do {
 #pragma unroll
-                    for (uint32_t d = 0; d < 4; d++) y[d] = t0 + d * step < n ? xld4(sl + (t0 + d * step) * (R * 4)) : make_uint4(0, 0, 0, 0);
+                    for (uint32_t d = 0; d < 4; d++)
+                        if (max(max(y[d].x, y[d].y), max(y[d].z, y[d].w)) == EMPTY) y[d] = xld4(sl + (t0 + d * step) * (R * 4));
                     uint32_t mx = 0;
 #pragma unroll
                     for (uint32_t d = 0; d < 4; d++) mx = max(max(mx, max(y[d].x, y[d].y)), max(y[d].z, y[d].w));
@@ -452,8 +454,8 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 const uint32_t row = m * 16 + rl;
                 float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (row_live(row)) {
-                    const int32_t ts = a.rows ? a.rows[row * 4] : a.tok_src[row];
-                    const uint32_t id = ts >= 0 ? (uint32_t)ts : a.sampled[row];
+                    const int32_t ts = a.rows ? a.rows[(row0 + row) * 4] : a.tok_src[row0 + row];
+                    const uint32_t id = ts >= 0 ? (uint32_t)ts : a.sampled[row0 + row];
                     if (id < a.vocab) {
                         const uint2 w = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(a.embedding) + (size_t)id * D + tile * 8 + h * 4);
                         x = make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u));
@@ -584,18 +586,18 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll
     for (uint32_t e = 0; e < 2 * MT; e++) a_live |= (eight_live(e) ? 1u : 0u) << e;
 
-    // The warp's share of NT tiles of projection `kind`; x: A fragments. What a phase spends its time on is dependent instructions, ~5 cycles each, so
-    // all that can be is done before the activations arrive: the weights are in registers, addresses are known.
-    auto pass = [&](auto nt_c, uint32_t x, const Kind& kind) {
-        constexpr uint32_t NT = decltype(nt_c)::value;
-        constexpr uint32_t CPG = MT == 1 && NT == 1 ? 2 : 1, DEPTH = CPG * PPC;   // chunks of a group (what a warp requests together), slices
+    // The warp's share of NT tiles of projection `kind`; x: A fragments. What a phase spends its time on is dependent instructions, ~5 cycles each, and
+    // round trips to L2, ~1 us each, so all that can be is done before the activations arrive: the weights are in registers, addresses are known.
+    // CPG: chunks of a group (what a warp requests together, as many as there are registers for). With K of one chunk the activations stay
+    // in v for the later passes over the same ones (loaded).
+    auto pass = [&](auto nt_c, auto cpg_c, uint32_t x, const Kind& kind, auto& v, bool loaded) {
+        constexpr uint32_t NT = decltype(nt_c)::value, CPG = decltype(cpg_c)::value, DEPTH = CPG * PPC;
         const uint32_t chunks = kind.chunks, slices = kind.slices, pitch = kind.pitch;
         // the warp's slices cw + NW i, i < nsl
         const uint32_t nsl = cw < slices ? (slices - cw + NW - 1) / NW : 0;
         const uint8_t* xl = a.xch + (x + cw * (MT * 1024) + frag_lane * 16);
         constexpr uint32_t STEP = NW * MT * 1024;
         const uint32_t w_off = (lane >> 2) * pitch + cw * 64 + (lane & 3) * 16;
-        uint4 v[DEPTH][MT][2];
         float acc[NT][MT][4];
 #pragma unroll
         for (uint32_t t = 0; t < NT; t++)
@@ -603,10 +605,6 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             for (uint32_t m = 0; m < MT; m++)
 #pragma unroll
                 for (int i = 0; i < 4; i++) acc[t][m][i] = 0.0f;
-#pragma unroll
-        for (uint32_t d = 0; d < DEPTH; d++)
-#pragma unroll
-            for (uint32_t e = 0; e < 2 * MT; e++) v[d][e >> 1][e & 1] = make_uint4(0, 0, 0, 0);
         auto issue = [&](uint32_t i0) {
 #pragma unroll
             for (uint32_t d = 0; d < DEPTH; d++)
@@ -623,7 +621,13 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 mbar_arrive(&empty_bar[q.s >= back ? q.s - back : q.s + slots - back]);
             }
         };
-        issue(0);
+        if (!loaded) {
+#pragma unroll
+            for (uint32_t d = 0; d < DEPTH; d++)
+#pragma unroll
+                for (uint32_t e = 0; e < 2 * MT; e++) v[d][e >> 1][e & 1] = make_uint4(0, 0, 0, 0);
+            issue(0);
+        }
 #pragma unroll 1
         for (uint32_t c0 = 0;;) {
             // the group's weights
@@ -666,7 +670,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                     if (d < left) {
 #pragma unroll
                         for (uint32_t e = 0; e < 2 * MT; e++)
-                            if (a_live >> e & 1u) v[d][e >> 1][e & 1] = xld4(xl + d * STEP + e * 512);
+                            if (v[d][e >> 1][e & 1].x == EMPTY) v[d][e >> 1][e & 1] = xld4(xl + d * STEP + e * 512);
                     }
             }
 #pragma unroll
@@ -708,12 +712,24 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     };
     auto gemm = [&](uint32_t x, const Kind& kind) {
         const uint32_t tiles = kind.n;
+        using std::integral_constant;
+        constexpr integral_constant<uint32_t, 1> one{};
+        uint4 kept[KEEP ? PPC : 1][MT][2];
+        const bool keep = KEEP && kind.chunks == 1;
 #pragma unroll 1
         for (uint32_t b = 0; b < tiles; b += TB) {
             const uint32_t nt = min(TB, tiles - b);
-            if (nt == 1) pass(std::integral_constant<uint32_t, 1>{}, x, kind);
-            else if (nt == 2) pass(std::integral_constant<uint32_t, 2>{}, x, kind);
-            else pass(std::integral_constant<uint32_t, 3>{}, x, kind);
+            auto of = [&](auto nt_c, auto cpg_c) {
+                if constexpr (KEEP) {
+                    pass(nt_c, one, x, kind, kept, keep && b > 0);
+                } else {
+                    uint4 v[decltype(cpg_c)::value * PPC][MT][2];
+                    pass(nt_c, cpg_c, x, kind, v, false);
+                }
+            };
+            if (nt == 1) of(one, integral_constant<uint32_t, MT == 1 ? 2 : 1>{});
+            else if (nt == 2) of(integral_constant<uint32_t, 2>{}, one);
+            else of(integral_constant<uint32_t, 3>{}, one);
         }
     };
 
@@ -754,7 +770,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     auto look_up = [&]() {   // the pool blocks of the walk's tile (lane 0)
         Walk& k = walk_sm[cw];
         const uint32_t p = k.b * UP;
-        const int32_t* bt = a.block_tables + (size_t)k.u.row * a.max_blocks + (k.u.p0 + p) / 16;
+        const int32_t* bt = a.block_tables + (size_t)(row0 + k.u.row) * a.max_blocks + (k.u.p0 + p) / 16;
         k.pb0 = (uint32_t)__ldg(bt);
         k.pb1 = UP > 16 && p + 16 < k.u.n ? (uint32_t)__ldg(bt + 1) : EMPTY;
     };
@@ -840,20 +856,20 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 const uint8_t* const src = qkv + ((size_t)u.row * 3 * D + u.head * HD + chunk * 8) * 4;
                 const float4* const rt = reinterpret_cast<const float4*>(a.rope + (size_t)pos * (HD / 2) + chunk * 4);
                 const float4 r0 = __ldg(rt), r1 = __ldg(rt + 1);
-                const uint32_t pb = owner ? (uint32_t)__ldg(a.block_tables + (size_t)u.row * a.max_blocks + pos / 16) : 0u;
+                const uint32_t pb = owner ? (uint32_t)__ldg(a.block_tables + (size_t)(row0 + u.row) * a.max_blocks + pos / 16) : 0u;
                 uint4 qa[NS], kn = make_uint4(0, 0, 0, 0), vn = kn;
                 {
-                    uint4 x[6];
+                    uint4 x[6] = {};
                     uint32_t n = 0;
                     Waiter w = wt;
 #pragma unroll
-                    for (int i = 0; i < 6; i++) x[i] = make_uint4(0, 0, 0, 0);
+                    for (int i = 0; i < 6; i++) x[i].x = i < 2 || owner ? EMPTY : 0u;
                     bool lack;
 #pragma unroll 1
                     do {
 #pragma unroll
                         for (int i = 0; i < 6; i++)
-                            if (i < 2 || owner) x[i] = xld4(src + (size_t)(i >> 1) * D * 4 + (i & 1) * 16);
+                            if (x[i].x == EMPTY) x[i] = xld4(src + (size_t)(i >> 1) * D * 4 + (i & 1) * 16);
                         lack = max(max(x[0].x, x[1].x), max(max(x[2].x, x[3].x), max(x[4].x, x[5].x))) == EMPTY;
                     } while (__any_sync(0xffffffffu, lack) && !__any_sync(0xffffffffu, w.give_up(n)));
                     auto packed = [&](const uint4& lo, const uint4& hi, bool rotate) {
@@ -1190,11 +1206,11 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             bar_sync<64>(BAR_FLAT);
             if (lane == 0) {
                 const uint32_t tok = n < a.vocab && !flat_sm ? n : 0u;   // (no logit above -inf, or all 0: 0)
-                a.sampled[cta] = tok;
-                if (a.sampled_host) a.sampled_host[cta] = tok;
+                a.sampled[row0 + cta] = tok;
+                if (a.sampled_host) a.sampled_host[row0 + cta] = tok;
                 if (cta == (uint32_t)__ffs(live) - 1) {   // every SM has published its best, so has read them
-                    a.state->set = (e0 + L + 1) % SETS;
-                    a.state->counted += clears_of_step(L) * a.sms;
+                    state->set = (e0 + L + 1) % SETS;
+                    state->counted += clears_of_step(L) * a.sms;
                 }
             }
         }
@@ -1209,7 +1225,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 }
 
 template <int HD, int MT, bool SPLIT, int PARTS>
-int launch_batch_t(cudaStream_t st, const BatchArgs* parts, const Plan& p, uint32_t blocks) {
+int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p, uint32_t blocks) {
     {
         static bool attr_set[64] = {};
         int dev = 0;
@@ -1220,8 +1236,6 @@ int launch_batch_t(cudaStream_t st, const BatchArgs* parts, const Plan& p, uint3
             attr_set[dev & 63] = true;
         }
     }
-    Parts<PARTS> step;
-    for (int i = 0; i < PARTS; i++) step.part[i] = parts[i];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(THREADS);
@@ -1232,7 +1246,7 @@ int launch_batch_t(cudaStream_t st, const BatchArgs* parts, const Plan& p, uint3
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    AK_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel<HD, MT, SPLIT, PARTS>, step, p.slots, p.wpi));
+    AK_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel<HD, MT, SPLIT, PARTS>, a, p.slots, p.wpi));
     AK_COUNT_LAUNCH();
     return AK_OK;
 }
@@ -1259,21 +1273,20 @@ bool batch_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads,
 
 size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len) { return sets_bytes(dim, ffn, heads, seqs, max_len); }
 
-int launch_batch(cudaStream_t st, const BatchArgs* parts, uint32_t n, uint32_t missing) {
-    const BatchArgs& a = parts[0];
-    const uint32_t blocks = n * a.sms - missing;
-    const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.seqs, a.max_len, a.sms);
-    const bool two = m_tiles(a.seqs) == 2, split = has_splits(a.max_len, a.dim / a.heads), hd64 = a.dim / a.heads == 64;
+int launch_batch(cudaStream_t st, const BatchArgs& a, uint32_t missing) {
+    const uint32_t n = parts_of(a.seqs), blocks = n * a.sms - missing;
+    const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.part_seqs, a.max_len, a.sms);
+    const bool two = m_tiles(a.part_seqs) == 2, split = has_splits(a.max_len, a.dim / a.heads), hd64 = a.dim / a.heads == 64;
     if (n == 2) {   // (17 to 32 rows each)
-        if (hd64) return split ? launch_batch_t<64, 2, true, 2>(st, parts, p, blocks) : launch_batch_t<64, 2, false, 2>(st, parts, p, blocks);
-        return split ? launch_batch_t<128, 2, true, 2>(st, parts, p, blocks) : launch_batch_t<128, 2, false, 2>(st, parts, p, blocks);
+        if (hd64) return split ? launch_batch_t<64, 2, true, 2>(st, a, p, blocks) : launch_batch_t<64, 2, false, 2>(st, a, p, blocks);
+        return split ? launch_batch_t<128, 2, true, 2>(st, a, p, blocks) : launch_batch_t<128, 2, false, 2>(st, a, p, blocks);
     }
     if (hd64) {
-        if (split) return two ? launch_batch_t<64, 2, true, 1>(st, parts, p, blocks) : launch_batch_t<64, 1, true, 1>(st, parts, p, blocks);
-        return two ? launch_batch_t<64, 2, false, 1>(st, parts, p, blocks) : launch_batch_t<64, 1, false, 1>(st, parts, p, blocks);
+        if (split) return two ? launch_batch_t<64, 2, true, 1>(st, a, p, blocks) : launch_batch_t<64, 1, true, 1>(st, a, p, blocks);
+        return two ? launch_batch_t<64, 2, false, 1>(st, a, p, blocks) : launch_batch_t<64, 1, false, 1>(st, a, p, blocks);
     }
-    if (split) return two ? launch_batch_t<128, 2, true, 1>(st, parts, p, blocks) : launch_batch_t<128, 1, true, 1>(st, parts, p, blocks);
-    return two ? launch_batch_t<128, 2, false, 1>(st, parts, p, blocks) : launch_batch_t<128, 1, false, 1>(st, parts, p, blocks);
+    if (split) return two ? launch_batch_t<128, 2, true, 1>(st, a, p, blocks) : launch_batch_t<128, 1, true, 1>(st, a, p, blocks);
+    return two ? launch_batch_t<128, 2, false, 1>(st, a, p, blocks) : launch_batch_t<128, 1, false, 1>(st, a, p, blocks);
 }
 
 int batch_status(unsigned int* out) {

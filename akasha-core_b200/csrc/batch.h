@@ -6,30 +6,28 @@
 
 namespace ak {
 
-constexpr uint32_t BATCH_ROWS = batch::ROWS;
+constexpr uint32_t BATCH_ROWS = batch::ROWS * batch::MAX_PARTS;
 
-// One part of a step: up to 32 of its sequences, on SMs of its own (batch_plan.h). The parts of a step differ in what belongs to their rows and sets.
 struct BatchArgs {
     const SoloLayer* layers;     // device array, one per layer; matrices [out, in] bf16
     const void* maps;            // device array of CUtensorMap (batch_maps): qkv, out, up, down of each layer, lm_head
     const void* embedding;
     const float* final_norm;
     const float2* rope;          // [max_len][head_dim / 2] (cos, sin)
-    uint8_t* xch;                // exchange sets, batch_sets_bytes(): all 0xff before the first launch
-    batch::State* state;         // zero before the first launch
-    uint32_t* sampled;           // [present]: the token fed back to a row with tok_src < 0 (its own last pick), overwritten by the row's greedy pick
+    uint8_t* xch;                // exchange sets of every part, batch_sets_bytes() each: all 0xff before the first launch
+    batch::State* state;         // of every part, zero before the first launch
+    uint32_t* sampled;           // [seqs]: the token fed back to a row with tok_src < 0 (its own last pick), overwritten by the row's greedy pick
     // The step, in device memory or (rows == nullptr) by value
-    const int32_t* rows;         // [present] of int4 {tok_src, pos, slot, seq}
-    const int32_t* kv_lens;      // [present]: positions attended to, the new one included; 0: the row is not there
+    const int32_t* rows;         // [seqs] of int4 {tok_src, pos, slot, seq}
+    const int32_t* kv_lens;      // [seqs]: positions attended to, the new one included; 0: the row is not there
     int32_t tok_src[BATCH_ROWS], lens[BATCH_ROWS];
-    const int32_t* block_tables; // [present][max_blocks]
-    uint32_t* sampled_host;      // where else the picks go: [present] in mapped host memory, or nullptr
+    const int32_t* block_tables; // [seqs][max_blocks]
+    uint32_t* sampled_host;      // where else the picks go: [seqs] in mapped host memory and behind them the status word, or nullptr
     uint32_t* status;            // device word: made non-zero when a wait runs out; a step that finds it so does nothing
-    uint32_t* status_host;       // the same for the host, or nullptr
     uint64_t max_cycles;         // time limit of the step, in SM clocks
-    uint32_t n_layers, dim, ffn, heads, vocab, max_blocks, max_len;
-    uint32_t seqs, present;      // rows of a part (the plan goes by them), rows that this one has
-    uint32_t sms;                // blocks the part is divided over
+    uint32_t n_layers, dim, ffn, heads, vocab, seqs, max_blocks, max_len;
+    uint32_t sms;                // blocks a part is divided over
+    uint32_t part_seqs, part_bytes;   // rows and bytes of sets of a part (batch_plan.h)
     float eps, scale;
 };
 
@@ -39,8 +37,8 @@ int batch_maps(void* out, const SoloLayer* layers, const void* lm_head, uint32_t
 // a part's sets; seqs: of a part
 size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t max_len);
 constexpr uint64_t BATCH_MAX_CYCLES = 1ull << 32;   // two seconds or so, for a step of milliseconds
-// n parts. missing: blocks left out, so that the others' waits run out (a drill)
-int launch_batch(cudaStream_t st, const BatchArgs* parts, uint32_t n, uint32_t missing = 0);
+// missing: blocks left out, so that the others' waits run out (a drill)
+int launch_batch(cudaStream_t st, const BatchArgs& a, uint32_t missing = 0);
 int batch_status(unsigned int* out);
 
 }  // namespace ak

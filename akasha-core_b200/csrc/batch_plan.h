@@ -147,7 +147,7 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
     const uint32_t splits = div_up(max_len, split_len(max_len, hd));
     const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms);
     if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * sms * (NW / p.wpi)) return false;
-    return p.slots >= 4 && sets_bytes(dim, ffn, heads, seqs, max_len) < (1ull << 32);
+    return p.slots >= 4 && MAX_PARTS * sets_bytes(dim, ffn, heads, seqs, max_len) < (1ull << 32);   // (offsets of 32 bits; four slots: what a pass holds at a time)
 }
 
 // SMs of a step with prompts beside it, whose chain of launches gets the others. The chain is the longer of the two in almost every such step, so the step

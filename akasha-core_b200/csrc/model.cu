@@ -399,70 +399,55 @@ int Runner::init_batch() {
     AK_TRY(batch_maps(host, solo_layers().data(), w_->lm_head, c.num_layers, c.dim, c.ffn_hidden, c.vocab_size));
     AK_CUDA(cudaMalloc(&d_batch_maps_, (4 * c.num_layers + 1) * 128));
     AK_CUDA(cudaMemcpyAsync(d_batch_maps_, host, (4 * c.num_layers + 1) * 128, cudaMemcpyHostToDevice, ctx_->stream));
-    const size_t bytes = batch_sets_bytes(c.dim, c.ffn_hidden, c.num_heads, batch::part_seqs(max_seqs_), max_seq_len_), part = bytes + sizeof(batch::State);
     const uint32_t parts = batch::parts_of(max_seqs_);
-    AK_CUDA(cudaMalloc((void**)&d_batch_xch_, parts * part));
-    AK_CUDA(cudaMemsetAsync(d_batch_xch_, 0xff, parts * part, ctx_->stream));
-    for (uint32_t i = 0; i < parts; i++) {
-        d_batch_state_[i] = reinterpret_cast<batch::State*>(d_batch_xch_ + i * part + bytes);
-        AK_CUDA(cudaMemsetAsync(d_batch_state_[i], 0, sizeof(batch::State), ctx_->stream));
-    }
+    batch_part_bytes_ = batch_sets_bytes(c.dim, c.ffn_hidden, c.num_heads, batch::part_seqs(max_seqs_), max_seq_len_);
+    const size_t bytes = parts * batch_part_bytes_, state = parts * sizeof(batch::State);
+    AK_CUDA(cudaMalloc((void**)&d_batch_xch_, bytes + state));
+    d_batch_state_ = reinterpret_cast<batch::State*>(d_batch_xch_ + bytes);
+    AK_CUDA(cudaMemsetAsync(d_batch_xch_, 0xff, bytes, ctx_->stream));
+    AK_CUDA(cudaMemsetAsync(d_batch_state_, 0, state, ctx_->stream));
     AK_CUDA(cudaStreamSynchronize(ctx_->stream));
     batch_ = true;
     return AK_OK;
 }
 
-uint32_t Runner::batch_args(BatchArgs* parts, bool beside) {
+BatchArgs Runner::batch_args() const {
     const ak_model_config& c = w_->cfg;
-    const uint32_t n = batch::parts_of(max_seqs_), seqs = batch::part_seqs(max_seqs_);
-    for (uint32_t i = 0; i < n; i++) {
-        BatchArgs& a = parts[i];
-        a = BatchArgs{};
-        const uint32_t r0 = i * seqs;
-        a.layers = d_batch_layers_;
-        a.embedding = w_->embedding;
-        a.final_norm = w_->final_norm;
-        a.maps = d_batch_maps_;
-        a.rope = rope_table_;
-        a.xch = d_batch_xch_ + i * (reinterpret_cast<uint8_t*>(d_batch_state_[0] + 1) - d_batch_xch_);
-        a.state = d_batch_state_[i];
-        a.sampled = d_sampled_ + r0;
-        a.block_tables = d_desc_ + d_.block_tables + (size_t)r0 * max_blocks_;
-        a.status = d_sampled_ + max_seqs_;
-        a.max_cycles = BATCH_MAX_CYCLES;
-        a.n_layers = c.num_layers; a.dim = c.dim; a.ffn = c.ffn_hidden; a.heads = c.num_heads; a.vocab = c.vocab_size;
-        a.max_blocks = max_blocks_; a.max_len = max_seq_len_;
-        a.seqs = seqs;
-        a.present = std::min(seqs, max_seqs_ - r0);
-        if (beside) {
-            a.rows = d_desc_ + d_.rows + r0 * 4;
-            a.kv_lens = d_desc_ + d_.kv_lens + r0;
-            a.sms = batch::sms_beside(c.dim, c.num_layers, c.num_heads, seqs, max_seq_len_, n);
-        } else {
-            for (uint32_t j = 0; j < a.present; j++) {
-                a.tok_src[j] = h_rows()[r0 + j].tok_src;
-                a.lens[j] = h_kv_lens()[r0 + j];
-            }
-            a.sampled_host = h_sampled_ + r0;
-            a.status_host = h_sampled_ + max_seqs_;
-            a.sms = B200_SMS / n;
-        }
-        a.eps = c.norm_eps;
-        a.scale = 1.0f / sqrtf((float)(c.dim / c.num_heads));
-    }
-    return n;
+    BatchArgs a{};
+    a.layers = d_batch_layers_;
+    a.embedding = w_->embedding;
+    a.final_norm = w_->final_norm;
+    a.maps = d_batch_maps_;
+    a.rope = rope_table_;
+    a.xch = d_batch_xch_;
+    a.state = d_batch_state_;
+    a.sampled = d_sampled_;
+    a.block_tables = d_desc_ + d_.block_tables;
+    a.status = d_sampled_ + max_seqs_;
+    a.max_cycles = BATCH_MAX_CYCLES;
+    a.n_layers = c.num_layers; a.dim = c.dim; a.ffn = c.ffn_hidden; a.heads = c.num_heads; a.vocab = c.vocab_size;
+    a.seqs = max_seqs_; a.max_blocks = max_blocks_; a.max_len = max_seq_len_;
+    a.part_seqs = batch::part_seqs(max_seqs_);
+    a.part_bytes = (uint32_t)batch_part_bytes_;
+    a.sms = B200_SMS / batch::parts_of(max_seqs_);
+    a.eps = c.norm_eps;
+    a.scale = 1.0f / sqrtf((float)(c.dim / c.num_heads));
+    return a;
 }
 
 // The block tables are on the device already: a sequence's were uploaded with its prompt's step, and they do not change. So neither a copy to
 // the device nor one back stands between two steps (162M model, 8 sequences: as a graph of copy, kernel, copy 15 us more per step).
 int Runner::run_decode_batch() {
     AK_CUDA(cudaSetDevice(ctx_->device));
-    BatchArgs parts[batch::MAX_PARTS];
-    const uint32_t n = batch_args(parts, false);
-    if (drill_cycles_)
-        for (BatchArgs& a : parts) a.max_cycles = drill_cycles_;
+    BatchArgs a = batch_args();
+    for (uint32_t i = 0; i < max_seqs_; i++) {
+        a.tok_src[i] = h_rows()[i].tok_src;
+        a.lens[i] = h_kv_lens()[i];
+    }
+    a.sampled_host = h_sampled_;
+    if (drill_cycles_) a.max_cycles = drill_cycles_;
     const auto h0 = std::chrono::steady_clock::now();
-    AK_TRY(launch_batch(ctx_->stream, parts, n, drill_cycles_ ? 1 : 0));
+    AK_TRY(launch_batch(ctx_->stream, a, drill_cycles_ ? 1 : 0));
     drill_cycles_ = 0;
     launch_host_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - h0).count();
     h2d_bytes += (size_t)max_seqs_ * 8;
@@ -671,9 +656,11 @@ int Runner::launch_layers(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, ui
             AK_CUDA(cudaStreamWaitEvent(st2_, ev_fork_, 0));
             rc = range(st2_, max_seqs_, T - max_seqs_, false, true);
             if (rc == AK_OK) {
-                BatchArgs parts[batch::MAX_PARTS];
-                const uint32_t n = batch_args(parts, true);
-                rc = launch_batch(st, parts, n);
+                BatchArgs a = batch_args();
+                a.rows = rows;
+                a.kv_lens = d_desc_ + d_.kv_lens;
+                a.sms = batch::sms_beside(c.dim, c.num_layers, c.num_heads, a.part_seqs, max_seq_len_, batch::parts_of(max_seqs_));
+                rc = launch_batch(st, a);
                 batch_ran_ = rc == AK_OK && !capturing;
             }
             AK_CUDA(cudaEventRecord(ev_join_, st2_));   // (what was launched is waited for whatever failed)

@@ -212,7 +212,8 @@ class Runner {
     uint8_t* d_batch_xch_ = nullptr;
     SoloLayer* d_batch_layers_ = nullptr;
     void* d_batch_maps_ = nullptr;
-    batch::State* d_batch_state_[batch::MAX_PARTS] = {};   // behind each part's exchange sets
+    batch::State* d_batch_state_ = nullptr;   // of every part, behind the exchange sets
+    size_t batch_part_bytes_ = 0;             // exchange sets of a part
     uint64_t drill_cycles_ = 0;
     bool batch_ran_ = false;            // a persistent step of the step being launched is on the stream
     int failed_ = 0;                    // the error after which this runner takes no step any more
@@ -220,7 +221,7 @@ class Runner {
     int launch_step(uint32_t T, uint32_t n_pf_rows, uint32_t n_pf_seqs, uint32_t max_pf_len, bool any_decode, uint32_t n_splits, size_t desc_bytes);
     std::vector<SoloLayer> solo_layers() const;
     int upload_layers(SoloLayer** out);
-    uint32_t batch_args(BatchArgs* parts, bool beside);   // the step's parts (beside: described in device memory, prompts' launches beside it); their number
+    BatchArgs batch_args() const;
     int run_decode_batch();             // a decode-only step: one launch, the step by value, the picks straight to the host
     size_t sampled_words() const { return max_seqs_ + 1; }   // the tokens, and the status word of the persistent step
     SoloArgs solo_args(int32_t tok_src, uint32_t pos);
