@@ -45,14 +45,17 @@ constexpr int THREADS = 512, FIRST_COMPUTE = 4;
 constexpr int REGS_FIRST = 80, REGS_COMPUTE = 144;
 static_assert(REGS_FIRST * 128 + REGS_COMPUTE * 384 <= 65536, "the split draws on the registers of the launch");
 constexpr uint32_t BLOCK_FAILED = 0xfffffffeu;   // in the place of the index of a block's best logit (0xffffffff: it has none)
-constexpr uint32_t REPLICAS = 4;         // copies of every exchanged value: an SM polls copy (SM mod 4). 148 SMs polling one 128-byte line
-                                         // occupy its L2 slice for ~300 cycles a round, and the store they wait for queues behind them
+// Copies of every exchanged value: an SM polls copy (SM mod copies), which spreads the polls over the L2. Since an SM asks only for what is missing, a copy
+// more costs about what it gives: bf16, 201 positions, 160.7 / 161.5 / 163.1 us a step with 1 / 2 / 4; f32 182.4 / 180.7 / 179.5, at 20 to 84 positions
+// (64 tokens generated) 13.24 / 13.19 / 13.29 ms.
+constexpr uint32_t MAX_REPLICAS = 2;
+template <typename T> __device__ constexpr uint32_t replicas() { return sizeof(T) == 4 ? MAX_REPLICAS : 1; }
 
 // ---- flagged exchange: {value, step} in one 64-bit word
-__device__ __forceinline__ void ll_put(uint64_t* p, size_t copy_stride, float v, uint32_t ep) {
+template <uint32_t N> __device__ __forceinline__ void ll_put(uint64_t* p, size_t copy_stride, float v, uint32_t ep) {
     const uint64_t word = (uint64_t)__float_as_uint(v) | ((uint64_t)ep << 32);
 #pragma unroll
-    for (uint32_t c = 0; c < REPLICAS; c++) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p + c * copy_stride), "l"(word) : "memory");
+    for (uint32_t c = 0; c < N; c++) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p + c * copy_stride), "l"(word) : "memory");
 }
 __device__ __forceinline__ void ll_ld2(const uint64_t* p, uint64_t& a, uint64_t& b) {
     asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
@@ -76,17 +79,19 @@ struct Waiter {   // bounds the polling of one thread; `dead` is sticky for the 
         return false;
     }
 };
-// n <= N value pairs at p, p + stride, ... (in words), all requested at once
+// n <= N value pairs at p, p + stride, ... (in words), all requested at once and then again as long as they are missing
 template <int N>
 __device__ __forceinline__ void poll_pairs(const uint64_t* p, uint32_t stride, uint32_t n, uint32_t ep, Waiter w, float2 (&v)[N]) {
     uint64_t a[N], b[N];
     uint32_t tries = 0;
     long long t0 = 0;
+#pragma unroll
+    for (int i = 0; i < N; i++) a[i] = b[i] = 0;   // (step 0 is none)
     for (;;) {
         bool ok = true;
 #pragma unroll
-        for (int i = 0; i < N; i++)
-            if ((uint32_t)i < n) ll_ld2(p + (size_t)i * stride, a[i], b[i]);
+        for (int i = 0; i < N; i++)   // what is not there yet (the polls of 148 SMs hold up each other and the stores they wait for)
+            if ((uint32_t)i < n && !(ll_ok(a[i], ep) && ll_ok(b[i], ep))) ll_ld2(p + (size_t)i * stride, a[i], b[i]);
 #pragma unroll
         for (int i = 0; i < N; i++)
             if ((uint32_t)i < n) ok = ok && ll_ok(a[i], ep) && ll_ok(b[i], ep);
@@ -174,6 +179,11 @@ template <> struct Vec<bf16> {
     }
 };
 
+__device__ __forceinline__ float redux_max(float v) {   // of the warp (a NaN is left out)
+    float m;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
+    return m;
+}
 // 1 / sqrt(m): the hardware's approximation and one Newton step (below 1 ulp). The step has no value where m is 0 or infinite (a
 // residual stream whose squares overflow): there the approximation is exact.
 __device__ __forceinline__ float inv_rms(float m) {
@@ -372,6 +382,7 @@ struct XchOff {   // word offsets inside a layer's exchange region
 
 template <typename T, int HD>
 __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant__ SoloArgs a, const uint32_t slots) {
+    constexpr uint32_t REPLICAS = replicas<T>();
     constexpr int EPV = Vec<T>::N;
     constexpr int VR = HD / EPV;             // 16-byte vectors per cache row
     constexpr int RPI = 32 / VR;             // rows a warp loads per instruction
@@ -487,23 +498,32 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
             if (ph == 1 && attends) {
                 bar_block();
                 // warps without a unit left max = -inf, sum = 0, accumulator 0
-                float f[NW], M = p_m[0], ls = 0.0f, o[HD / 32];
+                float f[NA], M, ls = 0.0f, o[HD / 32];
+                if constexpr (sizeof(T) == 4) {   // (an expf is long: lane i finds warp i's factor. With exponentials of the hardware that is no gain)
+                    const float pm = lane < NA ? p_m[lane] : -INFINITY;
+                    M = redux_max(pm);
+                    const float fl = ex(pm - M);
 #pragma unroll
-                for (int i = 1; i < NW; i++) M = fmaxf(M, p_m[i]);
+                    for (int i = 0; i < (int)NA; i++) f[i] = __shfl_sync(0xffffffffu, fl, i);
+                } else {
+                    M = p_m[0];
 #pragma unroll
-                for (int i = 0; i < NW; i++) f[i] = ex(p_m[i] - M);
+                    for (int i = 1; i < (int)NA; i++) M = fmaxf(M, p_m[i]);
+#pragma unroll
+                    for (int i = 0; i < (int)NA; i++) f[i] = ex(p_m[i] - M);
+                }
 #pragma unroll
                 for (int e = 0; e < HD / 32; e++) o[e] = 0.0f;
 #pragma unroll
-                for (int i = 0; i < NW; i++) {
+                for (int i = 0; i < (int)NA; i++) {
                     ls = fmaf(p_l[i], f[i], ls);
 #pragma unroll
                     for (int e = 0; e < HD / 32; e++) o[e] = fmaf(p_acc[i][e * 32 + lane], f[i], o[e]);
                 }
                 uint64_t* const out = xl + xo.att + (size_t)split * (D + 2 * H);
 #pragma unroll
-                for (int e = 0; e < HD / 32; e++) ll_put(out + head * HD + e * 32 + lane, copy, splits == 1 ? o[e] / ls : o[e], ep);
-                if (splits > 1 && lane < 2) ll_put(out + D + 2 * head + lane, copy, lane == 0 ? M : ls, ep);
+                for (int e = 0; e < HD / 32; e++) ll_put<REPLICAS>(out + head * HD + e * 32 + lane, copy, splits == 1 ? o[e] / ls : o[e], ep);
+                if (splits > 1 && lane < 2) ll_put<REPLICAS>(out + D + 2 * head + lane, copy, lane == 0 ? M : ls, ep);
             }
             const Kind& d = kinds[ph];
             uint64_t* const out = xl + (ph == 0 ? xo.qkv : ph == 1 ? xo.hid1 : ph == 2 ? xo.up : xo.hid2) + d.r0;
@@ -531,7 +551,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
                 if (mine) {
                     // (bf16 weights: off by 2^-17 of the value at most, and 0 below about -87)
                     if (ph == 2) v = sizeof(T) == 4 ? v / (1.0f + expf(-v)) : __fdividef(v, 1.0f + __expf(-v));
-                    ll_put(dst, copy, v, ep);
+                    ll_put<REPLICAS>(dst, copy, v, ep);
                 }
             }
         }
@@ -553,8 +573,8 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
         if (a.logits_host) bar_block();   // the logits are on the host
         uint64_t* const fin = a.xch + (size_t)L * xo.total;
         if (lane == 0) {
-            ll_put(fin + 2 * cta, copy, bv, ep);
-            ll_put(fin + 2 * cta + 1, copy, __uint_as_float(*(volatile uint32_t*)&dead ? BLOCK_FAILED : bi), ep);
+            ll_put<REPLICAS>(fin + 2 * cta, copy, bv, ep);
+            ll_put<REPLICAS>(fin + 2 * cta + 1, copy, __uint_as_float(*(volatile uint32_t*)&dead ? BLOCK_FAILED : bi), ep);
         }
         if (cta != 0) return;
         bv = -INFINITY;
@@ -979,7 +999,7 @@ bool solo_supported(uint32_t dtype, uint32_t dim, uint32_t ffn, uint32_t heads, 
 }
 
 size_t solo_xch_words(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t n_layers) {
-    return REPLICAS * ((size_t)n_layers * XchOff(dim, ffn, heads).total + 2 * B200_SMS);
+    return MAX_REPLICAS * ((size_t)n_layers * XchOff(dim, ffn, heads).total + 2 * B200_SMS);
 }
 
 template <typename T, int HD>
