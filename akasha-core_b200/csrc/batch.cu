@@ -1,14 +1,15 @@
-// One decode step of up to 32 sequences (bf16 weights and cache) as a single persistent kernel: embedding, every layer,
+// One decode step of up to 64 sequences (bf16 weights and cache) as a single persistent kernel: embedding, every layer,
 // lm_head, greedy argmax.
 //
 // What bounds it. A decode-only step as a chain of 88 launches is bound by the launches: each is a boundary of ~2 us plus the latencies
-// of its first loads, 3 to 5 us for work of 0.1 to 1 us (162M model, 8 sequences of 300: 0.39 ms; the bytes take 0.05 ms). Here, as in the
-// batch-1 step (solo.cu), a layer is five phases of one kernel and only activations cross the chip:
+// of its first loads, 3 to 5 us for work of 0.1 to 1 us (162M model, contexts of 300: 8 sequences 0.39 ms, 64 0.49; the bytes take 0.05 and
+// 0.15 ms). Here, as in the batch-1 step (solo.cu), a layer is five phases of one kernel and only activations cross the chip:
 //   qkv rows -> attention (sequence, head) -> out-proj rows -> ffn-up rows -> ffn-down rows.
-// That step takes 0.187 ms (1 sequence 0.17, 16 of 350 0.25, 32 of 350 0.334; 320-wide model, 21 sequences 0.22 -> 0.127; 1.4B model, 16 of 1600
-// 2.5 -> 2.1). With 64 sequences a form of it (since deleted) was slower than the chain: every SM reads all activations, 0.58 against 0.49 ms. Hence the
-// limit of 32. What is left is latency: per phase the way from a store to the last SM's poll, and dependent instructions (with everything
-// between two phases done by the same warps it was 0.29 ms).
+// That step takes 0.180 ms with 8 sequences, 0.219 with 16, 0.305 with 32, 0.414 with 64 (320-wide model, 21 sequences 0.126; 1.4B model, 16 of 1600
+// 1.85). What is left is latency: per phase the way from a store to the last SM's poll, and dependent instructions (with everything between
+// two phases done by the same warps it was 0.29 ms for 8).
+//   * Every SM reads all activations of a phase, which is what grows with the sequences. More than 32 are two parts: half of the sequences and half of
+//     the SMs each, all weights, nothing between the two. 64 sequences: 0.49 ms as launches, 0.58 with 64 rows on every SM, 0.414 in parts.
 //   * A producer thread per SM walks the SM's weight tiles of all phases in order and keeps a shared-memory ring of tensor loads full.
 //   * A phase's rows are dealt to the SMs in tiles of 8, all of K: no sum crosses SMs. The 12 compute warps split K and leave partial tiles in
 //     shared memory; three epilogue warps add them in warp order and publish, while the compute warps are already at the next phase. The
@@ -23,7 +24,7 @@
 //   * RMS norm: the producer of the residual stream publishes x * gain rounded to bf16 (one rounding, as of the normalised value) and
 //     the sums of squares of its columns; 1 / rms is a factor of the row sums of the next phase, found by the epilogue warps meanwhile.
 //   * The residual stream stays in shared memory of the SM that owns its columns (out-proj and ffn-down have the same tiles).
-//   * Attention: a unit is (sequence, head, split of split_len positions); units are dealt to groups of 4 or 12 warps in order of length. Keys
+//   * Attention: a unit is (sequence, head, split of split_len positions); units are dealt to groups of 2 to 12 warps in order of length. Keys
 //     and values go through per-warp shared-memory buffers, the next layer's first tiles already while this layer's ffn runs. Scores are
 //     mma.m16n8k16 (7/8 of it for nothing, but an eighth of the instructions of f32 FMAs); P V is f32 FMAs, the transposing loads that an
 //     MMA would need have 8-way bank conflicts on unswizzled tiles (32 sequences: 0.41 ms instead of 0.35).
@@ -123,7 +124,7 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {   // (a NaN become
 template <uint32_t N> __device__ __forceinline__ void bar_sync(uint32_t id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(N) : "memory"); }
 __device__ __forceinline__ void bar_sync_n(uint32_t id, uint32_t n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 template <uint32_t N> __device__ __forceinline__ void bar_arrive(uint32_t id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(N) : "memory"); }
-enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_GROUP = 4, BAR_FLAT = 7 };   // BAR_GROUP and the next two: by group
+enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_FLAT = 4, BAR_GROUP = 5 };   // BAR_GROUP and the next five: by group
 
 __device__ __forceinline__ uint64_t policy_evict_first() {
     uint64_t p;
@@ -193,7 +194,7 @@ constexpr uint32_t NO_LOGIT = 0x7fffffffu;   // in the place of the index of a b
 
 // SPLIT: sequences may be longer than an attention unit
 template <int HD, int MT, bool SPLIT, int PARTS>
-__global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant__ BatchArgs a, const uint32_t slots, const uint32_t wpi) {
+__global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant__ BatchArgs a, const uint32_t slots, const uint32_t wpi, const uint32_t inv_wpi) {
     constexpr uint32_t R = MT * 16;               // rows of the exchange buffers
     constexpr uint32_t PPC = CHUNK / NW;          // slices of a ring chunk that a warp has: 2
     constexpr bool KEEP = PARTS > 1;              // activations stay in registers for the passes of a phase (half of the SMs have twice the tiles)
@@ -735,8 +736,10 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 
     uint32_t tiles_done = 0;   // parity of the tiles worked through
     // ---- attention: units of this warp's group. What a warp keeps of it between layers is in shared memory (the projections need the registers).
-    auto group_of = [&]() { return wpi == NW ? 0u : cw >> 2; };     // wpi is 12 or 4
-    auto place_in = [&]() { return wpi == NW ? cw : cw & 3u; };
+    // (a multiplication by inv_wpi = 65536 / wpi + 1 divides the small numbers here)
+    auto group_of = [&]() { return cw * inv_wpi >> 16; };
+    auto in_group = [&](uint32_t i) { return i - (i * inv_wpi >> 16) * wpi; };   // i mod wpi
+    auto place_in = [&]() { return in_group(cw); };
     {   // unit j in lane j: row | head << 6 | split << 18
         const uint32_t grp = group_of();
         const uint32_t groups = a.sms * (NW / wpi), gid = grp * a.sms + cta;
@@ -852,7 +855,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             if (wg < u.nb) {
                 // This lane's 8 columns of the new token's query; of the newest tile's warp also of its key and value, which go to the pools and
                 // (below) into the tile. All of it, the rotation's factors and the place in the pools are asked for together.
-                const bool owner = newest && wg == (wpi == NW ? (u.nb - 1) % NW : (u.nb - 1) & 3u);
+                const bool owner = newest && wg == in_group(u.nb - 1);
                 const uint8_t* const src = qkv + ((size_t)u.row * 3 * D + u.head * HD + chunk * 8) * 4;
                 const float4* const rt = reinterpret_cast<const float4*>(a.rope + (size_t)pos * (HD / 2) + chunk * 4);
                 const float4 r0 = __ldg(rt), r1 = __ldg(rt + 1);
@@ -992,7 +995,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             }
             if (lane == 0) at_ml[buf][cw] = make_float2(m, l);
             bar_sync_n(BAR_GROUP + grp, wpi * 32);
-            if (wg == j % wpi) {   // one warp merges the group's, in warp order
+            if (wg == in_group(j)) {   // one warp merges the group's, in warp order
                 const float2 ml = lane < wpi ? at_ml[buf][grp * wpi + lane] : make_float2(-INFINITY, 0.0f);
                 const float M = redux_max(ml.x), f = ex2(ml.x - M), ls = warp_sum(ml.y * f);
                 float o[DL];
@@ -1000,7 +1003,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 for (uint32_t e = 0; e < DL; e++) o[e] = 0.0f;
                 const float* src = at_acc + (buf * NW + grp * wpi) * HD + lane * DL;
 #pragma unroll 4
-                for (uint32_t w = 0; w < wpi; w++) {   // (wpi is 4 or 12)
+                for (uint32_t w = 0; w < wpi; w++) {
                     const float fw = __shfl_sync(0xffffffffu, f, w);
 #pragma unroll
                     for (uint32_t e = 0; e < DL; e++) o[e] = fmaf(src[w * HD + e], fw, o[e]);
@@ -1246,7 +1249,7 @@ int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p, uint32_t 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    AK_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel<HD, MT, SPLIT, PARTS>, a, p.slots, p.wpi));
+    AK_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel<HD, MT, SPLIT, PARTS>, a, p.slots, p.wpi, 65536 / p.wpi + 1));
     AK_COUNT_LAUNCH();
     return AK_OK;
 }
@@ -1275,7 +1278,7 @@ size_t batch_sets_bytes(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seq
 
 int launch_batch(cudaStream_t st, const BatchArgs& a, uint32_t missing) {
     const uint32_t n = parts_of(a.seqs), blocks = n * a.sms - missing;
-    const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.part_seqs, a.max_len, a.sms);
+    const Plan p = make_plan(a.dim, a.n_layers, a.heads, a.part_seqs, a.max_len, a.sms, n);
     const bool two = m_tiles(a.part_seqs) == 2, split = has_splits(a.max_len, a.dim / a.heads), hd64 = a.dim / a.heads == 64;
     if (n == 2) {   // (17 to 32 rows each)
         if (hd64) return split ? launch_batch_t<64, 2, true, 2>(st, a, p, blocks) : launch_batch_t<64, 2, false, 2>(st, a, p, blocks);

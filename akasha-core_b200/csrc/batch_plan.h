@@ -94,15 +94,25 @@ struct Plan {
     uint32_t slots, wpi;
     size_t smem;
 };
-inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len, uint32_t sms = SMS) {
+// seqs: of a part; sms: blocks of a part
+inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len, uint32_t sms = SMS, uint32_t parts = 1) {
     const uint32_t hd = dim / heads;
     const size_t rest = NW * 2 * KV_BUF + (size_t)NW * TB * m_tiles(seqs) * 16 * 32 + 2 * NW * hd * 4 + TB * 32 * 2 * 16 + (size_t)(2 * n_layers + 1) * div_up(dim / 8, sms) * 32;
     Plan p;
     p.slots = (uint32_t)((MAX_DYN_SMEM - rest) / SLOT);
     if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
     p.smem = p.slots * SLOT + rest;
-    // Few units: all warps of an SM work on one; else four, so that an SM's units overlap. (Not by the step's blocks: a unit's sums depend on it.)
-    p.wpi = seqs * heads * div_up(max_len, split_len(max_len, hd)) <= SMS ? 12 : 4;
+    // Warps of an attention unit. Whole sequences: as many as leave a group for every unit, because a group's second unit starts when the first is done. Contexts
+    // of 300, us per step, with 12 or 4 warps (all there was) and now: 162M model, 13 sequences 233 / 218 (6 warps), 16 234 / 219 (6), 24 283 / 265 (4), 40
+    // 374 / 341 (3), 48 381 / 353 (3), 64 417 / 414 (2); 320-wide model, 32 sequences 151 / 143 (6). Cut sequences: 12 or 4.
+    // (Not by the step's blocks: a unit's sums depend on it.)
+    const uint32_t splits = div_up(max_len, split_len(max_len, hd)), own = SMS / parts;
+    p.wpi = splits == 1 ? 2 : 4;
+    for (uint32_t w = NW; w > p.wpi; w--)
+        if (NW % w == 0 && seqs * heads * splits <= own * (NW / w) && (splits == 1 || w == NW)) {
+            p.wpi = w;
+            break;
+        }
     return p;
 }
 
@@ -145,7 +155,7 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
     if (div_up(dim / 8, sms) > TB) return false;                           // the residual stream is worked on in one pass
     if (dim * m_tiles(seqs) * 16 * 2 > NW * 2 * KV_BUF) return false;      // the lm_head keeps x where the cache tiles were
     const uint32_t splits = div_up(max_len, split_len(max_len, hd));
-    const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms);
+    const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms, SMS / sms);
     if (splits > 16383 || (uint64_t)seqs * heads * splits > (uint64_t)MAX_UNITS * sms * (NW / p.wpi)) return false;
     return p.slots >= 4 && MAX_PARTS * sets_bytes(dim, ffn, heads, seqs, max_len) < (1ull << 32);   // (offsets of 32 bits; four slots: what a pass holds at a time)
 }
@@ -160,7 +170,7 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
 inline uint32_t sms_beside(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len, uint32_t parts = 1) {
     const uint64_t units = (uint64_t)seqs * heads * div_up(max_len, split_len(max_len, dim / heads));
     for (uint32_t sms = SMS_BESIDE; sms < SMS / parts; sms++) {
-        const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms);
+        const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms, parts);
         if (div_up(dim / 8, sms) <= TB && units <= (uint64_t)MAX_UNITS * sms * (NW / p.wpi) && p.slots >= 4) return sms;
     }
     return SMS / parts;
