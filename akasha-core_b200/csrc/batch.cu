@@ -369,6 +369,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         // squares of the norms, the clearing of exchange sets.
         const uint32_t ht = tid - 32, e = warp_ - 1, h = lane & 1;   // lane: row 16 m + lane / 2, columns 4 h .. 4 h + 3 of the tile
         const uint32_t rl = lane >> 1;
+        constexpr uint32_t PB = 12;   // partial sums read together
         auto clear = [&](uint32_t g) {
             uint4* p = reinterpret_cast<uint4*>(a.xch + set_of(g));
             const uint32_t n = (uint32_t)(so.total / 16);
@@ -483,7 +484,6 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             float f[MT];
 #pragma unroll
             for (uint32_t m = 0; m < MT; m++) f[m] = 1.0f;
-            if (norm && tiles) factors(ph == QKV ? set_of(e0 + l) + so.s1 : set + so.s2, f);
             if (ph == OUT) wait_cleared(clears_before_out(l));
             // A row without a sequence is published as zeros where a row of its eight has one (the consumers look at whole eights only). Here its
             // attention, by the SM with the row's number among its qkv tiles.
@@ -518,18 +518,22 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                     }
                 }
                 const float* const o = part + e * (R * 8) + lane * 4;
+                if (norm && b == 0) factors(ph == QKV ? set_of(e0 + l) + so.s1 : set + so.s2, f);
                 bar_sync<NCT + NHT>(BAR_PART);
                 if (has) {
 #pragma unroll
                     for (uint32_t m = 0; m < MT; m++) {
                         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                        for (uint32_t w0 = 0; w0 < NW; w0 += 4) {   // four at a time (registers), in pairs
-                            float4 y[4];
+                        for (uint32_t w0 = 0; w0 < NW; w0 += PB) {
+                            float4 y[PB];
 #pragma unroll
-                            for (uint32_t w = 0; w < 4; w++) y[w] = *reinterpret_cast<const float4*>(o + (w0 + w) * (TB * R * 8) + m * 128);
-                            v.x += (y[0].x + y[1].x) + (y[2].x + y[3].x); v.y += (y[0].y + y[1].y) + (y[2].y + y[3].y);
-                            v.z += (y[0].z + y[1].z) + (y[2].z + y[3].z); v.w += (y[0].w + y[1].w) + (y[2].w + y[3].w);
+                            for (uint32_t w = 0; w < PB; w++) y[w] = *reinterpret_cast<const float4*>(o + (w0 + w) * (TB * R * 8) + m * 128);
+#pragma unroll
+                            for (uint32_t w = 0; w < PB; w += 4) {   // in pairs
+                                v.x += (y[w].x + y[w + 1].x) + (y[w + 2].x + y[w + 3].x); v.y += (y[w].y + y[w + 1].y) + (y[w + 2].y + y[w + 3].y);
+                                v.z += (y[w].z + y[w + 1].z) + (y[w + 2].z + y[w + 3].z); v.w += (y[w].w + y[w + 1].w) + (y[w + 2].w + y[w + 3].w);
+                            }
                         }
                         const uint32_t row = m * 16 + rl;
                         if (!norm) {
