@@ -24,7 +24,7 @@
 //   * RMS norm: the producer of the residual stream publishes x * gain rounded to bf16 (one rounding, as of the normalised value) and
 //     the sums of squares of its columns; 1 / rms is a factor of the row sums of the next phase, found by the epilogue warps meanwhile.
 //   * The residual stream stays in shared memory of the SM that owns its columns (out-proj and ffn-down have the same tiles).
-//   * Attention: a unit is (sequence, head, split of split_len positions); units are dealt to groups of 2 to 12 warps in order of length. Keys
+//   * Attention: a unit is (sequence, head, split of split_len positions); units are dealt to groups of 4, 6 or 12 warps in order of length. Keys
 //     and values go through per-warp shared-memory buffers, the next layer's first tiles already while this layer's ffn runs. Scores are
 //     mma.m16n8k16 (7/8 of it for nothing, but an eighth of the instructions of f32 FMAs); P V is f32 FMAs, the transposing loads that an
 //     MMA would need have 8-way bank conflicts on unswizzled tiles (32 sequences: 0.41 ms instead of 0.35).
@@ -124,12 +124,17 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {   // (a NaN become
 template <uint32_t N> __device__ __forceinline__ void bar_sync(uint32_t id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(N) : "memory"); }
 __device__ __forceinline__ void bar_sync_n(uint32_t id, uint32_t n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 template <uint32_t N> __device__ __forceinline__ void bar_arrive(uint32_t id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(N) : "memory"); }
-enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_FLAT = 4, BAR_GROUP = 5 };   // BAR_GROUP and the next five: by group
+enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_FLAT = 4, BAR_GROUP = 5 };   // BAR_GROUP and the next two: by group
 
 __device__ __forceinline__ uint64_t policy_evict_first() {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
     return p;
+}
+__device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t pol) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
+                 : "memory");
 }
 __device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -194,8 +199,9 @@ constexpr uint32_t NO_LOGIT = 0x7fffffffu;   // in the place of the index of a b
 
 // SPLIT: sequences may be longer than an attention unit
 template <int HD, int MT, bool SPLIT, int PARTS>
-__global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant__ BatchArgs a, const uint32_t slots, const uint32_t wpi, const uint32_t inv_wpi) {
+__global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant__ BatchArgs a, const uint32_t slots, const uint32_t wpi, const uint32_t inv_wpi, const uint32_t ahead) {
     constexpr uint32_t R = MT * 16;               // rows of the exchange buffers
+    constexpr bool CAN_AHEAD = can_ahead(HD, MT);
     constexpr uint32_t PPC = CHUNK / NW;          // slices of a ring chunk that a warp has: 2
     constexpr bool KEEP = PARTS > 1;              // activations stay in registers for the passes of a phase (half of the SMs have twice the tiles)
     constexpr uint32_t Q = R / 4, TPL = 32 / Q;   // lanes that read a tile's sums of squares, tiles per load
@@ -307,6 +313,30 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         Cursor q;
         uint32_t sent = 0;
         bool ok = true;
+        // `ahead` chunks further on, the weights are brought into L2 (a walk of its own over phase, first tile of a pass, chunk, tile of the pass)
+        struct { uint32_t i, b, c, t; } pf = {0, 0, 0, 0};
+        auto skip_empty = [&]() {
+#pragma unroll 1
+            while (pf.i < 4 * L && kinds[pf.i & 3].n == 0) pf.i++;
+        };
+        auto prefetch_next = [&](bool fetch) {
+            if (pf.i >= 4 * L) return;
+            const Kind& k = kinds[pf.i & 3];
+            if (fetch) tma_prefetch_rows(map + pf.i, pf.c * k.pieces, (k.t0 + pf.b + pf.t) * 8);
+            if (++pf.t < min(TB, k.n - pf.b)) return;
+            pf.t = 0;
+            if (++pf.c < k.chunks) return;
+            pf.c = 0;
+            if ((pf.b += TB) < k.n) return;
+            pf.b = 0;
+            pf.i++;
+            skip_empty();
+        };
+        if constexpr (CAN_AHEAD) {
+            skip_empty();
+#pragma unroll 1
+            for (uint32_t n = 0; ahead && n < slots + ahead; n++) prefetch_next(n >= slots);
+        }
 #pragma unroll 1
         for (uint32_t i = 0; i < 4 * L && ok; i++) {
             const Kind& d = kinds[i & 3];
@@ -323,6 +353,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                         tma_load_rows(smem + q.s * SLOT, map + i, c * d.pieces, (d.t0 + b + t) * 8, &full_bar[q.s], pol);
                         sent++;
                         q.advance(1, slots);
+                        if (CAN_AHEAD && ahead) prefetch_next(true);
                     }
                 }
             }
@@ -795,8 +826,9 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             uint8_t* dst = values ? vbuf : kbuf;
             constexpr uint32_t TILE = 16 * HD * 2;
             mbar_expect_tx(bar, UP > 16 && pb1 != EMPTY ? 2 * TILE : TILE);
-            bulk_g2s(dst, pool + (size_t)pb0 * H * (16 * HD), TILE, bar);
-            if (UP > 16 && pb1 != EMPTY) bulk_g2s(dst + TILE, pool + (size_t)pb1 * H * (16 * HD), TILE, bar);
+            const uint64_t pol = policy_evict_first();   // (read once a step; the exchange sets and weights stay in L2: 64 sequences 398 instead of 408 us)
+            bulk_g2s_hint(dst, pool + (size_t)pb0 * H * (16 * HD), TILE, bar, pol);
+            if (UP > 16 && pb1 != EMPTY) bulk_g2s_hint(dst + TILE, pool + (size_t)pb1 * H * (16 * HD), TILE, bar, pol);
             k.asked = !values;
             if (values) {
                 k.sent++;
@@ -1253,7 +1285,7 @@ int launch_batch_t(cudaStream_t st, const BatchArgs& a, const Plan& p, uint32_t 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    AK_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel<HD, MT, SPLIT, PARTS>, a, p.slots, p.wpi, 65536 / p.wpi + 1));
+    AK_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel<HD, MT, SPLIT, PARTS>, a, p.slots, p.wpi, 65536 / p.wpi + 1, ahead_of(a.dim, a.ffn, a.heads, a.part_seqs, a.sms, p.slots)));
     AK_COUNT_LAUNCH();
     return AK_OK;
 }

@@ -102,18 +102,24 @@ inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t 
     p.slots = (uint32_t)((MAX_DYN_SMEM - rest) / SLOT);
     if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
     p.smem = p.slots * SLOT + rest;
-    // Warps of an attention unit. Whole sequences: as many as leave a group for every unit, because a group's second unit starts when the first is done. Contexts
-    // of 300, us per step, with 12 or 4 warps (all there was) and now: 162M model, 13 sequences 233 / 218 (6 warps), 16 234 / 219 (6), 24 283 / 265 (4), 40
-    // 374 / 341 (3), 48 381 / 353 (3), 64 417 / 414 (2); 320-wide model, 32 sequences 151 / 143 (6). Cut sequences: 12 or 4.
+    // Warps of an attention unit. Whole sequences: 12, 6 or 4, the most that leave a group for every unit, because a group's second unit starts when the first is done
+    // (where four do not either, long units share a group with short ones). Contexts of 300, us per step, with 12 or 4 and now 6: 162M model, 13 sequences
+    // 233 / 218, 16 234 / 219, 24 283 / 265; 320-wide model, 32 sequences 151 / 143. Fewer than four give 64 equal sequences 417 / 414, but a
+    // long one among others then takes long: 128 ragged sequences through 64 slots 359 / 375 ms. Cut sequences: 12 or 4.
     // (Not by the step's blocks: a unit's sums depend on it.)
-    const uint32_t splits = div_up(max_len, split_len(max_len, hd)), own = SMS / parts;
-    p.wpi = splits == 1 ? 2 : 4;
-    for (uint32_t w = NW; w > p.wpi; w--)
-        if (NW % w == 0 && seqs * heads * splits <= own * (NW / w) && (splits == 1 || w == NW)) {
-            p.wpi = w;
-            break;
-        }
+    const uint32_t splits = div_up(max_len, split_len(max_len, hd)), units = seqs * heads * splits, own = SMS / parts;
+    p.wpi = units <= own ? 12 : units <= 2 * own && splits == 1 ? 6 : 4;
     return p;
+}
+// Chunks of weights that are brought into L2 ahead of the ring of `slots`. Where the ring holds about a layer and the layer is short (16 rows at most), four more
+// close its gaps: 162M model, contexts of 300, us per step without / with: 1 sequence 160 / 147, 8 176 / 163, 16 211 / 202 (with 8 chunks 164 and 203, with 16
+// 166 and 205); 320-wide, 8 sequences 102 / 100. With 32 rows 294 / 295, 64 sequences 397 / 401, and models that stream many rings a layer
+// (1.4B, 4 sequences of 500: 961 / 977; for head size 128 the walk is left out) are without.
+AK_PLAN_FN constexpr bool can_ahead(uint32_t hd, uint32_t mt) { return hd == 64 && mt == 1; }
+AK_PLAN_FN constexpr uint32_t ahead_of(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t seqs, uint32_t sms, uint32_t slots) {
+    const uint32_t kd = div_up(dim, CHUNK * 32), kf = div_up(ffn, CHUNK * 32);
+    const uint32_t layer = (div_up(3 * dim / 8, sms) + div_up(dim / 8, sms) + div_up(ffn / 8, sms)) * kd + div_up(dim / 8, sms) * kf;
+    return can_ahead(dim / heads, m_tiles(seqs)) && layer <= 2 * slots ? 4 : 0;
 }
 
 // An attention unit: positions p0 .. p0 + n of (row, head), nb tiles.

@@ -37,6 +37,10 @@ __device__ __forceinline__ void tma_load_rows(void* smem_dst, const CUtensorMap*
         "l"(tmap), "r"(smem_u32(bar)), "r"(0), "r"(piece), "r"(row), "l"(pol)
         : "memory");
 }
+// The same box brought into L2
+__device__ __forceinline__ void tma_prefetch_rows(const CUtensorMap* tmap, int32_t piece, int32_t row) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];" ::"l"(tmap), "r"(0), "r"(piece), "r"(row) : "memory");
+}
 // Tiled 2-D store from shared memory (elements outside the tensor are not written), and the same adding into f32. The
 // shared-memory writes must be ordered before it with tma_store_fence() in the writing threads and a barrier.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, const void* smem_src, int32_t x, int32_t y) {
