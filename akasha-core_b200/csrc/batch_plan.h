@@ -16,10 +16,10 @@ namespace ak {
 namespace batch {
 
 constexpr uint32_t SMS = 148;             // one block per SM
-constexpr uint32_t SMS_BESIDE = 48;       // the fewest blocks of a step beside prompts
+constexpr uint32_t SMS_BESIDE = 48, SMS_BESIDE_PARTS = 34;   // the fewest blocks of a step beside prompts; of each of its parts
 constexpr uint32_t ROWS = 32;             // most sequences of a part
 constexpr uint32_t MAX_PARTS = 2;
-static_assert(SMS_BESIDE >= ROWS, "block r picks the token of row r");
+static_assert(SMS_BESIDE_PARTS >= ROWS && SMS_BESIDE >= ROWS, "block r picks the token of row r");
 constexpr uint32_t NW = 12;               // compute warps
 constexpr uint32_t NH = 3;                // epilogue warps
 constexpr uint32_t TB = 3;                // weight tiles of a pass (accumulators, partial sums)
@@ -172,10 +172,11 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
 // 33.1, 60 32.7, 48 30.7 (all rows through the chain, which shares its launches then: 31.2); 8 slots, prompts of 16 to 448, 2 tokens: 20.8, 19.2, 18.9,
 // 18.9, 18.5 (19.8); 320-wide model, 32 slots: 20.8, 16.7, 16.0, 15.9, 15.9 (17.2); 1.4B model (86 SMs at least), 16 slots, prompts of 1 to
 // 64, 4 tokens: 57.5, 55.8, 54.9 (53.9: both read all weights), prompts of 128 to 1024: 128.7, 129.3, 127.9 (128.8).
-// (of a part; seqs: the part's)
+// Of each of two parts (seqs: the part's), 64 slots of the 162M model, with 34 / 48 / 60 / 74 SMs: 192 prompts of 1 to 24, 8 tokens on average, 17.7 / 18.9 / 20.4 /
+// 20.8 ms (all rows through the chain 18.3); of 16 to 448, 4 tokens 21.5 / 21.5 / 22.0 / 22.4 (22.3), 32 tokens 89.9 / 92.7 / 97.7 / 101.1 (101.2).
 inline uint32_t sms_beside(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t seqs, uint32_t max_len, uint32_t parts = 1) {
     const uint64_t units = (uint64_t)seqs * heads * div_up(max_len, split_len(max_len, dim / heads));
-    for (uint32_t sms = SMS_BESIDE; sms < SMS / parts; sms++) {
+    for (uint32_t sms = parts == 1 ? SMS_BESIDE : SMS_BESIDE_PARTS; sms < SMS / parts; sms++) {
         const Plan p = make_plan(dim, n_layers, heads, seqs, max_len, sms, parts);
         if (div_up(dim / 8, sms) <= TB && units <= (uint64_t)MAX_UNITS * sms * (NW / p.wpi) && p.slots >= 4) return sms;
     }
