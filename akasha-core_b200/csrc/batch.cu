@@ -126,11 +126,6 @@ __device__ __forceinline__ void bar_sync_n(uint32_t id, uint32_t n) { asm volati
 template <uint32_t N> __device__ __forceinline__ void bar_arrive(uint32_t id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(N) : "memory"); }
 enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_FLAT = 4, BAR_GROUP = 5 };   // BAR_GROUP and the next two: by group
 
-__device__ __forceinline__ uint64_t policy_evict_first() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
 __device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t pol) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(smem_u32(dst)),
                  "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
@@ -309,7 +304,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         // bulk copies of their own took 0.6 us to issue: 3 TB/s over the chip)
         if (lane != 0) return;
         const CUtensorMap* const map = reinterpret_cast<const CUtensorMap*>(a.maps);
-        const uint64_t pol = policy_evict_first();
+        const uint64_t pol = stays_in_l2(step_weight_bytes(2, D, F, L, a.vocab)) ? policy_evict_normal() : policy_evict_first();
         Cursor q;
         uint32_t sent = 0;
         bool ok = true;

@@ -139,11 +139,6 @@ __device__ __forceinline__ void bar_block() { asm volatile("bar.sync 1, %0;" ::"
 __device__ __forceinline__ void bar_ss_arrive() { asm volatile("bar.arrive 2, %0;" ::"n"(NC) : "memory"); }
 __device__ __forceinline__ void bar_ss_wait() { asm volatile("bar.sync 2, %0;" ::"n"(NC) : "memory"); }
 
-__device__ __forceinline__ uint64_t policy_evict_first() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
 __device__ __forceinline__ void bulk_g2s_stream(void* dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t pol) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(smem_u32(dst)),
                  "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
@@ -437,7 +432,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_kernel(const __grid_constant_
     if (warp_ == 0) {
         // ---------------- producer: this SM's weight rows, in the order the compute warps use them (lane 0), and the cache
         // tiles of its attention share (lane i: those of compute warp i)
-        const uint64_t pol = policy_evict_first();
+        const uint64_t pol = stays_in_l2(step_weight_bytes(sizeof(T), D, F, L, V)) ? policy_evict_normal() : policy_evict_first();
         Cursor q;
         uint32_t sent = 0, kv_sent = 0;
         bool ok = true;
