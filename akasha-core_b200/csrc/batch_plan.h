@@ -105,10 +105,12 @@ inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t 
     // Warps of an attention unit. Whole sequences: 12, 6 or 4, the most that leave a group for every unit, because a group's second unit starts when the first is done
     // (where four do not either, long units share a group with short ones). Contexts of 300, us per step, with 12 or 4 and now 6: 162M model, 13 sequences
     // 233 / 218, 16 234 / 219, 24 283 / 265; 320-wide model, 32 sequences 151 / 143. Fewer than four give 64 equal sequences 417 / 414, but a
-    // long one among others then takes long: 128 ragged sequences through 64 slots 359 / 375 ms. Cut sequences: 12 or 4.
+    // long one among others then takes long: 128 ragged sequences through 64 slots 359 / 375 ms. Cut sequences: 12 up to one unit per SM, else 4, or
+    // 3 of head size 128, whose units are 16 tiles: 1.4B model, with 4 / 3 / 2 warps: 16 sequences of 128 to 3072 positions 1944 / 1880 / 2026, 8 1441 / 1383 / 1477,
+    // 16 of 1600 1793 / 1794 / 1830 (head size 64, 2048 positions: 8 sequences 266 / 290 / 254, 32 641 / 621 / 667, 320-wide model, 21 188 / 207 / 181).
     // (Not by the step's blocks: a unit's sums depend on it.)
     const uint32_t splits = div_up(max_len, split_len(max_len, hd)), units = seqs * heads * splits, own = SMS / parts;
-    p.wpi = units <= own ? 12 : units <= 2 * own && splits == 1 ? 6 : 4;
+    p.wpi = units <= own ? 12 : splits > 1 ? (hd == 128 ? 3 : 4) : units <= 2 * own ? 6 : 4;
     return p;
 }
 // Chunks of weights that are brought into L2 ahead of the ring of `slots`. Where the ring holds about a layer and the layer is short (16 rows at most), four more
