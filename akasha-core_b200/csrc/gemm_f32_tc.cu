@@ -7,8 +7,11 @@
 // with ordinary f32 additions; the others', 2^-8 of it, runs through a segment.
 //
 // What bounded the FMA kernel it replaces is the FMA pipe and the shared-memory words that feed it (a 512-token prefill of the 162M model ran at 40 % of
-// 74 TFLOP/s). Here a K block of a 128 x 128 tile takes 24 MMAs of 64 cycles and about as many issue slots for the split and the additions (warps of
-// their own for each), and 64 KB from L2; a 128 x 64 tile asks for half as much again of both per product and ran at 0.6 of the rate.
+// 74 TFLOP/s). Here a K block of a 128 x 128 tile takes 1.9 us: 24 MMAs of 64 cycles (1536), and about 3300 cycles of shared memory, which both operands
+// go through as f32, as pieces, and as what the MMAs read; the split and the additions have warps of their own and as many issue slots as the MMAs have
+// cycles. A 128 x 64 tile asks for half as much again per product and ran at 0.6 of the rate. A launch costs about 7 us beside its blocks (its
+// shared memory leaves the next one no room to start early). m x n x k 512 x 2304 x 768: 52 -> 20 us, 512 x 768 x 3072 60 -> 26, 64 x 3072 x 768 17.7 ->
+// 11.4, 64 x 768 x 768 9.6 -> 10.8; error against 64 bits (2-norm) at k = 768 1.85e-7 -> 0.88e-7, 3072 3.6e-7 -> 1.0e-7.
 //
 // The order of a row's sum is a function of (n, k) alone: K is cut into g x h segments of `per` blocks; a segment's blocks are added in order, h
 // segments make a group, and the groups are added in order. Who does it depends on m: one CTA (many rows), a cluster of g CTAs with a group each,
