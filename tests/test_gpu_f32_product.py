@@ -76,3 +76,30 @@ def test_rows_that_are_not_finite(ak, ctx):
         assert np.array_equal(a[rows], b[rows]) and not np.isfinite(b[130]).any()
     ctx.check_device_status()
     s.close(); w.close()
+
+
+def test_results_that_are_not_finite_or_nearly_so(ak, ctx):
+    """Values of layer 0 (products alone, no rotation): a weight that rounds to an infinity in 16 bits but whose products are finite, an infinite one, a NaN."""
+    cfg = ak.ModelConfig(50, 320, 5, 1, 300, 1280)
+    params = ak.synthetic_weights(cfg, seed=3, std=0.05)
+    params[1][17] = 0.05                            # (the factor of the largest weight stays below 1)
+    value = params[2][:, 2 * cfg.dim:]
+    value[:, 5] = 0
+    value[17, 5] = 3.4e38
+    value[23, 9] = -np.inf
+    value[300, 130] = np.nan
+    w = ak.ModelWeights.from_params(ctx, cfg, params, ak.AK_F32)
+    s = ak.InferenceSession(ctx, w, 300)
+    for n in (2, 9, 130, 300):
+        toks = ak.uniform_tokens(n, 50, seed=n)
+        want = forward64(cfg, params, toks)[1][0]
+        s.replace_cache()
+        s.prefill(toks)
+        got = np.asarray(s.read_cache(0)[1], np.float64).reshape(n, -1)
+        assert np.array_equal(np.isnan(got), np.isnan(want)) and np.isnan(got[:, 130]).all()
+        assert np.array_equal(got[:, 9], want[:, 9]) and np.isinf(got[:, 9]).all()
+        for cols in ([5], [c for c in range(cfg.dim) if c not in (5, 9, 130)]):
+            assert np.isfinite(got[:, cols]).all()
+            assert np.linalg.norm(got[:, cols] - want[:, cols]) < 1e-6 * np.linalg.norm(want[:, cols])   # (one product, as above)
+    ctx.check_device_status()
+    s.close(); w.close()
