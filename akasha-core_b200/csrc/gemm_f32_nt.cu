@@ -1,8 +1,8 @@
 // True-fp32 product with the weight matrix K-major: C[m,n] (op)= A[m,k] @ Wt[n,k]^T, the layout the runner keeps its f32 projections
 // in (each output column's weights contiguous, so that a batch-1 step streams whole rows).
 //
-// GEMM: gemm_f32_tc.cu where rows and operands are 16-byte aligned. Else on the FMA pipe: 64 x 128 tile per CTA, 128 threads, 8 x 8 outputs per thread as
-// packed pairs (fma.rn.f32x2: two IEEE fused multiply-adds per instruction), K blocks of 16 double-buffered in shared memory with
+// GEMM: gemm_f32_tc.cu where rows and operands are 16-byte aligned and (n, k) is not small. Else on the FMA pipe: 64 x 128 tile per CTA, 128 threads, 8 x 8
+// outputs per thread as packed pairs (fma.rn.f32x2: two IEEE fused multiply-adds per instruction), K blocks of 16 double-buffered in shared memory with
 // the next block's global loads in flight; K is split over a thread-block cluster and the partial tiles are added through distributed
 // shared memory in rank order. Either way the order of a sum is a function of (n, k) only: it does not depend on how many rows share the launch.
 // GEMV: a warp per output, the weights streamed once with 128-bit loads. Its order of sums is another one, so it is only for rows that
@@ -36,18 +36,24 @@ __device__ __forceinline__ uint64_t dup2(float v) {
     return r;
 }
 
-// 4 consecutive k of one row
+// 4 consecutive k of one row; k % 4 == 0 and 16-byte rows unless SCALAR
+template <bool SCALAR>
 __device__ __forceinline__ float4 load4(const float* __restrict__ p, uint32_t row, uint32_t rows, uint32_t k0, uint32_t k_end, uint32_t ld) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row >= rows) return v;
     const float* s = p + (size_t)row * ld + k0;
-    if (k0 < k_end) v.x = s[0];
-    if (k0 + 1 < k_end) v.y = s[1];
-    if (k0 + 2 < k_end) v.z = s[2];
-    if (k0 + 3 < k_end) v.w = s[3];
+    if (!SCALAR) {
+        if (k0 < k_end) v = *reinterpret_cast<const float4*>(s);
+    } else {
+        if (k0 < k_end) v.x = s[0];
+        if (k0 + 1 < k_end) v.y = s[1];
+        if (k0 + 2 < k_end) v.z = s[2];
+        if (k0 + 3 < k_end) v.w = s[3];
+    }
     return v;
 }
 
+template <bool SCALAR>
 __global__ void __launch_bounds__(THREADS, 3)
 gemm_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ c, uint32_t m, uint32_t n, uint32_t k, uint32_t flags) {
     __shared__ __align__(16) Smem sm;
@@ -64,11 +70,11 @@ gemm_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __r
     float4 ra[2], rb[4];
     auto fetch_b = [&](uint32_t k0) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) rb[i] = load4(w, n0 + lr + 32 * i, n, k0 + 4 * lq, k_end, k);
+        for (int i = 0; i < 4; i++) rb[i] = load4<SCALAR>(w, n0 + lr + 32 * i, n, k0 + 4 * lq, k_end, k);
     };
     auto fetch_a = [&](uint32_t k0) {
 #pragma unroll
-        for (int i = 0; i < 2; i++) ra[i] = load4(a, m0 + lr + 32 * i, m, k0 + 4 * lq, k_end, k);
+        for (int i = 0; i < 2; i++) ra[i] = load4<SCALAR>(a, m0 + lr + 32 * i, m, k0 + 4 * lq, k_end, k);
     };
     auto put = [&](uint32_t buf) {
 #pragma unroll
@@ -211,7 +217,12 @@ int launch_gemm_f32_nt(cudaStream_t st, const float* a, const float* wt, float* 
         const uint32_t ctas = cdiv(n, GV_WARPS), room = B200_SMS * 8;
         return launch_k(gemv_kernel, dim3(ctas < room ? ctas : room), dim3(GV_WARPS * 32), 0, st, NO_CLUSTER, a, wt, c, n, k, flags, (uint32_t)vec);
     }
-    if (vec) return launch_gemm_f32_tc(st, a, wt, c, m, n, k, flags);
+    // Where a launch is short anyway the FMA pipe is quicker to the end of it (an SM's whole shared and tensor memory are set up for nothing). Four products of a
+    // layer, this kernel / tensor cores, us, with 4, 128 and 1024 rows: 64-wide model 26 / 25, 32 / 43, 33 / 45; 128-wide 26.7 / 30.0, 38.5 / 42.7, 43.1 / 44.0
+    // (2048 rows 57 / 45); 256-wide, of which only 256 x 256 is small, 30.5 / 29.8, 37.3 / 39.5, 72 / 50. Steps of a 128-wide model of 2 layers with
+    // 8 sequences 88 / 101.
+    const bool small = k <= 128 || (uint64_t)n * k <= 65536;
+    if (vec && !small) return launch_gemm_f32_tc(st, a, wt, c, m, n, k, flags);
     // K is split so that one row tile occupies every SM, at most eight ways (a portable cluster), never less than 64 of K per CTA
     const uint32_t tn = cdiv(n, BN);
     uint32_t ks = B200_SMS / tn;
@@ -219,7 +230,8 @@ int launch_gemm_f32_nt(cudaStream_t st, const float* a, const float* wt, float* 
     if (ks > k / 64) ks = k / 64;
     if (ks < 1) ks = 1;
     const dim3 grid(tn, cdiv(m, BM), ks), cluster(1, 1, ks);
-    return launch_k(gemm_kernel, grid, dim3(THREADS), 0, st, cluster, a, wt, c, m, n, k, flags);
+    if (vec) return launch_k(gemm_kernel<false>, grid, dim3(THREADS), 0, st, cluster, a, wt, c, m, n, k, flags);
+    return launch_k(gemm_kernel<true>, grid, dim3(THREADS), 0, st, cluster, a, wt, c, m, n, k, flags);
 }
 
 }  // namespace ak

@@ -13,9 +13,9 @@
 // shared memory leaves the next one no room to start early). m x n x k 512 x 2304 x 768: 52 -> 20 us, 512 x 768 x 3072 60 -> 26, 64 x 3072 x 768 17.7 ->
 // 11.4, 64 x 768 x 768 9.6 -> 10.8; error against 64 bits (2-norm) at k = 768 1.85e-7 -> 0.88e-7, 3072 3.6e-7 -> 1.0e-7.
 //
-// The order of a row's sum is a function of (n, k) alone: K is cut into g x h segments of `per` blocks; a segment's blocks are added in order, h
-// segments make a group, and the groups are added in order. Who does it depends on m: one CTA (many rows), a cluster of g CTAs with a group each,
-// or of g h CTAs with a segment each (few rows); the partial tiles are read through distributed shared memory.
+// The order of a row's sum is a function of (n, k) alone: K is cut into segments of `per` blocks; a segment's blocks are added in order, h segments make
+// a group, of which there are two, and the groups are added. Who does it depends on m: one CTA (many rows), a cluster of two CTAs with a group each,
+// or of a CTA for each segment (few rows); the partial tiles are read through distributed shared memory.
 //
 // A result that is not finite (infinite or NaN operands and those that round to an infinite piece, or sums past the largest f32) is computed again with FMAs,
 // by a warp for each (a thread for each before): 512 x 768 x 3072, 26 us, with a NaN in one column of the weights 710 -> 53 us, in one row of the activations
@@ -42,7 +42,7 @@ constexpr uint32_t NCW = 8, NPW = 8;                      // warps that split, w
 constexpr uint32_t THREADS = 128 + 32 * (NCW + NPW);
 constexpr int REGS_FIRST = 64, REGS_SPLIT = 64, REGS_ADD = 144;   // of 640 x 96 at launch
 static_assert(REGS_FIRST * 128 + REGS_SPLIT * 32 * NCW + REGS_ADD * 32 * NPW <= THREADS * 96, "the split draws on the registers of the launch");
-constexpr uint32_t MAX_SEGS = 5;
+constexpr uint32_t MAX_SEGS = 6;
 
 // the pair (x, y) as three bf16 pairs
 __device__ __forceinline__ void split2(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
@@ -139,7 +139,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
     const uint32_t cs = gridDim.z, rank = blockIdx.z;   // CTAs of the cluster: 1, groups or segments
-    const uint32_t kb_total = (k + TK - 1) / TK, mine = cut.segs / cs * cut.per;
+    const uint32_t kb_total = (k + TK - 1) / TK, mine = (cs == 1 ? cut.segs : cs == cut.segs ? 1 : cut.h) * cut.per;
     const uint32_t kb0 = min(rank * mine, kb_total), nkb = min(kb0 + mine, kb_total) - kb0;
 
     const uint32_t halves = 2 * nkb, pre = min(halves, STAGES), tx = (a_box * HALF + TN * HALF) * 4;
@@ -419,24 +419,28 @@ static uint32_t resident_ctas(uint32_t cs) {
 // 16-byte rows (k % 4 == 0) and aligned operands, see launch_gemm_f32_nt()
 int launch_gemm_f32_tc(cudaStream_t st, const float* a, const float* wt, float* c, uint32_t m, uint32_t n, uint32_t k, uint32_t flags) {
     const uint32_t tn = cdiv(n, TN), tm = cdiv(m, TM), kb = cdiv(k, TK), a_box = m < TM ? m : TM;
-    // Segments: as many as let one row tile occupy the SMs, at most five (with six, clusters of which only 22 run at a time, 512 x 768 x 768 took 20.6 us,
-    // 512 x 768 x 3072 42.5).
+    // Segments: as many as let one row tile occupy the SMs, at most five, or six where K or n is small and a K block more is a good part of the
+    // launch: 4 x 1536 x 384 8.3 -> 6.8 us, the four products of a layer of a 384-wide model with 4, 128 and 512 rows 37.7, 51.4, 63.2 -> 33.3, 44.7, 57.2. (With
+    // six everywhere, clusters of which only 22 run at a time: 512 x 768 x 768 12.6 -> 20.6, 512 x 768 x 3072 25.7 -> 42.5; with eight, and partial
+    // tiles of as many to add, everything is 1 to 3 % slower.) Five segments are groups of three and two, so that a cluster of two can take more than
+    // the one wave that clusters of five have: 512 x 960 x 320 17.6 -> 13.8 us, a prompt of 480 tokens of the 320-wide model 1270 -> 1007.
+    const uint32_t most = k <= 384 || n <= 256 ? MAX_SEGS : 5;
     uint32_t segs = B200_SMS / tn;
-    if (segs > MAX_SEGS) segs = MAX_SEGS;
+    if (segs > most) segs = most;
     if (segs > kb) segs = kb;
     if (segs < 1) segs = 1;
     Cut cut;
     cut.per = cdiv(kb, segs);
     cut.segs = cdiv(kb, cut.per);
-    cut.h = cut.segs % 2 == 0 ? cut.segs / 2 : 1;
+    cut.h = cdiv(cut.segs, 2);
     // Who adds them: the choice with the shortest way to the end, a CTA per SM at a time. In 0.1 us: 9 for a K block, up to 10 more for the split
     // of its activations, 65 for the rest of a tile, 10 more in a cluster.
     uint32_t cs = 0, best = 0;
-    for (uint32_t o : {1u, cut.segs / cut.h, cut.segs}) {
+    for (uint32_t o : {1u, cut.segs > 2 ? 2u : 1u, cut.segs}) {
         const uint32_t room = resident_ctas(o);
         AK_REQUIRE(room || o > 1, AK_ERR_CUDA, "f32 product: the kernel does not fit an SM");
         if (!room) continue;
-        const uint32_t cost = cdiv(tn * tm * o, room) * (cut.segs / o * cut.per * (9 + 10 * a_box / TM) + 65 + (o > 1 ? 10 : 0));
+        const uint32_t cost = cdiv(tn * tm * o, room) * ((o == 1 ? cut.segs : o == cut.segs ? 1 : cut.h) * cut.per * (9 + 10 * a_box / TM) + 65 + (o > 1 ? 10 : 0));
         if (!cs || cost < best) { cs = o; best = cost; }
     }
     CUtensorMap tmA, tmB;

@@ -35,9 +35,10 @@ def forward64(cfg, params, toks):
     return ks, vs, (norm(h[-1:], P[1 + 6 * L]) @ P[2 + 6 * L])[0].numpy()
 
 
-# K of one block and of several, not a multiple of a block (64) nor of a half (32); one segment to five, in one group and in two; columns that end inside
-# a tile; rows at the edges of the 128-row tile and of the eight rows a warp splits
-@pytest.mark.parametrize("dim,heads,ffn,vocab", [(64, 1, 100, 33), (132, 3, 260, 129), (320, 5, 1280, 997), (768, 12, 3072, 1000), (1088, 17, 36, 64)])
+# K of several blocks, not a multiple of a block (64) nor of a half (32); two segments to six, in groups of one to three; columns that end inside
+# a tile; rows at the edges of the 128-row tile and of the eight rows a warp splits. 64: (n, k) that stay on the FMA pipe; 65 and 101: K that is no multiple of 4
+@pytest.mark.parametrize("dim,heads,ffn,vocab", [(64, 1, 100, 33), (132, 3, 260, 129), (320, 5, 1280, 997), (768, 12, 3072, 1000), (1088, 17, 36, 64),
+                                                 (64, 1, 65, 33), (320, 5, 1281, 129), (384, 6, 700, 513), (256, 4, 1540, 1000)])
 def test_prompt_against_64_bits(ak, ctx, dim, heads, ffn, vocab):
     cfg = ak.ModelConfig(vocab, dim, heads, 2, 600, ffn)
     params = ak.synthetic_weights(cfg, seed=dim, std=0.05)
@@ -54,6 +55,25 @@ def test_prompt_against_64_bits(ak, ctx, dim, heads, ffn, vocab):
             k, v = s.read_cache(l)
             assert err(k, ks[l]) < 2e-6 and err(v, vs[l]) < 2e-6, (n, l)
         assert err(logits, want) < 2e-6, n
+    ctx.check_device_status()
+    s.close(); w.close()
+
+
+@pytest.mark.parametrize("dim,heads,ffn", [(64, 1, 256), (128, 2, 512), (320, 5, 1280), (384, 6, 1536), (768, 12, 3072)])
+def test_rows_do_not_depend_on_their_number(ak, ctx, dim, heads, ffn):
+    """Bits: whoever adds the segments of K (a CTA, a cluster of two, a CTA each), and on either pipe."""
+    cfg = ak.ModelConfig(97, dim, heads, 2, 600, ffn)
+    w = ak.ModelWeights.from_params(ctx, cfg, ak.synthetic_weights(cfg, seed=dim, std=0.05), ak.AK_F32)
+    s = ak.InferenceSession(ctx, w, 600)
+    toks = ak.uniform_tokens(600, 97, seed=1)
+    def prefix(n):
+        s.replace_cache()
+        s.prefill(toks[:n])
+        return [np.asarray(x).reshape(n, -1).copy() for x in s.read_cache(0)]
+    full = prefix(600)
+    for n in (1, 2, 9, 40, 64, 65, 128, 129, 300, 385, 520):
+        for a, b in zip(prefix(n), full):
+            assert np.array_equal(a, b[:n]), n
     ctx.check_device_status()
     s.close(); w.close()
 
