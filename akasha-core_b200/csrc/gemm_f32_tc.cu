@@ -1,17 +1,19 @@
 // f32 product on the tensor cores: C[m,n] (op)= A[m,k] @ Wt[n,k]^T, f32 operands, f32-accurate sums.
 //
 // Every operand is split, on its way into shared memory, into three bf16 pieces x = x0 + x1 + x2 (each the rounding of what is left: 3 x 8 bits hold
-// the 24 of an f32 exactly), and six of the nine products are taken: x0 y0, and x0 y1 + x1 y0 + x1 y1 + x0 y2 + x2 y0. What is left out is at most 2^-25
-// of a product and of either sign. The large products and the others have accumulators of their own in tensor memory. The tensor core's
+// the 24 of an f32 exactly, unless it is so small that the third piece falls below bf16's smallest numbers: x is off by 2^-134 at most, 1e-7 of it at 2^-111,
+// 1e-4 at 2^-121), and six of the nine products are taken: x0 y0, and x0 y1 + x1 y0 + x1 y1 + x0 y2 + x2 y0. What is left out, x1 y2 + x2 y1 + x2 y2, is
+// at most about 2^-24 of a product and of either sign. The large products and the others have accumulators of their own in tensor memory. The tensor core's
 // additions cut instead of rounding, so the large products' accumulator is fresh for every K block of 64 (4 MMAs) and is added in registers
-// with ordinary f32 additions; the others', 2^-8 of it, runs through a segment.
+// with ordinary f32 additions; the others', at most 2^-7 of it, runs through a segment.
 //
 // What bounded the FMA kernel it replaces is the FMA pipe and the shared-memory words that feed it (a 512-token prefill of the 162M model ran at 40 % of
 // 74 TFLOP/s). Here a K block of a 128 x 128 tile takes 1.9 us: 24 MMAs of 64 cycles (1536), and about 3300 cycles of shared memory, which both operands
 // go through as f32, as pieces, and as what the MMAs read; the split and the additions have warps of their own and as many issue slots as the MMAs have
 // cycles. A 128 x 64 tile asks for half as much again per product and ran at 0.6 of the rate. A launch costs about 7 us beside its blocks (its
 // shared memory leaves the next one no room to start early). m x n x k 512 x 2304 x 768: 52 -> 20 us, 512 x 768 x 3072 60 -> 26, 64 x 3072 x 768 17.7 ->
-// 11.4, 64 x 768 x 768 9.6 -> 10.8; error against 64 bits (2-norm) at k = 768 1.85e-7 -> 0.88e-7, 3072 3.6e-7 -> 1.0e-7.
+// 11.4, 64 x 768 x 768 9.6 -> 10.8; error against 64 bits (2-norm), normal operands, at k = 768 1.85e-7 -> 0.88e-7, 3072 3.6e-7 -> 1.0e-7. With operands
+// all of one sign, whose sums rounding hardly touches, cutting shows: k = 320 0.66e-7 -> 0.84e-7, 768 0.73e-7 -> 0.85e-7, 3072 1.17e-7 -> 0.86e-7.
 //
 // The order of a row's sum is a function of (n, k) alone: K is cut into segments of `per` blocks; a segment's blocks are added in order, h segments make
 // a group, of which there are two, and the groups are added. Who does it depends on m: one CTA (many rows), a cluster of two CTAs with a group each,

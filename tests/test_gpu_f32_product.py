@@ -123,3 +123,33 @@ def test_results_that_are_not_finite_or_nearly_so(ak, ctx):
             assert np.linalg.norm(got[:, cols] - want[:, cols]) < 1e-6 * np.linalg.norm(want[:, cols])   # (one product, as above)
     ctx.check_device_status()
     s.close(); w.close()
+
+
+@pytest.mark.parametrize("case", ["one sign", "2^-112", "2^-118"])
+def test_operands_of_one_sign_and_tiny_ones(ak, ctx, case):
+    """Values of layer 0 against 64 bits. Of one sign: the cut additions of the tensor cores all err the same way. Tiny weights: their third piece is lost, up
+    to half of bf16's smallest number (2^-134), in 768 roundings of either sign."""
+    cfg = ak.ModelConfig(50, 768, 12, 1, 200, 3072)
+    params = ak.synthetic_weights(cfg, seed=3, std=0.05)
+    value = params[2][:, 2 * cfg.dim:]
+    if case == "one sign":
+        params[0][:] = np.abs(params[0])
+        value[:] = np.abs(value)
+        bound = 4e-7       # 64 products: 16 of an MMA cut to 2^-24 of the largest sum each time, 4 MMAs; 0.85e-7 measured
+    else:
+        e = int(case[2:])
+        value[:] = np.sign(value) * np.float32(2.0) ** e * (1 + np.abs(value))
+        bound = 4e-7 + 2.0 ** (-134 - e)
+    w = ak.ModelWeights.from_params(ctx, cfg, params, ak.AK_F32)
+    s = ak.InferenceSession(ctx, w, 200)
+    for n in (3, 150):
+        toks = ak.uniform_tokens(n, 50, seed=n)
+        want = forward64(cfg, params, toks)[1][0]
+        s.replace_cache()
+        s.prefill(toks)
+        got = np.asarray(s.read_cache(0)[1], np.float64).reshape(n, -1)
+        err = np.linalg.norm(got - want) / np.linalg.norm(want)
+        print(case, n, err)
+        assert err < bound
+    ctx.check_device_status()
+    s.close(); w.close()
