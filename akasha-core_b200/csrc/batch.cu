@@ -213,13 +213,13 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     __shared__ float2 at_ml[2][NW];
     __shared__ Walk walk_sm[NW];
     __shared__ uint32_t units[NW][MAX_UNITS];
-    __shared__ uint32_t len_sm[32], by_len[32], pre_sm[33];
+    __shared__ uint32_t len_sm[32], by_len[32], pre_sm[33], slot_sm[PARTS > 1 ? 32 : 1];   // slot_sm: the slots of a part's rows
     __shared__ Expiry expiry;
     __shared__ uint32_t failed_sm, flat_sm, live_sm, use_sm[MAX_SLOTS + MAX_EXTRA];   // use_sm: 1 + the number of the use a slot is in (lm_head only)
 
     const uint32_t tid = threadIdx.x, warp_ = tid >> 5, lane = tid & 31;
     // What tells the parts apart: rows, sets (an offset that set_of() adds), state. (As arguments of their own, chosen by the block, they cost 5 % of a step.)
-    const uint32_t part_no = PARTS > 1 && blockIdx.x >= a.sms ? 1u : 0u, row0 = PARTS > 1 ? part_no * a.part_seqs : 0u;
+    const uint32_t part_no = PARTS > 1 && blockIdx.x >= a.sms ? 1u : 0u;
     const uint32_t cta = PARTS > 1 ? blockIdx.x - part_no * a.sms : blockIdx.x;
     State* const state = PARTS > 1 ? a.state + part_no : a.state;
     const uint32_t D = a.dim, F = a.ffn, H = a.heads, L = a.n_layers;
@@ -246,18 +246,34 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     }
     if (tid >= 32 && tid < 32 + N_KINDS) make_kind(kinds[tid - 32], tid == 32 ? 3 * D : tid == 34 ? F : tid == 36 ? a.vocab : D, tid == 35 ? F : D, cta, a.sms);
     if (warp_ == 2) {   // the rows' lengths, the rows by length (the longest first), the attention splits of the rows before by that rank
-        const uint32_t n = lane < a.part_seqs && row0 + lane < a.seqs ? min((uint32_t)max(a.rows ? a.kv_lens[row0 + lane] : a.lens[row0 + lane], 0), a.max_len) : 0u;
-        uint32_t rank = 0;
+        uint32_t n[PARTS], key[PARTS], rank[PARTS] = {};   // of slot lane + 32 p
 #pragma unroll
-        for (uint32_t j = 0; j < 32; j++) {
-            const uint32_t o = __shfl_sync(0xffffffffu, n, j);
-            rank += o > n || (o == n && j < lane);
+        for (uint32_t p = 0; p < PARTS; p++) {
+            const uint32_t s = lane + 32 * p;
+            n[p] = s < a.seqs ? min((uint32_t)max(a.rows ? a.kv_lens[s] : a.lens[s], 0), a.max_len) : 0u;
+            key[p] = n[p] << 6 | (63 - s);   // (lengths are below 2^26)
         }
-        len_sm[lane] = n;
-        by_len[rank] = lane;
-        const uint32_t m = __ballot_sync(0xffffffffu, n > 0);
-        if (lane == 0) live_sm = m;
+#pragma unroll
+        for (uint32_t j = 0; j < 32 * PARTS; j++) {
+            const uint32_t o = __shfl_sync(0xffffffffu, key[j / 32], j % 32);
+#pragma unroll
+            for (uint32_t p = 0; p < PARTS; p++) rank[p] += o > key[p];
+        }
+#pragma unroll
+        for (uint32_t p = 0; p < PARTS; p++) {
+            if (PARTS == 1) {
+                len_sm[lane] = n[p];
+                by_len[rank[p]] = lane;
+            } else if (part_of_rank(rank[p]) == part_no) {   // (a part's rows are in order of length)
+                const uint32_t row = row_of_rank(rank[p]);
+                len_sm[row] = n[p];
+                slot_sm[row] = lane + 32 * p;
+                by_len[row] = row;
+            }
+        }
         __syncwarp();
+        const uint32_t m = __ballot_sync(0xffffffffu, len_sm[lane] > 0);
+        if (lane == 0) live_sm = m;
         const uint32_t mine = div_up(len_sm[by_len[lane]], SPLIT_LEN);
         uint32_t sum = mine;
 #pragma unroll
@@ -293,6 +309,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
     uint8_t* const extra_sm = kv_sm + D * R * 2;
     const uint32_t extra = min(MAX_EXTRA, (NW * 2 * KV_BUF - D * R * 2) / SLOT), head_slots = slots + extra;
     auto set_of = [&](uint32_t g) { return (g % SETS) * (uint32_t)so.total + (PARTS > 1 ? part_no * a.part_bytes : 0u); };   // byte offset; g = e0: the embedding, e0 + 1 + l: layer l
+    auto slot_of = [&](uint32_t r) { return PARTS > 1 ? slot_sm[r] : r; };
     auto row_live = [&](uint32_t r) { return (live >> r) & 1u; };
     auto eight_live = [&](uint32_t e) { return ((live >> (e * 8)) & 0xffu) != 0; };
     const Waiter wt{&expiry};
@@ -482,8 +499,8 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 const uint32_t row = m * 16 + rl;
                 float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (row_live(row)) {
-                    const int32_t ts = a.rows ? a.rows[(row0 + row) * 4] : a.tok_src[row0 + row];
-                    const uint32_t id = ts >= 0 ? (uint32_t)ts : a.sampled[row0 + row];
+                    const int32_t ts = a.rows ? a.rows[slot_of(row) * 4] : a.tok_src[slot_of(row)];
+                    const uint32_t id = ts >= 0 ? (uint32_t)ts : a.sampled[slot_of(row)];
                     if (id < a.vocab) {
                         const uint2 w = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(a.embedding) + (size_t)id * D + tile * 8 + h * 4);
                         x = make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u));
@@ -791,6 +808,9 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         if (lane == 0) walk_sm[cw].nu = n;
         __syncwarp();
     }
+    // (of two parts a unit's row has the slot above it)
+    auto row_in = [&](const Unit& u) { return PARTS > 1 ? u.row & 31u : u.row; };
+    auto slot_in = [&](const Unit& u) { return PARTS > 1 ? u.row >> 5 : u.row; };
     auto unit_at = [&](uint32_t j) {
         const uint32_t u = units[cw][j];
         Unit o;
@@ -798,12 +818,13 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
         o.p0 = o.split * SPLIT_LEN;
         o.n = min(SPLIT_LEN, len_sm[o.row] - o.p0);
         o.nb = (o.n + UP - 1) / UP;
+        if (PARTS > 1) o.row |= slot_sm[o.row] << 5;
         return o;
     };
     auto look_up = [&]() {   // the pool blocks of the walk's tile (lane 0)
         Walk& k = walk_sm[cw];
         const uint32_t p = k.b * UP;
-        const int32_t* bt = a.block_tables + (size_t)(row0 + k.u.row) * a.max_blocks + (k.u.p0 + p) / 16;
+        const int32_t* bt = a.block_tables + (size_t)slot_in(k.u) * a.max_blocks + (k.u.p0 + p) / 16;
         k.pb0 = (uint32_t)__ldg(bt);
         k.pb1 = UP > 16 && p + 16 < k.u.n ? (uint32_t)__ldg(bt + 1) : EMPTY;
     };
@@ -877,7 +898,7 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll 1
         for (uint32_t j = 0; j < nu; j++) {
             const Unit u = unit_at(j);
-            const uint32_t buf = j & 1, pos = len_sm[u.row] - 1;
+            const uint32_t buf = j & 1, pos = len_sm[row_in(u)] - 1;
             const bool newest = u.p0 + u.n == pos + 1;   // the unit holds the sequence's new position
             constexpr uint32_t KT = UP / 8, NS = HD / 32;   // eights of positions in a tile; k slices of a score
             float m = -INFINITY, l = 0.0f, acc[8];   // this lane's 8 columns, of its share of the positions
@@ -887,10 +908,10 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
                 // This lane's 8 columns of the new token's query; of the newest tile's warp also of its key and value, which go to the pools and
                 // (below) into the tile. All of it, the rotation's factors and the place in the pools are asked for together.
                 const bool owner = newest && wg == in_group(u.nb - 1);
-                const uint8_t* const src = qkv + ((size_t)u.row * 3 * D + u.head * HD + chunk * 8) * 4;
+                const uint8_t* const src = qkv + ((size_t)row_in(u) * 3 * D + u.head * HD + chunk * 8) * 4;
                 const float4* const rt = reinterpret_cast<const float4*>(a.rope + (size_t)pos * (HD / 2) + chunk * 4);
                 const float4 r0 = __ldg(rt), r1 = __ldg(rt + 1);
-                const uint32_t pb = owner ? (uint32_t)__ldg(a.block_tables + (size_t)(row0 + u.row) * a.max_blocks + pos / 16) : 0u;
+                const uint32_t pb = owner ? (uint32_t)__ldg(a.block_tables + (size_t)slot_in(u) * a.max_blocks + pos / 16) : 0u;
                 uint4 qa[NS], kn = make_uint4(0, 0, 0, 0), vn = kn;
                 {
                     uint4 x[6] = {};
@@ -1039,10 +1060,10 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
 #pragma unroll
                     for (uint32_t e = 0; e < DL; e++) o[e] = fmaf(src[w * HD + e], fw, o[e]);
                 }
-                if (!SPLIT || len_sm[u.row] <= SPLIT_LEN) {
-                    put_at(set, u.row, u.head, o, ls);
+                if (!SPLIT || len_sm[row_in(u)] <= SPLIT_LEN) {
+                    put_at(set, row_in(u), u.head, o, ls);
                 } else {
-                    uint8_t* dst = a.xch + set + so.part + ((size_t)(u.row * H + u.head) * splits + u.split) * (HD + 4) * 4;
+                    uint8_t* dst = a.xch + set + so.part + ((size_t)(row_in(u) * H + u.head) * splits + u.split) * (HD + 4) * 4;
                     if constexpr (DL == 2) xst2(dst + lane * 8, word(o[0]), word(o[1]));
                     else xst4(dst + lane * 16, word(o[0]), word(o[1]), word(o[DL - 2]), word(o[DL - 1]));
                     if (lane == 0) xst2(dst + HD * 4, word(M), word(ls));
@@ -1240,8 +1261,8 @@ __global__ void __launch_bounds__(THREADS, 1) batch_kernel(const __grid_constant
             bar_sync<64>(BAR_FLAT);
             if (lane == 0) {
                 const uint32_t tok = n < a.vocab && !flat_sm ? n : 0u;   // (no logit above -inf, or all 0: 0)
-                a.sampled[row0 + cta] = tok;
-                if (a.sampled_host) a.sampled_host[row0 + cta] = tok;
+                a.sampled[slot_of(cta)] = tok;
+                if (a.sampled_host) a.sampled_host[slot_of(cta)] = tok;
                 if (cta == (uint32_t)__ffs(live) - 1) {   // every SM has published its best, so has read them
                     state->set = (e0 + L + 1) % SETS;
                     state->counted += clears_of_step(L) * a.sms;

@@ -35,6 +35,12 @@ AK_PLAN_FN constexpr uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1
 // More than 32 sequences are two parts, each with half of the sequences and half of the SMs, that have nothing to do with each other
 AK_PLAN_FN constexpr uint32_t parts_of(uint32_t seqs) { return seqs <= ROWS ? 1 : MAX_PARTS; }
 AK_PLAN_FN constexpr uint32_t part_seqs(uint32_t seqs) { return div_up(seqs, parts_of(seqs)); }
+// The sequences of a step of two parts are dealt in order of length (rank 0: the longest), there and back: 0 1 1 0 0 1 1 0 ... Dealt by halves of the slots, the
+// part with the longer contexts set the step's time, and a queue that was half empty ran on half of the SMs: 162M model, 64 slots, us per step, so / now (as
+// launches): 32 running at 380 of 512 positions 430 / 317 (472), 48 439 / 408 (498), 64 440 / 444 (531); at 1900 of 2048 1037 / 632 (830), 1042 / 878 (950), 1055 / 1045
+// (1125); at 3900 of 4096 1824 / 1050 (1285), 1830 / 1470 (1510), 1873 / 1875 (1897); 128 ragged sequences through 64 slots 344 / 333 ms.
+AK_PLAN_FN constexpr uint32_t part_of_rank(uint32_t rank) { return (rank ^ (rank >> 1)) & 1u; }
+AK_PLAN_FN constexpr uint32_t row_of_rank(uint32_t rank) { return rank >> 1; }
 AK_PLAN_FN constexpr uint32_t m_tiles(uint32_t seqs) { return seqs <= 16 ? 1 : 2; }
 AK_PLAN_FN constexpr uint32_t tile_begin(uint32_t tiles, uint32_t cta, uint32_t sms) { return (tiles * cta) / sms; }   // of the step's sms blocks
 // Positions of an attention unit. Where all sequences fit in 128 KB of keys (1024 positions of head size 64, 512 of 128) they are whole, which saves

@@ -34,3 +34,32 @@ def test_which_shapes_are_two_parts(tmp_path_factory):
     assert shapes(768, 3072, 12, 12, 65, 512).startswith("0")
     assert shapes(1536, 6144, 12, 24, 64, 512).startswith("1")
     assert shapes(2048, 8192, 16, 24, 64, 512).startswith("0")   # 32 rows of x do not fit where the cache tiles were
+
+
+DEAL = r"""
+#include <stdio.h>
+#include <stdlib.h>
+#include "batch_plan.h"
+using namespace ak::batch;
+int main(int argc, char** argv) {   // the rows that argv[1] slots get, longest first: parts and rows, and the largest difference of the parts' sums
+    const uint32_t n = atoi(argv[1]);
+    unsigned long long seen[2] = {0, 0}, sum[2] = {0, 0};
+    for (uint32_t rank = 0; rank < ROWS * MAX_PARTS; rank++) {
+        const uint32_t p = part_of_rank(rank), r = row_of_rank(rank);
+        if (p >= MAX_PARTS || r >= ROWS || (seen[p] >> r & 1)) { printf("rank %u", rank); return 0; }
+        seen[p] |= 1ull << r;
+        if (rank < n && r >= part_seqs(n)) { printf("row %u", r); return 0; }
+        sum[p] += rank < n ? (unsigned long long)(n - rank) * (n - rank) : 0;   // (lengths n^2, (n - 1)^2 ... 1)
+    }
+    const unsigned long long d = sum[0] > sum[1] ? sum[0] - sum[1] : sum[1] - sum[0];
+    printf("%s", d <= (unsigned long long)n * n ? "ok" : "uneven");
+    return 0;
+}
+"""
+
+
+def test_sequences_are_dealt_evenly(tmp_path_factory):
+    """Every row of both parts is written, whatever is running; the parts' positions differ by the longest sequence at most."""
+    deal = build(tmp_path_factory, DEAL)
+    for n in range(33, 65):
+        assert deal(n) == "ok", n
