@@ -163,6 +163,11 @@ inline bool shape_supported(uint32_t dim, uint32_t ffn, uint32_t heads, uint32_t
     const uint32_t hd = heads ? dim / heads : 0;
     if ((hd != 64 && hd != 128) || dim != heads * hd || heads > 4095) return false;
     if (seqs < 1 || seqs > ROWS * MAX_PARTS || n_layers < 1 || n_layers > MAX_LAYERS || dim < 96 || dim % 32 || ffn % 32 || ffn > 65536) return false;
+    // Two parts where K is one chunk of the ring, so that activations stay in registers for the passes of a phase. Wider models were slower so than as launches:
+    // 64 slots, 12 layers, us per step as launches / in parts: 768 wide, heads of 128, 1 to 64 running at 380 positions 438 .. 520 / 314 .. 442; 1024 wide 494 .. 700 /
+    // 497 .. 744, at 1900 693 .. 1490 / 518 .. 1452 (48 running 1145 / 1234); heads of 64 491 .. 711 / 385 .. 675, 32 long and 32 short ones 962 / 1017;
+    // 1536 wide 702 .. 975 / 796 .. 1052, heads of 64, 64 running at 1900 2046 / 2179.
+    if (parts_of(seqs) > 1 && div_up(dim, CHUNK * 32) > 1) return false;
     const uint32_t sms = SMS / parts_of(seqs);
     seqs = part_seqs(seqs);
     if (ffn / 8 < SMS) return false;                                       // every SM has ffn-up rows (the clearing of the sets counts on it)

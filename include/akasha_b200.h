@@ -369,8 +369,8 @@ typedef struct ak_engine_config {
     uint32_t use_cuda_graph;   /* capture steps in CUDA graphs, one per shape (a decode-only step that is one kernel is launched as such) */
     uint32_t stop_on_eos;      /* 0: run every sequence to its max_len              */
     uint32_t attn_timing;      /* record CUDA events around layer 0's decode attention and the captured steps. With bf16 weights and up to
-                                * 64 slots a decode step is otherwise one kernel; with this it is the launch chain of larger
-                                * engines, whose sums are in another order (tokens may differ where two logits are all but equal) */
+                                * 32 slots (64 of models up to 768 wide) a decode step is otherwise one kernel; with this it is the
+                                * launch chain of larger engines, whose sums are in another order (tokens may differ where two logits are all but equal) */
     uint32_t async_steps;      /* 1: ak_engine_step returns once step N is LAUNCHED and step N-1's tokens are on the
                                 * host, so describing and launching a step overlaps the previous step's GPU time.
                                 * Needs stop_on_eos == 0 (sequence ends must be known without the tokens);

@@ -51,7 +51,7 @@ def main():
     mine = list(range(n_seqs)) if tp > 1 else sharding.shard_round_robin(n_seqs, rank, world)
     prompts = [ak.uniform_tokens(int(lens[i]), cfg.vocab_size, seed=50_000 + i) for i in mine]
     max_len = 3072 + gen
-    # up to 64 slots a decode step is one kernel, unless its attention is to be timed
+    # up to 32 slots a decode step is one kernel, unless its attention is to be timed
     timing = max_seqs > 32 or tp > 1
     eng = ak.Engine(ctx, w, max_seqs=max_seqs, max_seq_len=max_len, max_batch_tokens=max_seqs + 16384,
                     use_cuda_graph=True, attn_timing=timing, async_steps=(tp == 1))

@@ -32,8 +32,11 @@ def test_which_shapes_are_two_parts(tmp_path_factory):
     assert shapes(768, 3072, 12, 12, 33, 512) == "1 2 17"
     assert shapes(768, 3072, 12, 12, 64, 512) == "1 2 32"
     assert shapes(768, 3072, 12, 12, 65, 512).startswith("0")
-    assert shapes(1536, 6144, 12, 24, 64, 512).startswith("1")
-    assert shapes(2048, 8192, 16, 24, 64, 512).startswith("0")   # 32 rows of x do not fit where the cache tiles were
+    assert shapes(768, 3072, 6, 12, 64, 2048).startswith("1")
+    assert shapes(832, 3328, 13, 12, 32, 512).startswith("1")
+    for dim, heads in ((832, 13), (1024, 8), (1536, 12)):         # K of more than a chunk: launches are faster
+        assert shapes(dim, 4 * dim, heads, 12, 33, 512).startswith("0")
+    assert shapes(2048, 8192, 16, 24, 64, 512).startswith("0")
 
 
 DEAL = r"""
