@@ -24,7 +24,7 @@
 //   * RMS norm: the producer of the residual stream publishes x * gain rounded to bf16 (one rounding, as of the normalised value) and
 //     the sums of squares of its columns; 1 / rms is a factor of the row sums of the next phase, found by the epilogue warps meanwhile.
 //   * The residual stream stays in shared memory of the SM that owns its columns (out-proj and ffn-down have the same tiles).
-//   * Attention: a unit is (sequence, head, split of split_len positions); units are dealt to groups of 3 to 12 warps in order of length. Keys
+//   * Attention: a unit is (sequence, head, split of split_len positions); units are dealt to groups of 4 to 12 warps in order of length. Keys
 //     and values go through per-warp shared-memory buffers, the next layer's first tiles already while this layer's ffn runs. Scores are
 //     mma.m16n8k16 (7/8 of it for nothing, but an eighth of the instructions of f32 FMAs); P V is f32 FMAs, the transposing loads that an
 //     MMA would need have 8-way bank conflicts on unswizzled tiles (32 sequences: 0.41 ms instead of 0.35).
@@ -124,7 +124,7 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {   // (a NaN become
 template <uint32_t N> __device__ __forceinline__ void bar_sync(uint32_t id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(N) : "memory"); }
 __device__ __forceinline__ void bar_sync_n(uint32_t id, uint32_t n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 template <uint32_t N> __device__ __forceinline__ void bar_arrive(uint32_t id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(N) : "memory"); }
-enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_FLAT = 4, BAR_GROUP = 5 };   // BAR_GROUP and the next three: by group
+enum { BAR_PART = 1, BAR_HELP = 2, BAR_HEAD = 3, BAR_FLAT = 4, BAR_GROUP = 5 };   // BAR_GROUP and the next two: by group
 
 __device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t pol) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(smem_u32(dst)),

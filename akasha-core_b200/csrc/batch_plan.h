@@ -111,12 +111,13 @@ inline Plan make_plan(uint32_t dim, uint32_t n_layers, uint32_t heads, uint32_t 
     // Warps of an attention unit. Whole sequences: 12, 6 or 4, the most that leave a group for every unit, because a group's second unit starts when the first is done
     // (where four do not either, long units share a group with short ones). Contexts of 300, us per step, with 12 or 4 and now 6: 162M model, 13 sequences
     // 233 / 218, 16 234 / 219, 24 283 / 265; 320-wide model, 32 sequences 151 / 143. Fewer than four give 64 equal sequences 417 / 414, but a
-    // long one among others then takes long: 128 ragged sequences through 64 slots 359 / 375 ms. Cut sequences: 12 up to one unit per SM, else 4, or
-    // 3 of head size 128, whose units are 16 tiles: 1.4B model, with 4 / 3 / 2 warps: 16 sequences of 128 to 3072 positions 1944 / 1880 / 2026, 8 1441 / 1383 / 1477,
-    // 16 of 1600 1793 / 1794 / 1830 (head size 64, 2048 positions: 8 sequences 266 / 290 / 254, 32 641 / 621 / 667, 320-wide model, 21 188 / 207 / 181).
+    // long one among others then takes long: 128 ragged sequences through 64 slots 359 / 375 ms. Cut sequences: 12 up to one unit per SM, else 4. With 3
+    // or 2 some shapes are faster and as many slower, by how the units of a step fall into rounds of the groups: heads of 64, 2048 positions, 4 / 3 / 2 warps, 8
+    // sequences 266 / 290 / 254, 32 641 / 621 / 667, 320-wide model, 21 188 / 207 / 181; heads of 128, 4 / 3, 768 wide, 12 layers, 16 sequences at 2000 positions 382 / 444,
+    // 24 534 / 513; 1.4B model, 16 at 540 1253 / 1336, 16 of random lengths up to 3072 1980, 1922, 1677 / 2008, 1897, 1769, 8 1315, 1446, 1438 / 1367, 1384, 1378.
     // (Not by the step's blocks: a unit's sums depend on it.)
     const uint32_t splits = div_up(max_len, split_len(max_len, hd)), units = seqs * heads * splits, own = SMS / parts;
-    p.wpi = units <= own ? 12 : splits > 1 ? (hd == 128 ? 3 : 4) : units <= 2 * own ? 6 : 4;
+    p.wpi = units <= own ? 12 : splits == 1 && units <= 2 * own ? 6 : 4;
     return p;
 }
 // Chunks of weights that are brought into L2 ahead of the ring of `slots`. Where the ring holds about a layer and the layer is short (16 rows at most), four more

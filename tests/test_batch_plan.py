@@ -142,7 +142,7 @@ using namespace ak::batch;
 int main() {
     int bad = 0, walks = 0;
     for (uint32_t up : {16u, 32u})
-        for (uint32_t wpi : {4u, 12u})
+        for (uint32_t wpi : {4u, 6u, 12u})
             for (uint32_t place = 0; place < wpi; place++)
                 for (uint32_t n0 = 1; n0 <= 512; n0 += n0 < 70 ? 1 : 61)
                     for (uint32_t n1 : {0u, 1u, 17u, 33u, 512u}) {
