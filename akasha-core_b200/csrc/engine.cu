@@ -398,7 +398,8 @@ int ak_engine_run(ak_engine* e, uint64_t max_steps, uint64_t* steps_done) {
     uint64_t most = 1;
     for (const auto& kv : e->all)
         if (!kv.second->finished) most += kv.second->prompt.size() + kv.second->max_total + 1;
-    const bool ahead = max_steps == 0 || max_steps >= most || e->async_ok();
+    // Ranks of a tensor-parallel engine stay in step with one another token by token unless asked for more (async_steps).
+    const bool ahead = e->async_ok() || (e->w->tp_size == 1 && (max_steps == 0 || max_steps >= most));
     for (;;) {
         if (max_steps && n >= max_steps) break;
         uint32_t running = 0, waiting = 0;

@@ -400,8 +400,8 @@ AK_API int ak_engine_step(ak_engine* e, uint32_t* n_running, uint32_t* n_waiting
 /* Steps until nothing is running or waiting (at most max_steps; 0 = no limit), then waits for the last
  * step. steps_done may be NULL. The loop the reference's `generate` runs per sequence
  * (src/nn/inference.rs:264-326), for the whole queue and without returning to the caller per token. Without a limit that it could reach every
- * step is launched before the tokens of the one before it are read, whatever async_steps and stop_on_eos say: a sequence that ends at
- * its end-of-sequence token keeps its slot one step longer (its tokens are the same, the steps may be a few more). */
+ * step is launched before the tokens of the one before it are read, whatever async_steps and stop_on_eos say (but for tensor-parallel engines): a
+ * sequence that ends at its end-of-sequence token keeps its slot one step longer (its tokens are the same, the steps may be a few more). */
 AK_API int ak_engine_run(ak_engine* e, uint64_t max_steps, uint64_t* steps_done);
 /* Has the sequence finished? Its generated tokens (prompt excluded) are copied to out (capacity
  * cap); n_out gets the count generated so far. */
