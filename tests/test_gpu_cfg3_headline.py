@@ -21,6 +21,8 @@ Checked here, at that size:
 import numpy as np
 import pytest
 
+from test_gpu_batch_step import step_by_step
+
 pytestmark = pytest.mark.gpu
 
 N_SEQS, MAX_SEQS, TOTAL_LEN, LEN_LO, LEN_HI = 256, 64, 512, 16, 448
@@ -44,7 +46,7 @@ def run(ak, ctx, w, prompts, async_steps, prefill_chunk_rows=0):
     e = ak.Engine(ctx, w, max_seqs=MAX_SEQS, max_seq_len=TOTAL_LEN, use_cuda_graph=True, stop_on_eos=False,
                   async_steps=async_steps, prefill_chunk_rows=prefill_chunk_rows)
     ids = [e.submit(p, TOTAL_LEN) for p in prompts]
-    steps = e.run_to_completion()
+    steps = e.run_to_completion() if async_steps else step_by_step(e)
     outs, tables = [], []
     for i in ids:
         t, fin = e.poll(i, TOTAL_LEN)

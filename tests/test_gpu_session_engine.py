@@ -5,6 +5,8 @@ bf16-emulating mode and batch invariance."""
 import numpy as np
 import pytest
 
+from test_gpu_batch_step import step_by_step
+
 pytestmark = pytest.mark.gpu
 
 LOGIT_TOL = 2e-2
@@ -198,7 +200,7 @@ def run_engine(ak, ctx, w, prompts, total_len, max_seqs, graph, max_seq_len=None
     e = ak.Engine(ctx, w, max_seqs=max_seqs, max_seq_len=max_seq_len or total_len, use_cuda_graph=graph,
                   async_steps=async_steps, prefill_chunk_rows=prefill_chunk_rows)
     ids = [e.submit(p, total_len) for p in prompts]
-    steps = e.run_to_completion(100000)
+    steps = e.run_to_completion(100000) if async_steps else step_by_step(e)
     outs, tables = [], []
     for i in ids:
         t, fin = e.poll(i)
