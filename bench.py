@@ -240,10 +240,17 @@ def main():
 
     CHECK = (0, 63, 64, 150, N_SEQS - 1)   # sequences whose ids the two timed legs must agree on
 
+    def run_queue():
+        if not args.sync_steps:
+            eng.run_to_completion()
+        else:
+            while eng.step() != (0, 0):
+                pass
+
     def job(collect: bool):
         """One pass through the public API: submit (host prompts), step until done, poll outputs."""
         ids = [eng.submit(p, TOTAL_LEN) for p in prompts]
-        eng.run_to_completion()
+        run_queue()
         n, kept = 0, {}
         if collect:
             for k, i in enumerate(ids):
@@ -277,7 +284,7 @@ def main():
         ids = [eng.submit(p, TOTAL_LEN) for p in prompts]
         with torch.cuda.stream(ext):
             e0.record()
-        eng.run_to_completion()
+        run_queue()
         with torch.cuda.stream(ext):
             e1.record()
         e1.synchronize()
@@ -352,23 +359,23 @@ def main():
                     "h2d_bytes_per_step": (st2["h2d_bytes"] - st["h2d_bytes"]) / args.steps,
                     "d2h_bytes_per_step": (st2["d2h_bytes"] - st["d2h_bytes"]) / args.steps},
             "gpu_launches": int(st["kernel_launches"]),
-            "roofline": {"bound": "hbm", "kernel": "attn_decode_paged_kernel<bf16,64,2> (layer 0, every decode-only step of a job behind the timed legs, as a chain of launches)",
-                         "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "peak_source": peak_kind,
-                         # two CUDA events per step, recorded on a side stream of the captured step: "the qkv projection
+            # a step of the timed leg: decode-only, one launch of the persistent kernel; the few steps with prompts are in the mean
+            "roofline": {"bound": "hbm", "kernel": "batch_kernel<64, 2, false, 2> (a decode step of the timed leg)",
+                         "achieved": step_achieved, "peak": peak, "unit": "GB/s", "frac": step_achieved / peak, "peak_source": peak_kind,
+                         "bytes_per_step": step_bytes, "ms_per_step": step_ms, "steps_timed": st["steps"],
+                         # The decode attention as a launch of its own (layer 0, every decode-only step of a job behind the timed legs, whose steps are chains
+                         # of launches). Two CUDA events per step, recorded on a side stream of the captured step: "the qkv projection
                          # before it has completed" and "the attention launch has completed". The kernel keeps its
                          # launch overlap: its CTAs are resident and have requested their first K/V tiles before the
                          # first event, so this is the launch's share of the step's critical path, shorter than the
                          # same launch timed alone (16.1 us, 0.69 of peak: python microbench.py attn --rows 64 --min-len 232)
-                         "timing": "events on a side stream inside the captured step: predecessor complete -> launch complete",
-                         # DRAM bytes per launch: 1.059 x the algorithmic bytes, the ratio ncu measured
-                         # (dram__bytes_read.sum + dram__bytes_write.sum) on a smaller launch of the same
-                         # kernel; traffic grows in proportion to the K/V bytes
-                         "traffic": 1.059 * attn_bytes,
-                         "bytes_per_launch": attn_bytes, "ms_per_launch": attn_ms, "launches_timed": tst["attn_launches_timed"],
-                         # a step of the timed leg (decode-only: one launch of the persistent kernel) against the same peak
-                         "step": {"achieved": step_achieved, "frac": step_achieved / peak, "unit": "GB/s",
-                                  "bytes_per_step": step_bytes, "ms_per_step": step_ms, "steps_timed": st["steps"]}},
+                         "attention_launch": {"kernel": "attn_decode_paged_kernel<bf16,64,2>", "achieved": achieved, "frac": achieved / peak, "unit": "GB/s",
+                                              "timing": "events on a side stream inside the captured step: predecessor complete -> launch complete",
+                                              # DRAM bytes per launch: 1.059 x the algorithmic bytes, the ratio ncu measured
+                                              # (dram__bytes_read.sum + dram__bytes_write.sum) on a smaller launch of the same
+                                              # kernel; traffic grows in proportion to the K/V bytes
+                                              "traffic": 1.059 * attn_bytes, "bytes_per_launch": attn_bytes, "ms_per_launch": attn_ms,
+                                              "launches_timed": tst["attn_launches_timed"]}},
             "clocks": clocks,
             "engine": {"decode_tokens": st["decode_tokens"], "prefill_tokens": st["prefill_tokens"],
                        "graph_launches": st["graph_launches"], "eager_steps": st["eager_steps"],
