@@ -5,11 +5,11 @@
 // of its first loads, 3 to 5 us for work of 0.1 to 1 us (162M model, contexts of 300: 8 sequences 0.39 ms, 64 0.49; the bytes take 0.05 and
 // 0.15 ms). Here, as in the batch-1 step (solo.cu), a layer is five phases of one kernel and only activations cross the chip:
 //   qkv rows -> attention (sequence, head) -> out-proj rows -> ffn-up rows -> ffn-down rows.
-// That step takes 0.180 ms with 8 sequences, 0.219 with 16, 0.305 with 32, 0.414 with 64 (320-wide model, 21 sequences 0.126; 1.4B model, 16 of 1600
-// 1.85). What is left is latency: per phase the way from a store to the last SM's poll, and dependent instructions (with everything between
+// That step takes 0.162 ms with 8 sequences, 0.202 with 16, 0.295 with 32, 0.400 with 64 (320-wide model, 21 sequences 0.120; 1.4B model, 16 of 1600
+// 1.8). What is left is latency: per phase the way from a store to the last SM's poll, and dependent instructions (with everything between
 // two phases done by the same warps it was 0.29 ms for 8).
 //   * Every SM reads all activations of a phase, which is what grows with the sequences. More than 32 (of models up to 768 wide) are two parts: half of the
-//     sequences and half of the SMs each, all weights, nothing between the two. 64 sequences: 0.49 ms as launches, 0.58 with 64 rows on every SM, 0.414 in parts.
+//     sequences and half of the SMs each, all weights, nothing between the two. 64 sequences: 0.49 ms as launches, 0.58 with 64 rows on every SM, 0.400 in parts.
 //   * A producer thread per SM walks the SM's weight tiles of all phases in order and keeps a shared-memory ring of tensor loads full.
 //   * A phase's rows are dealt to the SMs in tiles of 8, all of K: no sum crosses SMs. The 12 compute warps split K and leave partial tiles in
 //     shared memory; three epilogue warps add them in warp order and publish, while the compute warps are already at the next phase. The

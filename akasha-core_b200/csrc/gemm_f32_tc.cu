@@ -12,7 +12,7 @@
 // go through as f32, as pieces, and as what the MMAs read; the split and the additions have warps of their own and as many issue slots as the MMAs have
 // cycles. A 128 x 64 tile asks for half as much again per product and ran at 0.6 of the rate. A launch costs about 7 us beside its blocks (its
 // shared memory leaves the next one no room to start early). m x n x k 512 x 2304 x 768: 52 -> 20 us, 512 x 768 x 3072 60 -> 26, 64 x 3072 x 768 17.7 ->
-// 11.4, 64 x 768 x 768 9.6 -> 10.8; error against 64 bits (2-norm), normal operands, at k = 768 1.85e-7 -> 0.88e-7, 3072 3.6e-7 -> 1.0e-7. With operands
+// 11.4, 64 x 768 x 768 9.6 -> 10.8; 512-token prompts of small models see launch_gemm_f32_nt(). It spills 64 bytes, behind its loops. Error against 64 bits (2-norm), normal operands, at k = 768 1.85e-7 -> 0.88e-7, 3072 3.6e-7 -> 1.0e-7. With operands
 // all of one sign, whose sums rounding hardly touches, cutting shows: k = 320 0.66e-7 -> 0.84e-7, 768 0.73e-7 -> 0.85e-7, 3072 1.17e-7 -> 0.86e-7.
 //
 // The order of a row's sum is a function of (n, k) alone: K is cut into segments of `per` blocks; a segment's blocks are added in order, h segments make

@@ -118,7 +118,8 @@ def test_sums_of_squares_that_overflow(ak, ctx):
 
 
 def test_many_runs_give_the_same_tokens(ak, ctx):
-    for dim, heads, slots, total in ((320, 5, 21, 512), (256, 2, 8, 620), (768, 12, 32, 512), (768, 12, 32, 1200), (320, 5, 32, 1200), (320, 5, 9, 1200), (256, 2, 20, 768)):
+    for dim, heads, slots, total in ((320, 5, 21, 512), (256, 2, 8, 620), (768, 12, 32, 512), (768, 12, 32, 1200), (320, 5, 32, 1200), (320, 5, 9, 1200), (256, 2, 20, 768),
+                                    (320, 5, 9, 512), (256, 2, 8, 500), (256, 2, 20, 500)):   # every form of a step of one part
         cfg = ak.ModelConfig(1000, dim, heads, 4, total, 4 * dim if dim > 300 else 1184)
         w = ak.ModelWeights(ctx, cfg, ak.AK_BF16)
         w.init_synthetic(3, 0.05)
